@@ -193,7 +193,7 @@ struct spn_batch {
     // per vertex class (vertex_class): work lists, prefixes, shared memory, grid
     int off_cv[kVertexClasses] = {}, n_cv[kVertexClasses] = {}, off_cp[kVertexClasses] = {}, total_cv[kVertexClasses] = {};
     int warp_area[kVertexClasses] = {}, nl_max = 1, vgrid[kVertexClasses] = {}, sched_ints[kVertexClasses] = {};
-    int nseg_v[kVertexClasses] = {};  // classes 6-8: the largest RPA segment count of the list
+    int nseg_v[kVertexClasses] = {};  // the CTA-per-triple classes: the largest RPA segment count of the list
     // per grouped class: subgroup member table, item prefix, grid
     int off_gm[kGroupClasses] = {}, off_gp[kGroupClasses] = {}, n_sg[kGroupClasses] = {}, total_g[kGroupClasses] = {};
     int nseg_g[kGroupClasses] = {}, ggrid[kGroupClasses] = {};
@@ -294,12 +294,12 @@ struct spn_batch {
             const int c = class_of(f.h->nl);
             measure.push_back(int(i));
             cm[c].push_back(int(i));
-            const int vc = vertex_class(f.h->nl);
+            const int vc = vertex_class(f.h->nl, f.h->inv_kind);
             n_max = std::max(n_max, f.h->n);
             nl_max = std::max(nl_max, f.h->nl);
             if (f.phase == kPhaseFlowing) {
                 flowing.push_back(int(i));
-                if (min_group > 0 && vc < kGroupClasses && group_vertex_eligible(f.h->nl))
+                if (min_group > 0 && vc < kGroupClasses && group_vertex_eligible(f.h->nl, f.h->inv_kind))
                     buckets[{f.share_id, f.step}].push_back(int(i));
                 else
                     cv[vc].push_back(int(i));
@@ -315,19 +315,19 @@ struct spn_batch {
         }
         for (auto &kv : buckets) {
             const std::vector<int> &v = kv.second;
-            const int vc = vertex_class(flows[v[0]].h->nl);
+            const int vc = vertex_class(flows[v[0]].h->nl, 0);
             if (int(v.size()) < min_group) {
                 cv[vc].insert(cv[vc].end(), v.begin(), v.end());
                 continue;
             }
-            const int gmax = group_vertex_gmax(vc);
+            const int gmax = group_vertex_gmax();
             const int cap = std::max(1, gmax / group_cap_div);
             const int parts = (int(v.size()) + cap - 1) / cap;
             size_t at = 0;
             for (int q = 0; q < parts; ++q) {
                 const size_t take = (v.size() - at) / size_t(parts - q);  // balanced sizes
                 for (int m = 0; m < gmax; ++m) gm[vc].push_back(m < int(take) ? v[at + m] : -1);
-                const long long next = gp[vc].back() + flows[v[at]].h->fn;
+                const long long next = gp[vc].back() + vertex_work_items(flows[v[at]].h->n, flows[v[at]].h->nl, 0);
                 if (next >= (1ll << 31)) throw Error(ErrorType::Unsupported, "batch work list beyond 2^31 items");
                 gp[vc].push_back(int(next));
                 for (size_t m = 0; m < take; ++m) nseg_g[vc] = std::max(nseg_g[vc], flows[v[at + m]].h->rpa_n_seg);
@@ -356,10 +356,10 @@ struct spn_batch {
             int sched = 0, nseg = 0;
             for (int i : cv[c]) {
                 const spn_su2 *h = flows[i].h;
-                const long long next = prefix.back() + h->fn;
+                const long long next = prefix.back() + vertex_work_items(h->n, h->nl, h->inv_kind);
                 if (next >= (1ll << 31)) throw Error(ErrorType::Unsupported, "batch work list beyond 2^31 items");
                 prefix.push_back(int(next));
-                if (c < 6) area = std::max(area, batch_vertex_warp_area(h->nl, h->rpa_n_seg, npi));
+                if (!vertex_class_big(c)) area = std::max(area, batch_vertex_warp_area(h->nl, h->rpa_n_seg, h->inv_kind));
                 sched = std::max(sched, rpa_smem_ints(h->args().rpa, h->nl));
                 nseg = std::max(nseg, h->rpa_n_seg);
             }
@@ -369,12 +369,12 @@ struct spn_batch {
             warp_area[c] = int((area + 15) / 16 * 16);
             // each warp stages its flow's RPA schedule when the largest one is small (warp-per-
             // triple classes; the CTA-per-triple classes 6-8 read it from global memory)
-            sched_ints[c] = (c < 6 && stage_sched && sched <= kBatchSchedMaxInts) ? sched : 0;
+            sched_ints[c] = (!vertex_class_big(c) && stage_sched && sched <= kBatchSchedMaxInts) ? sched : 0;
             vgrid[c] = 0;
             if (n_cv[c] > 0) {
-                const size_t smem = c >= 6 ? batch_big_smem_bytes(c, nseg_v[c])
+                const size_t smem = vertex_class_big(c) ? batch_big_smem_bytes(c, nseg_v[c])
                                            : batch_vertex_smem_bytes(n_max, warp_area[c], sched_ints[c]);
-                const int per_sm = batch_vertex_blocks_per_sm(c, npi, smem);
+                const int per_sm = batch_vertex_blocks_per_sm(c, smem);
                 cudaGetLastError();
                 if (per_sm < 1) throw Error(ErrorType::Unsupported, "batched vertex-flow kernel does not fit for this batch");
                 vgrid[c] = sms * per_sm;
@@ -444,7 +444,7 @@ struct spn_batch {
                 b.warp_area = warp_area[c];
                 b.sched_ints = sched_ints[c];
                 b.n_seg_max = nseg_v[c];
-                launch_batch_vertex(b, c, npi, vgrid[c], stream);
+                launch_batch_vertex(b, c, vgrid[c], stream);
             }
             for (int c = 0; c < kGroupClasses; ++c) {
                 if (n_sg[c] == 0) continue;
@@ -454,7 +454,7 @@ struct spn_batch {
                 g.prefix = L + off_gp[c];
                 g.n_sg = n_sg[c];
                 g.total = total_g[c];
-                g.gmax = group_vertex_gmax(c);
+                g.gmax = group_vertex_gmax();
                 g.counter = d_counters + kVertexClasses + c;
                 g.n_seg_max = nseg_g[c];
                 launch_group_vertex(g, c, ggrid[c], stream);
@@ -783,9 +783,9 @@ extern "C" int spn_batch_remove(spn_batch *b, int flow_id) {
 }
 
 // Times the vertex flow of the batch's current flows under each candidate configuration and
-// keeps the fastest: nodes per group iteration of the per-flow kernel (1, 2) x its RPA schedule
+// keeps the fastest: the per-flow kernel with its RPA schedule
 // (read from global memory, staged per warp in shared memory: more shared memory, fewer
-// resident blocks) without sharing, and, when the caller enabled sharing, (1, 2) x cross-flow
+// resident blocks) without sharing, and, when the caller enabled sharing, cross-flow
 // sharing in subgroups of the grouped kernel's full block or of half of it.  The front of a
 // step runs once first (self-energy flow and node tables of the current states); the timed
 // launches write only the flows' vertex-flow buffers, which hold nothing between steps, so
@@ -801,8 +801,7 @@ extern "C" int spn_batch_autotune(spn_batch *b, int reps, int *npi, int *min_gro
             int npi, min_group, cap;
             bool stage;
         };
-        const Cand cands[] = {{1, 0, 1, false}, {2, 0, 1, false}, {1, 0, 1, true}, {2, 0, 1, true},
-                              {1, 2, 1, false}, {2, 2, 1, false}, {1, 2, 2, false}, {2, 2, 2, false}};
+        const Cand cands[] = {{b->npi, 0, 1, false}, {b->npi, 0, 1, true}, {b->npi, 2, 1, false}, {b->npi, 2, 2, false}};
         const Cand keep{b->npi, b->min_group, b->group_cap_div, b->stage_sched};
         // sharing is a candidate only when the caller enabled it (spn_batch_set_grouping): on
         // a scan it wins in the first steps and loses in the later ones, which dominate

@@ -54,6 +54,7 @@ struct FlowArgsT {
     double *dv2d;          // FP64 self-energy flow
     int fp64_sigma;
     const int *sites, *inv_sites, *ov_ptr, *ov_r1, *ov_r2, *range_rid, *range_inv;
+    int inv_kind;  // site_exchange_kind of sites and inv_sites
     T *node_wp, *node_c;
     int *node_cnt;
     int *work_counter;
@@ -104,13 +105,23 @@ struct BatchFlow {
     unsigned flags;
 };
 
+// Site exchange of a flow: 0, every site's pair and its exchanged pair are the site's own; 1,
+// site j's pair is pair j and the exchange is an involution that fixes pair 0 (every lattice of
+// the factory is one of these); 2, any other tables.
+inline int site_exchange_kind(int nl, const int *sites, const int *inv_sites) {
+    bool ident = inv_sites[0] == 0, same = true;
+    for (int j = 0; j < nl; ++j) {
+        ident = ident && sites[j] == j && inv_sites[inv_sites[j]] == j;
+        same = same && inv_sites[j] == j;
+    }
+    return ident ? (same ? 0 : 1) : 2;
+}
 // Vertex-flow kernel (su2_vertex.cu): dynamic shared memory per block, the number of blocks
-// per SM it achieves, and the launch.
-// `npi`: loop-frequency nodes a site group evaluates per iteration (1 or 2); whether the RPA
-// schedule is staged in shared memory is a.rpa.in_smem.  Both are chosen per flow by timing.
-size_t vertex_flow_smem_bytes(int nl, const RpaSchedule &rpa, int npi);
-int vertex_flow_blocks_per_sm(int nl, const RpaSchedule &rpa, int npi);
-void launch_vertex_flow(const FlowArgs &a, int npi, int grid, cudaStream_t stream);
+// per SM it achieves, and the launch.  Whether the RPA schedule is staged in shared memory is
+// a.rpa.in_smem, chosen per flow by timing.
+size_t vertex_flow_smem_bytes(int nl, const RpaSchedule &rpa, int inv_kind);
+int vertex_flow_blocks_per_sm(int nl, const RpaSchedule &rpa, int inv_kind);
+void launch_vertex_flow(const FlowArgs &a, int grid, cudaStream_t stream);
 // FP64 flow (su2_vertex64.cu): one warp per triple over a persistent grid.
 void launch_vertex_flow_f64(const FlowArgsT<double> &a, int grid, cudaStream_t stream);
 int vertex_flow_f64_blocks_per_sm(int nl);
@@ -120,7 +131,7 @@ constexpr int kRpaSmemMaxInts = 8192;
 
 // Batched vertex flow: one persistent launch over the ragged work list of all flows of one
 // vertex class (vertex_class below).  Work item w belongs to flow list[f] with
-// prefix[f] <= w < prefix[f+1] (prefix[f+1] - prefix[f] = that flow's triple count).
+// prefix[f] <= w < prefix[f+1] (prefix[f+1] - prefix[f] = that flow's vertex_work_items).
 // `warp_area` is the per-warp shared-memory bytes the largest flow of the list needs.
 // `sched_ints` > 0: each warp stages the RPA schedule of its current flow in shared memory
 // (room for that many ints; every flow of the list must fit), else it reads global memory.
@@ -135,8 +146,8 @@ struct BatchVertexArgs {
 };
 // Grouped batches (flows sharing mesh, lattice tables and cutoff; see su2_vertex.cu): one
 // persistent launch per vertex class 0..3 over (subgroup, triple) items.  A subgroup holds up
-// to group_vertex_gmax(cls) flows: members[sg * gmax + q] is the record index of member q, -1
-// after the last; its items are prefix[sg] .. prefix[sg + 1] - 1 (its flows' F_N triples).
+// to group_vertex_gmax() flows: members[sg * gmax + q] is the record index of member q, -1
+// after the last; its items are prefix[sg] .. prefix[sg + 1] - 1 (its flows' vertex_work_items).
 // n_seg_max: the largest RPA segment count of the flows in the launch.
 struct GroupVertexArgs {
     BatchFlow *flows;
@@ -145,21 +156,23 @@ struct GroupVertexArgs {
     int *counter;
     int n_seg_max;
 };
-bool group_vertex_eligible(int nl);  // 5 <= nl <= 32
-int group_vertex_gmax(int cls);
+bool group_vertex_eligible(int nl, int inv_kind);  // 5 <= nl <= 32, every pair its own exchange
+int group_vertex_gmax();  // flows of a subgroup
 size_t group_vertex_smem_bytes(int cls, int n_seg_max);
 int group_vertex_blocks_per_sm(int cls, int n_seg_max);
 void launch_group_vertex(const GroupVertexArgs &g, int cls, int grid, cudaStream_t stream);
-size_t batch_vertex_warp_area(int nl, int n_seg, int npi);
+size_t batch_vertex_warp_area(int nl, int n_seg, int inv_kind);
 size_t batch_vertex_smem_bytes(int n_max, size_t warp_area, int sched_ints);
-int batch_vertex_blocks_per_sm(int cls, int npi, size_t smem);
-void launch_batch_vertex(const BatchVertexArgs &b, int cls, int npi, int grid, cudaStream_t stream);
-int vertex_spt(int nl);  // sites per lane of a flow with nl sites
-// Vertex-kernel class of a flow (one kernel instance per class): 0-3 for nl <= 32 (outer-product
-// RPA with w = 8, 16, 24, 32, a warp per triple), 6-10 for 33 <= nl <= 128 (outer-product RPA
-// with w = 48, 64, 80, 96, 128, a CTA per triple); 4 and 5 are unused.
-constexpr int kVertexClasses = 11;
-int vertex_class(int nl);
+int batch_vertex_blocks_per_sm(int cls, size_t smem);
+void launch_batch_vertex(const BatchVertexArgs &b, int cls, int grid, cudaStream_t stream);
+// Vertex-kernel class of a flow (one kernel instance per class): for nl <= 32 (outer-product RPA with
+// w = 8, 16, 24, 32) 0-3, a warp per item of three triples (site_exchange_kind 0), or 11-14, a warp
+// per triple; 6-10 for 33 <= nl <= 128 (outer-product RPA with w = 48, 64, 80, 96, 128, a CTA per
+// triple); 4 and 5 are unused.
+constexpr int kVertexClasses = 15;
+int vertex_class(int nl, int inv_kind);
+bool vertex_class_big(int cls);  // 6-10
+long long vertex_work_items(int n, int nl, int inv_kind);  // items of the vertex kernel's work counter
 // Lanes of the RPA schedule the vertex kernel of an nl-site flow walks: 32 (a warp per triple)
 // or the CTA's threads (33 to 128 sites).
 int vertex_rpa_lanes(int nl);

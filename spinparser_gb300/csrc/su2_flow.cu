@@ -210,7 +210,7 @@ int copy_grid(long long n) { return int(std::min<long long>((n + 255) / 256, 409
 
 void launch_vertex(spn_su2 *h) {
     if (h->fp64()) launch_vertex_flow_f64(h->args64(), h->vertex_grid, h->stream);
-    else launch_vertex_flow(h->args(), h->vertex_npi, h->vertex_grid, h->stream);
+    else launch_vertex_flow(h->args(), h->vertex_grid, h->stream);
     cuda_check(cudaGetLastError(), "vertex flow launch");
 }
 
@@ -247,9 +247,10 @@ void download_pairs64(S *ss, S *dd, const double2 *src, size_t count, cudaStream
     }
 }
 
-// Selects a vertex-flow variant: nodes per iteration and where the RPA schedule lives (all
-// variants give the same bits); the persistent grid fills every SM to the variant's
-// occupancy.  Returns false if it cannot run.
+// Selects a vertex-flow variant: where the RPA schedule lives (all variants give the same bits);
+// the persistent grid fills every SM to the variant's occupancy.  `npi` (1 or 2 nodes per
+// iteration) is kept as the caller set it; one kernel serves both.  Returns false if it cannot
+// run.
 bool select_variant(spn_su2 *h, int npi, int in_smem) {
     if (h->fp64()) {  // one FP64 kernel
         const int per_sm = vertex_flow_f64_blocks_per_sm(h->nl);
@@ -266,7 +267,7 @@ bool select_variant(spn_su2 *h, int npi, int in_smem) {
     }
     const int old_smem = h->rpa_in_smem;
     h->rpa_in_smem = in_smem;
-    const int per_sm = vertex_flow_blocks_per_sm(h->nl, h->args().rpa, npi);
+    const int per_sm = vertex_flow_blocks_per_sm(h->nl, h->args().rpa, h->inv_kind);
     cudaGetLastError();
     if (per_sm < 1) {
         h->rpa_in_smem = old_smem;
@@ -559,6 +560,7 @@ spn_su2 *spn::create_flow(const spn_su2_desc *d, cudaStream_t stream) {
             h->flags = d->flags;
             h->spin = d->spin_length;
             h->max_nodes = 2 * h->n + 8;
+            h->inv_kind = site_exchange_kind(h->nl, d->sites_rid, d->inv_sites_rid);
             if (stream) {
                 h->stream = stream;
                 h->own_stream = false;
@@ -822,32 +824,30 @@ extern "C" int spn_su2_autotune(spn_su2 *h, int reps, int *npi, int *sched_in_sm
         const bool prof = h->profiling;
         h->profiling = false;
         float best = 0.0f;
-        int best_npi = h->vertex_npi, best_smem = h->rpa_in_smem;
+        int best_smem = h->rpa_in_smem;
         try {
             // the node tables of the current cutoff (compute_step leaves the state untouched)
             cuda_check(spn_su2_compute_step(h) == 0 ? cudaSuccess : cudaErrorUnknown, "autotune step");
-            for (int npi = 1; npi <= 2; ++npi)
-                for (int sm = 0; sm <= 1; ++sm) {
-                    if (!select_variant(h, npi, sm)) continue;
-                    std::vector<float> ms;
-                    for (int r = 0; r <= reps; ++r) {
-                        cuda_check(cudaMemsetAsync(h->work_counter, 0, sizeof(int), h->stream), "memset counter");
-                        cuda_check(cudaEventRecord(e0, h->stream), "record");
-                        launch_vertex(h);
-                        cuda_check(cudaEventRecord(e1, h->stream), "record");
-                        cuda_check(cudaEventSynchronize(e1), "sync");
-                        float t = 0.0f;
-                        cuda_check(cudaEventElapsedTime(&t, e0, e1), "elapsed");
-                        if (r > 0) ms.push_back(t);  // first launch warms caches
-                    }
-                    std::sort(ms.begin(), ms.end());
-                    const float med = ms[ms.size() / 2];
-                    if (best == 0.0f || med < best) {
-                        best = med;
-                        best_npi = npi;
-                        best_smem = sm;
-                    }
+            for (int sm = 0; sm <= 1; ++sm) {
+                if (!select_variant(h, h->vertex_npi, sm)) continue;
+                std::vector<float> ms;
+                for (int r = 0; r <= reps; ++r) {
+                    cuda_check(cudaMemsetAsync(h->work_counter, 0, sizeof(int), h->stream), "memset counter");
+                    cuda_check(cudaEventRecord(e0, h->stream), "record");
+                    launch_vertex(h);
+                    cuda_check(cudaEventRecord(e1, h->stream), "record");
+                    cuda_check(cudaEventSynchronize(e1), "sync");
+                    float t = 0.0f;
+                    cuda_check(cudaEventElapsedTime(&t, e0, e1), "elapsed");
+                    if (r > 0) ms.push_back(t);  // first launch warms caches
                 }
+                std::sort(ms.begin(), ms.end());
+                const float med = ms[ms.size() / 2];
+                if (best == 0.0f || med < best) {
+                    best = med;
+                    best_smem = sm;
+                }
+            }
         } catch (...) {
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
@@ -857,7 +857,7 @@ extern "C" int spn_su2_autotune(spn_su2 *h, int reps, int *npi, int *sched_in_sm
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         h->profiling = prof;
-        if (!select_variant(h, best_npi, best_smem)) throw Error(ErrorType::Internal, "autotune: chosen variant unavailable");
+        if (!select_variant(h, h->vertex_npi, best_smem)) throw Error(ErrorType::Internal, "autotune: chosen variant unavailable");
         if (npi) *npi = h->vertex_npi;
         if (sched_in_smem) *sched_in_smem = h->rpa_in_smem;
         if (grid) *grid = h->vertex_grid;

@@ -48,7 +48,8 @@ struct spn_su2 {
     int *rpa_sched = nullptr, *rpa_count = nullptr, *rpa_slot_base = nullptr, *rpa_seg_ptr = nullptr;  // into rpa_image
     int rpa_image_bytes = 0;
     int rpa_lanes = 0, rpa_n_seg = 0, rpa_len = 0, rpa_in_smem = 0;
-    int vertex_npi = 1;       // loop-frequency nodes per site-group iteration
+    int inv_kind = 0;         // site_exchange_kind
+    int vertex_npi = 1;       // nodes per iteration as set (one kernel serves both settings)
     int sms = 0;
     bool profiling = false;
     std::vector<cudaEvent_t> ev_pool;
@@ -77,6 +78,7 @@ struct spn_su2 {
         a.fp64_sigma = (flags & SPN_SU2_FP64_SELF_ENERGY) ? 1 : 0;
         a.sites = sites;
         a.inv_sites = inv_sites;
+        a.inv_kind = inv_kind;
         a.ov_ptr = ov_ptr;
         a.ov_r1 = ov_r1;
         a.ov_r2 = ov_r2;
@@ -127,6 +129,7 @@ struct spn_su2 {
         a.fp64_sigma = 0;
         a.sites = f.sites;
         a.inv_sites = f.inv_sites;
+        a.inv_kind = f.inv_kind;
         a.ov_ptr = f.ov_ptr;
         a.ov_r1 = f.ov_r1;
         a.ov_r2 = f.ov_r2;

@@ -7,28 +7,34 @@
 // Katanin integrals, with propagators folded into c) depend only on the channel's transfer
 // frequency and are built per step by su2_node_table_kernel.
 //
-// Work distribution: a persistent grid; each warp pulls triples from a device atomic
-// counter.  For a triple and channel, nodes are handled in batches of 32:
-//   phase A, lane = node: the node's interpolation supports (access buffers: folding, mesh
-//            searches, weights) are computed once and written to shared memory as a
-//            NodeDesc; for the t channel the four site-local vertex values are gathered too;
+// Work distribution: a persistent grid; each warp pulls items from a device atomic counter.  An
+// item is three mesh indices p >= q >= r: the three triples (p, q, r), (p, r, q), (q, p, r),
+// whose nine channel integrals read the slabs of three transfer frequencies (su2_item.cuh).  For
+// a transfer frequency, nodes are handled in batches of 32:
+//   phase A, lane = node: the node's interpolation supports (mesh searches, weights, signs, site
+//            exchange) are computed once and written to shared memory as an ItemDesc;
 //   phase B, lane = (node group, site): each group of W lanes (W = next power of two >= Nl)
-//            takes one node at a time, reads its descriptor (broadcast), gathers the four
-//            interpolated vertex slabs for its sites (coalesced: a slab is Nl contiguous
-//            floats) and forms K_X.
+//            takes one node at a time, reads its descriptor (broadcast), gathers the node's six
+//            interpolated planes for its sites (coalesced: a slab is Nl contiguous pairs) and adds
+//            the node's terms to the three triples.
 // The t channel's RPA lattice sum sum_i A[rid1_i] B[rid2_i] (A, B: the third and fourth slab
-// of the node) is linear in the node, so for Nl <= 32 the warp first accumulates the matrix
+// of the node) is linear in the node, so the warp first accumulates the matrix
 //   M = sum over the channel's nodes of (c A) x B        (Nl x Nl, spin and density)
 // in registers -- the 32 lanes own an 8 x 4 grid of blocks, updated with packed f32x2 FMAs
-// from a per-node shared-memory panel -- and then walks the merged pair list once per triple,
-// sum m M[rid1][rid2] per rid (every (rid1, rid2) occurs: the pair matrix is dense).  For
-// Nl > 32 each node walks the merged pair list itself.  Both walks follow a lane-balanced
-// schedule with deterministic segment partials (no divergent per-rid loops).
-// Accumulation over nodes is Kahan-compensated FP32 for the local terms (the RPA matrix sums
-// are plain FP32); group partials are combined by shuffles.
+// from a per-node shared-memory panel -- and then walks the merged pair list once per t channel,
+// sum m M[rid1][rid2] per rid (every (rid1, rid2) occurs: the pair matrix is dense).  The walk
+// follows a lane-balanced schedule (host/rpa_schedule.hpp).  Lattices of 33 to 128 sites take a
+// CTA per triple (su2_vertex_big_kernel below).
+//
+// What bounds it (cubic r6, N = 64, cutoff 2.24): the L1 data path (77 % busy: 25 segment loads of
+// 3.1 wavefronts and 24 shared loads per node) and, at 12 resident warps, dependent-issue and L1
+// latency (issue 48 %).  Evaluated triple by triple, each channel with its own gathers, the same
+// launch took 5.73 ms (the L1 data path at 95 %); by items it takes 3.56 ms.  Padding the slabs to
+// whole cache lines takes the loads to 2.0 wavefronts but not the time down (3.55 ms).
 #include <type_traits>
 #include "su2_common.cuh"
 #include "su2_device.cuh"
+#include "su2_item.cuh"
 
 namespace spn {
 namespace {
@@ -61,16 +67,6 @@ struct Transfer {
     float s, t, u, w1p, w1, w2p, w2;
     int si, ti, ui;  // mesh indices of s, t, u: the channel coordinate's offset in every buffer
 };
-
-// Packed single-precision pairs (fma.rn.f32x2): per element the same IEEE round-to-nearest
-// result as fmaf.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("{\n\t.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
-        "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n}"
-        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return d;
-}
 
 // Stores buffer i of a node; returns its sign bits (bit 4 + 4i + q set when sw[q] = -w[q], the
 // density weight of a swapped slab; sw is exactly +-w, so the pair is rebuilt without loss).
@@ -151,119 +147,6 @@ __device__ __forceinline__ void make_desc(const FlowArgs &a, const float *pos, c
     d.c = c;
 }
 
-// Supports of the four site-local access buffers of a t-channel node (the values cbs ... icad2
-// of make_desc are local_pair of these with a flow's state).
-struct LocDesc {
-    int4 off[4];
-    float4 w[4];
-    float4 sw[4];
-};
-
-// Phase A for flows that share the mesh, the lattice tables and the cutoff (a grouped batch):
-// the node's supports only, as make_desc builds them (same access buffers, same arguments);
-// the coefficient and the t channel's site-local values are per flow (group_local_values).
-template <int CH>
-__device__ __forceinline__ void make_supports(const FlowArgs &a, const float *pos, const Transfer &f, float wp, NodeDesc &d,
-                                              LocDesc &loc) {
-    AB4 ab;
-    int exch = 0;
-    const int nl = a.nl, n = a.n;
-    const MeshIndex m{pos, a.n, a.mesh_lo, a.mesh_base, a.mesh_shift};
-    if (CH == kS) {
-        {  // buffers 0 and 2 interpolate |w1 + wp| and |w2 + wp|
-            const Interp<float> iA = interp_abs(m, f.w1 + wp), iB = interp_abs(m, f.w2 + wp);
-            access4i<kS>(n, nl, f.s, -f.w1 - wp, -f.w2 - wp, iA, iB, f.si, ab); exch |= put_ab(d, 0, ab) | (int(ab.exch) << 0);
-            access4i<kS>(n, nl, f.s, f.w2 + wp, f.w1 + wp, iB, iA, f.si, ab); exch |= put_ab(d, 2, ab) | (int(ab.exch) << 2);
-        }
-        {  // buffers 1 and 3: |w1p + wp| and |w2p + wp|
-            const Interp<float> iP = interp_abs(m, f.w1p + wp), iQ = interp_abs(m, f.w2p + wp);
-            access4i<kS>(n, nl, f.s, f.w1p + wp, -f.w2p - wp, iP, iQ, f.si, ab); exch |= put_ab(d, 1, ab) | (int(ab.exch) << 1);
-            access4i<kS>(n, nl, f.s, -f.w2p - wp, f.w1p + wp, iQ, iP, f.si, ab); exch |= put_ab(d, 3, ab) | (int(ab.exch) << 3);
-        }
-    } else if (CH == kT) {
-        auto put_loc = [&](int i) {
-            loc.off[i] = make_int4(ab.off[0], ab.off[1], ab.off[2], ab.off[3]);
-            loc.w[i] = make_float4(ab.w[0], ab.w[1], ab.w[2], ab.w[3]);
-            loc.sw[i] = make_float4(ab.sw[0], ab.sw[1], ab.sw[2], ab.sw[3]);
-        };
-        {
-            const Interp<float> iC = interp_abs(m, f.w1 - wp), iP = interp_abs(m, f.w1p + wp);
-            access4i<kT>(n, nl, f.w1 - wp, f.t, f.w1p + wp, iC, iP, f.ti, ab); exch |= put_ab(d, 0, ab) | (int(ab.exch) << 0);
-            access4i<kT>(n, nl, f.w1p + wp, f.t, f.w1 - wp, iP, iC, f.ti, ab); exch |= put_ab(d, 2, ab) | (int(ab.exch) << 2);
-            access4i<kU>(n, nl, f.w1 - wp, -f.w1p - wp, -f.t, iC, iP, f.ti, ab); put_loc(1);
-            access4i<kU>(n, nl, f.w1p + wp, wp - f.w1, -f.t, iP, iC, f.ti, ab); put_loc(3);
-        }
-        {
-            const Interp<float> iD = interp_abs(m, f.w2p - wp), iB = interp_abs(m, f.w2 + wp);
-            access4i<kT>(n, nl, f.w2p - wp, f.t, -f.w2 - wp, iD, iB, f.ti, ab); exch |= put_ab(d, 1, ab) | (int(ab.exch) << 1);
-            access4i<kT>(n, nl, f.w2 + wp, f.t, wp - f.w2p, iB, iD, f.ti, ab); exch |= put_ab(d, 3, ab) | (int(ab.exch) << 3);
-            access4i<kU>(n, nl, f.w2p - wp, -f.w2 - wp, f.t, iD, iB, f.ti, ab); put_loc(0);
-            access4i<kU>(n, nl, f.w2 + wp, wp - f.w2p, f.t, iB, iD, f.ti, ab); put_loc(2);
-        }
-    } else {
-        {  // buffers 0 and 2: |w1 + wp| and |w2p - wp|
-            const Interp<float> iA = interp_abs(m, f.w1 + wp), iD = interp_abs(m, f.w2p - wp);
-            access4i<kU>(n, nl, f.w1 + wp, wp - f.w2p, f.u, iA, iD, f.ui, ab); exch |= put_ab(d, 0, ab) | (int(ab.exch) << 0);
-            access4i<kU>(n, nl, f.w2p - wp, -f.w1 - wp, f.u, iD, iA, f.ui, ab); exch |= put_ab(d, 2, ab) | (int(ab.exch) << 2);
-        }
-        {  // buffers 1 and 3: |w1p + wp| and |w2 - wp|
-            const Interp<float> iP = interp_abs(m, f.w1p + wp), iE = interp_abs(m, f.w2 - wp);
-            access4i<kU>(n, nl, f.w1p + wp, f.w2 - wp, f.u, iP, iE, f.ui, ab); exch |= put_ab(d, 1, ab) | (int(ab.exch) << 1);
-            access4i<kU>(n, nl, f.w2 - wp, f.w1p + wp, f.u, iE, iP, f.ui, ab); exch |= put_ab(d, 3, ab) | (int(ab.exch) << 3);
-        }
-    }
-    d.exch = exch;
-    d.c = 0.0f;
-}
-
-// make_supports split over the four threads of a quad (q = 0..3), for a CTA that builds 32
-// nodes with 128 threads.  Thread q builds main buffer b(q) and, in the t channel, local buffer
-// l(q), from the two magnitudes (y1, y2) that those buffers interpolate; the coordinates come
-// from selects, so the quad runs one instruction stream.  Every coordinate is the value
-// make_supports passes (negations are exact), so the supports are the same bits.  Returns the
-// exchange and sign bits of the thread's buffer; the quad ORs them into d.exch.
-template <int CH>
-__device__ __forceinline__ int make_part(const FlowArgs &a, const float *pos, const Transfer &f, float wp, int q,
-                                         NodeDesc &d, LocDesc &loc) {
-    AB4 ab;
-    const int nl = a.nl, n = a.n;
-    const MeshIndex m{pos, a.n, a.mesh_lo, a.mesh_base, a.mesh_shift};
-    const bool lo2 = q < 2, odd = q & 1;
-    if (CH == kS) {
-        // buffers (t, u): 0 (-A, -B), 1 (P, -Q), 2 (B, A), 3 (-Q, P); (y1, y2) = (A, B) or (P, Q)
-        const float y1 = odd ? f.w1p + wp : f.w1 + wp, y2 = odd ? f.w2p + wp : f.w2 + wp;
-        const Interp<float> i1 = interp_abs(m, y1), i2 = interp_abs(m, y2);
-        const float t = lo2 ? (odd ? y1 : -y1) : (odd ? -y2 : y2);
-        const float u = lo2 ? -y2 : y1;
-        access4i<kS>(n, nl, f.s, t, u, lo2 ? i1 : i2, lo2 ? i2 : i1, f.si, ab);
-        return put_ab(d, q, ab) | (int(ab.exch) << q);
-    } else if (CH == kU) {
-        // buffers (s, t): 0 (A, -D), 1 (P, E), 2 (D, -A), 3 (E, P); (y1, y2) = (A, D) or (P, E)
-        const float y1 = odd ? f.w1p + wp : f.w1 + wp, y2 = odd ? f.w2 - wp : f.w2p - wp;
-        const Interp<float> i1 = interp_abs(m, y1), i2 = interp_abs(m, y2);
-        const float sv = lo2 ? y1 : y2;
-        const float t = lo2 ? (odd ? y2 : -y2) : (odd ? y1 : -y1);
-        access4i<kU>(n, nl, sv, t, f.u, lo2 ? i1 : i2, lo2 ? i2 : i1, f.ui, ab);
-        return put_ab(d, q, ab) | (int(ab.exch) << q);
-    } else {
-        // main buffers (s, u): 0 (C, P), 2 (P, C), 1 (D, -B), 3 (B, -D); local buffers (s, t, u):
-        // 1 (C, -P, -t), 3 (P, -C, -t), 0 (D, -B, t), 2 (B, -D, t); (y1, y2) = (C, P), (P, C),
-        // (D, B), (B, D) for q = 0..3
-        const float C = f.w1 - wp, P = f.w1p + wp, D = f.w2p - wp, B = f.w2 + wp;
-        const float x1 = lo2 ? C : D, x2 = lo2 ? P : B;
-        const float y1 = odd ? x2 : x1, y2 = odd ? x1 : x2;
-        const Interp<float> i1 = interp_abs(m, y1), i2 = interp_abs(m, y2);
-        const int bi = (int(odd) << 1) | (q >> 1), li = (int(odd) << 1) | (1 - (q >> 1));
-        access4i<kT>(n, nl, y1, f.t, lo2 ? y2 : -y2, i1, i2, f.ti, ab);
-        const int bits = put_ab(d, bi, ab) | (int(ab.exch) << bi);
-        access4i<kU>(n, nl, y1, -y2, lo2 ? -f.t : f.t, i1, i2, f.ti, ab);
-        loc.off[li] = make_int4(ab.off[0], ab.off[1], ab.off[2], ab.off[3]);
-        loc.w[li] = make_float4(ab.w[0], ab.w[1], ab.w[2], ab.w[3]);
-        loc.sw[li] = make_float4(ab.sw[0], ab.sw[1], ab.sw[2], ab.sw[3]);
-        return bits;
-    }
-}
-
 // make_desc split over the two threads of a lane pair (h = 0, 1), for a CTA that builds 128
 // nodes with 256 threads.  Thread h builds the two main buffers that share its pair of
 // interpolated magnitudes, buffers h and h + 2 (and in the t channel the two local buffers of
@@ -316,23 +199,6 @@ __device__ __forceinline__ int make_pair(const FlowArgs &a, const float *pos, co
         d.lv[odd ? 5 : 7] = v1;
     }
     return bits;
-}
-
-// The t channel's eight site-local values of one node for one flow's state (make_desc's
-// local_pair of each local buffer, in the same order).
-__device__ __forceinline__ void group_local_values(const float2 *sd, const LocDesc &loc, float *lv) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int4 o = loc.off[i];
-        const float4 w = loc.w[i], sw = loc.sw[i];
-        float2 g = make_float2(0.0f, 0.0f);
-        g = fma2(make_float2(w.x, sw.x), __ldg(sd + o.x), g);
-        g = fma2(make_float2(w.y, sw.y), __ldg(sd + o.y), g);
-        g = fma2(make_float2(w.z, sw.z), __ldg(sd + o.z), g);
-        g = fma2(make_float2(w.w, sw.w), __ldg(sd + o.w), g);
-        lv[2 * i] = g.x;
-        lv[2 * i + 1] = g.y;
-    }
 }
 
 // Phase B: interpolated slab of buffer i for this lane's sites (getValueSuperbundle): per
@@ -486,11 +352,431 @@ __device__ __forceinline__ void node_term(const A &a, const NodeView *v, const L
     }
 }
 
+// Adds the outer products of the panels of nodes k = r * G + gg < nb (ascending k) to the lane's
+// block of M.  `pan`: the warp's first panel; panel gg starts 2 w float2 later per step.
+template <int MB>
+__device__ __forceinline__ void outer_update(const float2 *pan, int lane, int r, int G, int nb, OuterAcc<MB> &M) {
+    constexpr int W = 8 * MB;
+    const int rb = lane >> 2, cb = lane & 3;
+    for (int gg = 0; gg < G; ++gg) {
+        if (r * G + gg >= nb) break;
+        const float2 *A = pan + gg * 2 * W + rb * MB;
+        const float2 *B = pan + gg * 2 * W + W + cb * 2 * MB;
+        float2 av[MB], bv[2 * MB];
+#pragma unroll
+        for (int i = 0; i < MB; ++i) av[i] = A[i];
+#pragma unroll
+        for (int j = 0; j < 2 * MB; ++j) bv[j] = B[j];
+#pragma unroll
+        for (int i = 0; i < MB; ++i)
+#pragma unroll
+            for (int j = 0; j < 2 * MB; ++j) M.m[i][j] = fma2(av[i], bv[j], M.m[i][j]);
+    }
+}
+
+// ------------------------------------------------------------------------------------
+// Bulk copies global -> shared through the copy engine (cp.async.bulk) completing on an
+// mbarrier.  Addresses and sizes are multiples of 16 bytes.
+// ------------------------------------------------------------------------------------
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return unsigned(__cvta_generic_to_shared(p)); }
+
+__device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+
+__device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long *bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void bulk_copy_g2s(void *dst, const void *src, unsigned bytes, unsigned long long *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+
+// Waits for phase `parity` of the barrier to complete, at most kStageSpin polls; false on timeout.
+constexpr int kStageSpin = 1 << 20;
+__device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned parity) {
+    for (int i = 0; i < kStageSpin; ++i) {
+        unsigned done;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.b32 %0, 1, 0, p;\n}"
+                     : "=r"(done)
+                     : "r"(smem_u32(bar)), "r"(parity)
+                     : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+// Shared memory of the single-flow kernel: frequency mesh; the RPA schedule when it is staged;
+// then per warp: 32 node descriptors and, per node group, a panel of 2 w float2.  The same warp
+// area holds, after a t channel, the matrix M (w x w float2) and the n_seg segment partials of
+// the pair walk.
+__host__ __device__ inline size_t align16(size_t x) { return (x + 15) / 16 * 16; }
+// A node's sites are held by W lanes, one site each, so a warp evaluates G = 32/W nodes at once.
+// Two sites per lane (half the address arithmetic, descriptor reads and control per node) need so
+// many more registers that they lose: cubic r6 at a mid cutoff 4.32 ms against 3.61.
+constexpr int kSpt = 1;
+// CTAs per SM the register budget is sized for: M takes 4 MB^2 registers a lane, and a budget that
+// spills loses more than the resident warps gain (ms at a mid cutoff with 2, 3, 4 CTAs: 20 sites
+// (MB 3) 4.41, 3.69, 5.06; 31 sites (MB 4) 9.70, 12.26, 16.84; 12 sites (MB 2) 0.96, 0.76, 0.82;
+// 6 sites (MB 1) 0.125, 0.125, 0.133).
+constexpr int vertex_min_blocks(int MB) { return MB <= 3 ? 3 : 2; }
+__host__ __device__ constexpr int lanes_of(int MB) { return MB == 1 ? 8 : (MB == 2 ? 16 : 32); }
+__host__ __device__ inline size_t warp_bytes(int MB, int n_seg) {
+    const size_t w = 8 * MB, G = 32 / lanes_of(MB);
+    const size_t main = kBatch * sizeof(ItemDesc) + G * sizeof(float2) * 2 * w;
+    const size_t st = align16(sizeof(float2) * (w * w + n_seg));
+    return main > st ? main : st;
+}
+__host__ __device__ inline size_t sched_bytes(const RpaSchedule &r, int nl) {
+    return r.in_smem ? align16(sizeof(int) * size_t(rpa_smem_ints(r, nl))) : 0;
+}
+
+// What one warp needs to evaluate items of one flow: lane roles, site indices, its shared-memory
+// area and the RPA schedule (shared or global memory).
+struct WarpCtx {
+    ItemDesc *desc;
+    float2 *panel;  // first panel (A2[w], B2[w]) of the warp; the lane's group has panel g
+    const int *sched, *count, *slot_base, *seg_ptr;
+    SiteRef sr[kSpt];
+    int g, jl;
+};
+
+template <int MB>
+__device__ __forceinline__ void setup_ctx(const FlowArgs &a, int lane, unsigned char *area, const int *sched,
+                                          const int *count, const int *slot_base, const int *seg_ptr, WarpCtx &c) {
+    constexpr int W = lanes_of(MB), G = 32 / W;
+    c.desc = reinterpret_cast<ItemDesc *>(area);
+    c.panel = reinterpret_cast<float2 *>(area + kBatch * sizeof(ItemDesc));
+    c.sched = sched;
+    c.count = count;
+    c.slot_base = slot_base;
+    c.seg_ptr = seg_ptr;
+    c.g = lane / W;
+    c.jl = lane - c.g * W;
+    // panel entries of sites >= Nl are never written; they enter only rows and columns of M that no pair names
+    for (int i = lane; i < G * 16 * MB; i += 32) c.panel[i] = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int k = 0; k < kSpt; ++k) {
+        const int j = min(c.jl + k * W, a.nl - 1);
+        c.sr[k].site = a.sites[j];
+        c.sr[k].isite = a.inv_sites[j];
+    }
+    __syncwarp();
+}
+
+// After a t channel: the lane's block of M goes to Ms (the warp area: descriptors and panels are
+// free then), the warp walks the merged pair
+// list once (segment partials after M), and group 0 adds its rid's sum s2 * sum m M[rid1][rid2]
+// (spin) and s8 * ... (density) to the triple's accumulators.
+template <int MB>
+__device__ __forceinline__ void outer_gather(const FlowArgs &a, const WarpCtx &c, float2 *Ms, int lane,
+                                             const OuterAcc<MB> &M, Acc (&acc)[kSpt]) {
+    constexpr int W = 8 * MB;
+    float2 *slots = Ms + W * W;
+    const int rb = lane >> 2, cb = lane & 3;
+#pragma unroll
+    for (int i = 0; i < MB; ++i)
+#pragma unroll
+        for (int j = 0; j < 2 * MB; ++j) Ms[(rb * MB + i) * W + cb * 2 * MB + j] = M.m[i][j];
+    __syncwarp();
+    const int lanes = a.rpa.lanes;
+    const int cnt = c.count[lane];
+    int slot = c.slot_base[lane];
+    const int *sched = c.sched + lane;
+    const char *mb = reinterpret_cast<const char *>(Ms);
+    float2 sum = make_float2(0.0f, 0.0f);
+    auto step = [&](int e, float2 v) {
+        const float m = float((e >> 16) & 0xff);
+        sum = fma2(make_float2(m, m), v, sum);
+        if (e < 0) {  // last pair of a segment
+            slots[slot++] = sum;
+            sum = make_float2(0.0f, 0.0f);
+        }
+    };
+    constexpr int kU = 4;
+    int i = 0;
+    for (; i + kU <= cnt; i += kU) {
+        int e[kU];
+        float2 v[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) e[u] = sched[(i + u) * lanes];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) v[u] = *reinterpret_cast<const float2 *>(mb + (e[u] & 0xffff));
+#pragma unroll
+        for (int u = 0; u < kU; ++u) step(e[u], v[u]);
+    }
+    for (; i < cnt; ++i) {
+        const int e = sched[i * lanes];
+        step(e, *reinterpret_cast<const float2 *>(mb + (e & 0xffff)));
+    }
+    __syncwarp();
+    if (c.g == 0) {
+        const float2 f = make_float2(2.0f * a.spin, 8.0f * a.spin);  // SU2FrgCore.cpp:265-266
+#pragma unroll
+        for (int k = 0; k < kSpt; ++k) {
+            const int j = c.jl + k * lanes_of(MB);
+            if (j < a.nl) {
+                float2 s = make_float2(0.0f, 0.0f);
+                for (int q = c.seg_ptr[j]; q < c.seg_ptr[j + 1]; ++q) s = add2(s, slots[q]);
+                acc[k].add(f, s);
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// The nodes desc[0 .. nb) of a transfer frequency: adds their terms to the accumulators and their
+// panels to M.  coef(k): the node's coefficient for this flow.
+template <int MB, class Coef>
+__device__ __forceinline__ void item_nodes(const float2 *sd, int nl, const ItemDesc *desc, int nb, int step,
+                                           const WarpCtx &c, int lane, Coef &&coef, Acc (&A)[kSpt], Acc (&B)[kSpt],
+                                           Acc (&T)[kSpt], OuterAcc<MB> &M) {
+    constexpr int W = lanes_of(MB), G = 32 / W;
+    const int trips = (nb + G - 1) / G;
+#pragma unroll 1
+    for (int t = 0; t < trips; ++t) {
+        const int k = t * G + c.g;  // group g: nodes g, g + G, g + 2 G, ...
+        const bool active = G == 1 || k < nb;
+        const int kk = active ? k : 0;
+        float2 pa[kSpt], pb[kSpt];
+        node_eval<kSpt, W, false>(sd, desc[kk], coef(kk), step, active, 0, c.sr, c.jl, nullptr, A, B, T, pa, pb);
+        float2 *pan = c.panel + c.g * 16 * MB + c.jl;
+#pragma unroll
+        for (int s = 0; s < kSpt; ++s)
+            if (c.jl + s * W < nl) {
+                pan[s * W] = pa[s];
+                pan[8 * MB + s * W] = pb[s];
+            }
+        __syncwarp();  // panels written
+        outer_update<MB>(c.panel, lane, t, G, nb, M);
+        __syncwarp();  // panels read
+    }
+}
+
+// The flow of triple (s, t, u): the node groups' sums in xor-shuffle order, over 2 pi.
+template <int MB>
+__device__ __forceinline__ void store_triple(const FlowArgs &a, float2 *dsd, unsigned *status, const WarpCtx &c,
+                                             const Acc (&acc)[kSpt], int s, int t, int u) {
+    constexpr int W = lanes_of(MB);
+    const float two_pi = 2.0f * float(kPi);
+#pragma unroll
+    for (int k = 0; k < kSpt; ++k) {
+        float2 v = acc[k].value();
+#pragma unroll
+        for (int o = W; o < 32; o <<= 1)
+            v = add2(v, make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o)));
+        const int j = c.jl + k * W;
+        if (c.g == 0 && j < a.nl) {
+            const float os = v.x / two_pi, od = v.y / two_pi;
+            dsd[(size_t(su_index(s, u)) * a.n + t) * a.nl + j] = make_float2(os, od);
+            if (isnan(os) || isnan(od)) atomicOr(status, kStatusNaN);
+        }
+    }
+}
+
+template <int MB>
+__device__ __forceinline__ void clear_outer(OuterAcc<MB> &M) {
+#pragma unroll
+    for (int i = 0; i < MB; ++i)
+#pragma unroll
+        for (int j = 0; j < 2 * MB; ++j) M.m[i][j] = make_float2(0.0f, 0.0f);
+}
+
+// Transfer frequency `step` of item (p, q, r) and its pair: transfer p has the targets (p,q,r),
+// (p,r,q) and the t channel of (q,p,r); transfer q (q,p,r), (p,r,q), t of (p,q,r); transfer r
+// (q,p,r), (p,q,r), t of (p,r,q).  With accumulators A, B, T for the first and second target and
+// the t channel, A and T trade places after the first, B and T after the second transfer, and A
+// ends as (q,p,r), B as (p,q,r), T as (p,r,q).
+__device__ __forceinline__ ItemFreq item_step(const float *pos, int step, int p, int q, int r) {
+    return item_freq(pos, step == 0 ? p : (step == 1 ? q : r), step == 0 ? q : p, step == 2 ? q : r, step == 2);
+}
+__device__ __forceinline__ void turn_accs(int step, Acc (&A)[kSpt], Acc (&B)[kSpt], Acc (&T)[kSpt]) {
+#pragma unroll
+    for (int k = 0; k < kSpt; ++k) {
+        if (step == 0) swap_acc(A[k], T[k]);
+        if (step == 1) swap_acc(B[k], T[k]);
+    }
+}
+
+// The three triples of an item of flow `a` (all lanes of the warp take part).  The single-flow and
+// the batched kernel both evaluate items with this function, so a flow's result does not depend
+// on the kernel, the launch or the other flows of a batch.
+template <int MB>
+__device__ __forceinline__ void vertex_item(const FlowArgs &a, const float *pos, int item, const WarpCtx &c, int lane) {
+    int p, q, r;
+    decode_item(item, p, q, r);
+    Acc A[kSpt], B[kSpt], T[kSpt];
+#pragma unroll
+    for (int k = 0; k < kSpt; ++k) {
+        A[k].clear();
+        B[k].clear();
+        T[k].clear();
+    }
+#pragma unroll 1
+    for (int step = 0; step < 3; ++step) {
+        const ItemFreq f = item_step(pos, step, p, q, r);
+        OuterAcc<MB> M;
+        clear_outer(M);
+        const int cnt = __ldg(a.node_cnt + f.xi);
+        const float *nwp = a.node_wp + size_t(f.xi) * a.max_nodes;
+        const float *nc = a.node_c + size_t(f.xi) * a.max_nodes;
+        for (int b0 = 0; b0 < cnt; b0 += kBatch) {
+            const int nb = min(kBatch, cnt - b0);
+            if (lane < nb) make_item(a, pos, f, __ldg(nwp + b0 + lane), __ldg(nc + b0 + lane), c.desc[lane]);
+            __syncwarp();
+            item_nodes<MB>(a.sd, a.nl, c.desc, nb, step, c, lane, [&](int k) { return c.desc[k].c; }, A, B,
+                                T, M);
+        }
+        outer_gather<MB>(a, c, reinterpret_cast<float2 *>(c.desc), lane, M, T);
+        turn_accs(step, A, B, T);
+    }
+    store_triple<MB>(a, a.dsd, a.status, c, B, p, q, r);
+    if (q != r) store_triple<MB>(a, a.dsd, a.status, c, T, p, r, q);
+    if (p != q) store_triple<MB>(a, a.dsd, a.status, c, A, q, p, r);
+}
+
+template <int MB>
+__global__ void __launch_bounds__(kThreads, vertex_min_blocks(MB)) su2_vertex_flow_kernel(FlowArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ __align__(8) unsigned long long stage_bar;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned char *sbase = smem_raw + kMaxFreq * sizeof(float);
+
+    // Stage the frequency mesh and (if selected) the RPA schedule image in shared memory with
+    // the bulk-copy engine: one thread arms an mbarrier with the byte count and issues the
+    // copies; every thread waits on the barrier (bounded; on timeout the kernel records
+    // kStatusStageTimeout and reads the global copies instead).
+    const unsigned pos_bytes = (unsigned(a.n) * sizeof(float) + 15u) & ~15u;
+    const unsigned img_bytes = a.rpa.in_smem ? unsigned(a.rpa.image_bytes) : 0u;
+    if (threadIdx.x == 0) {
+        mbar_init(&stage_bar, 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        mbar_arrive_expect_tx(&stage_bar, pos_bytes + img_bytes);
+        bulk_copy_g2s(smem_raw, a.freq, pos_bytes, &stage_bar);
+        if (img_bytes) bulk_copy_g2s(sbase, a.rpa.image, img_bytes, &stage_bar);
+    }
+    const bool staged = mbar_wait(&stage_bar, 0);
+    if (!staged) atomicOr(a.status, kStatusStageTimeout);
+
+    const float *pos = staged ? reinterpret_cast<const float *>(smem_raw) : a.freq;
+    const int *sched, *count, *slot_base, *seg_ptr;
+    if (a.rpa.in_smem && staged) {
+        const int *s = reinterpret_cast<const int *>(sbase);
+        const int ns = a.rpa.len * a.rpa.lanes, nc = a.rpa.lanes;
+        sched = s;
+        count = s + ns;
+        slot_base = s + ns + nc;
+        seg_ptr = s + ns + 2 * nc;
+    } else {
+        sched = a.rpa.sched;
+        count = a.rpa.count;
+        slot_base = a.rpa.slot_base;
+        seg_ptr = a.rpa.seg_ptr;
+    }
+    WarpCtx c;
+    setup_ctx<MB>(a, lane, sbase + sched_bytes(a.rpa, a.nl) + warp * warp_bytes(MB, a.rpa.n_seg), sched, count,
+                  slot_base, seg_ptr, c);
+    __syncthreads();
+
+    const int items = vertex_items(a.n);
+    for (;;) {
+        int it = 0;
+        if (lane == 0) it = atomicAdd(a.work_counter, 1);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= items) break;
+        vertex_item<MB>(a, pos, it, c, lane);
+    }
+    // a copy that timed out must still land before the block's shared memory is released
+    if (!staged && threadIdx.x == 0) mbar_wait(&stage_bar, 0);
+}
+
+// Batched vertex flow: a persistent grid over the ragged list of (flow, item) pairs of all flows
+// of one site class.  A warp keeps the flow it works on (argument block, frequency mesh, lane
+// roles) in its own shared-memory area and reloads it only when an item of another flow comes
+// up; items are numbered flow by flow, so that happens rarely.  The RPA schedule is read from
+// global memory (it differs between flows) unless every flow's fits the warp's area.
+template <int MB>
+__global__ void __launch_bounds__(kThreads, vertex_min_blocks(MB)) su2_vertex_batch_kernel(BatchVertexArgs b) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t fa_bytes = align16(sizeof(FlowArgs)), pos_bytes = align16(sizeof(float) * b.n_max);
+    const size_t sch_bytes = align16(sizeof(int) * size_t(b.sched_ints));
+    unsigned char *wbase = smem_raw + size_t(warp) * (fa_bytes + pos_bytes + sch_bytes + b.warp_area);
+    FlowArgs *fa = reinterpret_cast<FlowArgs *>(wbase);
+    float *pos = reinterpret_cast<float *>(wbase + fa_bytes);
+    int *sch = reinterpret_cast<int *>(wbase + fa_bytes + pos_bytes);
+    unsigned char *area = wbase + fa_bytes + pos_bytes + sch_bytes;
+
+    WarpCtx c;
+    int cur = -1, base = 0;
+    bool skip = false;
+    for (;;) {
+        int w = 0;
+        if (lane == 0) w = atomicAdd(b.counter, 1);
+        w = __shfl_sync(0xffffffffu, w, 0);
+        if (w >= b.total) break;
+        int lo = 0, hi = b.n_list - 1;  // last f with prefix[f] <= w
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (__ldg(b.prefix + mid) <= w) lo = mid;
+            else hi = mid - 1;
+        }
+        if (lo != cur) {
+            cur = lo;
+            base = __ldg(b.prefix + lo);
+            const BatchFlow *bf = b.flows + __ldg(b.list + lo);
+            __syncwarp();
+            const int *src = reinterpret_cast<const int *>(&bf->a);
+            int *dst = reinterpret_cast<int *>(fa);
+            for (int i = lane; i < int(sizeof(FlowArgs) / sizeof(int)); i += 32) dst[i] = src[i];
+            skip = bf->phase != kPhaseFlowing;
+            __syncwarp();
+            for (int i = lane; i < fa->n; i += 32) pos[i] = fa->freq[i];
+            if (b.sched_ints > 0) {  // the host checked that every flow's schedule fits
+                const RpaSchedule &r = fa->rpa;
+                const int ns = r.len * r.lanes, nc = r.lanes;
+                for (int i = lane; i < ns; i += 32) sch[i] = __ldg(r.sched + i);
+                for (int i = lane; i < nc; i += 32) {
+                    sch[ns + i] = __ldg(r.count + i);
+                    sch[ns + nc + i] = __ldg(r.slot_base + i);
+                }
+                for (int i = lane; i <= fa->nl; i += 32) sch[ns + 2 * nc + i] = __ldg(r.seg_ptr + i);
+                setup_ctx<MB>(*fa, lane, area, sch, sch + ns, sch + ns + nc, sch + ns + 2 * nc, c);
+            } else {
+                setup_ctx<MB>(*fa, lane, area, fa->rpa.sched, fa->rpa.count, fa->rpa.slot_base, fa->rpa.seg_ptr, c);
+            }
+            __syncwarp();
+        }
+        if (skip) continue;
+        vertex_item<MB>(*fa, pos, w - base, c, lane);
+    }
+}
+
+// ------------------------------------------------------------------------------------
+// Triple by triple, a warp per triple, for lattices of at most 32 sites on which some pair differs
+// from its exchanged pair (site_exchange_kind > 0, e.g. pyrochlore).  By items such a flow is faster
+// too (pyrochlore r5, N = 64, late: 10.7 ms against 14.4), but rounds the interpolation coordinates
+// otherwise than the reference (one operation each, in the order of each channel).  Late in a
+// strongly coupled flow the self-energy flow of these lattices cancels to a part in 10^3 and the
+// vertex grows by its square in every step, which takes the difference to 10^-5 .. 10^-4 of the
+// final correlations (either form is that far from the exact flow there), so they keep the
+// reference's coordinates.
+// ------------------------------------------------------------------------------------
+namespace triple {
+constexpr int SPT = 1, NPI = 1;  // one site per lane, one node per group and step
+
 // Adds the outer products of the panels of nodes k = (r*NPI+n)*G+gg < nb (ascending k) to the
 // lane's block of M.  `pan`: the warp's first panel; panel (gg, n) starts pstride float2 later
 // per step of gg * NPI + n.
-template <int NPI, int MB>
-__device__ __forceinline__ void outer_update(const float2 *pan, int pstride, int lane, int r, int G, int nb,
+template <int MB>
+__device__ __forceinline__ void triple_outer_update(const float2 *pan, int pstride, int lane, int r, int G, int nb,
                                              OuterAcc<MB> &M) {
     constexpr int W = 8 * MB;
     const int rb = lane >> 2, cb = lane & 3;
@@ -513,7 +799,7 @@ __device__ __forceinline__ void outer_update(const float2 *pan, int pstride, int
         }
 }
 
-template <int CH, int SPT, int NPI, int MB>
+template <int CH, int MB>
 __device__ __forceinline__ void channel_sum(const FlowArgs &a, const float *pos, const Transfer &f, int xi, int lane, int g,
                                             int G, int jl, const Lane<SPT> &ln, NodeDesc *desc, const TExchange *tx,
                                             const float2 *pan, int pstride, OuterAcc<MB> &M,
@@ -557,7 +843,7 @@ __device__ __forceinline__ void channel_sum(const FlowArgs &a, const float *pos,
                 }
             if constexpr (CH == kT && SPT == 1) {
                 __syncwarp();  // panels written
-                outer_update<NPI, MB>(pan, pstride, lane, r, G, nb, M);
+                triple_outer_update<MB>(pan, pstride, lane, r, G, nb, M);
                 __syncwarp();  // panels read
             }
         }
@@ -565,72 +851,18 @@ __device__ __forceinline__ void channel_sum(const FlowArgs &a, const float *pos,
     }
 }
 
-// ------------------------------------------------------------------------------------
-// Bulk copies global -> shared through the copy engine (cp.async.bulk) completing on an
-// mbarrier.  Addresses and sizes are multiples of 16 bytes.
-// ------------------------------------------------------------------------------------
-__device__ __forceinline__ unsigned smem_u32(const void *p) { return unsigned(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long *bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void bulk_copy_g2s(void *dst, const void *src, unsigned bytes, unsigned long long *bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-
-// Waits for phase `parity` of the barrier to complete, at most kStageSpin polls; false on timeout.
-constexpr int kStageSpin = 1 << 20;
-__device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned parity) {
-    for (int i = 0; i < kStageSpin; ++i) {
-        unsigned done;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                     "selp.b32 %0, 1, 0, p;\n}"
-                     : "=r"(done)
-                     : "r"(smem_u32(bar)), "r"(parity)
-                     : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-
-// Shared memory of the single-flow kernel: frequency mesh; the RPA schedule when it is staged;
-// then per warp: 32 node descriptors and, per node group, NPI t-channel exchange areas (Nl <=
-// 32: a panel of 2 w float2; otherwise four arrays of W*SPT sites and n_seg slots).  For Nl <=
-// 32 the same warp area holds, between the t and the u channel, the matrix M (w x w float2)
-// and the n_seg segment partials of the pair walk.
-__host__ __device__ inline size_t node_area_bytes(int wsite, int spt, int n_seg, int w) {
-    if (spt == 1) return sizeof(float2) * 2 * size_t(w);  // w is a multiple of 8: 16-byte aligned
-    return (sizeof(float) * 4 * size_t(wsite) * spt + sizeof(float2) * n_seg + 15) / 16 * 16;
-}
-__host__ __device__ inline size_t group_area_bytes(int wsite, int spt, int npi, int n_seg, int w) {
-    return (32 / wsite) * npi * node_area_bytes(wsite, spt, n_seg, w);
-}
-__host__ __device__ inline size_t outer_stage_bytes(int w, int n_seg) {
-    return (sizeof(float2) * (size_t(w) * w + n_seg) + 15) / 16 * 16;
-}
-__host__ __device__ inline size_t warp_bytes(int wsite, int spt, int npi, int n_seg, int w) {
-    const size_t main = kBatch * sizeof(NodeDesc) + group_area_bytes(wsite, spt, npi, n_seg, w);
-    if (spt != 1) return main;
-    const size_t st = outer_stage_bytes(w, n_seg);
+// Shared memory per warp: 32 node descriptors and, per node group, a t-channel panel of 2 w float2;
+// the same area holds, between the t and the u channel, the matrix M (w x w float2) and the n_seg
+// segment partials of the pair walk.
+__host__ __device__ inline size_t triple_warp_bytes(int wsite, int n_seg, int w) {
+    const size_t main = kBatch * sizeof(NodeDesc) + (32 / wsite) * sizeof(float2) * 2 * size_t(w);
+    const size_t st = align16(sizeof(float2) * (size_t(w) * w + n_seg));
     return main > st ? main : st;
 }
-__host__ __device__ inline size_t sched_bytes(const RpaSchedule &r, int nl) {
-    return r.in_smem ? (sizeof(int) * size_t(rpa_smem_ints(r, nl)) + 15) / 16 * 16 : 0;
-}
-__host__ __device__ inline size_t align16(size_t x) { return (x + 15) / 16 * 16; }
 
 // What one warp needs to evaluate triples of one flow: lane roles, site indices and the
 // shared-memory areas.
-template <int SPT, int NPI>
-struct WarpCtx {
+struct TripleCtx {
     NodeDesc *desc;
     TExchange tx[NPI];
     Lane<SPT> ln;
@@ -640,16 +872,16 @@ struct WarpCtx {
 };
 
 // `groups`: the warp's node-group areas; sched..seg_ptr: the RPA schedule (shared or global).
-template <int SPT, int NPI, int MB>
-__device__ __forceinline__ void setup_ctx(const FlowArgs &a, int lane, NodeDesc *desc, unsigned char *groups,
+template <int MB>
+__device__ __forceinline__ void triple_ctx(const FlowArgs &a, int lane, NodeDesc *desc, unsigned char *groups,
                                           const int *sched, const int *count, const int *slot_base, const int *seg_ptr,
-                                          WarpCtx<SPT, NPI> &c) {
+                                          TripleCtx &c) {
     c.desc = desc;
     c.W = (SPT == 1) ? a.wsite : 32;
     c.G = 32 / c.W;
     c.g = lane / c.W;
     c.jl = lane - c.g * c.W;
-    const size_t nab = node_area_bytes(c.W, SPT, a.rpa.n_seg, 8 * MB);
+    const size_t nab = sizeof(float2) * 16 * MB;
     c.panel = reinterpret_cast<float2 *>(groups);
     c.pstride = int(nab / sizeof(float2));
     if (SPT == 1) {  // panel entries of sites >= Nl stay zero
@@ -685,8 +917,8 @@ __device__ __forceinline__ void setup_ctx(const FlowArgs &a, int lane, NodeDesc 
 // Nl <= 32, after the t channel: the lane's block of M goes to the warp area, the warp walks
 // the merged pair list once (segment partials after M), and group 0 adds its rid's sum
 // s2 * sum m M[rid1][rid2] (spin) and s8 * ... (density) to its accumulators.
-template <int SPT, int NPI, int MB>
-__device__ __forceinline__ void outer_gather(const FlowArgs &a, const WarpCtx<SPT, NPI> &c, int lane,
+template <int MB>
+__device__ __forceinline__ void triple_outer_gather(const FlowArgs &a, const TripleCtx &c, int lane,
                                              const OuterAcc<MB> &M, float *acc_s, float *cmp_s, float *acc_d,
                                              float *cmp_d) {
     constexpr int W = 8 * MB;
@@ -743,8 +975,8 @@ __device__ __forceinline__ void outer_gather(const FlowArgs &a, const WarpCtx<SP
     __syncwarp();
 }
 
-template <int SPT, int NPI, int MB>
-__device__ __forceinline__ void vertex_triple(const FlowArgs &a, const float *pos, int it, const WarpCtx<SPT, NPI> &c,
+template <int MB>
+__device__ __forceinline__ void vertex_triple(const FlowArgs &a, const float *pos, int it, const TripleCtx &c,
                                               int lane) {
     const float two_pi = 2.0f * float(kPi);
     const int su = it / a.n, ti = it - su * a.n;
@@ -773,12 +1005,12 @@ __device__ __forceinline__ void vertex_triple(const FlowArgs &a, const float *po
     for (int i = 0; i < (MB > 0 ? MB : 1); ++i)
 #pragma unroll
         for (int j = 0; j < (MB > 0 ? 2 * MB : 1); ++j) M.m[i][j] = make_float2(0.0f, 0.0f);
-    channel_sum<kS, SPT, NPI, MB>(a, pos, f, si, lane, c.g, c.G, c.jl, c.ln, c.desc, c.tx, c.panel, c.pstride, M, acc_s,
+    channel_sum<kS, MB>(a, pos, f, si, lane, c.g, c.G, c.jl, c.ln, c.desc, c.tx, c.panel, c.pstride, M, acc_s,
                                   cmp_s, acc_d, cmp_d);
-    channel_sum<kT, SPT, NPI, MB>(a, pos, f, ti, lane, c.g, c.G, c.jl, c.ln, c.desc, c.tx, c.panel, c.pstride, M, acc_s,
+    channel_sum<kT, MB>(a, pos, f, ti, lane, c.g, c.G, c.jl, c.ln, c.desc, c.tx, c.panel, c.pstride, M, acc_s,
                                   cmp_s, acc_d, cmp_d);
-    if constexpr (SPT == 1) outer_gather<SPT, NPI, MB>(a, c, lane, M, acc_s, cmp_s, acc_d, cmp_d);
-    channel_sum<kU, SPT, NPI, MB>(a, pos, f, ui, lane, c.g, c.G, c.jl, c.ln, c.desc, c.tx, c.panel, c.pstride, M, acc_s,
+    if constexpr (SPT == 1) triple_outer_gather<MB>(a, c, lane, M, acc_s, cmp_s, acc_d, cmp_d);
+    channel_sum<kU, MB>(a, pos, f, ui, lane, c.g, c.G, c.jl, c.ln, c.desc, c.tx, c.panel, c.pstride, M, acc_s,
                                   cmp_s, acc_d, cmp_d);
 
 #pragma unroll
@@ -796,8 +1028,8 @@ __device__ __forceinline__ void vertex_triple(const FlowArgs &a, const float *po
     }
 }
 
-template <int SPT, int NPI, int MB>
-__global__ void __launch_bounds__(kThreads) su2_vertex_flow_kernel(FlowArgs a) {
+template <int MB>
+__global__ void __launch_bounds__(kThreads) su2_triple_flow_kernel(FlowArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long stage_bar;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -839,9 +1071,9 @@ __global__ void __launch_bounds__(kThreads) su2_vertex_flow_kernel(FlowArgs a) {
         slot_base = a.rpa.slot_base;
         seg_ptr = a.rpa.seg_ptr;
     }
-    unsigned char *wbase = sbase + sched_bytes(a.rpa, a.nl) + warp * warp_bytes(W, SPT, NPI, n_seg, 8 * MB);
-    WarpCtx<SPT, NPI> c;
-    setup_ctx<SPT, NPI, MB>(a, lane, reinterpret_cast<NodeDesc *>(wbase), wbase + kBatch * sizeof(NodeDesc), sched, count,
+    unsigned char *wbase = sbase + sched_bytes(a.rpa, a.nl) + warp * triple_warp_bytes(W, n_seg, 8 * MB);
+    TripleCtx c;
+    triple_ctx<MB>(a, lane, reinterpret_cast<NodeDesc *>(wbase), wbase + kBatch * sizeof(NodeDesc), sched, count,
                             slot_base, seg_ptr, c);
     __syncthreads();
 
@@ -850,32 +1082,27 @@ __global__ void __launch_bounds__(kThreads) su2_vertex_flow_kernel(FlowArgs a) {
         if (lane == 0) it = atomicAdd(a.work_counter, 1);
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= a.fn) break;
-        vertex_triple<SPT, NPI, MB>(a, pos, it, c, lane);
+        vertex_triple<MB>(a, pos, it, c, lane);
     }
     // a copy that timed out must still land before the block's shared memory is released
     if (!staged && threadIdx.x == 0) mbar_wait(&stage_bar, 0);
 }
 
-// Batched vertex flow: a persistent grid over the ragged list of (flow, triple) items of all
-// flows of one site class.  A warp keeps the flow it works on (argument block, frequency
-// mesh, lane roles) in its own shared-memory area and reloads it only when an item of another
-// flow comes up; items are numbered flow by flow, so that happens rarely.  The RPA schedule
-// is read from global memory (it differs between flows).
-template <int SPT, int NPI, int MB>
-__global__ void __launch_bounds__(kThreads) su2_vertex_batch_kernel(BatchVertexArgs b) {
+template <int MB>
+__global__ void __launch_bounds__(kThreads) su2_triple_batch_kernel(BatchVertexArgs b) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const size_t fa_bytes = align16(sizeof(FlowArgs)), pos_bytes = align16(sizeof(float) * b.n_max);
     const size_t sch_bytes = align16(sizeof(int) * size_t(b.sched_ints));
     unsigned char *wbase =
-        smem_raw + size_t(warp) * (fa_bytes + pos_bytes + sch_bytes + kBatch * sizeof(NodeDesc) + b.warp_area);
+        smem_raw + size_t(warp) * (fa_bytes + pos_bytes + sch_bytes + b.warp_area);
     FlowArgs *fa = reinterpret_cast<FlowArgs *>(wbase);
     float *pos = reinterpret_cast<float *>(wbase + fa_bytes);
     int *sch = reinterpret_cast<int *>(wbase + fa_bytes + pos_bytes);
     NodeDesc *desc = reinterpret_cast<NodeDesc *>(wbase + fa_bytes + pos_bytes + sch_bytes);
     unsigned char *groups = wbase + fa_bytes + pos_bytes + sch_bytes + kBatch * sizeof(NodeDesc);
 
-    WarpCtx<SPT, NPI> c;
+    TripleCtx c;
     int cur = -1, base = 0;
     bool skip = false;
     for (;;) {
@@ -909,127 +1136,72 @@ __global__ void __launch_bounds__(kThreads) su2_vertex_batch_kernel(BatchVertexA
                     sch[ns + nc + i] = __ldg(r.slot_base + i);
                 }
                 for (int i = lane; i <= fa->nl; i += 32) sch[ns + 2 * nc + i] = __ldg(r.seg_ptr + i);
-                setup_ctx<SPT, NPI, MB>(*fa, lane, desc, groups, sch, sch + ns, sch + ns + nc, sch + ns + 2 * nc, c);
+                triple_ctx<MB>(*fa, lane, desc, groups, sch, sch + ns, sch + ns + nc, sch + ns + 2 * nc, c);
             } else {
-                setup_ctx<SPT, NPI, MB>(*fa, lane, desc, groups, fa->rpa.sched, fa->rpa.count, fa->rpa.slot_base,
+                triple_ctx<MB>(*fa, lane, desc, groups, fa->rpa.sched, fa->rpa.count, fa->rpa.slot_base,
                                         fa->rpa.seg_ptr, c);
             }
             __syncwarp();
         }
         if (skip) continue;
-        vertex_triple<SPT, NPI, MB>(*fa, pos, w - base, c, lane);
+        vertex_triple<MB>(*fa, pos, w - base, c, lane);
     }
 }
+
+}  // namespace triple
 
 // ------------------------------------------------------------------------------------
 // Grouped batches: flows that share the frequency mesh, the lattice tables and the current
 // cutoff (a parameter scan's members of one lattice, range and frequency count, started
 // together) have the same loop-frequency node positions and the same interpolation supports
-// for every (triple, node); only the state, the node coefficients (through the self-energy)
-// and the t channel's site-local values differ.  A CTA takes one triple for a subgroup of up to
-// kGroupWarps * 32 / W flows: its threads build each node's supports once, in chunks of 32
-// nodes, and every warp evaluates them for 32 / W flows at once, lane = (flow, site).
-//
-// The result of every flow is the single-flow kernel's, bit for bit: a flow's W lanes keep the
-// single-flow kernel's G = 32 / W Kahan accumulator pairs (node k of a channel adds into pair
-// k mod G, the RPA term into pair 0 after the t channel) and combine them in its order, and
-// the outer-product matrix M adds the nodes' panels in ascending order.  The pair walk follows
-// the same 32-chunk schedule, each of the flow's W lanes walking chunks l, l + W, ...
+// for every (item, node); only the state and the node coefficients (through the self-energy)
+// differ.  A CTA takes one item for a subgroup of up to kGroupWarps flows: its threads build
+// each node's supports once, one node per thread, and every warp evaluates them for its own flow
+// with the single-flow kernel's code, so every flow's result is the single-flow kernel's, bit for
+// bit.
 // ------------------------------------------------------------------------------------
 constexpr int kGroupWarps = 4;
-constexpr int kGroupChunk = 32;  // nodes whose supports the CTA builds at once (four threads per node)
-static_assert(kGroupWarps * 32 == 4 * kGroupChunk, "the grouped kernel builds a chunk with four threads per node");
-
-// What a lane of a grouped warp needs of its flow (node_term reads a.sd and a.spin).
-struct GroupLaneArgs {
-    const float2 *sd;
-    float spin;
-};
-
-__host__ __device__ constexpr int group_cb(int W) { return W == 8 ? 2 : 4; }
-
-// Adds the outer product of the flow's panel (A2 = c * third slab, B2 = fourth slab; w entries
-// each) to the lane's R x C block of M; the flow's W lanes form a (W / Cb) x Cb grid.
-template <int W, int MB>
-__device__ __forceinline__ void group_outer_update(const float2 *pan, int jl, float2 (*m)[8 * MB / group_cb(W)]) {
-    constexpr int w = 8 * MB, Cb = group_cb(W), Rb = W / Cb, R = w / Rb, C = w / Cb;
-    const int rb = jl / Cb, cb = jl % Cb;
-    float2 av[R], bv[C];
-#pragma unroll
-    for (int i = 0; i < R; ++i) av[i] = pan[rb * R + i];
-#pragma unroll
-    for (int j = 0; j < C; ++j) bv[j] = pan[w + cb * C + j];
-#pragma unroll
-    for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int j = 0; j < C; ++j) m[i][j] = fma2(av[i], bv[j], m[i][j]);
-}
-
-template <int W, int MB>
-struct GroupShape {
-    static constexpr int F = 32 / W;                 // flows per warp
-    static constexpr int GMAX = kGroupWarps * F;     // flows per CTA
-    static constexpr int G = 32 / W;                 // single-flow node groups (accumulator pairs)
-    static constexpr int w = 8 * MB;                 // outer-product width
-    static constexpr int Cb = group_cb(W), R = w / (W / Cb), C = w / Cb;
-};
+constexpr int kGroupChunk = kGroupWarps * 32;  // nodes whose supports the CTA builds at once
+static_assert(kGroupChunk % kBatch == 0, "node k must fall to the same node group as in the single-flow kernel");
 
 // Shared-memory layout of the grouped kernel (bytes from the dynamic base, all 16-aligned).
 struct GroupSmem {
-    size_t fa, ptrs, pos, build_desc, build_loc, build_c, build_lv, stage, panels, total;
+    size_t fa, ptrs, pos, desc, coef, warps, warp_size, total;
 };
-__host__ __device__ inline GroupSmem group_smem_layout(int W, int MB, int n_seg_max) {
-    const int F = 32 / W, GMAX = kGroupWarps * F, w = 8 * MB;
+__host__ __device__ inline GroupSmem group_smem_layout(int MB, int n_seg_max) {
     GroupSmem L;
     size_t o = 0;
     L.fa = o; o += align16(sizeof(FlowArgs));
-    L.ptrs = o; o += align16(size_t(GMAX) * (2 * sizeof(void *) + sizeof(void *) + sizeof(void *) + sizeof(int)));
+    L.ptrs = o; o += align16(size_t(kGroupWarps) * (4 * sizeof(void *) + sizeof(int)));
     L.pos = o; o += align16(sizeof(float) * kMaxFreq);
-    // union: the chunk build area, or (after the t channel) each flow's staged M and slots
-    const size_t u0 = o;
-    L.build_desc = o; o += kGroupChunk * sizeof(NodeDesc);
-    L.build_loc = o; o += kGroupChunk * sizeof(LocDesc);
-    L.build_c = o; o += align16(sizeof(float) * kGroupChunk * GMAX);
-    L.build_lv = o; o += align16(sizeof(float) * 8 * kGroupChunk * GMAX);
-    const size_t build_end = o;
-    L.stage = u0;
-    const size_t stage_end = u0 + align16(sizeof(float2) * size_t(GMAX) * (size_t(w) * w + n_seg_max));
-    o = build_end > stage_end ? build_end : stage_end;
-    L.panels = o; o += align16(sizeof(float2) * size_t(GMAX) * 2 * w);
-    L.total = o;
+    L.desc = o; o += kGroupChunk * sizeof(ItemDesc);
+    L.coef = o; o += align16(sizeof(float) * kGroupChunk * kGroupWarps);
+    L.warps = o;  // per warp: as the single-flow kernel's area (its descriptors only as room for M)
+    L.warp_size = warp_bytes(MB, n_seg_max);
+    L.total = o + kGroupWarps * L.warp_size;
     return L;
 }
 
-template <int W, int MB>
-__global__ void __launch_bounds__(kGroupWarps * 32) su2_vertex_group_kernel(GroupVertexArgs g) {
-    using S = GroupShape<W, MB>;
-    constexpr int F = S::F, GMAX = S::GMAX, G = S::G, w = S::w, R = S::R, C = S::C;
+template <int MB>
+__global__ void __launch_bounds__(kGroupWarps * 32, vertex_min_blocks(MB)) su2_vertex_group_kernel(GroupVertexArgs g) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_item;
-    const GroupSmem L = group_smem_layout(W, MB, g.n_seg_max);
+    const GroupSmem L = group_smem_layout(MB, g.n_seg_max);
     FlowArgs *fa = reinterpret_cast<FlowArgs *>(smem_raw + L.fa);
     unsigned char *pb = smem_raw + L.ptrs;
     const float2 **m_sd = reinterpret_cast<const float2 **>(pb);
-    float2 **m_dsd = reinterpret_cast<float2 **>(pb + GMAX * sizeof(void *));
-    const float **m_nc = reinterpret_cast<const float **>(pb + 2 * GMAX * sizeof(void *));
-    unsigned **m_status = reinterpret_cast<unsigned **>(pb + 3 * GMAX * sizeof(void *));
-    int *m_on = reinterpret_cast<int *>(pb + 4 * GMAX * sizeof(void *));  // member flowing this step
+    float2 **m_dsd = reinterpret_cast<float2 **>(pb + kGroupWarps * sizeof(void *));
+    const float **m_nc = reinterpret_cast<const float **>(pb + 2 * kGroupWarps * sizeof(void *));
+    unsigned **m_status = reinterpret_cast<unsigned **>(pb + 3 * kGroupWarps * sizeof(void *));
+    int *m_on = reinterpret_cast<int *>(pb + 4 * kGroupWarps * sizeof(void *));  // member flowing this step
     float *pos = reinterpret_cast<float *>(smem_raw + L.pos);
-    NodeDesc *desc = reinterpret_cast<NodeDesc *>(smem_raw + L.build_desc);
-    LocDesc *loc = reinterpret_cast<LocDesc *>(smem_raw + L.build_loc);
-    float *ctab = reinterpret_cast<float *>(smem_raw + L.build_c);   // [node][member]
-    float *lvtab = reinterpret_cast<float *>(smem_raw + L.build_lv);  // [node][member][8]
-    float2 *stage = reinterpret_cast<float2 *>(smem_raw + L.stage);
-    float2 *panels = reinterpret_cast<float2 *>(smem_raw + L.panels);
+    ItemDesc *desc = reinterpret_cast<ItemDesc *>(smem_raw + L.desc);
+    float *ctab = reinterpret_cast<float *>(smem_raw + L.coef);  // [member][node]
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int gg = lane / W, jl = lane - gg * W;  // flow slot in the warp, site
-    const int fs = warp * F + gg;                 // member index in the subgroup
-    float2 *pan = panels + size_t(fs) * 2 * w;
-    // panel entries of sites >= Nl are never written and stay zero
-    for (int i = tid; i < GMAX * 2 * w; i += blockDim.x) panels[i] = make_float2(0.0f, 0.0f);
-
-    int cur = -1, base = 0, nf = 0;
+    unsigned char *area = smem_raw + L.warps + warp * L.warp_size;
+    WarpCtx c;
+    int cur = -1, base = 0;
     bool live = false;
     for (;;) {
         __syncthreads();  // the previous item is finished with the shared areas
@@ -1048,23 +1220,22 @@ __global__ void __launch_bounds__(kGroupWarps * 32) su2_vertex_group_kernel(Grou
             base = __ldg(g.prefix + lo);
             // leader: the first member that is flowing this step (its node tables are current)
             int lead = -1, cnt = 0;
-            for (int q = 0; q < GMAX; ++q) {
-                const int fi = __ldg(g.members + size_t(lo) * GMAX + q);
+            for (int q = 0; q < kGroupWarps; ++q) {
+                const int fi = __ldg(g.members + size_t(lo) * kGroupWarps + q);
                 if (fi < 0) break;
                 ++cnt;
                 if (lead < 0 && g.flows[fi].phase == kPhaseFlowing) lead = fi;
             }
-            nf = cnt;
             live = lead >= 0;
             if (live) {
                 const BatchFlow *lf = g.flows + lead;
                 const int *src = reinterpret_cast<const int *>(&lf->a);
                 int *dst = reinterpret_cast<int *>(fa);
                 for (int i = tid; i < int(sizeof(FlowArgs) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
-                if (tid < GMAX) {
-                    const int fi = tid < cnt ? __ldg(g.members + size_t(lo) * GMAX + tid) : -1;
+                if (tid < kGroupWarps) {
+                    const int fi = tid < cnt ? __ldg(g.members + size_t(lo) * kGroupWarps + tid) : -1;
                     const bool on = fi >= 0 && g.flows[fi].phase == kPhaseFlowing;
-                    const BatchFlow *bf = g.flows + (on ? fi : lead);  // idle slots read the leader's data
+                    const BatchFlow *bf = g.flows + (on ? fi : lead);  // idle warps have no flow of their own
                     m_sd[tid] = bf->a.sd;
                     m_dsd[tid] = bf->a.dsd;
                     m_nc[tid] = bf->a.node_c;
@@ -1073,183 +1244,49 @@ __global__ void __launch_bounds__(kGroupWarps * 32) su2_vertex_group_kernel(Grou
                 }
             }
             __syncthreads();
-            if (live)
+            if (live) {
                 for (int i = tid; i < fa->n; i += blockDim.x) pos[i] = fa->freq[i];
+                setup_ctx<MB>(*fa, lane, area, fa->rpa.sched, fa->rpa.count, fa->rpa.slot_base, fa->rpa.seg_ptr, c);
+            }
             __syncthreads();
         }
         if (!live) continue;
-        const int it = item - base;
         const FlowArgs &a = *fa;
-
-        // the triple (as vertex_triple decodes it)
-        const int su = it / a.n, ti = it - su * a.n;
-        int si = int((sqrtf(8.0f * float(su) + 1.0f) - 1.0f) * 0.5f);
-        while (si * (si + 1) / 2 > su) --si;
-        while ((si + 1) * (si + 2) / 2 <= su) ++si;
-        const int ui = su - si * (si + 1) / 2;
-        Transfer f;
-        f.s = pos[si];
-        f.t = pos[ti];
-        f.u = pos[ui];
-        f.w1p = 0.5f * (f.s + f.t + f.u);
-        f.w1 = 0.5f * (f.s - f.t + f.u);
-        f.w2p = 0.5f * (f.s - f.t - f.u);
-        f.w2 = 0.5f * (f.s + f.t - f.u);
-        f.si = si;
-        f.ti = ti;
-        f.ui = ui;
-
-        const bool mine = fs < nf && m_on[fs];
-        const GroupLaneArgs la{m_sd[fs < nf ? fs : 0], a.spin};
-        Lane<1> ln;
-        ln.j[0] = jl;
-        ln.valid[0] = jl < a.nl;
-        ln.site[0] = ln.valid[0] ? a.sites[jl] : 0;
-        ln.isite[0] = ln.valid[0] ? a.inv_sites[jl] : 0;
-        TExchange tx;
-        tx.A2 = pan;
-        tx.B2 = pan + w;
-
-        float acc_s[G], cmp_s[G], acc_d[G], cmp_d[G];
+        const bool mine = m_on[warp] != 0;
+        int p, q, r;
+        decode_item(item - base, p, q, r);
+        Acc A[kSpt], B[kSpt], T[kSpt];
 #pragma unroll
-        for (int q = 0; q < G; ++q) acc_s[q] = cmp_s[q] = acc_d[q] = cmp_d[q] = 0.0f;
-        float2 M[R][C];
-#pragma unroll
-        for (int i = 0; i < R; ++i)
-#pragma unroll
-            for (int j = 0; j < C; ++j) M[i][j] = make_float2(0.0f, 0.0f);
-
-        // node k of a channel adds into pair k mod G: the pairs rotate after every node, and
-        // pair 0 is realigned at the end of each channel
-        auto rotate = [&]() {
-#pragma unroll
-            for (int q = 0; q + 1 < G; ++q) {
-                float t;
-                t = acc_s[q]; acc_s[q] = acc_s[q + 1]; acc_s[q + 1] = t;
-                t = cmp_s[q]; cmp_s[q] = cmp_s[q + 1]; cmp_s[q + 1] = t;
-                t = acc_d[q]; acc_d[q] = acc_d[q + 1]; acc_d[q + 1] = t;
-                t = cmp_d[q]; cmp_d[q] = cmp_d[q + 1]; cmp_d[q + 1] = t;
-            }
-        };
-
-        auto channel = [&](auto chc, int xi) {
-            constexpr int CH = decltype(chc)::value;
-            const int cnt = __ldg(a.node_cnt + xi);
-            const float *nwp = a.node_wp + size_t(xi) * a.max_nodes;
+        for (int k = 0; k < kSpt; ++k) {
+            A[k].clear();
+            B[k].clear();
+            T[k].clear();
+        }
+#pragma unroll 1
+        for (int step = 0; step < 3; ++step) {
+            const ItemFreq f = item_step(pos, step, p, q, r);
+            OuterAcc<MB> M;
+            clear_outer(M);
+            const int cnt = __ldg(a.node_cnt + f.xi);
+            const float *nwp = a.node_wp + size_t(f.xi) * a.max_nodes;
             for (int b0 = 0; b0 < cnt; b0 += kGroupChunk) {
                 const int nb = min(kGroupChunk, cnt - b0);
                 __syncthreads();  // the previous chunk is consumed
-                {  // four threads per node build its supports (the CTA's 128 threads: 32 nodes)
-                    const int k = tid >> 2, q = tid & 3;
-                    int bits = 0;
-                    if (k < nb) bits = make_part<CH>(a, pos, f, __ldg(nwp + b0 + k), q, desc[k], loc[k]);
-                    bits |= __shfl_xor_sync(0xffffffffu, bits, 1);
-                    bits |= __shfl_xor_sync(0xffffffffu, bits, 2);
-                    if (k < nb && q == 0) {
-                        desc[k].exch = bits;
-                        desc[k].c = 0.0f;
-                    }
-                    for (int p = tid; p < nb * GMAX; p += blockDim.x) {
-                        const int kk = p / GMAX, qq = p - kk * GMAX;
-                        float c = __ldg(m_nc[qq] + size_t(xi) * a.max_nodes + b0 + kk);
-                        if (CH == kU) c = -c;
-                        ctab[p] = c;
-                    }
-                }
+                if (tid < nb) make_item(a, pos, f, __ldg(nwp + b0 + tid), 0.0f, desc[tid]);
+                for (int k = lane; k < nb; k += 32)
+                    ctab[warp * kGroupChunk + k] = __ldg(m_nc[warp] + size_t(f.xi) * a.max_nodes + b0 + k);
                 __syncthreads();
-                if constexpr (CH == kT) {
-                    for (int p = tid; p < nb * GMAX; p += blockDim.x) {
-                        const int k = p / GMAX, q = p - k * GMAX;
-                        group_local_values(m_sd[q], loc[k], lvtab + size_t(p) * 8);
-                    }
-                    __syncthreads();
-                }
-                for (int k = 0; k < nb; ++k) {
-                    const int p = k * GMAX + fs;
-                    NodeView v{&desc[k], ctab[p], lvtab + size_t(p) * 8};
-                    float rs[1][1], rd[1][1];
-                    node_term<CH, 1, 1>(la, &v, ln, jl, &tx, rs, rd);
-                    kahan_add(acc_s[0], cmp_s[0], v.c * rs[0][0]);
-                    kahan_add(acc_d[0], cmp_d[0], v.c * rd[0][0]);
-                    rotate();
-                    if constexpr (CH == kT) {
-                        __syncwarp();  // panel written
-                        group_outer_update<W, MB>(pan, jl, M);
-                        __syncwarp();  // panel read
-                    }
-                }
+                if (mine)
+                    item_nodes<MB>(m_sd[warp], a.nl, desc, nb, step, c, lane,
+                                         [&](int k) { return ctab[warp * kGroupChunk + k]; }, A, B, T, M);
             }
-            // realign: pair 0 holds residue 0 again
-            const int extra = (G - cnt % G) % G;
-            for (int r = 0; r < extra; ++r) rotate();
-        };
-
-        channel(std::integral_constant<int, kS>{}, si);
-        channel(std::integral_constant<int, kT>{}, ti);
-
-        // RPA term: stage each flow's M, walk the 32-chunk schedule (chunks jl, jl + W, ...)
-        __syncthreads();  // the build area is free
-        {
-            float2 *Ms = stage + size_t(fs) * (size_t(w) * w + g.n_seg_max);
-            float2 *slots = Ms + w * w;
-            const int rb = jl / S::Cb, cb = jl % S::Cb;
-#pragma unroll
-            for (int i = 0; i < R; ++i)
-#pragma unroll
-                for (int j = 0; j < C; ++j) Ms[(rb * R + i) * w + cb * C + j] = M[i][j];
-            __syncwarp();
-            const int lanes = a.rpa.lanes;
-            const char *mb = reinterpret_cast<const char *>(Ms);
-            for (int ch = jl; ch < lanes; ch += W) {
-                const int cntq = __ldg(a.rpa.count + ch);
-                int slot = __ldg(a.rpa.slot_base + ch);
-                const int *sched = a.rpa.sched + ch;
-                float2 acc = make_float2(0.0f, 0.0f);
-                for (int i = 0; i < cntq; ++i) {
-                    const int e = __ldg(sched + size_t(i) * lanes);
-                    const float2 v = *reinterpret_cast<const float2 *>(mb + (e & 0xffff));
-                    const float m = float((e >> 16) & 0xff);
-                    acc = fma2(make_float2(m, m), v, acc);
-                    if (e < 0) {
-                        slots[slot++] = acc;
-                        acc = make_float2(0.0f, 0.0f);
-                    }
-                }
-            }
-            __syncwarp();
-            if (ln.valid[0]) {
-                float os = 0.0f, od = 0.0f;
-                for (int q = __ldg(a.rpa.seg_ptr + jl); q < __ldg(a.rpa.seg_ptr + jl + 1); ++q) {
-                    const float2 p = slots[q];
-                    os += p.x;
-                    od += p.y;
-                }
-                kahan_add(acc_s[0], cmp_s[0], (2.0f * a.spin) * os);  // SU2FrgCore.cpp:265-266
-                kahan_add(acc_d[0], cmp_d[0], (8.0f * a.spin) * od);
-            }
+            if (mine) outer_gather<MB>(a, c, reinterpret_cast<float2 *>(area), lane, M, T);
+            turn_accs(step, A, B, T);
         }
-        channel(std::integral_constant<int, kU>{}, ui);
-
-        // the single-flow kernel's combination of its groups: xor-shuffle order
-        float vs[G], vd[G];
-#pragma unroll
-        for (int q = 0; q < G; ++q) {
-            vs[q] = acc_s[q] - cmp_s[q];
-            vd[q] = acc_d[q] - cmp_d[q];
-        }
-        float ts = vs[0], td = vd[0];
-        if constexpr (G == 2) {
-            ts = vs[0] + vs[1];
-            td = vd[0] + vd[1];
-        } else if constexpr (G == 4) {
-            ts = (vs[0] + vs[1]) + (vs[2] + vs[3]);
-            td = (vd[0] + vd[1]) + (vd[2] + vd[3]);
-        }
-        if (mine && ln.valid[0]) {
-            const float two_pi = 2.0f * float(kPi);
-            const float os = ts / two_pi, od = td / two_pi;
-            m_dsd[fs][size_t(it) * a.nl + jl] = make_float2(os, od);
-            if (isnan(os) || isnan(od)) atomicOr(m_status[fs], kStatusNaN);
+        if (mine) {
+            store_triple<MB>(a, m_dsd[warp], m_status[warp], c, B, p, q, r);
+            if (q != r) store_triple<MB>(a, m_dsd[warp], m_status[warp], c, T, p, r, q);
+            if (p != q) store_triple<MB>(a, m_dsd[warp], m_status[warp], c, A, q, p, r);
         }
     }
 }
@@ -1554,17 +1591,6 @@ __global__ void __launch_bounds__(NT, big_min_blocks(R, NT)) su2_vertex_big_batc
     }
 }
 
-int spt_of(int nl) { return nl <= 32 ? 1 : (nl <= 64 ? 2 : 4); }
-
-int wsite_of(int nl) {
-    if (nl > 32) return 32;
-    int w = 1;
-    while (w < nl) w <<= 1;
-    return w;
-}
-
-int outer_w_of(int nl) { return nl <= 32 ? rpa_outer_width(nl) : 0; }
-
 }  // namespace
 
 // Lattices of 33 to 128 sites use the CTA-per-triple kernel: w = 16 R >= Nl, R = 3 with 128
@@ -1575,11 +1601,18 @@ int big_r_of(int nl) {
 int big_class_r(int cls) { return cls == 6 ? 3 : (cls == 7 ? 4 : (cls == 8 ? 5 : (cls == 9 ? 6 : 8))); }
 int big_threads(int r) { return r <= 3 ? 128 : 256; }
 
+// items of three triples, or single triples
+long long vertex_work_items(int n, int nl, int inv_kind) {
+    return big_r_of(nl) || inv_kind ? (long long)n * n * (n + 1) / 2 : vertex_items(n);
+}
+
 int vertex_rpa_lanes(int nl) { return big_r_of(nl) ? big_threads(big_r_of(nl)) : 32; }
 
-int vertex_class(int nl) {
+bool vertex_class_big(int cls) { return cls >= 6 && cls <= 10; }
+
+int vertex_class(int nl, int inv_kind) {
     switch (big_r_of(nl)) {
-        case 0: return rpa_outer_width(nl) / 8 - 1;  // 0..3: a warp per triple, blocks of 1..4 rows
+        case 0: return (inv_kind ? 11 : 0) + rpa_outer_width(nl) / 8 - 1;
         case 3: return 6;
         case 4: return 7;
         case 5: return 8;
@@ -1588,25 +1621,33 @@ int vertex_class(int nl) {
     }
 }
 
-size_t vertex_flow_smem_bytes(int nl, const RpaSchedule &rpa, int npi) {
+namespace {
+size_t warp_area_bytes(int nl, int n_seg, int inv_kind) {
+    const int w = rpa_outer_width(nl);
+    if (!inv_kind) return warp_bytes(w / 8, n_seg);
+    int wsite = 1;
+    while (wsite < nl) wsite <<= 1;
+    return triple::triple_warp_bytes(wsite, n_seg, w);
+}
+}  // namespace
+
+size_t vertex_flow_smem_bytes(int nl, const RpaSchedule &rpa, int inv_kind) {
     if (const int r = big_r_of(nl)) return big_smem_layout(r, big_threads(r), rpa.n_seg).total;
-    const int spt = spt_of(nl);
-    return kMaxFreq * sizeof(float) + sched_bytes(rpa, nl) +
-           kWarps * warp_bytes(spt == 1 ? wsite_of(nl) : 32, spt, npi, rpa.n_seg, outer_w_of(nl));
+    return kMaxFreq * sizeof(float) + sched_bytes(rpa, nl) + kWarps * warp_area_bytes(nl, rpa.n_seg, inv_kind);
 }
 
 namespace {
 using VertexKernel = void (*)(FlowArgs);
-template <int SPT, int MB>
-VertexKernel vertex_kernel_npi(int npi) {
-    return npi == 1 ? su2_vertex_flow_kernel<SPT, 1, MB> : su2_vertex_flow_kernel<SPT, 2, MB>;
-}
-VertexKernel vertex_kernel(int cls, int npi) {
+VertexKernel vertex_kernel(int cls) {
     switch (cls) {
-        case 0: return vertex_kernel_npi<1, 1>(npi);
-        case 1: return vertex_kernel_npi<1, 2>(npi);
-        case 2: return vertex_kernel_npi<1, 3>(npi);
-        case 3: return vertex_kernel_npi<1, 4>(npi);
+        case 0: return su2_vertex_flow_kernel<1>;
+        case 1: return su2_vertex_flow_kernel<2>;
+        case 2: return su2_vertex_flow_kernel<3>;
+        case 3: return su2_vertex_flow_kernel<4>;
+        case 11: return triple::su2_triple_flow_kernel<1>;
+        case 12: return triple::su2_triple_flow_kernel<2>;
+        case 13: return triple::su2_triple_flow_kernel<3>;
+        case 14: return triple::su2_triple_flow_kernel<4>;
         case 6: return su2_vertex_big_kernel<3, 128>;
         case 7: return su2_vertex_big_kernel<4, 256>;
         case 8: return su2_vertex_big_kernel<5, 256>;
@@ -1614,54 +1655,48 @@ VertexKernel vertex_kernel(int cls, int npi) {
         default: return su2_vertex_big_kernel<8, 256>;
     }
 }
-int threads_of(int cls) { return cls >= 6 ? big_threads(big_class_r(cls)) : kThreads; }
+int threads_of(int cls) { return vertex_class_big(cls) ? big_threads(big_class_r(cls)) : kThreads; }
 }  // namespace
 
-// The CTA-per-triple kernel (33..128 sites) has no variants: nodes per iteration and the
-// schedule's place do not apply, and every setting launches the same kernel.
-int vertex_flow_blocks_per_sm(int nl, const RpaSchedule &rpa, int npi) {
-    const size_t smem = vertex_flow_smem_bytes(nl, rpa, npi);
-    const int cls = vertex_class(nl);
-    VertexKernel k = vertex_kernel(cls, npi);
+// The CTA-per-triple kernel (33..128 sites) reads the schedule from global memory wherever
+// rpa.in_smem says.
+int vertex_flow_blocks_per_sm(int nl, const RpaSchedule &rpa, int inv_kind) {
+    const size_t smem = vertex_flow_smem_bytes(nl, rpa, inv_kind);
+    const int cls = vertex_class(nl, inv_kind);
+    VertexKernel k = vertex_kernel(cls);
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -1;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads_of(cls), smem) != cudaSuccess) return -1;
     return per_sm;
 }
 
-void launch_vertex_flow(const FlowArgs &a, int npi, int grid, cudaStream_t stream) {
-    const size_t smem = vertex_flow_smem_bytes(a.nl, a.rpa, npi);
-    const int cls = vertex_class(a.nl);
-    VertexKernel k = vertex_kernel(cls, npi);
+void launch_vertex_flow(const FlowArgs &a, int grid, cudaStream_t stream) {
+    const size_t smem = vertex_flow_smem_bytes(a.nl, a.rpa, a.inv_kind);
+    const int cls = vertex_class(a.nl, a.inv_kind);
+    VertexKernel k = vertex_kernel(cls);
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     k<<<grid, threads_of(cls), smem, stream>>>(a);
 }
 
-int vertex_spt(int nl) { return spt_of(nl); }
-
-size_t batch_vertex_warp_area(int nl, int n_seg, int npi) {
-    const int spt = spt_of(nl);
-    // everything after the descriptors: the group areas, or the outer-product stage
-    return warp_bytes(spt == 1 ? wsite_of(nl) : 32, spt, npi, n_seg, outer_w_of(nl)) - kBatch * sizeof(NodeDesc);
-}
+size_t batch_vertex_warp_area(int nl, int n_seg, int inv_kind) { return warp_area_bytes(nl, n_seg, inv_kind); }
 
 size_t batch_vertex_smem_bytes(int n_max, size_t warp_area, int sched_ints) {
     return kWarps * (align16(sizeof(FlowArgs)) + align16(sizeof(float) * n_max) + align16(sizeof(int) * size_t(sched_ints)) +
-                     kBatch * sizeof(NodeDesc) + warp_area);
+                     warp_area);
 }
 
 namespace {
 using BatchKernel = void (*)(BatchVertexArgs);
-template <int SPT, int MB>
-BatchKernel batch_kernel_npi(int npi) {
-    return npi == 1 ? su2_vertex_batch_kernel<SPT, 1, MB> : su2_vertex_batch_kernel<SPT, 2, MB>;
-}
-BatchKernel batch_kernel(int cls, int npi) {
+BatchKernel batch_kernel(int cls) {
     switch (cls) {
-        case 0: return batch_kernel_npi<1, 1>(npi);
-        case 1: return batch_kernel_npi<1, 2>(npi);
-        case 2: return batch_kernel_npi<1, 3>(npi);
-        case 3: return batch_kernel_npi<1, 4>(npi);
+        case 0: return su2_vertex_batch_kernel<1>;
+        case 1: return su2_vertex_batch_kernel<2>;
+        case 2: return su2_vertex_batch_kernel<3>;
+        case 3: return su2_vertex_batch_kernel<4>;
+        case 11: return triple::su2_triple_batch_kernel<1>;
+        case 12: return triple::su2_triple_batch_kernel<2>;
+        case 13: return triple::su2_triple_batch_kernel<3>;
+        case 14: return triple::su2_triple_batch_kernel<4>;
         case 6: return su2_vertex_big_batch_kernel<3, 128>;
         case 7: return su2_vertex_big_batch_kernel<4, 256>;
         case 8: return su2_vertex_big_batch_kernel<5, 256>;
@@ -1676,8 +1711,8 @@ size_t batch_big_smem_bytes(int cls, int n_seg_max) {
     return big_smem_layout(r, big_threads(r), n_seg_max).total;
 }
 
-int batch_vertex_blocks_per_sm(int cls, int npi, size_t smem) {
-    BatchKernel k = batch_kernel(cls, npi);
+int batch_vertex_blocks_per_sm(int cls, size_t smem) {
+    BatchKernel k = batch_kernel(cls);
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -1;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads_of(cls), smem) != cudaSuccess) return -1;
@@ -1686,32 +1721,29 @@ int batch_vertex_blocks_per_sm(int cls, int npi, size_t smem) {
 
 // The kernel's shared-memory limit is raised by batch_vertex_blocks_per_sm when the plan is
 // built, so this launch can be captured into a graph.
-void launch_batch_vertex(const BatchVertexArgs &b, int cls, int npi, int grid, cudaStream_t stream) {
-    const size_t smem = cls >= 6 ? batch_big_smem_bytes(cls, b.n_seg_max)
+void launch_batch_vertex(const BatchVertexArgs &b, int cls, int grid, cudaStream_t stream) {
+    const size_t smem = vertex_class_big(cls) ? batch_big_smem_bytes(cls, b.n_seg_max)
                                  : batch_vertex_smem_bytes(b.n_max, size_t(b.warp_area), b.sched_ints);
-    batch_kernel(cls, npi)<<<grid, threads_of(cls), smem, stream>>>(b);
+    batch_kernel(cls)<<<grid, threads_of(cls), smem, stream>>>(b);
 }
 
 namespace {
 using GroupKernel = void (*)(GroupVertexArgs);
 GroupKernel group_kernel(int cls) {
     switch (cls) {
-        case 0: return su2_vertex_group_kernel<8, 1>;
-        case 1: return su2_vertex_group_kernel<16, 2>;
-        case 2: return su2_vertex_group_kernel<32, 3>;
-        default: return su2_vertex_group_kernel<32, 4>;
+        case 0: return su2_vertex_group_kernel<1>;
+        case 1: return su2_vertex_group_kernel<2>;
+        case 2: return su2_vertex_group_kernel<3>;
+        default: return su2_vertex_group_kernel<4>;
     }
 }
-int group_w(int cls) { return cls == 0 ? 8 : (cls == 1 ? 16 : 32); }
 }  // namespace
 
-bool group_vertex_eligible(int nl) { return nl >= 5 && nl <= 32; }
+bool group_vertex_eligible(int nl, int inv_kind) { return nl >= 5 && nl <= 32 && inv_kind == 0; }
 
-int group_vertex_gmax(int cls) { return kGroupWarps * (32 / group_w(cls)); }
+int group_vertex_gmax() { return kGroupWarps; }
 
-size_t group_vertex_smem_bytes(int cls, int n_seg_max) {
-    return group_smem_layout(group_w(cls), cls + 1, n_seg_max).total;
-}
+size_t group_vertex_smem_bytes(int cls, int n_seg_max) { return group_smem_layout(cls + 1, n_seg_max).total; }
 
 int group_vertex_blocks_per_sm(int cls, int n_seg_max) {
     GroupKernel k = group_kernel(cls);
