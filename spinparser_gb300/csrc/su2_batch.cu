@@ -53,11 +53,11 @@ __global__ void __launch_bounds__(128) batch_self_energy_kernel(const BatchFlow 
     self_energy_body(a, blockIdx.x);
 }
 
-__global__ void batch_node_table_kernel(const BatchFlow *flows, const int *list) {
+__global__ void __launch_bounds__(kNodeThreads) batch_node_table_kernel(const BatchFlow *flows, const int *list) {
     const BatchFlow &f = flows[list[blockIdx.y]];
     if (f.phase != kPhaseFlowing) return;
     const FlowArgs a = f.a;
-    if (int(blockIdx.x * blockDim.x) >= a.n) return;
+    if (int(blockIdx.x) >= a.n) return;
     node_table_body(a, blockIdx.x);
 }
 
@@ -69,7 +69,7 @@ __device__ __forceinline__ CorrArgs batch_corr_args(const BatchFlow &f) {
 }
 
 template <int SPT>
-__global__ void __launch_bounds__(128) batch_corr_inner_kernel(const BatchFlow *flows, const int *list) {
+__global__ void __launch_bounds__(kCorrThreads) batch_corr_inner_kernel(const BatchFlow *flows, const int *list) {
     const BatchFlow &f = flows[list[blockIdx.y]];
     if (f.phase == kPhaseDone) return;
     const CorrArgs c = batch_corr_args(f);
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(128) batch_corr_inner_kernel(const BatchFlow *
     corr_inner_body<SPT>(c, PairedState<float>{c.sd}, blockIdx.x);
 }
 
-__global__ void batch_corr_final_kernel(const BatchFlow *flows, const int *list) {
+__global__ void __launch_bounds__(kCorrThreads) batch_corr_final_kernel(const BatchFlow *flows, const int *list) {
     const BatchFlow &f = flows[list[blockIdx.x]];
     if (f.phase == kPhaseDone) return;
     corr_final_body(batch_corr_args(f));
@@ -424,7 +424,7 @@ struct spn_batch {
                                                                                                n_measure, d_counters);
         if (n_flowing > 0) {
             batch_self_energy_kernel<<<dim3(n_max, n_flowing), 128, 0, stream>>>(d_flows, L + off_flowing);
-            batch_node_table_kernel<<<dim3((n_max + 63) / 64, n_flowing), 64, 0, stream>>>(d_flows, L + off_flowing);
+            batch_node_table_kernel<<<dim3(n_max, n_flowing), kNodeThreads, 0, stream>>>(d_flows, L + off_flowing);
         }
     }
 
@@ -467,12 +467,12 @@ struct spn_batch {
         for (int c = 0; c < kClasses; ++c) {
             if (n_cm[c] == 0) continue;
             const dim3 g(2 * n_max + 4, n_cm[c]);
-            if (c == 0) batch_corr_inner_kernel<1><<<g, 128, 0, stream>>>(d_flows, L + off_cm[c]);
-            else if (c == 1) batch_corr_inner_kernel<2><<<g, 128, 0, stream>>>(d_flows, L + off_cm[c]);
-            else batch_corr_inner_kernel<4><<<g, 128, 0, stream>>>(d_flows, L + off_cm[c]);
+            if (c == 0) batch_corr_inner_kernel<1><<<g, kCorrThreads, 0, stream>>>(d_flows, L + off_cm[c]);
+            else if (c == 1) batch_corr_inner_kernel<2><<<g, kCorrThreads, 0, stream>>>(d_flows, L + off_cm[c]);
+            else batch_corr_inner_kernel<4><<<g, kCorrThreads, 0, stream>>>(d_flows, L + off_cm[c]);
         }
         if (n_measure > 0)
-            batch_corr_final_kernel<<<n_measure, 128, 2 * nl_max * sizeof(double), stream>>>(d_flows, L + off_measure);
+            batch_corr_final_kernel<<<n_measure, kCorrThreads, corr_final_smem(2 * nl_max), stream>>>(d_flows, L + off_measure);
         if (n_flowing > 0) batch_euler_kernel<<<dim3(48, n_flowing), 256, 0, stream>>>(d_flows, L + off_flowing);
         batch_advance_kernel<<<(std::max(n_measure, 1) + 127) / 128, 128, 0, stream>>>(d_flows, L + off_measure, n_measure);
         cuda_check(cudaGetLastError(), "batch step launch");

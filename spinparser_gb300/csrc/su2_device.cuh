@@ -462,66 +462,70 @@ SPN_HDI T value_none(const T *pos, int n, int nl, const S &v, bool density, int 
 }
 
 // ---- trapezoid quadrature nodes (ImplicitIntegrator, src/lib/Integrator.hpp:137-287) ----
-// Each rule calls emit(wp, weight) once per integrand evaluation of the reference, in the
-// same order, with weight = 0.5 * (the float node spacing the reference multiplies by).
+// A rule's nodes are its lower end (if it has one), the points um .. ux of the symmetric mesh and
+// its upper end (if it has one), in the reference's order; node k's weight is 0.5 * (the float
+// node spacing the reference multiplies by).  Each node is a function of its number, so the
+// threads of a block evaluate them side by side.
+template <class T>
+struct QuadRule {
+    const T *pos;
+    int n, um, ux, count;
+    bool has_min, has_max, two;  // two: the range holds no inner spacing, only the points p0 and p1
+    T min, max, p0, p1;
+    SPN_HDI T point(int i) const { return full_value(pos, n, i); }
+    SPN_HDI void pair(T first, T second, T hi, T lo) {
+        two = true;
+        count = 2;
+        p0 = first;
+        p1 = second;
+        max = hi;
+        min = lo;
+    }
+    SPN_HDI void node(int k, T &w, double &weight) const {
+        if (two) {
+            w = k == 0 ? p0 : p1;
+            weight = double(rn_mul(T(0.5), rn_sub(max, min)));
+            return;
+        }
+        const int i = um + k - int(has_min);
+        if (i < um) {
+            w = min;
+            weight = 0.5 * double(rn_sub(point(um), min));
+        } else if (i > ux) {
+            w = max;
+            weight = 0.5 * double(rn_sub(max, point(ux)));
+        } else {
+            const T lo = i > um ? point(i - 1) : (has_min ? min : point(um));
+            const T hi = i < ux ? point(i + 1) : (has_max ? max : point(ux));
+            w = point(i);
+            weight = 0.5 * double(rn_sub(hi, lo));
+        }
+    }
+};
 
 // integrateWithObscureLeftBoundary(min, last)
-template <class T, class Emit>
-__host__ __device__ void nodes_left(const T *pos, int n, T min, Emit &&emit) {
-    const int maxi = 2 * n - 1;
-    int um = full_greater(pos, n, min);
-    if (um != maxi) {
-        emit(min, 0.5 * double(rn_sub(full_value(pos, n, um), min)));
-        emit(full_value(pos, n, um), 0.5 * double(rn_sub(full_value(pos, n, um + 1), min)));
-        while (++um != maxi)
-            emit(full_value(pos, n, um), 0.5 * double(rn_sub(full_value(pos, n, um + 1), full_value(pos, n, um - 1))));
-        emit(full_value(pos, n, um), 0.5 * double(rn_sub(full_value(pos, n, um), full_value(pos, n, um - 1))));
-    } else {
-        const double w = double(rn_mul(T(0.5), rn_sub(full_value(pos, n, um), min)));
-        emit(min, w);
-        emit(full_value(pos, n, um), w);
-    }
+template <class T>
+SPN_HDI QuadRule<T> rule_left(const T *pos, int n, T min) {
+    QuadRule<T> r{pos, n, full_greater(pos, n, min), 2 * n - 1, 0, true, false, false, min, T(0), T(0), T(0)};
+    r.count = r.ux - r.um + 2;
+    if (r.um == r.ux) r.pair(min, r.point(r.um), r.point(r.um), min);
+    return r;
 }
-
 // integrateWithObscureRightBoundary(beginNegative, max)
-template <class T, class Emit>
-__host__ __device__ void nodes_right(const T *pos, int n, T max, Emit &&emit) {
-    int um = 0;
-    const int ux = full_lesser(pos, n, max);
-    if (um != ux) {
-        emit(full_value(pos, n, um), 0.5 * double(rn_sub(full_value(pos, n, um + 1), full_value(pos, n, um))));
-        while (++um != ux)
-            emit(full_value(pos, n, um), 0.5 * double(rn_sub(full_value(pos, n, um + 1), full_value(pos, n, um - 1))));
-        emit(full_value(pos, n, um), 0.5 * double(rn_sub(max, full_value(pos, n, um - 1))));
-        emit(max, 0.5 * double(rn_sub(max, full_value(pos, n, um))));
-    } else {
-        const double w = double(rn_mul(T(0.5), rn_sub(max, full_value(pos, n, um))));
-        emit(max, w);
-        emit(full_value(pos, n, um), w);
-    }
+template <class T>
+SPN_HDI QuadRule<T> rule_right(const T *pos, int n, T max) {
+    QuadRule<T> r{pos, n, 0, full_lesser(pos, n, max), 0, false, true, false, T(0), max, T(0), T(0)};
+    r.count = r.ux + 2;
+    if (r.ux == 0) r.pair(max, r.point(0), max, r.point(0));
+    return r;
 }
-
 // integrateWithObscureBoundaries(min, max)
-template <class T, class Emit>
-__host__ __device__ void nodes_both(const T *pos, int n, T min, T max, Emit &&emit) {
-    int um = full_greater(pos, n, min);
-    const int ux = full_lesser(pos, n, max);
-    if (ux >= um) {
-        emit(min, 0.5 * double(rn_sub(full_value(pos, n, um), min)));
-        if (ux != um) {
-            emit(full_value(pos, n, um), 0.5 * double(rn_sub(full_value(pos, n, um + 1), min)));
-            while (++um != ux)
-                emit(full_value(pos, n, um), 0.5 * double(rn_sub(full_value(pos, n, um + 1), full_value(pos, n, um - 1))));
-            emit(full_value(pos, n, um), 0.5 * double(rn_sub(max, full_value(pos, n, um - 1))));
-        } else {
-            emit(full_value(pos, n, um), 0.5 * double(rn_sub(max, min)));
-        }
-        emit(max, 0.5 * double(rn_sub(max, full_value(pos, n, um))));
-    } else {
-        const double w = double(rn_mul(T(0.5), rn_sub(max, min)));
-        emit(max, w);
-        emit(min, w);
-    }
+template <class T>
+SPN_HDI QuadRule<T> rule_both(const T *pos, int n, T min, T max) {
+    QuadRule<T> r{pos, n, full_greater(pos, n, min), full_lesser(pos, n, max), 0, true, true, false, min, max, T(0), T(0)};
+    r.count = r.ux - r.um + 3;
+    if (r.ux < r.um) r.pair(max, min, max, min);
+    return r;
 }
 
 }  // namespace dev

@@ -44,32 +44,32 @@ namespace {
 // ------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) su2_self_energy_kernel(FlowArgs a) { self_energy_body(a, blockIdx.x); }
 
-__global__ void su2_node_table_kernel(FlowArgs a) { node_table_body(a, blockIdx.x); }
+__global__ void __launch_bounds__(kNodeThreads) su2_node_table_kernel(FlowArgs a) { node_table_body(a, blockIdx.x); }
 
 template <int SPT>
-__global__ void __launch_bounds__(128) su2_corr_inner_kernel(CorrArgs a) {
+__global__ void __launch_bounds__(kCorrThreads) su2_corr_inner_kernel(CorrArgs a) {
     corr_inner_body<SPT>(a, PairedState<float>{a.sd}, blockIdx.x);
 }
 
 // the allocation-free measurement: the caller's separate spin and density arrays
 template <int SPT>
-__global__ void __launch_bounds__(128) su2_corr_inner_split_kernel(CorrArgs a) {
+__global__ void __launch_bounds__(kCorrThreads) su2_corr_inner_split_kernel(CorrArgs a) {
     corr_inner_body<SPT>(a, SplitState<float>{a.ss, a.dd}, blockIdx.x);
 }
 
-__global__ void su2_corr_final_kernel(CorrArgs a) { corr_final_body(a); }
+__global__ void __launch_bounds__(kCorrThreads) su2_corr_final_kernel(CorrArgs a) { corr_final_body(a); }
 
 // FP64 flow (SPN_SU2_FP64): the same bodies in double
 __global__ void __launch_bounds__(128) su2_self_energy_f64_kernel(FlowArgsT<double> a) { self_energy_body(a, blockIdx.x); }
 
-__global__ void su2_node_table_f64_kernel(FlowArgsT<double> a) { node_table_body(a, blockIdx.x); }
+__global__ void __launch_bounds__(kNodeThreads) su2_node_table_f64_kernel(FlowArgsT<double> a) { node_table_body(a, blockIdx.x); }
 
 template <int SPT>
-__global__ void __launch_bounds__(128) su2_corr_inner_f64_kernel(CorrArgsT<double> a) {
+__global__ void __launch_bounds__(kCorrThreads) su2_corr_inner_f64_kernel(CorrArgsT<double> a) {
     corr_inner_body<SPT>(a, PairedState<double>{a.sd}, blockIdx.x);
 }
 
-__global__ void su2_corr_final_f64_kernel(CorrArgsT<double> a) { corr_final_body(a); }
+__global__ void __launch_bounds__(kCorrThreads) su2_corr_final_f64_kernel(CorrArgsT<double> a) { corr_final_body(a); }
 
 // ------------------------------------------------------------------------------------
 // Euler step  x += step * dx  (rounded like the reference: product, then sum)
@@ -493,9 +493,15 @@ extern "C" int spn_quadrature_nodes(const float *pos, int n, int rule, float min
         if (rule < 0 || rule > 2 || !count || cap < 0 || (cap > 0 && (!wp || !weight)))
             throw Error(ErrorType::Argument, "spn_quadrature_nodes: bad argument");
         NodeList emit{wp, weight, cap, 0};
-        if (rule == 0) dev::nodes_left(pos, n, min, emit);
-        else if (rule == 1) dev::nodes_right(pos, n, max, emit);
-        else dev::nodes_both(pos, n, min, max, emit);
+        const dev::QuadRule<float> r = rule == 0   ? dev::rule_left(pos, n, min)
+                                       : rule == 1 ? dev::rule_right(pos, n, max)
+                                                   : dev::rule_both(pos, n, min, max);
+        for (int k = 0; k < r.count; ++k) {
+            float x;
+            double c;
+            r.node(k, x, c);
+            emit(x, c);
+        }
         *count = emit.k;
     });
 }
@@ -772,13 +778,13 @@ extern "C" int spn_su2_compute_step(spn_su2 *h) {
             const FlowArgsT<double> a = h->args64();
             su2_self_energy_f64_kernel<<<h->n, 128, 0, h->stream>>>(a);
             cuda_check(cudaGetLastError(), "self-energy launch");
-            su2_node_table_f64_kernel<<<(h->n + 63) / 64, 64, 0, h->stream>>>(a);
+            su2_node_table_f64_kernel<<<h->n, kNodeThreads, 0, h->stream>>>(a);
             cuda_check(cudaGetLastError(), "node table launch");
         } else {
             const FlowArgs a = h->args();
             su2_self_energy_kernel<<<h->n, 128, 0, h->stream>>>(a);
             cuda_check(cudaGetLastError(), "self-energy launch");
-            su2_node_table_kernel<<<(h->n + 63) / 64, 64, 0, h->stream>>>(a);
+            su2_node_table_kernel<<<h->n, kNodeThreads, 0, h->stream>>>(a);
             cuda_check(cudaGetLastError(), "node table launch");
         }
         if (h->profiling) {
@@ -981,22 +987,22 @@ void launch_correlation(spn_su2 *h) {
             const CorrArgsT<double> a = corr_args64(h);
             const int spt = spt_for(h->nl);
             const int blocks = 2 * h->n + 4;
-            if (spt == 1) su2_corr_inner_f64_kernel<1><<<blocks, 128, 0, h->stream>>>(a);
-            else if (spt == 2) su2_corr_inner_f64_kernel<2><<<blocks, 128, 0, h->stream>>>(a);
-            else su2_corr_inner_f64_kernel<4><<<blocks, 128, 0, h->stream>>>(a);
+            if (spt == 1) su2_corr_inner_f64_kernel<1><<<blocks, kCorrThreads, 0, h->stream>>>(a);
+            else if (spt == 2) su2_corr_inner_f64_kernel<2><<<blocks, kCorrThreads, 0, h->stream>>>(a);
+            else su2_corr_inner_f64_kernel<4><<<blocks, kCorrThreads, 0, h->stream>>>(a);
             cuda_check(cudaGetLastError(), "correlation launch");
-            su2_corr_final_f64_kernel<<<1, 128, 2 * h->nl * sizeof(double), h->stream>>>(a);
+            su2_corr_final_f64_kernel<<<1, kCorrThreads, corr_final_smem(2 * h->nl), h->stream>>>(a);
             cuda_check(cudaGetLastError(), "correlation final launch");
             return;
         }
         const CorrArgs a = corr_args(h);
         const int spt = spt_for(h->nl);
         const int blocks = 2 * h->n + 4;
-        if (spt == 1) su2_corr_inner_kernel<1><<<blocks, 128, 0, h->stream>>>(a);
-        else if (spt == 2) su2_corr_inner_kernel<2><<<blocks, 128, 0, h->stream>>>(a);
-        else su2_corr_inner_kernel<4><<<blocks, 128, 0, h->stream>>>(a);
+        if (spt == 1) su2_corr_inner_kernel<1><<<blocks, kCorrThreads, 0, h->stream>>>(a);
+        else if (spt == 2) su2_corr_inner_kernel<2><<<blocks, kCorrThreads, 0, h->stream>>>(a);
+        else su2_corr_inner_kernel<4><<<blocks, kCorrThreads, 0, h->stream>>>(a);
         cuda_check(cudaGetLastError(), "correlation launch");
-        su2_corr_final_kernel<<<1, 128, 2 * h->nl * sizeof(double), h->stream>>>(a);
+        su2_corr_final_kernel<<<1, kCorrThreads, corr_final_smem(2 * h->nl), h->stream>>>(a);
         cuda_check(cudaGetLastError(), "correlation final launch");
 }
 
@@ -1247,11 +1253,11 @@ extern "C" int spn_su2_correlation_noalloc(int n_freq, const float *freq, int n_
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         const int spt = spt_for(n_sites);
         const int blocks = 2 * n_freq + 4;
-        if (spt == 1) su2_corr_inner_split_kernel<1><<<blocks, 128, 0, s>>>(a);
-        else if (spt == 2) su2_corr_inner_split_kernel<2><<<blocks, 128, 0, s>>>(a);
-        else su2_corr_inner_split_kernel<4><<<blocks, 128, 0, s>>>(a);
+        if (spt == 1) su2_corr_inner_split_kernel<1><<<blocks, kCorrThreads, 0, s>>>(a);
+        else if (spt == 2) su2_corr_inner_split_kernel<2><<<blocks, kCorrThreads, 0, s>>>(a);
+        else su2_corr_inner_split_kernel<4><<<blocks, kCorrThreads, 0, s>>>(a);
         cuda_check(cudaGetLastError(), "correlation launch");
-        su2_corr_final_kernel<<<1, 128, 2 * n_sites * sizeof(double), s>>>(a);
+        su2_corr_final_kernel<<<1, kCorrThreads, corr_final_smem(2 * n_sites), s>>>(a);
         cuda_check(cudaGetLastError(), "correlation final launch");
     });
 }

@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(128) tri_self_energy_kernel(TriArgs a) {
 }
 
 // Loop-frequency node tables: the SU(2) core's body on an argument block of this flow.
-__global__ void tri_node_table_kernel(FlowArgs f) { node_table_body(f, blockIdx.x); }
+__global__ void __launch_bounds__(kNodeThreads) tri_node_table_kernel(FlowArgs f) { node_table_body(f, blockIdx.x); }
 
 // ------------------------------------------------------------------------------------
 // vertex flow
@@ -658,22 +658,41 @@ __global__ void __launch_bounds__(kThreads) tri_vertex_kernel(TriArgs a) {
 // ------------------------------------------------------------------------------------
 __constant__ int kOutComp[kCorrOut] = {0, 1, 2, 4, 5, 6, 8, 9, 10, 15};
 
-__global__ void __launch_bounds__(128) tri_corr_inner_kernel(TriArgs a) {
+// Linear in the vertex, as the SU(2) core's (corr_inner_body): sums of g * vertex per site and
+// component and, a thread per node and component, of the egg diagram's site-local reads (lane 0
+// alone took 320 reads a node: 289 us at N = 32, 28 sites, now 29).
+constexpr int kCorrTWarps = 8, kCorrTThreads = 32 * kCorrTWarps;
+
+__global__ void __launch_bounds__(kCorrTThreads) tri_corr_inner_kernel(TriArgs a) {
     __shared__ float pos[kMaxFreq];
     __shared__ float nwp[kMaxCorrNodes];
-    __shared__ double nw[kMaxCorrNodes];
-    __shared__ int ncnt;
-    extern __shared__ double red[];  // [kWarps][kCorrOut][nl]
+    __shared__ double nw[kMaxCorrNodes], ng[kMaxCorrNodes];
+    __shared__ double egg[kCorrTThreads];
+    extern __shared__ double red[];  // [kCorrTWarps][kCorrOut][nl]
     for (int i = threadIdx.x; i < a.n; i += blockDim.x) pos[i] = a.freq[i];
     __syncthreads();
-    if (threadIdx.x == 0) ncnt = corr_nodes(pos, a.n, a.cutoff, nwp, nw);
-    __syncthreads();
+    const int ncnt = corr_nodes(pos, a.n, a.cutoff, nwp, nw, ng, [&](float x) { return odd_interp(pos, a.n, a.v2, x); });
     const int ia = blockIdx.x;
     if (ia >= ncnt) return;
     const float w = nwp[ia];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nl = a.nl;
-    const double dw = double(w) + odd_interp(pos, a.n, a.v2, w);
+    {  // site-local vertex component tid & 15 at nodes tid >> 4, ...
+        const int c = threadIdx.x & 15;
+        double sum = 0.0;
+        for (int b = threadIdx.x >> 4; b < ncnt; b += kCorrTThreads / 16) {
+            const float wp = nwp[b];
+            TAB8 ab;
+            tri_access8(pos, a.n, nl, w + wp + 0.0f, w - wp, 0.0f, ab);
+            sum += nw[b] * ng[b] * double(tri_local(a.v4, nl, ab, c >> 2, c & 3));
+        }
+        egg[threadIdx.x] = sum;
+        __syncthreads();
+        if (threadIdx.x < 16) {
+            for (int q = 16 + threadIdx.x; q < kCorrTThreads; q += 16) sum += egg[q];
+            egg[threadIdx.x] = sum;
+        }
+    }
     for (int j0 = 0; j0 < nl; j0 += 32) {
         const int j = j0 + lane;
         const bool valid = j < nl;
@@ -682,76 +701,61 @@ __global__ void __launch_bounds__(128) tri_corr_inner_kernel(TriArgs a) {
         double acc[kCorrOut];
 #pragma unroll
         for (int q = 0; q < kCorrOut; ++q) acc[q] = 0.0;
-        for (int b = warp; b < ncnt; b += kWarps) {
+        for (int b = warp; b < ncnt; b += kCorrTWarps) {
             const float wp = nwp[b];
-            TAB8 ab, ab1;
+            TAB8 ab;
             tri_access8(pos, a.n, nl, w + wp + 0.0f, 0.0f, w - wp, ab);
-            const double dwp = double(wp) + odd_interp(pos, a.n, a.v2, wp);
-            const double cw = nw[b] / (dw * dw * dwp * dwp * (4.0 * kPiD * kPiD));
+            const double cw = nw[b] * ng[b];
             if (!valid) continue;
             const bool ex = ab.fl & kFlExch;
-            double rr[kCorrOut];
 #pragma unroll
-            for (int q = 0; q < kCorrOut; ++q) {
-                const int c = kOutComp[q];
-                const float g = tri_bundle(a.v4, nl, ab, c, ex ? r1 : r0, ex ? p1 : p0);
-                rr[q] = c == 15 ? -4.0 * double(g) : -double(g);  // dumbbell
-            }
-            if (j == 0) {  // egg diagram, TRIMeasurementCorrelation.cpp:211-251
-                tri_access8(pos, a.n, nl, w + wp + 0.0f, w - wp, 0.0f, ab1);
-#pragma unroll
-                for (int q = 0; q < kCorrOut; ++q) {
-                    const int c = kOutComp[q];
-                    const double f = c == 15 ? 2.0 : 0.5;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const int lam = tri::inner(k), rho = (c >> 2) ^ (c & 3) ^ lam;
-                        const int sg = tri::egg_sign(c, lam);
-                        if (sg != 0) rr[q] += f * sg * double(tri_local(a.v4, nl, ab1, lam, rho));
-                    }
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < kCorrOut; ++q) acc[q] += cw * rr[q];
+            for (int q = 0; q < kCorrOut; ++q)
+                acc[q] += cw * double(tri_bundle(a.v4, nl, ab, kOutComp[q], ex ? r1 : r0, ex ? p1 : p0));
         }
         if (valid)
             for (int q = 0; q < kCorrOut; ++q) red[(size_t(warp) * kCorrOut + q) * nl + j] = acc[q];
     }
     __syncthreads();
+    const double norm = ng[ia] / (4.0 * kPiD * kPiD);
     for (int e = threadIdx.x; e < kCorrOut * nl; e += blockDim.x) {
+        const int q = e / nl, c = kOutComp[q];
         double sum = 0.0;
-        for (int q = 0; q < kWarps; ++q) sum += red[size_t(q) * kCorrOut * nl + e];
-        a.partial[size_t(ia) * kCorrOut * nl + e] = sum;
+        for (int k = 0; k < kCorrTWarps; ++k) sum += red[size_t(k) * kCorrOut * nl + e];
+        sum *= c == 15 ? -4.0 : -1.0;  // dumbbell
+        if (e == q * nl) {             // egg diagram, TRIMeasurementCorrelation.cpp:211-251
+            const double f = c == 15 ? 2.0 : 0.5;
+            for (int k = 0; k < 4; ++k) {
+                const int lam = tri::inner(k), rho = (c >> 2) ^ (c & 3) ^ lam;
+                sum += f * tri::egg_sign(c, lam) * egg[4 * lam + rho];
+            }
+        }
+        a.partial[size_t(ia) * kCorrOut * nl + e] = sum * norm;
     }
 }
 
-__global__ void tri_corr_final_kernel(TriArgs a) {
+// Shared memory of the final kernel: chi[16][nl], then the reduction's slices.
+size_t tri_final_smem(int nl) { return 16 * size_t(nl) * sizeof(double) + corr_final_smem(kCorrOut * nl); }
+
+__global__ void __launch_bounds__(kCorrThreads) tri_corr_final_kernel(TriArgs a) {
     __shared__ float pos[kMaxFreq];
     __shared__ float nwp[kMaxCorrNodes];
-    __shared__ double nw[kMaxCorrNodes];
-    __shared__ int ncnt;
+    __shared__ double nw[kMaxCorrNodes], ng[kMaxCorrNodes];
     extern __shared__ double chi[];  // [16][nl]
     for (int i = threadIdx.x; i < a.n; i += blockDim.x) pos[i] = a.freq[i];
     __syncthreads();
-    if (threadIdx.x == 0) ncnt = corr_nodes(pos, a.n, a.cutoff, nwp, nw);
-    __syncthreads();
+    const int ncnt = corr_nodes(pos, a.n, a.cutoff, nwp, nw, ng, [&](float x) { return odd_interp(pos, a.n, a.v2, x); });
     const int nl = a.nl;
+    double *sums = chi + 16 * nl;
+    column_sums(ncnt, kCorrOut * nl, sums, [&](int ia, int e) { return nw[ia] * a.partial[size_t(ia) * kCorrOut * nl + e]; });
     for (int e = threadIdx.x; e < 16 * nl; e += blockDim.x) chi[e] = 0.0;
     __syncthreads();
-    for (int e = threadIdx.x; e < kCorrOut * nl; e += blockDim.x) {
-        const int q = e / nl, j = e - q * nl, c = kOutComp[q];
-        double sum = 0.0;
-        for (int ia = 0; ia < ncnt; ++ia) {
-            double v = a.partial[size_t(ia) * kCorrOut * nl + e];
-            if (j == 0 && (c == 0 || c == 5 || c == 10 || c == 15)) {  // on-site term
-                const float w = nwp[ia];
-                const double dw = double(w) + odd_interp(pos, a.n, a.v2, w);
-                const double t1 = 1.0 / (dw * dw);
-                v += c == 15 ? t1 / kPiD : t1 / (4.0 * kPiD);
-            }
-            sum += nw[ia] * v;
-        }
-        chi[c * nl + j] = sum;
+    for (int e = threadIdx.x; e < kCorrOut * nl; e += blockDim.x) chi[kOutComp[e / nl] * nl + e % nl] = sums[e];
+    __syncthreads();
+    if (threadIdx.x < 32) {  // on-site term
+        double s = 0.0;
+        for (int k = threadIdx.x; k < ncnt; k += 32) s += nw[k] * ng[k];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (threadIdx.x < 4) chi[5 * threadIdx.x * nl] += threadIdx.x == 3 ? s / kPiD : s / (4.0 * kPiD);
     }
     __syncthreads();
     for (int e = threadIdx.x; e < 16 * nl; e += blockDim.x) a.out[size_t(kCorrOut) * a.n_corr + e] = float(chi[e]);
@@ -924,9 +928,12 @@ std::vector<int> order_rpa_pairs(const spn_tri_desc *d) {
 
 void launch_correlation(spn_tri *h) {
     const TriArgs a = h->args();
-    tri_corr_inner_kernel<<<2 * h->n + 4, 128, size_t(kWarps) * kCorrOut * h->nl * sizeof(double), h->stream>>>(a);
+    const size_t smem = size_t(kCorrTWarps) * kCorrOut * h->nl * sizeof(double);
+    check_cuda(cudaFuncSetAttribute(tri_corr_inner_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
+               "shared memory limit");
+    tri_corr_inner_kernel<<<2 * h->n + 4, kCorrTThreads, smem, h->stream>>>(a);
     check_cuda(cudaGetLastError(), "correlation launch");
-    tri_corr_final_kernel<<<1, 128, 16 * h->nl * sizeof(double), h->stream>>>(a);
+    tri_corr_final_kernel<<<1, kCorrThreads, tri_final_smem(h->nl), h->stream>>>(a);
     check_cuda(cudaGetLastError(), "correlation final launch");
 }
 
@@ -1068,7 +1075,7 @@ extern "C" int spn_tri_compute_step(spn_tri *h) {
         const TriArgs a = h->args();
         tri_self_energy_kernel<<<h->n, 128, 0, h->stream>>>(a);
         check_cuda(cudaGetLastError(), "self-energy launch");
-        tri_node_table_kernel<<<(h->n + 63) / 64, 64, 0, h->stream>>>(h->node_args());
+        tri_node_table_kernel<<<h->n, kNodeThreads, 0, h->stream>>>(h->node_args());
         check_cuda(cudaGetLastError(), "node table launch");
         check_cuda(cudaFuncSetAttribute(tri_vertex_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(vertex_smem(h->nl, h->rpa_n_seg))),
                    "shared memory limit");

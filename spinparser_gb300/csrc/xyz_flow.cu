@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(128) xyz_self_energy_kernel(XyzArgs a) {
 }
 
 // Loop-frequency node tables: the SU(2) core's body on an argument block of this flow.
-__global__ void xyz_node_table_kernel(FlowArgs f) { node_table_body(f, blockIdx.x); }
+__global__ void __launch_bounds__(kNodeThreads) xyz_node_table_kernel(FlowArgs f) { node_table_body(f, blockIdx.x); }
 
 // ------------------------------------------------------------------------------------
 // vertex flow
@@ -503,16 +503,19 @@ SPN_HDI void bundle8(const XyzArgs &a, const AB8 &ab, int r, int p, float g[4]) 
     }
 }
 
-__global__ void __launch_bounds__(128) xyz_corr_inner_kernel(XyzArgs a) {
+// Linear in the vertex, as the SU(2) core's (corr_inner_body): sums of g * vertex per site and, a
+// thread per node, of the on-site reads.
+constexpr int kCorrXWarps = 8, kCorrXThreads = 32 * kCorrXWarps;
+
+__global__ void __launch_bounds__(kCorrXThreads) xyz_corr_inner_kernel(XyzArgs a) {
     __shared__ float pos[kMaxFreq];
     __shared__ float nwp[kMaxCorrNodes];
-    __shared__ double nw[kMaxCorrNodes];
-    __shared__ int ncnt;
-    __shared__ double red[kWarps][4][32 * kSpt];
+    __shared__ double nw[kMaxCorrNodes], ng[kMaxCorrNodes];
+    __shared__ double red[kCorrXWarps][4][32 * kSpt];
+    __shared__ double egg[kCorrXWarps][4];
     for (int i = threadIdx.x; i < a.n; i += blockDim.x) pos[i] = a.freq[i];
     __syncthreads();
-    if (threadIdx.x == 0) ncnt = corr_nodes(pos, a.n, a.cutoff, nwp, nw);
-    __syncthreads();
+    const int ncnt = corr_nodes(pos, a.n, a.cutoff, nwp, nw, ng, [&](float x) { return odd_interp(pos, a.n, a.v2, x); });
     const int ia = blockIdx.x;
     if (ia >= ncnt) return;
     const float w = nwp[ia];
@@ -529,74 +532,76 @@ __global__ void __launch_bounds__(128) xyz_corr_inner_kernel(XyzArgs a) {
         ln.irid[k] = ln.valid[k] ? a.inv_sites[j] : 0;
         ln.iprm[k] = ln.valid[k] ? a.inv_sites_perm[j] : 0;
     }
-    const double dw = double(w) + odd_interp(pos, a.n, a.v2, w);
+    double e[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int q = threadIdx.x; q < 4 * ncnt; q += blockDim.x) {  // a thread per node and component
+        const int c = q & 3, b = q >> 2;
+        const float wp = nwp[b];
+        const double v = nw[b] * ng[b] * double(value4(pos, a, c, 0, 0, w + wp + 0.0f, w - wp, 0.0f));
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k == c) e[k] += v;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        for (int o = 16; o > 0; o >>= 1) e[c] += __shfl_xor_sync(0xffffffffu, e[c], o);
+        if (lane == 0) egg[warp][c] = e[c];
+    }
     double acc[kSpt][4];
 #pragma unroll
     for (int k = 0; k < kSpt; ++k)
         for (int c = 0; c < 4; ++c) acc[k][c] = 0.0;
-    for (int b = warp; b < ncnt; b += kWarps) {
+    for (int b = warp; b < ncnt; b += kCorrXWarps) {
         const float wp = nwp[b];
         AB8 ab;
         access8(pos, a.n, nl, w + wp + 0.0f, 0.0f, w - wp, ab);
-        float vv[4];
-        for (int c = 0; c < 4; ++c) vv[c] = value4(pos, a, c, 0, 0, w + wp + 0.0f, w - wp, 0.0f);
-        const double dwp = double(wp) + odd_interp(pos, a.n, a.v2, wp);
-        const double cw = nw[b] / (dw * dw * dwp * dwp * (4.0 * kPiD * kPiD));
+        const double cw = nw[b] * ng[b];
 #pragma unroll
         for (int k = 0; k < kSpt; ++k) {
             if (!ln.valid[k]) continue;
             float g[4];
             bundle8(a, ab, ab.exch ? ln.irid[k] : ln.rid[k], ab.exch ? ln.iprm[k] : ln.prm[k], g);
-            double rr[4] = {-double(g[0]), -double(g[1]), -double(g[2]), -4.0 * double(g[3])};  // dumbbell
-            if (ln.j[k] == 0) {  // egg diagram
-                rr[0] += 0.5 * (double(vv[0]) - vv[1] - vv[2] + vv[3]);
-                rr[1] += 0.5 * (-double(vv[0]) + vv[1] - vv[2] + vv[3]);
-                rr[2] += 0.5 * (-double(vv[0]) - vv[1] + vv[2] + vv[3]);
-                rr[3] += 2.0 * (double(vv[0]) + vv[1] + vv[2] + vv[3]);
-            }
-            for (int c = 0; c < 4; ++c) acc[k][c] += cw * rr[c];
+            for (int c = 0; c < 4; ++c) acc[k][c] += cw * double(g[c]);
         }
     }
 #pragma unroll
     for (int k = 0; k < kSpt; ++k)
         for (int c = 0; c < 4; ++c) red[warp][c][lane + 32 * k] = acc[k][c];
     __syncthreads();
-    for (int e = threadIdx.x; e < 4 * nl; e += blockDim.x) {
-        const int c = e / nl, j = e - c * nl;
+    const double norm = ng[ia] / (4.0 * kPiD * kPiD);
+    for (int p = threadIdx.x; p < 4 * nl; p += blockDim.x) {
+        const int c = p / nl, j = p - c * nl;
         double sum = 0.0;
-        for (int q = 0; q < kWarps; ++q) sum += red[q][c][j];
-        a.partial[(size_t(ia) * 4 + c) * nl + j] = sum;
+        for (int q = 0; q < kCorrXWarps; ++q) sum += red[q][c][j];
+        sum *= c == D ? -4.0 : -1.0;  // dumbbell
+        if (j == 0) {                 // egg diagram
+            double v[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int q = 0; q < kCorrXWarps; ++q)
+                for (int k = 0; k < 4; ++k) v[k] += egg[q][k];
+            if (c == D) sum += 2.0 * (v[0] + v[1] + v[2] + v[3]);
+            else sum += 0.5 * (2.0 * v[c] - v[0] - v[1] - v[2] + v[3]);
+        }
+        a.partial[(size_t(ia) * 4 + c) * nl + j] = sum * norm;
     }
 }
 
-__global__ void xyz_corr_final_kernel(XyzArgs a) {
+__global__ void __launch_bounds__(kCorrThreads) xyz_corr_final_kernel(XyzArgs a) {
     __shared__ float pos[kMaxFreq];
     __shared__ float nwp[kMaxCorrNodes];
-    __shared__ double nw[kMaxCorrNodes];
-    __shared__ int ncnt;
-    extern __shared__ double chi[];  // [4][nl]
+    __shared__ double nw[kMaxCorrNodes], ng[kMaxCorrNodes];
+    extern __shared__ double chi[];  // [4][nl] and the reduction's slices
     for (int i = threadIdx.x; i < a.n; i += blockDim.x) pos[i] = a.freq[i];
     __syncthreads();
-    if (threadIdx.x == 0) ncnt = corr_nodes(pos, a.n, a.cutoff, nwp, nw);
-    __syncthreads();
+    const int ncnt = corr_nodes(pos, a.n, a.cutoff, nwp, nw, ng, [&](float x) { return odd_interp(pos, a.n, a.v2, x); });
     const int nl = a.nl;
-    for (int e = threadIdx.x; e < 4 * nl; e += blockDim.x) {
-        const int c = e / nl, j = e - c * nl;
-        double sum = 0.0;
-        for (int ia = 0; ia < ncnt; ++ia) {
-            double v = a.partial[(size_t(ia) * 4 + c) * nl + j];
-            if (j == 0) {  // on-site term
-                const float w = nwp[ia];
-                const double dw = double(w) + odd_interp(pos, a.n, a.v2, w);
-                const double t1 = 1.0 / (dw * dw);
-                v += c == D ? t1 / kPiD : t1 / (4.0 * kPiD);
-            }
-            sum += nw[ia] * v;
-        }
-        chi[e] = sum;
-        a.out[4 * size_t(a.n_corr) + e] = float(sum);
+    column_sums(ncnt, 4 * nl, chi, [&](int ia, int e) { return nw[ia] * a.partial[size_t(ia) * 4 * nl + e]; });
+    if (threadIdx.x < 32) {  // on-site term
+        double s = 0.0;
+        for (int k = threadIdx.x; k < ncnt; k += 32) s += nw[k] * ng[k];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (threadIdx.x < 4) chi[threadIdx.x * nl] += threadIdx.x == D ? s / kPiD : s / (4.0 * kPiD);
     }
     __syncthreads();
+    for (int e = threadIdx.x; e < 4 * nl; e += blockDim.x) a.out[4 * size_t(a.n_corr) + e] = float(chi[e]);
     for (int q = threadIdx.x; q < a.n_corr; q += blockDim.x) {
         const int r = a.corr_rid[q], p = a.corr_perm[q];
         for (int c = 0; c < 3; ++c) a.out[size_t(c) * a.n_corr + q] = float(chi[perm_c(p, c) * nl + r]);
@@ -785,9 +790,9 @@ size_t vertex_smem(int nl, int n_seg) {
 
 void launch_correlation(spn_xyz *h) {
     const XyzArgs a = h->args();
-    xyz_corr_inner_kernel<<<2 * h->n + 4, 128, 0, h->stream>>>(a);
+    xyz_corr_inner_kernel<<<2 * h->n + 4, kCorrXThreads, 0, h->stream>>>(a);
     check_cuda(cudaGetLastError(), "correlation launch");
-    xyz_corr_final_kernel<<<1, 128, 4 * h->nl * sizeof(double), h->stream>>>(a);
+    xyz_corr_final_kernel<<<1, kCorrThreads, corr_final_smem(4 * h->nl), h->stream>>>(a);
     check_cuda(cudaGetLastError(), "correlation final launch");
 }
 
@@ -954,7 +959,7 @@ extern "C" int spn_xyz_compute_step(spn_xyz *h) {
         const XyzArgs a = h->args();
         xyz_self_energy_kernel<<<h->n, 128, 0, h->stream>>>(a);
         check_cuda(cudaGetLastError(), "self-energy launch");
-        xyz_node_table_kernel<<<(h->n + 63) / 64, 64, 0, h->stream>>>(h->node_args());
+        xyz_node_table_kernel<<<h->n, kNodeThreads, 0, h->stream>>>(h->node_args());
         check_cuda(cudaGetLastError(), "node table launch");
         check_cuda(cudaFuncSetAttribute(vertex_kernel(h->spt), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         int(vertex_smem(h->nl, h->rpa_n_seg))),
