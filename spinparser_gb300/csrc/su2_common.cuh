@@ -122,9 +122,9 @@ inline int site_exchange_kind(int nl, const int *sites, const int *inv_sites) {
 size_t vertex_flow_smem_bytes(int nl, const RpaSchedule &rpa, int inv_kind);
 int vertex_flow_blocks_per_sm(int nl, const RpaSchedule &rpa, int inv_kind);
 void launch_vertex_flow(const FlowArgs &a, int grid, cudaStream_t stream);
-// FP64 flow (su2_vertex64.cu): one warp per triple over a persistent grid.
+// FP64 flow (su2_vertex64.cu): a warp per item of three triples (nl <= 32) or per triple, over a persistent grid.
 void launch_vertex_flow_f64(const FlowArgsT<double> &a, int grid, cudaStream_t stream);
-int vertex_flow_f64_blocks_per_sm(int nl);
+int vertex_flow_f64_blocks_per_sm(int nl, const RpaSchedule &rpa);
 
 // Largest schedule staged in shared memory; larger ones are read from global memory.
 constexpr int kRpaSmemMaxInts = 8192;

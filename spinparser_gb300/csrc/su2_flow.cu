@@ -253,7 +253,7 @@ void download_pairs64(S *ss, S *dd, const double2 *src, size_t count, cudaStream
 // run.
 bool select_variant(spn_su2 *h, int npi, int in_smem) {
     if (h->fp64()) {  // one FP64 kernel
-        const int per_sm = vertex_flow_f64_blocks_per_sm(h->nl);
+        const int per_sm = vertex_flow_f64_blocks_per_sm(h->nl, h->args().rpa);
         cudaGetLastError();
         if (per_sm < 1 || npi != 1 || in_smem) return false;
         h->vertex_npi = 1;
