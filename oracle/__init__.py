@@ -216,6 +216,7 @@ class XyzOracle:
         pp = C.POINTER(C.POINTER(C.c_float))
         dsc = C.POINTER(XyzOracleDesc)
         lib.oracle_xyz_rhs_f32.argtypes = [dsc, C.c_float, fp, pp, fp, pp, i4]
+        lib.oracle_xyz_vertex_f32.argtypes = [dsc, C.c_float, fp, fp, pp, pp, i4]
         lib.oracle_xyz_correlation_f32.argtypes = [dsc, C.c_float, fp, pp, pp]
         lib.oracle_xyz_flow_f32.argtypes = [dsc, fp, i4, fp, pp, pp, i4]
         self.freq = np.ascontiguousarray(freq, np.float32)
@@ -247,6 +248,15 @@ class XyzOracle:
         assert self.lib.oracle_xyz_rhs_f32(C.byref(self.desc), cutoff, _p(v2, C.c_float), self._pp(v4), _p(dv2, C.c_float),
                                            self._pp(dv4), threads) == 0
         return dv2, np.stack(dv4)
+
+    def vertex(self, cutoff, v2, dv2, v4, threads: int = 0):
+        """dv4[4][F_N*Nl] of the state with the given self-energy flow dv2[N]."""
+        v2, dv2 = np.ascontiguousarray(v2, np.float32), np.ascontiguousarray(dv2, np.float32)
+        v4 = [np.ascontiguousarray(x, np.float32).reshape(-1) for x in v4]
+        dv4 = [np.empty(self.fn * self.nl, np.float32) for _ in range(4)]
+        assert self.lib.oracle_xyz_vertex_f32(C.byref(self.desc), cutoff, _p(v2, C.c_float), _p(dv2, C.c_float), self._pp(v4),
+                                              self._pp(dv4), threads) == 0
+        return np.stack(dv4)
 
     def correlation(self, cutoff, v2, v4):
         v2 = np.ascontiguousarray(v2, np.float32)
@@ -316,6 +326,7 @@ class TriOracle:
         fp, i4 = C.POINTER(C.c_float), C.c_int
         dsc = C.POINTER(XyzOracleDesc)
         lib.oracle_tri_rhs_f32.argtypes = [dsc, C.c_float, fp, fp, fp, fp, i4]
+        lib.oracle_tri_vertex_f32.argtypes = [dsc, C.c_float, fp, fp, fp, fp, i4]
         lib.oracle_tri_correlation_f32.argtypes = [dsc, C.c_float, fp, fp, fp]
         lib.oracle_tri_flow_f32.argtypes = [dsc, fp, i4, fp, fp, fp, i4]
         lib.oracle_tri_tables.argtypes = [C.POINTER(C.c_int)]
@@ -353,6 +364,16 @@ class TriOracle:
         assert self.lib.oracle_tri_rhs_f32(C.byref(self.desc), cutoff, _p(v2, C.c_float), _p(v4, C.c_float),
                                            _p(dv2, C.c_float), _p(dv4, C.c_float), threads) == 0
         return dv2, dv4
+
+    def vertex(self, cutoff, v2, dv2, v4, threads: int = 0):
+        """dv4[F_N*16*Nl] of the state with the given self-energy flow dv2[N]."""
+        v2, dv2 = np.ascontiguousarray(v2, np.float32), np.ascontiguousarray(dv2, np.float32)
+        v4 = np.ascontiguousarray(v4, np.float32).reshape(-1)
+        assert v4.size == self.size
+        dv4 = np.empty(self.size, np.float32)
+        assert self.lib.oracle_tri_vertex_f32(C.byref(self.desc), cutoff, _p(v2, C.c_float), _p(dv2, C.c_float),
+                                              _p(v4, C.c_float), _p(dv4, C.c_float), threads) == 0
+        return dv4
 
     def correlation(self, cutoff, v2, v4):
         """chi[16][Nl] at the state (the mixed spin/density components are zero)."""

@@ -740,17 +740,13 @@ int oracle_tri_tables(int *rows) {
     return n;
 }
 
-// One flow right-hand side: self-energy flow dv2[N], then the vertex flow dv4[F_N*16*Nl].
-int oracle_tri_rhs_f32(const TriOracleDesc *d, float cutoff, const float *v2, const float *v4, float *dv2, float *dv4,
-                       int nthreads) {
+// The vertex flow dv4[F_N*16*Nl] with a given self-energy flow dv2[N].
+int oracle_tri_vertex_f32(const TriOracleDesc *d, float cutoff, const float *v2, const float *dv2, const float *v4, float *dv4,
+                          int nthreads) {
     if (!d || d->n_freq < 2 || d->n_sites < 1) return -2;
     if (tables().bad) return -3;
     const int N = d->n_freq, Nl = d->n_sites;
     const int FN = N * N * (N + 1) / 2;
-    {
-        Tri core(*d, v2, nullptr, v4);
-        for (int i = 0; i < N; ++i) dv2[i] = core.self_energy_flow(i, cutoff);
-    }
     Tri core(*d, v2, dv2, v4);
 #ifdef _OPENMP
     if (nthreads > 0) omp_set_num_threads(nthreads);
@@ -764,6 +760,18 @@ int oracle_tri_rhs_f32(const TriOracleDesc *d, float cutoff, const float *v2, co
         for (int it = 0; it < FN; ++it) core.vertex_flow(it, cutoff, sc, dv4 + (long long)it * 16 * Nl);
     }
     return 0;
+}
+
+// One flow right-hand side: self-energy flow dv2[N], then the vertex flow dv4[F_N*16*Nl].
+int oracle_tri_rhs_f32(const TriOracleDesc *d, float cutoff, const float *v2, const float *v4, float *dv2, float *dv4,
+                       int nthreads) {
+    if (!d || d->n_freq < 2 || d->n_sites < 1) return -2;
+    if (tables().bad) return -3;
+    {
+        Tri core(*d, v2, nullptr, v4);
+        for (int i = 0; i < d->n_freq; ++i) dv2[i] = core.self_energy_flow(i, cutoff);
+    }
+    return oracle_tri_vertex_f32(d, cutoff, v2, dv2, v4, dv4, nthreads);
 }
 
 // Static susceptibility chi[16][Nl] at the given cutoff (the mixed components stay zero).

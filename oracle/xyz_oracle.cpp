@@ -625,17 +625,12 @@ struct Xyz {
 
 extern "C" {
 
-// One flow right-hand side: self-energy flow dv2[N], then the vertex flow of the four
-// components dv4[c][F_N*Nl] (c = X, Y, Z, density).
-int oracle_xyz_rhs_f32(const XyzOracleDesc *d, float cutoff, const float *v2, const float *const *v4, float *dv2,
-                       float *const *dv4, int nthreads) {
+// The vertex flow of the four components dv4[c][F_N*Nl] (c = X, Y, Z, density) with a given self-energy flow dv2[N].
+int oracle_xyz_vertex_f32(const XyzOracleDesc *d, float cutoff, const float *v2, const float *dv2, const float *const *v4,
+                          float *const *dv4, int nthreads) {
     if (!d || d->n_freq < 2 || d->n_sites < 1) return -2;
     const int N = d->n_freq, Nl = d->n_sites;
     const int FN = N * N * (N + 1) / 2;
-    {
-        Xyz core(*d, v2, nullptr, v4[0], v4[1], v4[2], v4[3]);
-        for (int i = 0; i < N; ++i) dv2[i] = core.self_energy_flow(i, cutoff);
-    }
     Xyz core(*d, v2, dv2, v4[0], v4[1], v4[2], v4[3]);
 #ifdef _OPENMP
     if (nthreads > 0) omp_set_num_threads(nthreads);
@@ -653,6 +648,19 @@ int oracle_xyz_rhs_f32(const XyzOracleDesc *d, float cutoff, const float *v2, co
         }
     }
     return 0;
+}
+
+// One flow right-hand side: self-energy flow dv2[N], then the vertex flow of the four
+// components dv4[c][F_N*Nl] (c = X, Y, Z, density).
+int oracle_xyz_rhs_f32(const XyzOracleDesc *d, float cutoff, const float *v2, const float *const *v4, float *dv2,
+                       float *const *dv4, int nthreads) {
+    if (!d || d->n_freq < 2 || d->n_sites < 1) return -2;
+    const int N = d->n_freq;
+    {
+        Xyz core(*d, v2, nullptr, v4[0], v4[1], v4[2], v4[3]);
+        for (int i = 0; i < N; ++i) dv2[i] = core.self_energy_flow(i, cutoff);
+    }
+    return oracle_xyz_vertex_f32(d, cutoff, v2, dv2, v4, dv4, nthreads);
 }
 
 // Static susceptibility chi[c][Nl] per component at the given cutoff.

@@ -160,13 +160,12 @@ __device__ __forceinline__ int su_index(int i, int j) {
     return hi * (hi + 1) / 2 + lo;
 }
 
-// Builds the descriptor of node (w, c) of an item.
-__device__ __forceinline__ void make_item(const FlowArgs &a, const float *pos, const ItemFreq &f, float w, float c,
-                                          ItemDesc &d) {
-    const MeshIndex mi{pos, a.n, a.mesh_lo, a.mesh_base, a.mesh_shift};
+// Builds the descriptor of node (w, c) of an item; mi looks up the mesh, nl elements make a slab.
+template <class Mesh>
+__device__ __forceinline__ void make_item(const Mesh &mi, int nl, const ItemFreq &f, float w, float c, ItemDesc &d) {
     const float A = __fadd_rn(__fadd_rn(f.h[0], w), f.l[0]), B = __fadd_rn(__fadd_rn(f.h[1], w), f.l[1]);
     const float P = __fadd_rn(__fadd_rn(f.h[2], w), f.l[2]), Q = __fadd_rn(__fadd_rn(f.h[3], w), f.l[3]);
-    const int nl = a.nl, stepT = a.n * nl, x = f.xi;
+    const int stepT = mi.n * nl, x = f.xi;
     int flags = 0;
     const Interp<float> iA = interp_abs(mi, A), iB = interp_abs(mi, B), iP = interp_abs(mi, P), iQ = interp_abs(mi, Q);
     // outer-point weights with the density's sign; a diagonal point has sign +1 (s) or -1 (u)

@@ -529,6 +529,10 @@ __device__ __forceinline__ void outer_gather(const FlowArgs &a, const WarpCtx &c
     __syncwarp();
 }
 
+__device__ __forceinline__ MeshIndex mesh_of(const FlowArgs &a, const float *pos) {
+    return MeshIndex{pos, a.n, a.mesh_lo, a.mesh_base, a.mesh_shift};
+}
+
 // The nodes desc[0 .. nb) of a transfer frequency: adds their terms to the accumulators and their
 // panels to M.  coef(k): the node's coefficient for this flow.
 template <int MB, class Coef>
@@ -626,7 +630,7 @@ __device__ __forceinline__ void vertex_item(const FlowArgs &a, const float *pos,
         const float *nc = a.node_c + size_t(f.xi) * a.max_nodes;
         for (int b0 = 0; b0 < cnt; b0 += kBatch) {
             const int nb = min(kBatch, cnt - b0);
-            if (lane < nb) make_item(a, pos, f, __ldg(nwp + b0 + lane), __ldg(nc + b0 + lane), c.desc[lane]);
+            if (lane < nb) make_item(mesh_of(a, pos), a.nl, f, __ldg(nwp + b0 + lane), __ldg(nc + b0 + lane), c.desc[lane]);
             __syncwarp();
             item_nodes<MB>(a.sd, a.nl, c.desc, nb, step, c, lane, [&](int k) { return c.desc[k].c; }, A, B,
                                 T, M);
@@ -1272,7 +1276,7 @@ __global__ void __launch_bounds__(kGroupWarps * 32, vertex_min_blocks(MB)) su2_v
             for (int b0 = 0; b0 < cnt; b0 += kGroupChunk) {
                 const int nb = min(kGroupChunk, cnt - b0);
                 __syncthreads();  // the previous chunk is consumed
-                if (tid < nb) make_item(a, pos, f, __ldg(nwp + b0 + tid), 0.0f, desc[tid]);
+                if (tid < nb) make_item(mesh_of(a, pos), a.nl, f, __ldg(nwp + b0 + tid), 0.0f, desc[tid]);
                 for (int k = lane; k < nb; k += 32)
                     ctab[warp * kGroupChunk + k] = __ldg(m_nc[warp] + size_t(f.xi) * a.max_nodes + b0 + k);
                 __syncthreads();

@@ -26,6 +26,7 @@
 #include "su2_common.cuh"
 #include "su2_device.cuh"
 #include "su2_kernels.cuh"
+#include "su2_item.cuh"
 #include "cuda_host.cuh"
 #include "host/capi_common.hpp"
 #include "host/pair_order.hpp"
@@ -65,6 +66,10 @@ struct XyzArgs {
     // seg_ptr[j] .. seg_ptr[j + 1] - 1
     const int *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr;
     int rpa_n_seg;
+    // lattices of at most 32 sites: site_kind (below) and the same walk cut into kItemThreads chunks
+    int site_kind;
+    const int *item_sched, *item_count, *item_slot_base, *item_seg_ptr;
+    int item_n_seg;
     const int *range_rid, *range_inv;
     const float *node_wp, *node_c;
     const int *node_cnt;
@@ -488,6 +493,411 @@ __global__ void __launch_bounds__(kThreads) xyz_vertex_kernel(XyzArgs a) {
 }
 
 // ------------------------------------------------------------------------------------
+// Vertex flow of lattices of at most 32 sites: a CTA per item of three triples (su2_item.cuh).
+//
+// A warp takes a node, lane = site: it reads the node's six planes (24 segments of 16-byte elements)
+// and adds the node's s/u terms to two triples and its t terms to the third, with the site-local
+// vertices of the t channel from the lane that holds pair 0.  The t channel's lattice sum
+// sum over pairs of A[perm1 c][rid1] B[perm2 c][rid2] (A, B: the first and second slab) is linear in the node, so the
+// CTA accumulates, over the nodes of a transfer frequency, the matrix of products of every spin component of A
+// with every spin component of B (3w x 3w) and of the densities (w x w) in registers (a 16 x 16 grid of
+// threads, 6 x 6 + 2 x 2 elements each at w = 32), and walks the pairs once per transfer frequency instead of
+// once per node.
+//
+// Honeycomb r9 (28 sites, 2308 pairs), N = 48, cutoff 1: triple by triple, with the pairs walked for every node (577
+// wavefronts of 16-byte shared reads), 14.2 ms a launch, bound by the shared-memory path; by items 5.6 ms, bound by
+// instruction issue and the latency of the slab reads at two CTAs an SM.
+// ------------------------------------------------------------------------------------
+constexpr int kItemThreads = 256, kItemWarps = kItemThreads / 32;
+constexpr int kItemBatch = 64;  // node descriptors built at once
+
+// Exchange of a flow's pairs, as site_exchange_kind: 0 every pair is its own exchange with identity
+// spin maps, 1 the exchange is an involution of the sites that fixes pair 0 and the direct pairs have
+// identity spin maps, 2 any tables.
+int xyz_site_kind(int nl, const int *sites, const int *perm, const int *inv, const int *inv_perm) {
+    int kind = site_exchange_kind(nl, sites, inv);
+    for (int j = 0; j < nl; ++j) {
+        if (perm[j] != 0) return 2;
+        if (kind == 0 && inv_perm[j] != 0) kind = 1;
+    }
+    return kind;
+}
+
+// (X, Y) and (Z, density) of an element.
+struct Quad {
+    float2 a, b;
+};
+__device__ __forceinline__ Quad load_quad(const float4 *p) {
+    const float4 v = __ldg(p);
+    return Quad{make_float2(v.x, v.y), make_float2(v.z, v.w)};
+}
+__device__ __forceinline__ float2 dup(float x) { return make_float2(x, x); }
+// w1 * x + w2 * y, the density with its own weights
+__device__ __forceinline__ Quad quad_mix(float w1, float d1, const Quad &x, float w2, float d2, const Quad &y) {
+    return Quad{fma2(dup(w2), y.a, mul2(dup(w1), x.a)), fma2(make_float2(w2, d2), y.b, mul2(make_float2(w1, d1), x.b))};
+}
+__device__ __forceinline__ Quad quad_g(const ItemDesc &d, const float4 *v, int i, const float4 &wi, const float4 &wo) {
+    const int4 o = d.g[i];
+    const Quad x = quad_mix(wo.x, wo.y, load_quad(v + o.x), wo.z, wo.w, load_quad(v + o.z));
+    const Quad y = quad_mix(wo.x, wo.y, load_quad(v + o.y), wo.z, wo.w, load_quad(v + o.w));
+    return quad_mix(wi.x, wi.x, x, wi.z, wi.z, y);
+}
+// T plane i: the density of its off-diagonal supports in the first buffer (the second buffer's is the opposite).
+__device__ __forceinline__ Quad quad_t(const ItemDesc &d, const float4 *v, int i) {
+    const int4 o = d.t[i];
+    const float4 p = d.tw[i][0], q = d.tw[i][1];
+    const Quad x = quad_mix(p.x, p.y, load_quad(v + o.x), p.z, p.w, load_quad(v + o.y));
+    const Quad y = quad_mix(q.x, q.y, load_quad(v + o.z), q.z, q.w, load_quad(v + o.w));
+    return Quad{add2(x.a, y.a), add2(x.b, y.b)};
+}
+__device__ __forceinline__ float quad_t_diag(const ItemDesc &d, const float4 *v, int i) {
+    const int4 o = d.t[i];
+    const float4 w = d.td[i];
+    return __fmaf_rn(w.w, __ldg(&v[o.w].w), __fmaf_rn(w.z, __ldg(&v[o.z].w), __fmaf_rn(w.y, __ldg(&v[o.y].w), __fmul_rn(w.x, __ldg(&v[o.x].w)))));
+}
+// the density of G plane i with the u channel's sign on the diagonal
+__device__ __forceinline__ float quad_diag_u(const ItemDesc &d, const float4 *v, int i, const float4 &wi, const float4 &wo, float h) {
+    const int4 o = d.g[i];
+    const int bits = d.flags >> (kFlDiagShift + 2 * i);
+    if (bits & 1) h = __fmaf_rn(-2.0f * wo.x, __fmaf_rn(wi.z, __ldg(&v[o.y].w), __fmul_rn(wi.x, __ldg(&v[o.x].w))), h);
+    if (bits & 2) h = __fmaf_rn(-2.0f * wo.z, __fmaf_rn(wi.z, __ldg(&v[o.w].w), __fmul_rn(wi.x, __ldg(&v[o.z].w))), h);
+    return h;
+}
+// X, Y, Z replaced by components perm[p][0..2]
+__device__ __forceinline__ Quad quad_perm(const Quad &q, int p) {
+    const float4 v = make_float4(q.a.x, q.a.y, q.b.x, q.b.y);
+    return Quad{make_float2(comp_of(v, perm_c(p, 0)), comp_of(v, perm_c(p, 1))), make_float2(comp_of(v, perm_c(p, 2)), v.w)};
+}
+// adds the s/u integrand's products of a pair of slabs (s_terms)
+__device__ __forceinline__ void add_su(const Quad &p, const Quad &q, float4 &r) {
+    r.x = fmaf(p.b.y, q.a.x, fmaf(p.a.x, q.b.y, fmaf(-p.b.x, q.a.y, fmaf(-p.a.y, q.b.x, r.x))));
+    r.y = fmaf(p.b.y, q.a.y, fmaf(p.a.y, q.b.y, fmaf(-p.b.x, q.a.x, fmaf(-p.a.x, q.b.x, r.y))));
+    r.z = fmaf(p.b.y, q.b.x, fmaf(p.b.x, q.b.y, fmaf(-p.a.x, q.a.y, fmaf(-p.a.y, q.a.x, r.z))));
+    r.w = fmaf(p.b.y, q.b.y, fmaf(p.a.x, q.a.x, fmaf(p.a.y, q.a.y, fmaf(p.b.x, q.b.x, r.w))));
+}
+__device__ __forceinline__ void add_acc(float4 &acc, float c, float cd, const float4 &r) {
+    acc.x = fmaf(c, r.x, acc.x);
+    acc.y = fmaf(c, r.y, acc.y);
+    acc.z = fmaf(c, r.z, acc.z);
+    acc.w = fmaf(cd, r.w, acc.w);
+}
+// Factors of the t channel's slab components for one site-local vertex l (XYZFrgCore.cpp:347-417), its density with
+// the u channel's sign reversed: component c takes the two other spin components minus its own.
+__device__ __forceinline__ float4 local_factors(const Quad &l) {
+    const float x = l.a.x, y = l.a.y, z = l.b.x, h = l.b.y;
+    return make_float4(y + z - x + h, x + z - y + h, x + y - z + h, h - x - y - z);
+}
+__device__ __forceinline__ float4 shfl4(const float4 &v) {
+    constexpr unsigned kAll = 0xffffffffu;
+    return make_float4(__shfl_sync(kAll, v.x, 0), __shfl_sync(kAll, v.y, 0), __shfl_sync(kAll, v.z, 0), __shfl_sync(kAll, v.w, 0));
+}
+__device__ __forceinline__ Quad shfl_quad(const Quad &q, int src) {
+    constexpr unsigned kAll = 0xffffffffu;
+    return Quad{make_float2(__shfl_sync(kAll, q.a.x, src), __shfl_sync(kAll, q.a.y, src)),
+                make_float2(__shfl_sync(kAll, q.b.x, src), __shfl_sync(kAll, q.b.y, src))};
+}
+
+// One node at the lane's site, by a whole warp: adds the two s/u targets to acc1, acc2 and the t target's local terms
+// to acct, and returns the first two t slabs (a times c) for the lattice sum.
+__device__ __forceinline__ void xyz_node(const XyzArgs &a, const ItemDesc &d, int step, int rid, int prm, int irid, int iprm,
+                                         int lane, float4 &acc1, float4 &acc2, float4 &acct, Quad &pa, Quad &pb) {
+    const int fl = d.flags, kind = a.site_kind;
+    const float c = d.c, c1 = step == 2 ? -c : c, c2 = step == 0 ? c : -c;
+    const float4 wA = d.w[0], wB = d.w[1], wP = d.w[2], wQ = d.w[3];
+    auto at = [&](int bit) { return a.sd + (fl & bit ? irid : rid); };
+    auto site = [&](const Quad &q, int bit) {  // the site's components: its representative's, permuted
+        if (fl & bit) return kind ? quad_perm(q, iprm) : q;
+        return kind == 2 ? quad_perm(q, prm) : q;
+    };
+    const float4 *v0 = at(kFlE0), *v1 = at(kFlE1), *v2 = at(kFlE2), *v3 = at(kFlE3);
+    Quad R0 = quad_g(d, v0, 0, wA, wB), R1 = quad_g(d, v1, 1, wP, wQ), R2 = quad_g(d, v2, 2, wB, wA), R3 = quad_g(d, v3, 3, wQ, wP);
+    {
+        float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        add_su(site(R0, kFlE0), site(R1, kFlE1), r);
+        add_su(site(R2, kFlE2), site(R3, kFlE3), r);
+        add_acc(acc1, c, c1, r);
+    }
+    const bool diag = step != 2 && (fl & kFlDiag) != 0;
+    Quad U0 = R0, U1 = R1, U2 = R2, U3 = R3;  // densities with the u channel's signs
+    if (diag) {
+        U0.b.y = quad_diag_u(d, v0, 0, wA, wB, U0.b.y);
+        U1.b.y = quad_diag_u(d, v1, 1, wP, wQ, U1.b.y);
+        U2.b.y = quad_diag_u(d, v2, 2, wB, wA, U2.b.y);
+        U3.b.y = quad_diag_u(d, v3, 3, wQ, wP, U3.b.y);
+        if (step == 1) R0 = U0, R1 = U1, R2 = U2, R3 = U3;
+    }
+    // second target: a and b exchanged, G0 and G2 trade places with their own site exchange
+    {
+        Quad q0 = R0, q2 = R2;
+        const bool f0 = ((fl & kFlE0) != 0) != ((fl & kFlF0) != 0), f2 = ((fl & kFlE2) != 0) != ((fl & kFlF2) != 0);
+        if (kind == 1) {
+            if (f0) q0 = shfl_quad(q0, irid);
+            if (f2) q2 = shfl_quad(q2, irid);
+        } else if (kind == 2) {
+            const float4 *b0 = at(kFlF0), *b2 = at(kFlF2);
+            q0 = quad_g(d, b0, 0, wA, wB);
+            q2 = quad_g(d, b2, 2, wB, wA);
+            if (diag && step == 1) {
+                q0.b.y = quad_diag_u(d, b0, 0, wA, wB, q0.b.y);
+                q2.b.y = quad_diag_u(d, b2, 2, wB, wA, q2.b.y);
+            }
+        }
+        float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        add_su(site(q2, kFlF2), site(R1, kFlE1), r);
+        add_su(site(q0, kFlF0), site(R3, kFlE3), r);
+        add_acc(acc2, c, c2, r);
+    }
+    // t channel: buffers 0, 2 (1, 3) have equal spin slabs and opposite off-diagonal densities, and the local vertices
+    // of planes G2, G0 (G1, G3) at pair 0
+    if (kind == 2) {
+        U0 = quad_g(d, a.sd, 0, wA, wB);
+        U1 = quad_g(d, a.sd, 1, wP, wQ);
+        U2 = quad_g(d, a.sd, 2, wB, wA);
+        U3 = quad_g(d, a.sd, 3, wQ, wP);
+        if (diag) {
+            U0.b.y = quad_diag_u(d, a.sd, 0, wA, wB, U0.b.y);
+            U1.b.y = quad_diag_u(d, a.sd, 1, wP, wQ, U1.b.y);
+            U2.b.y = quad_diag_u(d, a.sd, 2, wB, wA, U2.b.y);
+            U3.b.y = quad_diag_u(d, a.sd, 3, wQ, wP, U3.b.y);
+        }
+    }
+    const float4 m0 = local_factors(U2), m1 = local_factors(U1), m2 = local_factors(U0), m3 = local_factors(U3);
+    const float4 k0 = shfl4(make_float4(m0.x + m2.x, m0.y + m2.y, m0.z + m2.z, m0.w - m2.w));
+    const float4 k1 = shfl4(make_float4(m1.x + m3.x, m1.y + m3.y, m1.z + m3.z, m1.w - m3.w));
+    const float4 *vt0 = at(kFlT0), *vt1 = at(kFlT1);
+    Quad T0 = site(quad_t(d, vt0, 0), kFlT0), T1 = site(quad_t(d, vt1, 1), kFlT1);
+    float4 r = make_float4(fmaf(k1.x, T1.a.x, k0.x * T0.a.x), fmaf(k1.y, T1.a.y, k0.y * T0.a.y),
+                           fmaf(k1.z, T1.b.x, k0.z * T0.b.x), fmaf(k1.w, T1.b.y, k0.w * T0.b.y));
+    if (fl & (kFlDiagT | kFlExT)) {
+        const float d0 = __shfl_sync(0xffffffffu, m0.w + m2.w, 0), d1 = __shfl_sync(0xffffffffu, m1.w + m3.w, 0);
+        const float e0 = quad_t_diag(d, vt0, 0), e1 = quad_t_diag(d, vt1, 1);
+        r.w = fmaf(d0, e0, fmaf(d1, e1, r.w));
+        if (fl & kFlExT) {  // the fourth buffer reads the other site
+            const float4 f = shfl4(m3);
+            const float4 *vt3 = at(kFlT3);
+            const Quad T3 = site(quad_t(d, vt3, 1), kFlT3);
+            const float e3 = quad_t_diag(d, vt3, 1);
+            r.x = fmaf(f.x, T3.a.x - T1.a.x, r.x);
+            r.y = fmaf(f.y, T3.a.y - T1.a.y, r.y);
+            r.z = fmaf(f.z, T3.b.x - T1.b.x, r.z);
+            r.w = fmaf(f.w, (e3 - T3.b.y) - (e1 - T1.b.y), r.w);
+        }
+        T0.b.y += e0;
+        T1.b.y += e1;
+    }
+    add_acc(acct, c, c, r);
+    pa = Quad{mul2(dup(c), T0.a), mul2(dup(c), T0.b)};
+    pb = T1;
+}
+
+struct XyzItemSmem {
+    size_t u, panels, parts, rpa, total;
+};
+__host__ __device__ inline XyzItemSmem xyz_item_smem(int R, int n_seg) {
+    const int w = 16 * R;
+    XyzItemSmem L;
+    size_t o = 0;
+    // union: a batch's descriptors, or (after a transfer frequency) the product matrices and the walk's partials
+    L.u = o;
+    const size_t d = kItemBatch * sizeof(ItemDesc), m = sizeof(float) * size_t(10 * w * w) + sizeof(float4) * size_t(n_seg);
+    o += ((d > m ? d : m) + 15) / 16 * 16;
+    L.panels = o; o += sizeof(float) * 2 * kItemWarps * 8 * size_t(w);  // 2 buffers x nodes x (A, B) x 4 components
+    L.parts = o; o += sizeof(float4) * 3 * kItemWarps * size_t(w);
+    L.rpa = o; o += sizeof(float4) * 3 * size_t(w);
+    L.total = o;
+    return L;
+}
+
+// Adds a panel to the thread's block of the product matrices.  Panel: A's components X, Y, Z, D of w sites each,
+// then B's.
+template <int R>
+__device__ __forceinline__ void xyz_outer(const float *pan, int tr, int tc, float2 (&S)[3 * R][(3 * R + 1) / 2],
+                                          float (&Dm)[R][R]) {
+    constexpr int w = 16 * R, K = 3 * R, K2 = (K + 1) / 2;
+    float av[K], ad[R], bd[R];
+    float2 bv[K2];
+    if constexpr (K % 2 == 0) {  // 8-byte reads
+        const float2 *pa = reinterpret_cast<const float2 *>(pan + tr * K), *pb = reinterpret_cast<const float2 *>(pan + 4 * w + tc * K);
+#pragma unroll
+        for (int i = 0; i < K2; ++i) {
+            const float2 v = pa[i];
+            av[2 * i] = v.x;
+            av[2 * i + 1] = v.y;
+            bv[i] = pb[i];
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < K; ++i) av[i] = pan[tr * K + i];
+#pragma unroll
+        for (int j = 0; j < K2; ++j)
+            bv[j] = make_float2(pan[4 * w + tc * K + 2 * j], 2 * j + 1 < K ? pan[4 * w + tc * K + 2 * j + 1] : 0.0f);
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        ad[i] = pan[3 * w + tr * R + i];
+        bd[i] = pan[7 * w + tc * R + i];
+    }
+#pragma unroll
+    for (int i = 0; i < K; ++i)
+#pragma unroll
+        for (int j = 0; j < K2; ++j) S[i][j] = fma2(dup(av[i]), bv[j], S[i][j]);
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < R; ++j) Dm[i][j] = fmaf(ad[i], bd[j], Dm[i][j]);
+}
+
+template <int R>
+__global__ void __launch_bounds__(kItemThreads, 2) xyz_item_kernel(XyzArgs a) {
+    constexpr int w = 16 * R, K = 3 * R, K2 = (K + 1) / 2;
+    extern __shared__ float4 xs[];
+    __shared__ float pos[kMaxFreq];
+    __shared__ int s_item;
+    unsigned char *smem = reinterpret_cast<unsigned char *>(xs);
+    const XyzItemSmem L = xyz_item_smem(R, a.item_n_seg);
+    ItemDesc *desc = reinterpret_cast<ItemDesc *>(smem + L.u);
+    float *Ms = reinterpret_cast<float *>(smem + L.u);  // spin (3w x 3w), then density (w x w)
+    float4 *slots = reinterpret_cast<float4 *>(Ms + 10 * w * w);
+    float *panels = reinterpret_cast<float *>(smem + L.panels);
+    float4 *parts = reinterpret_cast<float4 *>(smem + L.parts);
+    float4 *rpa = reinterpret_cast<float4 *>(smem + L.rpa);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tr = tid >> 4, tc = tid & 15;
+    const int n = a.n, nl = a.nl;
+    for (int i = tid; i < n; i += blockDim.x) pos[i] = a.freq[i];
+    const bool valid = lane < nl;
+    const int sc = min(lane, nl - 1);  // a lane without a site reads the last one's elements
+    const int rid = a.sites[sc], prm = a.sites_perm[sc], irid = a.inv_sites[sc], iprm = a.inv_sites_perm[sc];
+    const int rpa_cnt = a.item_count[tid], rpa_base = a.item_slot_base[tid];
+    const float two_pi = 2.0f * float(kPiD);
+    const int items = vertex_items(n);
+    const MeshSearch<float> mesh{pos, n};
+    int round = 0;
+    for (;;) {
+        __syncthreads();  // the previous item is finished with shared memory
+        if (tid == 0) s_item = atomicAdd(a.work_counter, 1);
+        __syncthreads();
+        const int item = s_item;
+        if (item >= items) break;
+        int p, q, r;
+        decode_item(item, p, q, r);
+        float4 A = make_float4(0.0f, 0.0f, 0.0f, 0.0f), B = A, T = A;
+        // transfer p: targets (p,q,r), (p,r,q) and the t channel of (q,p,r); q: (q,p,r), (p,r,q), t of (p,q,r);
+        // r: (q,p,r), (p,q,r), t of (p,r,q)
+#pragma unroll 1
+        for (int step = 0; step < 3; ++step) {
+            const ItemFreq f = item_freq(pos, step == 0 ? p : (step == 1 ? q : r), step == 0 ? q : p, step == 2 ? q : r, step == 2);
+            float2 S[K][K2];
+            float Dm[R][R];
+#pragma unroll
+            for (int i = 0; i < K; ++i)
+#pragma unroll
+                for (int j = 0; j < K2; ++j) S[i][j] = make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+#pragma unroll
+                for (int j = 0; j < R; ++j) Dm[i][j] = 0.0f;
+            const int cnt = __ldg(a.node_cnt + f.xi);
+            const float *nwp = a.node_wp + size_t(f.xi) * a.max_nodes;
+            const float *nc = a.node_c + size_t(f.xi) * a.max_nodes;
+#pragma unroll 1
+            for (int b0 = 0; b0 < cnt; b0 += kItemBatch) {
+                const int nb = min(kItemBatch, cnt - b0);
+                __syncthreads();  // the previous batch's descriptors (or the matrices) are no longer read
+                if (tid < nb) make_item(mesh, nl, f, __ldg(nwp + b0 + tid), __ldg(nc + b0 + tid), desc[tid]);
+                __syncthreads();
+#pragma unroll 1
+                for (int r0 = 0; r0 < nb; r0 += kItemWarps, ++round) {
+                    float *buf = panels + size_t(round & 1) * kItemWarps * 8 * w;
+                    if (r0 + warp < nb) {
+                        Quad pa, pb;
+                        xyz_node(a, desc[r0 + warp], step, rid, prm, irid, iprm, lane, A, B, T, pa, pb);
+                        if (valid) {
+                            float *pan = buf + warp * 8 * w + lane;
+                            pan[0] = pa.a.x;
+                            pan[w] = pa.a.y;
+                            pan[2 * w] = pa.b.x;
+                            pan[3 * w] = pa.b.y;
+                            pan[4 * w] = pb.a.x;
+                            pan[5 * w] = pb.a.y;
+                            pan[6 * w] = pb.b.x;
+                            pan[7 * w] = pb.b.y;
+                        }
+                    }
+                    __syncthreads();  // the round's panels are written
+                    const int np = min(kItemWarps, nb - r0);
+#pragma unroll 1
+                    for (int k = 0; k < np; ++k) xyz_outer<R>(buf + k * 8 * w, tr, tc, S, Dm);
+                }
+            }
+            __syncthreads();  // every descriptor read is done
+#pragma unroll
+            for (int i = 0; i < K; ++i)
+#pragma unroll
+                for (int j = 0; j < K; ++j) Ms[(tr * K + i) * 3 * w + tc * K + j] = (j & 1) ? S[i][j / 2].y : S[i][j / 2].x;
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+#pragma unroll
+                for (int j = 0; j < R; ++j) Ms[9 * w * w + (tr * R + i) * w + tc * R + j] = Dm[i][j];
+            __syncthreads();
+            {  // XYZFrgCore.cpp:282-305, every site's pairs in one walk
+                float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                int slot = rpa_base;
+                for (int i = 0; i < rpa_cnt; ++i) {
+                    const int e = __ldg(a.item_sched + kItemThreads * i + tid);
+                    const int r1 = e & 127, r2 = (e >> 7) & 127, p1 = (e >> 14) & 7, p2 = (e >> 17) & 7;
+                    sum.x += Ms[(perm_c(p1, 0) * w + r1) * 3 * w + perm_c(p2, 0) * w + r2];
+                    sum.y += Ms[(perm_c(p1, 1) * w + r1) * 3 * w + perm_c(p2, 1) * w + r2];
+                    sum.z += Ms[(perm_c(p1, 2) * w + r1) * 3 * w + perm_c(p2, 2) * w + r2];
+                    sum.w += Ms[9 * w * w + r1 * w + r2];
+                    if (e & (1 << 20)) {
+                        slots[slot++] = sum;
+                        sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    }
+                }
+            }
+            __syncthreads();
+            if (tid < nl) {
+                float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                for (int k = a.item_seg_ptr[tid]; k < a.item_seg_ptr[tid + 1]; ++k) {
+                    const float4 v = slots[k];
+                    sum.x += v.x;
+                    sum.y += v.y;
+                    sum.z += v.z;
+                    sum.w += v.w;
+                }
+                rpa[step * w + tid] = sum;
+            }
+            if (step == 0) { const float4 t = A; A = T; T = t; }
+            if (step == 1) { const float4 t = B; B = T; T = t; }
+        }
+        if (valid) {
+            parts[(0 * kItemWarps + warp) * w + lane] = B;  // (p,q,r), t channel of transfer q
+            parts[(1 * kItemWarps + warp) * w + lane] = T;  // (p,r,q), r
+            parts[(2 * kItemWarps + warp) * w + lane] = A;  // (q,p,r), p
+        }
+        __syncthreads();
+        for (int e = tid; e < 3 * nl; e += kItemThreads) {
+            const int k = e / nl, j = e - k * nl;
+            if ((k == 1 && q == r) || (k == 2 && p == q)) continue;  // the same triple again
+            float4 v[kItemWarps];
+#pragma unroll
+            for (int u = 0; u < kItemWarps; ++u) v[u] = parts[(k * kItemWarps + u) * w + j];
+#pragma unroll
+            for (int o = 1; o < kItemWarps; o <<= 1)
+#pragma unroll
+                for (int u = 0; u + o < kItemWarps; u += 2 * o)
+                    v[u] = make_float4(v[u].x + v[u + o].x, v[u].y + v[u + o].y, v[u].z + v[u + o].z, v[u].w + v[u + o].w);
+            const float4 g = rpa[((k + 1) % 3) * w + j];
+            const int ts = k == 2 ? q : p, tt = k == 0 ? q : (k == 1 ? r : p), tu = k == 1 ? q : r;
+            const float4 o = make_float4((v[0].x + 4.0f * g.x) / two_pi, (v[0].y + 4.0f * g.y) / two_pi,
+                                         (v[0].z + 4.0f * g.z) / two_pi, (v[0].w + 4.0f * g.w) / two_pi);
+            a.dsd[(size_t(su_index(ts, tu)) * n + tt) * nl + j] = o;
+            if (isnan(o.x) || isnan(o.y) || isnan(o.z) || isnan(o.w)) atomicOr(a.status, kStatusNaN);
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------
 // correlation measurement at nu = 0 (XYZMeasurementCorrelation.cpp:98-184): one CTA per
 // outer node accumulates the inner integral per site in FP64, a final CTA adds the outer
 // weights and the on-site term and scatters to (basis, site in range) entries.
@@ -641,7 +1051,6 @@ using cuh::h2d;
 
 struct spn_xyz {
     int device = 0, n = 0, nl = 0, n_range = 0, n_corr = 0, n_overlap = 0, max_nodes = 0, sms = 0, grid = 0;
-    int spt = 4;  // sites per lane of the vertex kernel
     long long fn = 0;
     float cutoff = 0.0f;
     cudaStream_t stream = nullptr;
@@ -650,8 +1059,9 @@ struct spn_xyz {
     float4 *sd = nullptr, *dsd = nullptr;
     int *ints = nullptr;  // all integer tables in one allocation
     int *sites, *sites_perm, *inv_sites, *inv_sites_perm, *range_rid, *range_inv, *corr_rid, *corr_perm, *node_cnt,
-        *work_counter, *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr;
-    int rpa_n_seg = 0;
+        *work_counter, *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr, *item_sched, *item_count, *item_slot_base,
+        *item_seg_ptr;
+    int rpa_n_seg = 0, item_n_seg = 0, site_kind = 0;
     unsigned *status = nullptr;
     double *partial = nullptr;
 
@@ -678,6 +1088,12 @@ struct spn_xyz {
         a.rpa_slot_base = rpa_slot_base;
         a.rpa_seg_ptr = rpa_seg_ptr;
         a.rpa_n_seg = rpa_n_seg;
+        a.site_kind = site_kind;
+        a.item_sched = item_sched;
+        a.item_count = item_count;
+        a.item_slot_base = item_slot_base;
+        a.item_seg_ptr = item_seg_ptr;
+        a.item_n_seg = item_n_seg;
         a.range_rid = range_rid;
         a.range_inv = range_inv;
         a.node_wp = node_wp;
@@ -762,12 +1178,14 @@ void validate(const spn_xyz_desc *d) {
     in_range(d->corr_perm, d->n_corr, 6, "corr_perm");
 }
 
-// the vertex kernel for SPT sites per lane (1 for Nl <= 32, 2 for Nl <= 64, else 4)
-const void *vertex_kernel(int spt) {
-    if (spt == 1) return reinterpret_cast<const void *>(&xyz_vertex_kernel<1>);
-    if (spt == 2) return reinterpret_cast<const void *>(&xyz_vertex_kernel<2>);
+// The vertex kernel: by items for Nl <= 32, else by triples with SPT sites per lane (2 for Nl <= 64, else 4).
+const void *vertex_kernel(int nl) {
+    if (nl <= 16) return reinterpret_cast<const void *>(&xyz_item_kernel<1>);
+    if (nl <= 32) return reinterpret_cast<const void *>(&xyz_item_kernel<2>);
+    if (nl <= 64) return reinterpret_cast<const void *>(&xyz_vertex_kernel<2>);
     return reinterpret_cast<const void *>(&xyz_vertex_kernel<4>);
 }
+int vertex_threads(int nl) { return nl <= 32 ? kItemThreads : kThreads; }
 
 // The RPA pairs of each site in the order of host/pair_order (against bank collisions of the
 // kernel's 16-byte reads of A6 and B6), packed rid1 | rid2 << 7 | perm1 << 14 | perm2 << 17.
@@ -784,8 +1202,9 @@ std::vector<int> order_rpa_pairs(const spn_xyz_desc *d) {
     return out;
 }
 
-size_t vertex_smem(int nl, int n_seg) {
-    return size_t(kWarps) * (kXBatch * sizeof(XDesc) + (12 * size_t(nl) + size_t(n_seg)) * sizeof(float4));
+size_t vertex_smem(const spn_xyz *h) {
+    if (h->nl <= 32) return xyz_item_smem(h->nl <= 16 ? 1 : 2, h->item_n_seg).total;
+    return size_t(kWarps) * (kXBatch * sizeof(XDesc) + (12 * size_t(h->nl) + size_t(h->rpa_n_seg)) * sizeof(float4));
 }
 
 void launch_correlation(spn_xyz *h) {
@@ -851,11 +1270,19 @@ extern "C" int spn_xyz_create(const spn_xyz_desc *d, spn_xyz **out) {
             put(rpa.count.data(), 32);
             put(rpa.slot_base.data(), 32);
             put(rpa.seg_ptr.data(), nl + 1);
+            h->site_kind = xyz_site_kind(nl, d->sites_rid, d->sites_perm, d->inv_sites_rid, d->inv_sites_perm);
+            const LaneSchedule items = lane_schedule(nl, d->overlap_ptr, packed, kItemThreads, 20);
+            h->item_n_seg = items.n_seg;
+            put(items.sched.data(), int(items.sched.size()));
+            put(items.count.data(), kItemThreads);
+            put(items.slot_base.data(), kItemThreads);
+            put(items.seg_ptr.data(), nl + 1);
             h->ints = dalloc<int>(img.size(), "alloc lattice tables");
             h2d(h->ints, img.data(), img.size(), h->stream);
             int **fields[] = {&h->sites, &h->sites_perm, &h->inv_sites, &h->inv_sites_perm, &h->range_rid, &h->range_inv,
                               &h->corr_rid, &h->corr_perm, &h->node_cnt, &h->work_counter, &h->rpa_sched,
-                              &h->rpa_count, &h->rpa_slot_base, &h->rpa_seg_ptr};
+                              &h->rpa_count, &h->rpa_slot_base, &h->rpa_seg_ptr, &h->item_sched, &h->item_count,
+                              &h->item_slot_base, &h->item_seg_ptr};
             for (size_t k = 0; k < at.size(); ++k) *fields[k] = h->ints + at[k];
             h2d(h->freq, d->freq, h->n, h->stream);
             check_cuda(cudaMemsetAsync(h->sd, 0, vsz * sizeof(float4), h->stream), "memset");
@@ -865,11 +1292,10 @@ extern "C" int spn_xyz_create(const spn_xyz_desc *d, spn_xyz **out) {
             check_cuda(cudaMemsetAsync(h->status, 0, sizeof(unsigned), h->stream), "memset");
             check_cuda(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device), "device attribute");
             int per_sm = 0;
-            h->spt = h->nl <= 32 ? 1 : (h->nl <= 64 ? 2 : 4);
-            const void *fn = vertex_kernel(h->spt);
-            check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(vertex_smem(h->nl, h->rpa_n_seg))),
+            const void *fn = vertex_kernel(h->nl);
+            check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(vertex_smem(h))),
                        "shared memory limit");
-            check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, vertex_smem(h->nl, h->rpa_n_seg)), "occupancy");
+            check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, vertex_threads(h->nl), vertex_smem(h)), "occupancy");
             if (per_sm < 1) throw Error(ErrorType::Unsupported, "XYZ vertex-flow kernel does not fit on this device");
             h->grid = h->sms * per_sm;
             check_cuda(cudaStreamSynchronize(h->stream), "create sync");
@@ -961,12 +1387,11 @@ extern "C" int spn_xyz_compute_step(spn_xyz *h) {
         check_cuda(cudaGetLastError(), "self-energy launch");
         xyz_node_table_kernel<<<h->n, kNodeThreads, 0, h->stream>>>(h->node_args());
         check_cuda(cudaGetLastError(), "node table launch");
-        check_cuda(cudaFuncSetAttribute(vertex_kernel(h->spt), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        int(vertex_smem(h->nl, h->rpa_n_seg))),
-                   "shared memory limit");
-        if (h->spt == 1) xyz_vertex_kernel<1><<<h->grid, kThreads, vertex_smem(h->nl, h->rpa_n_seg), h->stream>>>(a);
-        else if (h->spt == 2) xyz_vertex_kernel<2><<<h->grid, kThreads, vertex_smem(h->nl, h->rpa_n_seg), h->stream>>>(a);
-        else xyz_vertex_kernel<4><<<h->grid, kThreads, vertex_smem(h->nl, h->rpa_n_seg), h->stream>>>(a);
+        const void *fn = vertex_kernel(h->nl);
+        check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(vertex_smem(h))), "shared memory limit");
+        XyzArgs arg = a;
+        void *params[] = {&arg};
+        check_cuda(cudaLaunchKernel(fn, dim3(h->grid), dim3(vertex_threads(h->nl)), params, vertex_smem(h), h->stream), "vertex flow launch");
         check_cuda(cudaGetLastError(), "vertex flow launch");
     });
 }
