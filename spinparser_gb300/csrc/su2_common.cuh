@@ -11,6 +11,8 @@ constexpr unsigned kStatusNaN = 1u;           // a NaN was written into the flow
 constexpr unsigned kStatusNodeOverflow = 2u;  // a loop-frequency node table overflowed
 constexpr unsigned kStatusStageTimeout = 4u;  // a bulk copy to shared memory did not complete in
                                               // time; the kernel read global memory instead
+constexpr unsigned kStatusProductTimeout = 8u;  // a tensor-core product did not complete in time;
+                                                 // the flow is incomplete
 
 // Lane-balanced RPA schedule (built by host/rpa_schedule.cpp): the RPA pair lists of all
 // rids merged into distinct (rid, rid1, rid2) with their multiplicity, sorted by rid and cut

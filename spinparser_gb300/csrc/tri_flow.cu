@@ -26,7 +26,9 @@
 #include <vector>
 #include "su2_common.cuh"
 #include "su2_device.cuh"
+#include "su2_item.cuh"
 #include "su2_kernels.cuh"
+#include "umma.cuh"
 #include "tri_algebra.hpp"
 #include "cuda_host.cuh"
 #include "host/capi_common.hpp"
@@ -41,7 +43,8 @@ namespace {
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxSites = 128;
-constexpr int kTBatch = 4;  // nodes whose descriptors a warp builds at once (a quad of lanes each)
+constexpr int kTBatch = 4;  // nodes whose descriptors a warp builds at once (a quad of lanes each): above 32 sites
+constexpr int kSiteBatch = 8;  // at most 32 sites
 constexpr int kCorrOut = 10;  // XX XY XZ YX YY YZ ZX ZY ZZ DD
 
 // The six spin permutations (X,Y,Z) (X,Z,Y) (Y,X,Z) (Y,Z,X) (Z,X,Y) (Z,Y,X): 2 bits per image
@@ -69,10 +72,14 @@ struct TriArgs {
     // slot_base[l], ... and site j sums slots seg_ptr[j] .. seg_ptr[j + 1] - 1
     const int *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr;
     int rpa_n_seg;
+    // the same pairs for the lattice sum on the tensor cores (tri_lattice_kernel): words of the inner
+    // components (k2, k1) and site j at prod_words[4 prod_ptr[(4 k2 + k1) nl + j]] ..; the CTAs' operand scratch
+    const int *prod_ptr, *prod_words;
+    unsigned char *prod_scratch;
     const int *range_rid, *range_inv;
     const float *node_wp, *node_c;
     const int *node_cnt;
-    int *work_counter;
+    int *work_counter;  // two: the vertex-flow kernel's and tri_lattice_kernel's
     unsigned *status;
     const int *corr_rid, *corr_perm;
     double *partial;  // [kMaxCorrNodes][16][nl]
@@ -652,6 +659,546 @@ __global__ void __launch_bounds__(kThreads) tri_vertex_kernel(TriArgs a) {
 }
 
 // ------------------------------------------------------------------------------------
+// Lattices of at most 32 sites: a CTA per triple, whose warps take the nodes of all channels; lane = site
+// (8 or 16 lanes a node where they hold the sites, so a warp takes several nodes at once).
+//
+// A lane gathers its own site's components straight into registers and keeps its sums there.  Above 32 sites the
+// slabs go through shared memory with a warp per triple (tri_vertex_kernel); here that took 31.5 ms (28 sites,
+// N = 32, cutoff 0.5): 64 stores and loads a node and site, four triples' serial node chains at a time on small meshes.
+// ------------------------------------------------------------------------------------
+constexpr int kGoffRow = 20;  // gather offsets of a site: 16, rows 16 bytes aligned and in distinct banks
+constexpr int kCoefRow = 260;  // chalice coefficients of a node: 256
+
+__host__ __device__ inline int site_lanes(int nl) { return nl <= 8 ? 8 : (nl <= 16 ? 16 : 32); }
+
+// The 16 components of a slab at site j (gather_slab for one site).
+__device__ __forceinline__ void gather_site(const float *__restrict__ v4, const TAB4 &ab, const int *goff, int nl, int j, float (&x)[16]) {
+    const int fl = ab.fl;
+    const bool ex = fl & kFlExch, tu = fl & kFlTu;
+    float sw[4][4];  // [class: bit 0 a is a spin component, bit 1 b is][support]
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float za = (k & 1) ? -1.0f : 1.0f, zb = (k & 2) ? -1.0f : 1.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float sg = tu ? za * zb : 1.0f;
+            if ((fl >> i) & 1) sg *= -(ex ? za : zb);
+            sw[k][i] = sg * ab.w[i];
+        }
+    }
+    const int4 *g = reinterpret_cast<const int4 *>(goff + ((ex ? nl : 0) + j) * kGoffRow);
+    const float *p[4] = {v4 + ab.off[0], v4 + ab.off[1], v4 + ab.off[2], v4 + ab.off[3]};
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const int4 o4 = g[a];
+        const int o[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int k = (a < 3 ? 1 : 0) | (b < 3 ? 2 : 0);
+            float v = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v += sw[k][i] * ro_load(p[i] + o[b]);
+            x[4 * a + b] = v;
+        }
+    }
+}
+
+__device__ __forceinline__ void site_offsets(const TriArgs &a, int *goff) {
+    for (int i = threadIdx.x; i < 32 * a.nl; i += blockDim.x) {
+        const int e = i / (16 * a.nl), j = (i >> 4) % a.nl, c = i & 15;
+        const int r = e ? a.inv_sites[j] : a.sites[j], p = e ? a.inv_sites_perm[j] : a.sites_perm[j];
+        goff[(e * a.nl + j) * kGoffRow + c] = gather_offset(e, c, a.nl, r, p);
+    }
+}
+
+// The two ladders for one site (as ladder): X holds slabs (0, 2), Y slabs (1, 3), so a packed product takes both
+// slab pairs; terms of either sign are summed apart.  Adds cw times the result to acc.
+template <bool PH>
+__device__ __forceinline__ void site_ladder(const float2 (&X)[16], const float2 (&Y)[16], float cw, float (&acc)[16]) {
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+        float2 vp = make_float2(0.0f, 0.0f), vn = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int n = 0; n < 16; ++n) {
+            const int x = 15 - n, y = x ^ c ^ 15;
+            if ((PH ? tri::ph_sign(c, x) : tri::pp_sign(c, x)) > 0) vp = fma2(X[x], Y[y], vp);
+            else vn = fma2(X[x], Y[y], vn);
+        }
+        acc[c] += cw * ((vp.x + vp.y) - (vn.x + vn.y));
+    }
+}
+
+// The chalice diagrams are linear in a slab's components with coefficients that are sums of four
+// site-local values each, the same for all sites: slab q's coefficient of output c and component k is word
+// 64 q + 4 c + k, the indices of the four among the slab's 16 (4 bits) with their signs.
+__device__ __forceinline__ void chalice_words(int *words) {
+    for (int e = threadIdx.x; e < 256; e += blockDim.x) {
+        const int q = e >> 6, c = (e >> 2) & 15, k = e & 3;
+        int w = 0;
+        for (int i = 0; i < 4; ++i) {
+            const int l = (q & 1) ? 4 * i + (i ^ (c >> 2) ^ k) : 4 * i + ((c & 3) ^ k ^ i);
+            const int sg = (q & 1) ? tri::ichal_sign(c, l) : tri::chal_sign(c, k, i);
+            w |= (l | (sg < 0 ? 16 : 0)) << (5 * i);
+        }
+        words[e] = w;
+    }
+}
+// Site-local value e of a node (tri_local): those of slab q are 16 ((q & 1) 2 + (q >> 1)) .. + 15.
+__device__ __forceinline__ float local_value(const TriArgs &a, const TDesc &d, int e) {
+    return tri_local(a.v4, a.nl, d.ab[4 + (e >> 4)], (e & 15) >> 2, e & 3);
+}
+__device__ __forceinline__ int local_first(int q) { return ((q & 1) << 5) | ((q >> 1) << 4); }
+// A chalice coefficient from its slab's 16 site-local values.
+__device__ __forceinline__ float chalice_coef(const float *L, int w) {
+    float v = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = w >> (5 * i);
+        v += __int_as_float(__float_as_int(L[t & 15]) ^ ((t & 16) << 27));
+    }
+    return v;
+}
+// Adds a slab's chalice terms of one site to v: chalice (slabs 0, 2) over the second component, inverse (1, 3) over the
+// first.
+template <bool INVERSE>
+__device__ __forceinline__ void chalice_terms(const float (&x)[16], const float *coef, float (&v)[16]) {
+    const float4 *C = reinterpret_cast<const float4 *>(coef);
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+        const float4 k = C[c];
+        const int m = c >> 2, n = c & 3;
+        if (INVERSE) v[c] += x[n] * k.x + x[4 + n] * k.y + x[8 + n] * k.z + x[12 + n] * k.w;
+        else v[c] += x[4 * m] * k.x + x[4 * m + 1] * k.y + x[4 * m + 2] * k.z + x[4 * m + 3] * k.w;
+    }
+}
+
+// index triple of flow element `it`
+__device__ __forceinline__ void decode_triple(int it, int n, int &si, int &ti, int &ui) {
+    const int su = it / n;
+    ti = it - su * n;
+    si = int((sqrtf(8.0f * float(su) + 1.0f) - 1.0f) * 0.5f);
+    while (si * (si + 1) / 2 > su) --si;
+    while ((si + 1) * (si + 2) / 2 <= su) ++si;
+    ui = su - si * (si + 1) / 2;
+}
+
+// shared memory, in floats: head (gather offsets, chalice words, the warps' sums) and a warp's area
+__host__ __device__ inline size_t site_head_floats(int nl) { return 2 * size_t(nl) * kGoffRow + 256 + size_t(kWarps) * 512; }
+__host__ __device__ inline size_t site_warp_floats(int nl, int n_seg, bool walk) {
+    const size_t g = 32 / site_lanes(nl);
+    return kSiteBatch * (sizeof(TDesc) / sizeof(float)) + (walk ? g * (64 + kCoefRow + 64 * size_t(nl) + 16 * size_t(n_seg)) : 0);
+}
+
+// WALK: the t channel too, with the RPA pairs walked for every node; otherwise tri_lattice_kernel adds the t channel.
+template <bool WALK>
+__global__ void __launch_bounds__(kThreads, 4) tri_site_kernel(TriArgs a) {
+    __shared__ float pos[kMaxFreq];
+    __shared__ int s_item;
+    extern __shared__ __align__(16) float tsm[];
+    const int n = a.n, nl = a.nl, W = site_lanes(nl), G = 32 / W, n_seg = WALK ? a.rpa_n_seg : 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / W, jl = lane - sub * W, j = min(jl, nl - 1);
+    int *goff = reinterpret_cast<int *>(tsm), *words = goff + 2 * nl * kGoffRow;
+    float *red = reinterpret_cast<float *>(words + 256);
+    float *area = red + kWarps * 512 + warp * site_warp_floats(nl, n_seg, WALK);
+    TDesc *desc = reinterpret_cast<TDesc *>(area);
+    float *coef = area + kSiteBatch * (sizeof(TDesc) / sizeof(float));  // [G][kCoefRow]
+    float *L = coef + G * kCoefRow, *S = L + G * 64, *slots = S + G * 64 * nl;  // [G] of each
+    for (int i = threadIdx.x; i < n; i += blockDim.x) pos[i] = a.freq[i];
+    site_offsets(a, goff);
+    if (WALK) chalice_words(words);
+    const int rpa_cnt = WALK ? a.rpa_count[lane] : 0, rpa_base = WALK ? a.rpa_slot_base[lane] : 0;
+    const float two_pi = 2.0f * float(kPiD);
+
+    for (;;) {
+        __syncthreads();  // the previous triple's sums are read
+        if (threadIdx.x == 0) s_item = atomicAdd(a.work_counter, 1);
+        __syncthreads();
+        const int it = s_item;
+        if (it >= a.fn) break;
+        int si, ti, ui;
+        decode_triple(it, n, si, ti, ui);
+        const float s = pos[si], t = pos[ti], u = pos[ui];
+        const float w1p = 0.5f * (s + t + u), w1 = 0.5f * (s - t + u), w2p = 0.5f * (s - t - u), w2 = 0.5f * (s + t - u);
+        float acc[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) acc[c] = 0.0f;
+#pragma unroll 1
+        for (int ch = 0; ch < 3; ch += WALK ? 1 : 2) {
+            const int xi = ch == 0 ? si : (ch == 1 ? ti : ui);
+            const int mine = (a.node_cnt[xi] - warp + kWarps - 1) / kWarps;  // nodes warp, warp + kWarps, ...
+            const float *nwp = a.node_wp + size_t(xi) * a.max_nodes + warp, *nc = a.node_c + size_t(xi) * a.max_nodes + warp;
+#pragma unroll 1
+            for (int b0 = 0; b0 < mine; b0 += kSiteBatch) {
+                const int nb = min(kSiteBatch, mine - b0);
+                if ((lane >> 2) < nb) {  // a quad of lanes per node
+                    const int k = lane >> 2;
+                    make_tpart(a, pos, ch, xi, s, t, u, w1p, w1, w2p, w2, nwp[kWarps * (b0 + k)], lane & 3, desc[k]);
+                    if ((lane & 3) == 0) desc[k].c = nc[kWarps * (b0 + k)];
+                }
+                __syncwarp();
+#pragma unroll 1
+                for (int b = 0; b < nb; b += G) {
+                    const bool active = b + sub < nb;
+                    const TDesc &d = desc[active ? b + sub : b];
+                    if (!WALK || ch != 1) {
+                        float2 X[16], Y[16];
+                        {
+                            float x0[16], x1[16];
+                            gather_site(a.v4, d.ab[0], goff, nl, j, x0);
+                            gather_site(a.v4, d.ab[2], goff, nl, j, x1);
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) X[c] = make_float2(x0[c], x1[c]);
+                            gather_site(a.v4, d.ab[1], goff, nl, j, x0);
+                            gather_site(a.v4, d.ab[3], goff, nl, j, x1);
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) Y[c] = make_float2(x0[c], x1[c]);
+                        }
+                        if (active) {
+                            if (ch == 0) site_ladder<false>(X, Y, d.c, acc);
+                            else site_ladder<true>(X, Y, d.c, acc);
+                        }
+                    } else {
+                        float *Sn = S + sub * 64 * nl, *Ln = L + sub * 64, *Cn = coef + sub * kCoefRow;
+#pragma unroll 1
+                        for (int q = 0; q < 4; ++q) {
+                            float x[16];
+                            gather_site(a.v4, d.ab[q], goff, nl, j, x);
+                            if (jl < nl)
+#pragma unroll
+                                for (int c = 0; c < 16; ++c) Sn[(16 * q + c) * nl + jl] = x[c];
+                        }
+                        for (int e = jl; e < 64; e += W) Ln[e] = local_value(a, d, e);
+                        __syncwarp();
+                        for (int e = jl; e < 256; e += W) Cn[e] = chalice_coef(Ln + local_first(e >> 6), words[e]);
+                        for (int g = 0; g < min(G, nb - b); ++g)
+                            rpa_walk(a, S + g * 64 * nl, nl, lane, rpa_cnt, rpa_base, slots + g * 16 * n_seg);
+                        __syncwarp();
+                        if (active) {
+                            float v[16], x[16];
+                            const float *sl = slots + sub * 16 * n_seg;
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) v[c] = 0.0f;
+                            for (int q = a.rpa_seg_ptr[j]; q < a.rpa_seg_ptr[j + 1]; ++q)  // the site's run partials, in order
+#pragma unroll
+                                for (int c = 0; c < 16; ++c) v[c] += sl[16 * q + c];
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) v[c] *= 2.0f;
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) x[c] = Sn[c * nl + j];
+                            chalice_terms<false>(x, Cn, v);
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) x[c] = Sn[(16 + c) * nl + j];
+                            chalice_terms<true>(x, Cn + 64, v);
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) x[c] = Sn[(32 + c) * nl + j];
+                            chalice_terms<false>(x, Cn + 128, v);
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) x[c] = Sn[(48 + c) * nl + j];
+                            chalice_terms<true>(x, Cn + 192, v);
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) acc[c] += d.c * v[c];
+                        }
+                        __syncwarp();
+                    }
+                }
+                __syncwarp();
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 16; ++c) red[warp * 512 + c * 32 + lane] = acc[c];
+        __syncthreads();
+        float *dst = a.dv4 + size_t(it) * 16 * nl;
+        bool bad = false;
+        for (int e = threadIdx.x; e < 16 * nl; e += kThreads) {
+            const int c = e / nl, k = e - c * nl;
+            float v = 0.0f;
+            for (int w = 0; w < kWarps; ++w)
+                for (int g = 0; g < G; ++g) v += red[w * 512 + c * 32 + g * W + k];
+            const float o = v / two_pi;
+            dst[e] = o;
+            bad |= isnan(o);
+        }
+        if (bad) atomicOr(a.status, kStatusNaN);
+    }
+}
+
+// ------------------------------------------------------------------------------------
+// The t channel with its lattice sum on the tensor cores (use_products).
+//
+// For output (mu, nu) of site j the sum over its pairs and the inner index k of
+//   sign(mu, nu, k) A[rid1][P1 mu, P1 k] B[rid2][P2 k, P2 nu]
+// is linear in the node's slab products, so per triple the kernel forms, for the inner components k1 = P1 k and
+// k2 = P2 k that pairs have (10 of 16 at most: the density maps to itself),
+//   M = sum over nodes of c S0 x S1 + c S2 x S3      (4 Nl rows (rid1, P1 mu) x 4 Nl columns (rid2, P2 nu))
+// as a matrix product over K = 2 x nodes, and adds each pair's elements of M once per triple, where the walk
+// adds 128 products for every pair and node.
+//
+// A CTA takes a triple.  Its 16 worker warps gather the nodes' slabs, a slab at a time, add the chalice terms and leave
+// the slabs as operands (three bf16 terms of each FP32 value, umma.cuh) in a scratch that stays in L2.  Then one
+// thread copies the operands of every (k2, k1) to shared memory and issues the products, two chunks of K and two
+// accumulators ahead of the workers, which stage M in shared memory and add their outputs' elements.
+// ------------------------------------------------------------------------------------
+constexpr int kLatMinSites = 20;
+constexpr int kLatWarps = 16, kLatWorkers = 32 * kLatWarps, kLatThreads = kLatWorkers + 32;
+constexpr int kLatK = 48;        // slab pairs of a product
+constexpr int kLatNodes = kLatWorkers / 4;  // nodes whose descriptors are built at once (a quad of threads each)
+constexpr uint32_t kLatCols = 512;  // tensor memory: accumulator b's high products at column 256 b, low ones 128 on
+
+__host__ __device__ inline int lat_rows(int nl) { return (4 * nl + 15) / 16 * 16; }
+__host__ __device__ inline int lat_stride(int nl) { return lat_rows(nl) + 1; }  // of the staged M: an odd row stride
+// scratch of a CTA: [A of k1 = 0 .. 3, B of k2 = 0 .. 3][term][k / 8][row / 8][8 k][8 rows] bf16
+__host__ __device__ inline int lat_blocks(int max_nodes) { return (2 * max_nodes + 15) / 16 * 2; }
+__host__ __device__ inline size_t lat_scratch_bytes(int nl, int max_nodes) { return 24 * size_t(lat_blocks(max_nodes)) * lat_rows(nl) * 16; }
+
+struct LatSmem {
+    size_t words, u, locals, coef, stage, total;
+};
+__host__ __device__ inline LatSmem lat_smem(int nl) {
+    LatSmem L;
+    L.words = sizeof(int) * 2 * size_t(nl) * kGoffRow;
+    L.u = (L.words + sizeof(int) * 256 + 127) / 128 * 128;
+    // union: the nodes' descriptors and the warps' local values and coefficients, or two chunks of operands
+    L.locals = L.u + sizeof(TDesc) * kLatNodes;
+    L.coef = L.locals + sizeof(float) * 16 * kLatWarps;
+    const size_t g = L.coef + sizeof(float) * 64 * kLatWarps, m = L.u + 2 * 6 * size_t(lat_rows(nl)) * kLatK * 2;
+    L.stage = ((g > m ? g : m) + 127) / 128 * 128;
+    // union: the warps' sums, or M and a zero
+    const size_t red = sizeof(float) * 512 * kLatWarps, st = sizeof(float) * (lat_rows(nl) * size_t(lat_stride(nl)) + 1);
+    L.total = L.stage + (red > st ? red : st);
+    return L;
+}
+
+__device__ __forceinline__ void worker_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kLatWorkers) : "memory"); }
+
+// Stores the lane's rows 4 lane .. 4 lane + 3 of slab pair k, four operands of three terms: x[operand][row].
+__device__ __forceinline__ void lat_store(unsigned char *dst, int blocks, int rows, int k, int lane, const float (&x)[4][4]) {
+    unsigned char *p = dst + size_t(k >> 3) * rows * 16 + (lane >> 1) * 128 + (k & 7) * 16 + (lane & 1) * 8;
+    const size_t term = size_t(blocks) * rows * 16;
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+        uint2 h, m, l;
+        umma::split2(x[o][0], x[o][1], h.x, m.x, l.x);
+        umma::split2(x[o][2], x[o][3], h.y, m.y, l.y);
+        *reinterpret_cast<uint2 *>(p + 3 * o * term) = h;
+        *reinterpret_cast<uint2 *>(p + (3 * o + 1) * term) = m;
+        *reinterpret_cast<uint2 *>(p + (3 * o + 2) * term) = l;
+    }
+}
+
+__global__ void __launch_bounds__(kLatThreads, 1) tri_lattice_kernel(TriArgs a) {
+    extern __shared__ __align__(128) unsigned char psm[];
+    __shared__ float pos[kMaxFreq];
+    __shared__ uint64_t full[2], empty[2], done[2], drained[2];  // operands there / read, accumulator complete / read
+    __shared__ uint32_t tmem_slot;
+    __shared__ int s_item, s_combos[16], s_ncombo;
+    __shared__ int s_dead, s_late;  // a wait ran out: the copying thread's, a worker's
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n = a.n, nl = a.nl, rows = lat_rows(nl), stride = lat_stride(nl), blocks = lat_blocks(a.max_nodes);
+    const LatSmem L = lat_smem(nl);
+    int *goff = reinterpret_cast<int *>(psm), *words = reinterpret_cast<int *>(psm + L.words);
+    TDesc *desc = reinterpret_cast<TDesc *>(psm + L.u);
+    float *stage = reinterpret_cast<float *>(psm + L.stage), *red = stage;
+    unsigned char *scratch = a.prod_scratch + lat_scratch_bytes(nl, a.max_nodes) * blockIdx.x;
+    const size_t operand = size_t(blocks) * rows * 16;  // scratch bytes of an operand's term
+    for (int i = tid; i < n; i += kLatThreads) pos[i] = a.freq[i];
+    site_offsets(a, goff);
+    chalice_words(words);
+    if (warp == 0) umma::tmem_alloc(&tmem_slot, kLatCols);
+    if (tid == 0) {
+        for (int b = 0; b < 2; ++b) {
+            umma::bar_init(full + b);
+            umma::bar_init(empty + b);
+            umma::bar_init(done + b);
+            umma::bar_init(drained + b, kLatWarps);
+        }
+        s_dead = s_late = 0;
+        s_ncombo = 0;
+        for (int cb = 0; cb < 16; ++cb)
+            if (a.prod_ptr[cb * nl] != a.prod_ptr[(cb + 1) * nl]) s_combos[s_ncombo++] = cb;
+    }
+    umma::fence_before();
+    __syncthreads();
+    umma::fence_after();
+    const uint32_t tmem = tmem_slot;
+    const float two_pi = 2.0f * float(kPiD);
+    const int combos = s_ncombo;
+    const int j = tid >> 4, mu = (tid >> 2) & 3, nu = tid & 3;  // a worker's output
+    uint32_t chunk_no = 0, combo_no = 0;  // products and accumulators so far: their barriers' phases
+
+    while (!s_dead && !s_late) {
+        __syncthreads();  // the previous triple is finished with shared memory
+        if (tid == 0) s_item = atomicAdd(a.work_counter + 1, 1);
+        __syncthreads();
+        const int it = s_item;
+        if (it >= a.fn) break;
+        int si, ti, ui;
+        decode_triple(it, n, si, ti, ui);
+        const int cnt = a.node_cnt[ti], kn = (2 * cnt + 15) / 16 * 16, chunks = (kn + kLatK - 1) / kLatK;
+
+        if (warp < kLatWarps) {
+            const float s = pos[si], t = pos[ti], u = pos[ui];
+            const float w1p = 0.5f * (s + t + u), w1 = 0.5f * (s - t + u), w2p = 0.5f * (s - t - u), w2 = 0.5f * (s + t - u);
+            const float *nwp = a.node_wp + size_t(ti) * a.max_nodes, *nc = a.node_c + size_t(ti) * a.max_nodes;
+            float *Ln = reinterpret_cast<float *>(psm + L.locals) + warp * 16, *coef = reinterpret_cast<float *>(psm + L.coef) + warp * 64;
+            float acc[16];
+#pragma unroll
+            for (int c = 0; c < 16; ++c) acc[c] = 0.0f;
+#pragma unroll 1
+            for (int b0 = 0; b0 < cnt; b0 += kLatNodes) {
+                const int nb = min(kLatNodes, cnt - b0);
+                if (b0) worker_sync();  // the previous batch's descriptors are read
+                if ((tid >> 2) < nb) {
+                    const int k = tid >> 2;
+                    make_tpart(a, pos, 1, ti, s, t, u, w1p, w1, w2p, w2, nwp[b0 + k], tid & 3, desc[k]);
+                    if ((tid & 3) == 0) desc[k].c = nc[b0 + k];
+                }
+                worker_sync();
+#pragma unroll 1
+                for (int task = warp; task < 4 * nb; task += kLatWarps) {  // slab q of a node
+                    const int q = task & 3;
+                    const TDesc &d = desc[task >> 2];
+                    float x[16], v[16], y[4][4];
+                    gather_site(a.v4, d.ab[q], goff, nl, min(lane, nl - 1), x);
+                    if (lane < 16) Ln[lane] = local_value(a, d, local_first(q) + lane);
+                    __syncwarp();
+                    coef[lane] = chalice_coef(Ln, words[64 * q + lane]);
+                    coef[lane + 32] = chalice_coef(Ln, words[64 * q + 32 + lane]);
+                    __syncwarp();
+                    const float c1 = d.c;
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) v[c] = 0.0f;
+                    if (q & 1) {
+                        chalice_terms<true>(x, coef, v);
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) y[c >> 2][c & 3] = x[c];  // operand k, row nu
+                    } else {
+                        chalice_terms<false>(x, coef, v);
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) y[c & 3][c >> 2] = c1 * x[c];  // operand k, row mu
+                    }
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) acc[c] += c1 * v[c];
+                    if (lane < nl) lat_store(scratch + (q & 1) * 12 * operand, blocks, rows, 2 * (b0 + (task >> 2)) + (q >> 1), lane, y);
+                }
+            }
+            for (int task = warp + 4 * cnt; task < 2 * kn; task += kLatWarps) {  // zero up to a multiple of 16
+                const float y[4][4] = {};
+                if (lane < nl) lat_store(scratch + (task & 1) * 12 * operand, blocks, rows, task >> 1, lane, y);
+            }
+#pragma unroll
+            for (int c = 0; c < 16; ++c) red[warp * 512 + c * 32 + lane] = acc[c];
+            umma::fence_copies();
+        }
+        __syncthreads();
+
+        if (warp == kLatWarps) {
+            if (lane == 0 && chunks > 0) {
+                bool ok = true;
+                const int total = combos * chunks;
+                auto load = [&](int g) {
+                    const uint32_t b = (chunk_no + g) & 1, seq = (chunk_no + g) >> 1;
+                    if (seq) ok = ok && umma::bar_wait(empty + b, (seq - 1) & 1);
+                    if (!ok) return;
+                    const int cb = s_combos[g / chunks], k0 = g % chunks * kLatK;
+                    const uint32_t bytes = min(kLatK, kn - k0) * rows * 2, term = rows * kLatK * 2;
+                    const uint32_t dst = umma::smem_addr(psm + L.u) + b * 6 * term;
+                    const unsigned char *A = scratch + 3 * (cb & 3) * operand + size_t(k0) * rows * 2;
+                    const unsigned char *B = scratch + (12 + 3 * (cb >> 2)) * operand + size_t(k0) * rows * 2;
+                    umma::bar_expect(full + b, 6 * bytes);
+                    for (int t = 0; t < 3; ++t) {
+                        umma::bulk_load(dst + t * term, A + t * operand, bytes, full + b);
+                        umma::bulk_load(dst + (3 + t) * term, B + t * operand, bytes, full + b);
+                    }
+                };
+                if (total) load(0);
+                for (int g = 0; g < total && ok; ++g) {
+                    if (g + 1 < total) load(g + 1);
+                    const uint32_t b = (chunk_no + g) & 1, ci = combo_no + g / chunks, k0 = g % chunks * kLatK;
+                    const uint32_t d = tmem + 256 * (ci & 1), term = rows * kLatK * 2;
+                    if (k0 == 0 && ci >= 2) ok = ok && umma::bar_wait(drained + (ci & 1), ((ci >> 1) - 1) & 1);
+                    ok = ok && umma::bar_wait(full + b, ((chunk_no + g) >> 1) & 1);
+                    if (!ok) break;
+                    umma::fence_after();
+                    const uint32_t o = umma::smem_addr(psm + L.u) + b * 6 * term;
+                    umma::product<true>(d, d + 128, o, rows, term, o + 3 * term, rows, term, rows, min(kLatK, kn - int(k0)) / 16, k0 > 0);
+                    umma::commit(empty + b);
+                    if (g % chunks == chunks - 1) umma::commit(done + (ci & 1));
+                }
+                if (!ok) s_dead = 1;
+            }
+            __syncwarp();
+        } else {
+            float sum = 0.0f, rpa = 0.0f;
+            if (j < nl)
+                for (int w = 0; w < kLatWarps; ++w) sum += red[w * 512 + (tid & 15) * 32 + j];
+            worker_sync();  // M takes the place of the sums
+            if (tid == 0) stage[rows * stride] = 0.0f;  // for the padding words
+            for (int i = 0; i < combos && chunks > 0; ++i) {
+                const uint32_t ci = combo_no + i, b = ci & 1;
+                const int cb = s_combos[i];
+                int w0 = 0, w1 = 0;
+                if (j < nl) {
+                    w0 = __ldg(a.prod_ptr + cb * nl + j);
+                    w1 = __ldg(a.prod_ptr + cb * nl + j + 1);
+                }
+                if (!umma::bar_wait(done + b, (ci >> 1) & 1)) s_late = 1;
+                umma::fence_after();
+                const int row = (warp & 3) * 32 + lane;
+                for (int c0 = (warp >> 2) * 16; c0 < rows; c0 += 64) {
+                    float hi[16], lo[16];
+                    const uint32_t addr = tmem + 256 * b + (uint32_t(warp & 3) << 21) + c0;
+                    umma::load16(addr, hi);
+                    umma::load16(addr + 128, lo);
+                    umma::load_wait();
+                    if (row < rows)
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) stage[row * stride + c0 + k] = hi[k] + lo[k];
+                }
+                umma::fence_before();
+                __syncwarp();
+                if (lane == 0) umma::bar_arrive(drained + b);
+                worker_sync();
+                if (s_late) break;  // the workers write it before this barrier alone, so they agree
+                float p0 = 0.0f, p1 = 0.0f;
+                const int4 *list = reinterpret_cast<const int4 *>(a.prod_words);
+                auto element = [&](int w) {
+                    return stage[(w & 0x7fff) + ((w >> (15 + 2 * mu)) & 3) * stride + ((unsigned(w) >> (23 + 2 * nu)) & 3)];
+                };
+#pragma unroll 4
+                for (int e = w0; e < w1; ++e) {
+                    const int4 w = __ldg(list + e);
+                    p0 += element(w.x) + element(w.y);
+                    p1 += element(w.z) + element(w.w);
+                }
+                // tri::rpa_sign: the inner index is the density for k1 = 3 alone
+                const float part = p0 + p1;
+                rpa += (mu == 3) == (nu == 3) && ((cb & 3) == 3) != (mu == 3) ? -part : part;
+                worker_sync();  // M is read
+            }
+            if (j < nl) {
+                float *p = a.dv4 + size_t(it) * 16 * nl + (tid & 15) * nl + j;
+                const float o = *p + (sum + 2.0f * rpa) / two_pi;
+                *p = o;
+                if (isnan(o)) atomicOr(a.status, kStatusNaN);
+            }
+        }
+        chunk_no += combos * chunks;
+        if (chunks > 0) combo_no += combos;
+        __syncthreads();  // s_dead, s_late
+    }
+    if (s_dead || s_late) {  // a copy or a product did not complete in time: report it, and give them a last chance before the memory goes
+        if (tid == 0) atomicOr(a.status, kStatusProductTimeout);
+        if (tid < 2) umma::bar_wait(full + tid, 0) && umma::bar_wait(done + tid, 0);
+    }
+    umma::fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        umma::fence_after();
+        umma::tmem_free(tmem, kLatCols);
+    }
+}
+
+// ------------------------------------------------------------------------------------
 // correlation measurement at nu = 0 (TRIMeasurementCorrelation.cpp:147-285): one CTA per
 // outer node accumulates the inner integral per site and component in FP64, a final CTA adds
 // the outer weights and the on-site term and scatters to (basis, site in range) entries.
@@ -779,10 +1326,6 @@ using cuh::copy_grid;
 using cuh::dalloc;
 using cuh::h2d;
 
-size_t vertex_smem(int nl, int n_seg) {
-    return (tri_cta_head_floats(nl) + size_t(kWarps) * tri_warp_floats(nl, n_seg)) * sizeof(float);
-}
-
 }  // namespace
 
 struct spn_tri {
@@ -794,8 +1337,9 @@ struct spn_tri {
           *node_c = nullptr, *corr_out = nullptr;
     int *ints = nullptr;  // all integer tables in one allocation
     int *sites, *sites_perm, *inv_sites, *inv_sites_perm, *range_rid, *range_inv, *corr_rid,
-        *corr_perm, *node_cnt, *work_counter, *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr;
+        *corr_perm, *node_cnt, *work_counter, *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr, *prod_ptr, *prod_words;
     int rpa_n_seg = 0;
+    unsigned char *prod_scratch = nullptr;  // tri_lattice_kernel runs when not NULL
     unsigned *status = nullptr;
     double *partial = nullptr;
 
@@ -824,6 +1368,9 @@ struct spn_tri {
         a.rpa_slot_base = rpa_slot_base;
         a.rpa_seg_ptr = rpa_seg_ptr;
         a.rpa_n_seg = rpa_n_seg;
+        a.prod_ptr = prod_ptr;
+        a.prod_words = prod_words;
+        a.prod_scratch = prod_scratch;
         a.range_rid = range_rid;
         a.range_inv = range_inv;
         a.node_wp = node_wp;
@@ -859,7 +1406,7 @@ struct spn_tri {
 
     void release() {
         cudaSetDevice(device);
-        void *ptrs[] = {freq, v2, dv2, v4, dv4, node_wp, node_c, corr_out, ints, status, partial};
+        void *ptrs[] = {freq, v2, dv2, v4, dv4, node_wp, node_c, corr_out, ints, status, partial, prod_scratch};
         for (void *p : ptrs)
             if (p) cudaFree(p);
         if (stream) cudaStreamDestroy(stream);
@@ -906,6 +1453,41 @@ void validate(const spn_tri_desc *d) {
     in_range(d->range_inv_rid, d->n_range, nl, "range_inv_rid");
     in_range(d->corr_rid, d->n_corr, nl, "corr_rid");
     in_range(d->corr_perm, d->n_corr, 6, "corr_perm");
+}
+
+size_t vertex_smem(const spn_tri *h) {
+    const int nl = h->nl, n_seg = h->rpa_n_seg;
+    if (nl > 32) return (tri_cta_head_floats(nl) + size_t(kWarps) * tri_warp_floats(nl, n_seg)) * sizeof(float);
+    return (site_head_floats(nl) + size_t(kWarps) * site_warp_floats(nl, n_seg, !h->prod_scratch)) * sizeof(float);
+}
+void (*vertex_kernel(const spn_tri *h))(TriArgs) {
+    return h->nl > 32 ? tri_vertex_kernel : (h->prod_scratch ? tri_site_kernel<false> : tri_site_kernel<true>);
+}
+
+// Whether the t channel runs on the tensor cores (tri_lattice_kernel).
+bool use_products(int nl) { return nl >= kLatMinSites && nl <= 32; }
+
+// The RPA pairs by inner components and site, as tri_lattice_kernel reads them, four words at a time: the element of the
+// staged M (15 bits) and the images of the four components under perm1 and perm2 (2 bits each).  The last
+// four of a site are filled up with words of the zero behind M.
+void product_pairs(const spn_tri_desc *d, std::vector<int> &ptr, std::vector<int> &words) {
+    const int nl = d->n_sites, stride = lat_stride(nl);
+    ptr.assign(1, 0);
+    for (int k2 = 0; k2 < 4; ++k2)
+        for (int k1 = 0; k1 < 4; ++k1)
+            for (int j = 0; j < nl; ++j) {
+                for (int i = d->overlap_ptr[j]; i < d->overlap_ptr[j + 1]; ++i) {
+                    const int p1 = d->overlap_perm1[i], p2 = d->overlap_perm2[i];
+                    for (int k = 0; k < 4; ++k) {
+                        if (permc(p1, k) != k1 || permc(p2, k) != k2) continue;
+                        unsigned w = 4 * d->overlap_rid1[i] * stride + 4 * d->overlap_rid2[i];
+                        for (int q = 0; q < 4; ++q) w |= unsigned(permc(p1, q)) << (15 + 2 * q) | unsigned(permc(p2, q)) << (23 + 2 * q);
+                        words.push_back(int(w));
+                    }
+                }
+                while (words.size() % 4) words.push_back(lat_rows(nl) * stride);
+                ptr.push_back(int(words.size() / 4));
+            }
 }
 
 // The RPA pairs of each site in the order of host/pair_order (against bank collisions of the
@@ -986,16 +1568,21 @@ extern "C" int spn_tri_create(const spn_tri_desc *d, spn_tri **out) {
             put(d->corr_rid, nc);
             put(d->corr_perm, nc);
             put(nullptr, h->n);  // node counts
-            put(nullptr, 1);     // work counter
+            put(nullptr, 2);     // work counters
             put(rpa.sched.data(), int(rpa.sched.size()));
             put(rpa.count.data(), 32);
             put(rpa.slot_base.data(), 32);
             put(rpa.seg_ptr.data(), nl + 1);
+            std::vector<int> prod_ptr, prod_words;
+            if (use_products(nl)) product_pairs(d, prod_ptr, prod_words);
+            put(prod_ptr.data(), int(prod_ptr.size()));
+            img.resize((img.size() + 3) / 4 * 4);  // read four words at a time
+            put(prod_words.data(), int(prod_words.size()));
             h->ints = dalloc<int>(img.size(), "alloc lattice tables");
             h2d(h->ints, img.data(), img.size(), h->stream);
             int **fields[] = {&h->sites, &h->sites_perm, &h->inv_sites, &h->inv_sites_perm,
                               &h->range_rid, &h->range_inv, &h->corr_rid, &h->corr_perm, &h->node_cnt, &h->work_counter,
-                              &h->rpa_sched, &h->rpa_count, &h->rpa_slot_base, &h->rpa_seg_ptr};
+                              &h->rpa_sched, &h->rpa_count, &h->rpa_slot_base, &h->rpa_seg_ptr, &h->prod_ptr, &h->prod_words};
             for (size_t k = 0; k < at.size(); ++k) *fields[k] = h->ints + at[k];
             h2d(h->freq, d->freq, h->n, h->stream);
             check_cuda(cudaMemsetAsync(h->v4, 0, vsz * sizeof(float), h->stream), "memset");
@@ -1004,12 +1591,19 @@ extern "C" int spn_tri_create(const spn_tri_desc *d, spn_tri **out) {
             check_cuda(cudaMemsetAsync(h->dv2, 0, h->n * sizeof(float), h->stream), "memset");
             check_cuda(cudaMemsetAsync(h->status, 0, sizeof(unsigned), h->stream), "memset");
             check_cuda(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device), "device attribute");
+            if (use_products(nl)) {
+                // without the memory for the scratch, or room for the kernel, the pairs are walked
+                void *p = nullptr;
+                if (cudaFuncSetAttribute(tri_lattice_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(lat_smem(nl).total)) ==
+                        cudaSuccess &&
+                    cudaMalloc(&p, lat_scratch_bytes(nl, h->max_nodes) * size_t(h->sms)) == cudaSuccess)
+                    h->prod_scratch = static_cast<unsigned char *>(p);
+                else cudaGetLastError();
+            }
             int per_sm = 0;
-            check_cuda(cudaFuncSetAttribute(tri_vertex_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            int(vertex_smem(h->nl, h->rpa_n_seg))),
-                       "shared memory limit");
-            check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tri_vertex_kernel, kThreads, vertex_smem(h->nl, h->rpa_n_seg)),
-                       "occupancy");
+            const auto fn = vertex_kernel(h);
+            check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(vertex_smem(h))), "shared memory limit");
+            check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, vertex_smem(h)), "occupancy");
             if (per_sm < 1) throw Error(ErrorType::Unsupported, "TRI vertex-flow kernel does not fit on this device");
             h->grid = h->sms * per_sm;
             check_cuda(cudaStreamSynchronize(h->stream), "create sync");
@@ -1071,15 +1665,21 @@ extern "C" int spn_tri_compute_step(spn_tri *h) {
         if (!h) throw Error(ErrorType::Argument, "null handle");
         check_cuda(cudaSetDevice(h->device), "cudaSetDevice");
         check_cuda(cudaMemsetAsync(h->status, 0, sizeof(unsigned), h->stream), "memset status");
-        check_cuda(cudaMemsetAsync(h->work_counter, 0, sizeof(int), h->stream), "memset counter");
+        check_cuda(cudaMemsetAsync(h->work_counter, 0, 2 * sizeof(int), h->stream), "memset counter");
         const TriArgs a = h->args();
         tri_self_energy_kernel<<<h->n, 128, 0, h->stream>>>(a);
         check_cuda(cudaGetLastError(), "self-energy launch");
         tri_node_table_kernel<<<h->n, kNodeThreads, 0, h->stream>>>(h->node_args());
         check_cuda(cudaGetLastError(), "node table launch");
-        check_cuda(cudaFuncSetAttribute(tri_vertex_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(vertex_smem(h->nl, h->rpa_n_seg))),
-                   "shared memory limit");
-        tri_vertex_kernel<<<h->grid, kThreads, vertex_smem(h->nl, h->rpa_n_seg), h->stream>>>(a);
+        const auto fn = vertex_kernel(h);
+        check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(vertex_smem(h))), "shared memory limit");
+        fn<<<h->grid, kThreads, vertex_smem(h), h->stream>>>(a);
+        if (h->prod_scratch) {
+            check_cuda(cudaGetLastError(), "vertex flow launch");
+            const size_t smem = lat_smem(h->nl).total;
+            check_cuda(cudaFuncSetAttribute(tri_lattice_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)), "shared memory limit");
+            tri_lattice_kernel<<<h->sms, kLatThreads, smem, h->stream>>>(a);
+        }
         check_cuda(cudaGetLastError(), "vertex flow launch");
     });
 }
@@ -1121,6 +1721,7 @@ extern "C" int spn_tri_is_diverged(spn_tri *h, int *diverged) {
         check_cuda(cudaMemcpyAsync(&st, h->status, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream), "D2H");
         check_cuda(cudaStreamSynchronize(h->stream), "status sync");
         if (st & kStatusNodeOverflow) throw Error(ErrorType::Device, "loop-frequency node table overflow");
+        if (st & kStatusProductTimeout) throw Error(ErrorType::Device, "a tensor-core product of the vertex flow did not complete");
         *diverged = (st & kStatusNaN) ? 1 : 0;
     });
 }

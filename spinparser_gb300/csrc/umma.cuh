@@ -1,0 +1,144 @@
+// Fifth-generation tensor core products with FP32 accumulators in tensor memory (sm_103a): one
+// 128 x N x 16 bf16 product per instruction, operands in shared memory without swizzle.
+//
+// FP32 operands enter as three bf16 terms, x = h + m + l (8 mantissa bits each, so all 24 bits of a
+// normal x), and a product as h h plus the five terms h m, m h, m m, h l, l h; what is left out is
+// below 2^-26 of the product.  h h and the small terms accumulate in separate accumulators, so the small
+// ones are not rounded away against the large sum.
+//
+// Operand layout of one term, in 128-byte blocks of 8 rows x 8 k: block (row / 8, k / 8) at
+// (k / 8) * rows * 16 + (row / 8) * 128 bytes, and in a block element (row, k) at 16 row + 2 k (k contiguous) or
+// 16 k + 2 row (rows contiguous).
+#pragma once
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <cstdint>
+
+namespace spn {
+namespace dev {
+namespace umma {
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p) { return uint32_t(__cvta_generic_to_shared(p)); }
+
+// Tensor memory: `cols` columns (a power of two >= 32) of 128 lanes; a whole warp calls these.
+__device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(slot)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+}
+__device__ __forceinline__ void tmem_free(uint32_t addr, uint32_t cols) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols));
+}
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// shared-memory writes of this thread become visible to the tensor core's reads
+__device__ __forceinline__ void fence_operands() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// generic-proxy accesses of this thread, to shared and global memory, come before later bulk copies
+__device__ __forceinline__ void fence_copies() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+__device__ __forceinline__ void bar_init(uint64_t *bar, uint32_t arrivals = 1) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(arrivals) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+__device__ __forceinline__ void bar_expect(uint64_t *bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+// Bulk copy from global memory (addresses and size multiples of 16 bytes).
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes),
+                 "r"(smem_addr(bar))
+                 : "memory");
+}
+// Waits for phase `parity` of the barrier; false after kWaitPolls polls.
+constexpr int kWaitPolls = 1 << 20;
+__device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity) {
+    for (int i = 0; i < kWaitPolls; ++i) {
+        uint32_t done;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n}"
+                     : "=r"(done)
+                     : "r"(smem_addr(bar)), "r"(parity)
+                     : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+// The barrier completes a phase when this thread's products so far are done.
+__device__ __forceinline__ void commit(uint64_t *bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+// Shared-memory descriptor of a term's operand: `rows` rows allocated, starting at its k = 0 (or a
+// multiple of 8).  Fields: start >> 4, distance of the two 8-k units >> 4, distance of 8-row groups >> 4, version 1.
+__device__ __forceinline__ uint64_t operand(uint32_t addr, uint32_t rows) {
+    return uint64_t((addr >> 4) & 0x3fff) | (uint64_t((rows * 16) >> 4) << 16) | (uint64_t(128 >> 4) << 32) | (uint64_t(1) << 46);
+}
+// bf16 operands, both with k or (ROWS) rows contiguous, FP32 accumulator, M = 128.
+template <bool ROWS>
+__device__ __forceinline__ uint32_t instruction(uint32_t n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (ROWS ? 3u << 15 : 0u) | ((n >> 3) << 17) | (8u << 24);
+}
+
+// D[128 x N] (+)= A B^T over 16 k; one thread issues it.
+__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t inst, bool accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d),
+                 "l"(a), "l"(b), "r"(inst), "r"(uint32_t(accumulate))
+                 : "memory");
+}
+
+// D_hi, D_lo (+)= the product of `steps` x 16 k of A (arows rows allocated) and B (brows): the terms' operands
+// follow each other, a_term and b_term bytes apart.
+template <bool ROWS>
+__device__ __forceinline__ void product(uint32_t d_hi, uint32_t d_lo, uint32_t a, uint32_t arows, uint32_t a_term, uint32_t b,
+                                        uint32_t brows, uint32_t b_term, uint32_t n, int steps, bool accumulate) {
+    const uint32_t inst = instruction<ROWS>(n);
+    for (int s = 0; s < steps; ++s) {
+        const uint32_t ao = a + s * 32 * arows, bo = b + s * 32 * brows;
+        mma(d_hi, operand(ao, arows), operand(bo, brows), inst, accumulate || s > 0);
+    }
+    constexpr int ta[5] = {0, 1, 1, 0, 2}, tb[5] = {1, 0, 1, 2, 0};
+#pragma unroll
+    for (int t = 0; t < 5; ++t)
+        for (int s = 0; s < steps; ++s) {
+            const uint32_t ao = a + ta[t] * a_term + s * 32 * arows, bo = b + tb[t] * b_term + s * 32 * brows;
+            mma(d_lo, operand(ao, arows), operand(bo, brows), inst, accumulate || t > 0 || s > 0);
+        }
+}
+
+// Four columns of this thread's lane (lane 32 (warp % 4) + lane id of the addressed rows).
+__device__ __forceinline__ void load4(uint32_t addr, float (&v)[4]) {
+    uint32_t r[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
+}
+// The same for 16 columns.
+__device__ __forceinline__ void load16(uint32_t addr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(addr));
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// The three bf16 terms of two values.  An infinite, NaN or overflowing value keeps its leading term alone.
+__device__ __forceinline__ void split2(float u, float v, uint32_t &h, uint32_t &m, uint32_t &l) {
+    const __nv_bfloat162 p = __floats2bfloat162_rn(u, v);
+    const float ru = fabsf(u) < 3.3e38f ? u - __low2float(p) : 0.0f, rv = fabsf(v) < 3.3e38f ? v - __high2float(p) : 0.0f;
+    const __nv_bfloat162 q = __floats2bfloat162_rn(ru, rv);
+    const __nv_bfloat162 s = __floats2bfloat162_rn(ru - __low2float(q), rv - __high2float(q));
+    h = *reinterpret_cast<const uint32_t *>(&p);
+    m = *reinterpret_cast<const uint32_t *>(&q);
+    l = *reinterpret_cast<const uint32_t *>(&s);
+}
+
+}  // namespace umma
+}  // namespace dev
+}  // namespace spn
