@@ -13,12 +13,9 @@
 // constants in the unrolled loops.
 //
 // A step: the self-energy flow (one CTA per frequency), the loop-frequency node tables (the
-// SU(2) core's, shared), the vertex flow and the Euler update.  The vertex-flow kernel runs a
-// persistent grid whose warps take one (s,t,u) triple at a time from a device counter.  Per
-// channel, nodes go in batches of 16: a lane first builds one node's access buffers into a
-// shared-memory descriptor; then, node by node, the warp gathers the four 16-component slabs
-// of all sites into shared memory (t: and the 64 site-local values of the chalice diagrams),
-// and each lane evaluates the products for its sites from registers.
+// SU(2) core's, shared), the vertex flow and the Euler update.  The vertex-flow kernels run persistent
+// grids that take (s,t,u) triples from a device counter: a CTA per triple (tri_site_kernel and, for the t channel,
+// tri_lattice_kernel) for at most 32 sites, a warp per triple above (tri_vertex_kernel).
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstring>
@@ -72,9 +69,10 @@ struct TriArgs {
     // slot_base[l], ... and site j sums slots seg_ptr[j] .. seg_ptr[j + 1] - 1
     const int *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr;
     int rpa_n_seg;
-    // the same pairs for the lattice sum on the tensor cores (tri_lattice_kernel): words of the inner
-    // components (k2, k1) and site j at prod_words[4 prod_ptr[(4 k2 + k1) nl + j]] ..; the CTAs' operand scratch
-    const int *prod_ptr, *prod_words;
+    // the same pairs for the lattice sum on the tensor cores (tri_lattice_kernel): site j's are dealt to groups
+    // prod_group[j] .. prod_group[j + 1] - 1; the words of the inner components (k2, k1) and group g at
+    // prod_words[2 prod_ptr[(4 k2 + k1) kLatGroups + g]] ..; the CTAs' operand scratch
+    const int *prod_ptr, *prod_words, *prod_group;
     unsigned char *prod_scratch;
     const int *range_rid, *range_inv;
     const float *node_wp, *node_c;
@@ -571,6 +569,10 @@ __host__ __device__ constexpr size_t tri_warp_floats(int nl, int n_seg) {
 // per CTA: the gather offsets goff[2][16][nl] (ints), then the warps' areas
 __host__ __device__ constexpr size_t tri_cta_head_floats(int nl) { return (32 * size_t(nl) + 3) / 4 * 4; }
 
+// Above 32 sites.  Per channel, nodes go in batches of four: a quad of lanes builds one node's access buffers into a
+// shared-memory descriptor; then, node by node, the warp gathers the four 16-component slabs of all sites into shared
+// memory (t: and the 64 site-local values of the chalice diagrams), and each lane evaluates the products for its sites from
+// registers.
 __global__ void __launch_bounds__(kThreads) tri_vertex_kernel(TriArgs a) {
     __shared__ float pos[kMaxFreq];
     // per CTA: gather offsets goff[2][16][nl]; per warp: slabs S[4][16][nl], accumulator
@@ -663,8 +665,9 @@ __global__ void __launch_bounds__(kThreads) tri_vertex_kernel(TriArgs a) {
 // (8 or 16 lanes a node where they hold the sites, so a warp takes several nodes at once).
 //
 // A lane gathers its own site's components straight into registers and keeps its sums there.  Above 32 sites the
-// slabs go through shared memory with a warp per triple (tri_vertex_kernel); here that took 31.5 ms (28 sites,
-// N = 32, cutoff 0.5): 64 stores and loads a node and site, four triples' serial node chains at a time on small meshes.
+// slabs go through shared memory with a warp per triple (tri_vertex_kernel): 64 stores and loads a node and site, and on a
+// small mesh a warp's nodes one after the other.  The ladders of 28 sites, N = 32 take 3.35 ms here, about 8 there; all of
+// 8 sites, N = 15 0.47 ms, 1.3 there.
 // ------------------------------------------------------------------------------------
 constexpr int kGoffRow = 20;  // gather offsets of a site: 16, rows 16 bytes aligned and in distinct banks
 constexpr int kCoefRow = 260;  // chalice coefficients of a node: 256
@@ -699,6 +702,48 @@ __device__ __forceinline__ void gather_site(const float *__restrict__ v4, const 
 #pragma unroll
             for (int i = 0; i < 4; ++i) v += sw[k][i] * ro_load(p[i] + o[b]);
             x[4 * a + b] = v;
+        }
+    }
+}
+
+// Slabs q and q + 2 of a t-channel node at site j.  Their coordinates are the same two magnitudes with s and u
+// exchanged, and a slab is stored for s >= u alone, so both interpolate the same four stored slabs (supports 1
+// and 2 trade places); their site exchanges differ only where a loop frequency cancels to zero.
+__device__ __forceinline__ void gather_site_pair(const float *__restrict__ v4, const TAB4 &ab, const TAB4 &cd, const int *goff, int nl, int j,
+                                                 float (&x)[16], float (&y)[16]) {
+    if ((ab.fl ^ cd.fl) & kFlExch) {
+        gather_site(v4, ab, goff, nl, j, x);
+        gather_site(v4, cd, goff, nl, j, y);
+        return;
+    }
+    const bool ex = ab.fl & kFlExch;
+    float sx[4][4], sy[4][4];  // as gather_site's
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float za = (k & 1) ? -1.0f : 1.0f, zb = (k & 2) ? -1.0f : 1.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float sg = (ab.fl & kFlTu) ? za * zb : 1.0f, sh = (cd.fl & kFlTu) ? za * zb : 1.0f;
+            if ((ab.fl >> i) & 1) sg *= -(ex ? za : zb);
+            if ((cd.fl >> i) & 1) sh *= -(ex ? za : zb);
+            sx[k][i] = sg * ab.w[i];
+            sy[k][i] = sh * cd.w[i];
+        }
+    }
+    const int4 *g = reinterpret_cast<const int4 *>(goff + ((ex ? nl : 0) + j) * kGoffRow);
+    const float *p[4] = {v4 + ab.off[0], v4 + ab.off[1], v4 + ab.off[2], v4 + ab.off[3]};
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const int4 o4 = g[a];
+        const int o[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int k = (a < 3 ? 1 : 0) | (b < 3 ? 2 : 0);
+            float r[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) r[i] = ro_load(p[i] + o[b]);
+            x[4 * a + b] = sx[k][0] * r[0] + sx[k][1] * r[1] + sx[k][2] * r[2] + sx[k][3] * r[3];
+            y[4 * a + b] = sy[k][0] * r[0] + sy[k][1] * r[2] + sy[k][2] * r[1] + sy[k][3] * r[3];
         }
     }
 }
@@ -933,47 +978,68 @@ __global__ void __launch_bounds__(kThreads, 4) tri_site_kernel(TriArgs a) {
 // as a matrix product over K = 2 x nodes, and adds each pair's elements of M once per triple, where the walk
 // adds 128 products for every pair and node.
 //
-// A CTA takes a triple.  Its 16 worker warps gather the nodes' slabs, a slab at a time, add the chalice terms and leave
+// A CTA takes a triple.  Its 14 worker warps gather the nodes' slabs, a slab at a time, add the chalice terms and leave
 // the slabs as operands (three bf16 terms of each FP32 value, umma.cuh) in a scratch that stays in L2.  Then one
-// thread copies the operands of every (k2, k1) to shared memory and issues the products, two chunks of K and two
-// accumulators ahead of the workers, which stage M in shared memory and add their outputs' elements.
+// thread copies the operands of every (k2, k1) to shared memory in chunks of 32 slab pairs, another issues the products, up
+// to two accumulators ahead of the workers, which stage M in shared memory and add their outputs' elements.
+//
+// 28 sites, N = 32, cutoff 0.5: 6.7 ms, where the walk took about 19 of the vertex flow's 31.5.  A triple takes 117,000
+// cycles: 47,000 gather and split the slabs (latency of the slab reads, sectors written), 29,000 add the pairs' elements, 20,000
+// are the products (62 cycles each, the reads of their operands), the rest is waiting between the stages.
 // ------------------------------------------------------------------------------------
-constexpr int kLatMinSites = 20;
-constexpr int kLatWarps = 16, kLatWorkers = 32 * kLatWarps, kLatThreads = kLatWorkers + 32;
-constexpr int kLatK = 48;        // slab pairs of a product
+// From here on the products pay (honeycomb, N = 24, cutoff 0.5, a right-hand side): 8 sites 2.41 ms, with the pairs walked
+// 2.22; 11 sites 2.64 and 3.08; 28 sites 3.4 and 9.1.
+constexpr int kLatMinSites = 10;
+constexpr int kLatWarps = 14, kLatWorkers = 32 * kLatWarps, kLatThreads = kLatWorkers + 64;
+constexpr int kLatReaders = kLatWarps / 4 * 4;  // warps that stage M: every four of them, the 128 rows
+constexpr int kLatGroups = kLatWorkers / 4;  // groups of four threads, one for each mu, that share the sites' pairs
+constexpr int kLatAhead = 6;     // pairs of words loaded before M is complete
+constexpr int kLatK = 32;        // slab pairs of a chunk
+// Chunks of A in shared memory (as many as fit) and of B, which are kept for all products of a k2 where its K has no
+// more.
+constexpr int kLatStages = 4, kLatSlotsB = 3;
 constexpr int kLatNodes = kLatWorkers / 4;  // nodes whose descriptors are built at once (a quad of threads each)
 constexpr uint32_t kLatCols = 512;  // tensor memory: accumulator b's high products at column 256 b, low ones 128 on
 
 __host__ __device__ inline int lat_rows(int nl) { return (4 * nl + 15) / 16 * 16; }
-__host__ __device__ inline int lat_stride(int nl) { return lat_rows(nl) + 1; }  // of the staged M: an odd row stride
-// scratch of a CTA: [A of k1 = 0 .. 3, B of k2 = 0 .. 3][term][k / 8][row / 8][8 k][8 rows] bf16
+__host__ __device__ inline int lat_stride(int nl) { return lat_rows(nl) + 4; }  // of the staged M: an odd number of 16-byte units
+// scratch of a CTA: [A of k1 = 0 .. 3, B of k2 = 0 .. 3][term][k / 8][two row blocks] (umma.cuh)
+constexpr int kLatGroup = 2048;  // bytes of 8 slab pairs of 128 rows
 __host__ __device__ inline int lat_blocks(int max_nodes) { return (2 * max_nodes + 15) / 16 * 2; }
-__host__ __device__ inline size_t lat_scratch_bytes(int nl, int max_nodes) { return 24 * size_t(lat_blocks(max_nodes)) * lat_rows(nl) * 16; }
+__host__ __device__ inline size_t lat_scratch_bytes(int max_nodes) { return 24 * size_t(lat_blocks(max_nodes)) * kLatGroup; }
+
+constexpr int kLatSmemMax = 227 * 1024 - 2048;  // dynamic; the rest is the kernel's static variables
 
 struct LatSmem {
     size_t words, u, locals, coef, stage, total;
+    int stages;
 };
 __host__ __device__ inline LatSmem lat_smem(int nl) {
     LatSmem L;
     L.words = sizeof(int) * 2 * size_t(nl) * kGoffRow;
-    L.u = (L.words + sizeof(int) * 256 + 127) / 128 * 128;
-    // union: the nodes' descriptors and the warps' local values and coefficients, or two chunks of operands
+    L.u = (L.words + sizeof(int) * 256 + 1023) / 1024 * 1024;
+    // union: the nodes' descriptors and the warps' local values and coefficients, or the chunks of operands
     L.locals = L.u + sizeof(TDesc) * kLatNodes;
-    L.coef = L.locals + sizeof(float) * 16 * kLatWarps;
-    const size_t g = L.coef + sizeof(float) * 64 * kLatWarps, m = L.u + 2 * 6 * size_t(lat_rows(nl)) * kLatK * 2;
-    L.stage = ((g > m ? g : m) + 127) / 128 * 128;
-    // union: the warps' sums, or M and a zero
-    const size_t red = sizeof(float) * 512 * kLatWarps, st = sizeof(float) * (lat_rows(nl) * size_t(lat_stride(nl)) + 1);
-    L.total = L.stage + (red > st ? red : st);
+    L.coef = L.locals + sizeof(float) * 32 * kLatWarps;
+    const size_t red = sizeof(float) * 512 * kLatWarps, st = sizeof(float) * (lat_rows(nl) * size_t(lat_stride(nl)) + 4);
+    const size_t chunk = 3 * size_t(kLatGroup) * (kLatK / 8), tail = (red > st ? red : st) + 1024;  // aligned to 1024 in the kernel
+    const size_t gather = L.coef + sizeof(float) * 128 * kLatWarps;
+    for (L.stages = kLatStages;; --L.stages) {
+        const size_t ring = L.u + (L.stages + kLatSlotsB) * chunk;
+        L.stage = gather > ring ? (gather + 1023) / 1024 * 1024 : ring;
+        L.total = L.stage + tail;  // the stage is a union: the warps' sums, or M and four zeros
+        if (L.total <= kLatSmemMax || L.stages == 2) break;
+    }
     return L;
 }
 
 __device__ __forceinline__ void worker_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kLatWorkers) : "memory"); }
 
-// Stores the lane's rows 4 lane .. 4 lane + 3 of slab pair k, four operands of three terms: x[operand][row].
-__device__ __forceinline__ void lat_store(unsigned char *dst, int blocks, int rows, int k, int lane, const float (&x)[4][4]) {
-    unsigned char *p = dst + size_t(k >> 3) * rows * 16 + (lane >> 1) * 128 + (k & 7) * 16 + (lane & 1) * 8;
-    const size_t term = size_t(blocks) * rows * 16;
+// Stores the lane's rows 4 lane .. 4 lane + 3 of slab pair k, four operands of three terms: x[operand][row].  The lanes fill
+// whole sectors.
+__device__ __forceinline__ void lat_store(unsigned char *dst, int blocks, int k, int lane, const float (&x)[4][4]) {
+    unsigned char *p = dst + (k >> 3) * kLatGroup + (lane >> 4) * 1024 + umma::block_offset(lane & 15, k & 7);
+    const size_t term = size_t(blocks) * kLatGroup;
 #pragma unroll
     for (int o = 0; o < 4; ++o) {
         uint2 h, m, l;
@@ -985,36 +1051,52 @@ __device__ __forceinline__ void lat_store(unsigned char *dst, int blocks, int ro
     }
 }
 
+// Copies the three terms of a chunk.
+__device__ __forceinline__ void copy_terms(uint32_t dst, uint32_t dst_term, const unsigned char *src, size_t src_term, uint32_t bytes,
+                                           uint64_t *bar) {
+    umma::bar_expect(bar, 3 * bytes);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) umma::bulk_load(dst + t * dst_term, src + t * src_term, bytes, bar);
+}
+
 __global__ void __launch_bounds__(kLatThreads, 1) tri_lattice_kernel(TriArgs a) {
-    extern __shared__ __align__(128) unsigned char psm[];
+    extern __shared__ __align__(1024) unsigned char lat_sm[];
     __shared__ float pos[kMaxFreq];
-    __shared__ uint64_t full[2], empty[2], done[2], drained[2];  // operands there / read, accumulator complete / read
+    // chunk of A there / read, chunk of B, accumulator complete / read
+    __shared__ uint64_t full[kLatStages], empty[kLatStages], full_b[kLatSlotsB], empty_b[kLatSlotsB], done[2], drained[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int s_item, s_combos[16], s_ncombo;
-    __shared__ int s_dead, s_late;  // a wait ran out: the copying thread's, a worker's
+    __shared__ int s_dead, s_late;  // a wait ran out: the copying or issuing thread's, a worker's
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = a.n, nl = a.nl, rows = lat_rows(nl), stride = lat_stride(nl), blocks = lat_blocks(a.max_nodes);
     const LatSmem L = lat_smem(nl);
+    unsigned char *psm = lat_sm + (-umma::smem_addr(lat_sm) & 1023);
     int *goff = reinterpret_cast<int *>(psm), *words = reinterpret_cast<int *>(psm + L.words);
     TDesc *desc = reinterpret_cast<TDesc *>(psm + L.u);
     float *stage = reinterpret_cast<float *>(psm + L.stage), *red = stage;
-    unsigned char *scratch = a.prod_scratch + lat_scratch_bytes(nl, a.max_nodes) * blockIdx.x;
-    const size_t operand = size_t(blocks) * rows * 16;  // scratch bytes of an operand's term
+    unsigned char *scratch = a.prod_scratch + lat_scratch_bytes(a.max_nodes) * blockIdx.x;
+    const size_t operand = size_t(blocks) * kLatGroup;  // scratch bytes of an operand's term
     for (int i = tid; i < n; i += kLatThreads) pos[i] = a.freq[i];
     site_offsets(a, goff);
     chalice_words(words);
     if (warp == 0) umma::tmem_alloc(&tmem_slot, kLatCols);
     if (tid == 0) {
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < kLatStages; ++b) {
             umma::bar_init(full + b);
             umma::bar_init(empty + b);
+        }
+        for (int b = 0; b < kLatSlotsB; ++b) {
+            umma::bar_init(full_b + b);
+            umma::bar_init(empty_b + b);
+        }
+        for (int b = 0; b < 2; ++b) {
             umma::bar_init(done + b);
-            umma::bar_init(drained + b, kLatWarps);
+            umma::bar_init(drained + b, kLatReaders);
         }
         s_dead = s_late = 0;
         s_ncombo = 0;
         for (int cb = 0; cb < 16; ++cb)
-            if (a.prod_ptr[cb * nl] != a.prod_ptr[(cb + 1) * nl]) s_combos[s_ncombo++] = cb;
+            if (a.prod_ptr[cb * kLatGroups] != a.prod_ptr[(cb + 1) * kLatGroups]) s_combos[s_ncombo++] = cb;
     }
     umma::fence_before();
     __syncthreads();
@@ -1022,8 +1104,14 @@ __global__ void __launch_bounds__(kLatThreads, 1) tri_lattice_kernel(TriArgs a) 
     const uint32_t tmem = tmem_slot;
     const float two_pi = 2.0f * float(kPiD);
     const int combos = s_ncombo;
-    const int j = tid >> 4, mu = (tid >> 2) & 3, nu = tid & 3;  // a worker's output
-    uint32_t chunk_no = 0, combo_no = 0;  // products and accumulators so far: their barriers' phases
+    const int group = tid >> 2, mu = tid & 3;  // a worker's group of pairs and output row
+    const uint32_t term = kLatK / 8 * kLatGroup;  // bytes of an operand's term of a chunk
+    uint32_t combo_no = 0;                   // accumulators so far
+    const uint32_t ring = umma::smem_addr(psm + L.u), ring_b = ring + L.stages * 3 * term;
+    // the copying and the issuing thread's next chunk of A, its barrier's phase and those of B's slots (a bit each); the first
+    // wait for an empty slot passes
+    int stage_no = 0;
+    uint32_t phase = warp == kLatWarps ? 1 : 0, phase_b = warp == kLatWarps ? ~0u : 0;
 
     while (!s_dead && !s_late) {
         __syncthreads();  // the previous triple is finished with shared memory
@@ -1033,13 +1121,13 @@ __global__ void __launch_bounds__(kLatThreads, 1) tri_lattice_kernel(TriArgs a) 
         if (it >= a.fn) break;
         int si, ti, ui;
         decode_triple(it, n, si, ti, ui);
-        const int cnt = a.node_cnt[ti], kn = (2 * cnt + 15) / 16 * 16, chunks = (kn + kLatK - 1) / kLatK;
+        const int cnt = a.node_cnt[ti], kn = (2 * cnt + 15) / 16 * 16;
 
         if (warp < kLatWarps) {
             const float s = pos[si], t = pos[ti], u = pos[ui];
             const float w1p = 0.5f * (s + t + u), w1 = 0.5f * (s - t + u), w2p = 0.5f * (s - t - u), w2 = 0.5f * (s + t - u);
             const float *nwp = a.node_wp + size_t(ti) * a.max_nodes, *nc = a.node_c + size_t(ti) * a.max_nodes;
-            float *Ln = reinterpret_cast<float *>(psm + L.locals) + warp * 16, *coef = reinterpret_cast<float *>(psm + L.coef) + warp * 64;
+            float *Ln = reinterpret_cast<float *>(psm + L.locals) + warp * 32, *coef = reinterpret_cast<float *>(psm + L.coef) + warp * 128;
             float acc[16];
 #pragma unroll
             for (int c = 0; c < 16; ++c) acc[c] = 0.0f;
@@ -1054,36 +1142,44 @@ __global__ void __launch_bounds__(kLatThreads, 1) tri_lattice_kernel(TriArgs a) 
                 }
                 worker_sync();
 #pragma unroll 1
-                for (int task = warp; task < 4 * nb; task += kLatWarps) {  // slab q of a node
-                    const int q = task & 3;
-                    const TDesc &d = desc[task >> 2];
-                    float x[16], v[16], y[4][4];
-                    gather_site(a.v4, d.ab[q], goff, nl, min(lane, nl - 1), x);
-                    if (lane < 16) Ln[lane] = local_value(a, d, local_first(q) + lane);
+                for (int task = warp; task < 2 * nb; task += kLatWarps) {  // slabs q and q + 2 of a node
+                    const int q = task & 1, k = 2 * (b0 + (task >> 1));
+                    const TDesc &d = desc[task >> 1];
+                    float x[16], y[16], v[16], f[4][4], g[4][4];
+                    const float lv = local_value(a, d, 32 * q + lane);
+                    gather_site_pair(a.v4, d.ab[q], d.ab[q + 2], goff, nl, min(lane, nl - 1), x, y);
+                    Ln[lane] = lv;
                     __syncwarp();
-                    coef[lane] = chalice_coef(Ln, words[64 * q + lane]);
-                    coef[lane + 32] = chalice_coef(Ln, words[64 * q + 32 + lane]);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        coef[32 * e + lane] = chalice_coef(Ln + 16 * (e >> 1), words[64 * (q + (e & 2)) + 32 * (e & 1) + lane]);
                     __syncwarp();
                     const float c1 = d.c;
+                    unsigned char *dst = scratch + q * 12 * operand;
 #pragma unroll
                     for (int c = 0; c < 16; ++c) v[c] = 0.0f;
-                    if (q & 1) {
+                    if (q) {  // operand k, row nu
                         chalice_terms<true>(x, coef, v);
+                        chalice_terms<true>(y, coef + 64, v);
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) y[c >> 2][c & 3] = x[c];  // operand k, row nu
-                    } else {
+                        for (int c = 0; c < 16; ++c) f[c >> 2][c & 3] = x[c], g[c >> 2][c & 3] = y[c];
+                    } else {  // operand k, row mu
                         chalice_terms<false>(x, coef, v);
+                        chalice_terms<false>(y, coef + 64, v);
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) y[c & 3][c >> 2] = c1 * x[c];  // operand k, row mu
+                        for (int c = 0; c < 16; ++c) f[c & 3][c >> 2] = c1 * x[c], g[c & 3][c >> 2] = c1 * y[c];
+                    }
+                    if (lane < nl) {
+                        lat_store(dst, blocks, k, lane, f);
+                        lat_store(dst, blocks, k + 1, lane, g);
                     }
 #pragma unroll
                     for (int c = 0; c < 16; ++c) acc[c] += c1 * v[c];
-                    if (lane < nl) lat_store(scratch + (q & 1) * 12 * operand, blocks, rows, 2 * (b0 + (task >> 2)) + (q >> 1), lane, y);
                 }
             }
             for (int task = warp + 4 * cnt; task < 2 * kn; task += kLatWarps) {  // zero up to a multiple of 16
-                const float y[4][4] = {};
-                if (lane < nl) lat_store(scratch + (task & 1) * 12 * operand, blocks, rows, task >> 1, lane, y);
+                const float z[4][4] = {};
+                if (lane < nl) lat_store(scratch + (task & 1) * 12 * operand, blocks, task >> 1, lane, z);
             }
 #pragma unroll
             for (int c = 0; c < 16; ++c) red[warp * 512 + c * 32 + lane] = acc[c];
@@ -1091,60 +1187,90 @@ __global__ void __launch_bounds__(kLatThreads, 1) tri_lattice_kernel(TriArgs a) 
         }
         __syncthreads();
 
+        const bool keep = kn <= kLatSlotsB * kLatK;  // the whole B of a k2 stays in shared memory
         if (warp == kLatWarps) {
-            if (lane == 0 && chunks > 0) {
+            if (lane == 0) {  // copies
                 bool ok = true;
-                const int total = combos * chunks;
-                auto load = [&](int g) {
-                    const uint32_t b = (chunk_no + g) & 1, seq = (chunk_no + g) >> 1;
-                    if (seq) ok = ok && umma::bar_wait(empty + b, (seq - 1) & 1);
-                    if (!ok) return;
-                    const int cb = s_combos[g / chunks], k0 = g % chunks * kLatK;
-                    const uint32_t bytes = min(kLatK, kn - k0) * rows * 2, term = rows * kLatK * 2;
-                    const uint32_t dst = umma::smem_addr(psm + L.u) + b * 6 * term;
-                    const unsigned char *A = scratch + 3 * (cb & 3) * operand + size_t(k0) * rows * 2;
-                    const unsigned char *B = scratch + (12 + 3 * (cb >> 2)) * operand + size_t(k0) * rows * 2;
-                    umma::bar_expect(full + b, 6 * bytes);
-                    for (int t = 0; t < 3; ++t) {
-                        umma::bulk_load(dst + t * term, A + t * operand, bytes, full + b);
-                        umma::bulk_load(dst + (3 + t) * term, B + t * operand, bytes, full + b);
+                int slot = 0;
+                for (int i = 0; i < combos && ok; ++i) {
+                    const int cb = s_combos[i];
+                    const bool with_b = !keep || i == 0 || s_combos[i - 1] >> 2 != cb >> 2;
+                    const unsigned char *src_a = scratch + 3 * (cb & 3) * operand, *src_b = scratch + (12 + 3 * (cb >> 2)) * operand;
+                    if (keep) slot = 0;
+                    for (int k0 = 0; k0 < kn; k0 += kLatK) {
+                        const uint32_t bytes = min(kLatK, kn - k0) / 8 * kLatGroup;
+                        if (with_b) {
+                            ok = umma::bar_wait(empty_b + slot, phase_b >> slot & 1);
+                            if (!ok) break;
+                            phase_b ^= 1u << slot;
+                            copy_terms(ring_b + slot * 3 * term, term, src_b, operand, bytes, full_b + slot);
+                        }
+                        ok = umma::bar_wait(empty + stage_no, phase);
+                        if (!ok) break;
+                        copy_terms(ring + stage_no * 3 * term, term, src_a, operand, bytes, full + stage_no);
+                        src_a += bytes;
+                        src_b += bytes;
+                        if (++slot == kLatSlotsB) slot = 0;
+                        if (++stage_no == L.stages) stage_no = 0, phase ^= 1;
                     }
-                };
-                if (total) load(0);
-                for (int g = 0; g < total && ok; ++g) {
-                    if (g + 1 < total) load(g + 1);
-                    const uint32_t b = (chunk_no + g) & 1, ci = combo_no + g / chunks, k0 = g % chunks * kLatK;
-                    const uint32_t d = tmem + 256 * (ci & 1), term = rows * kLatK * 2;
-                    if (k0 == 0 && ci >= 2) ok = ok && umma::bar_wait(drained + (ci & 1), ((ci >> 1) - 1) & 1);
-                    ok = ok && umma::bar_wait(full + b, ((chunk_no + g) >> 1) & 1);
-                    if (!ok) break;
-                    umma::fence_after();
-                    const uint32_t o = umma::smem_addr(psm + L.u) + b * 6 * term;
-                    umma::product<true>(d, d + 128, o, rows, term, o + 3 * term, rows, term, rows, min(kLatK, kn - int(k0)) / 16, k0 > 0);
-                    umma::commit(empty + b);
-                    if (g % chunks == chunks - 1) umma::commit(done + (ci & 1));
+                }
+                if (!ok) s_dead = 1;
+            }
+            __syncwarp();
+        } else if (warp == kLatWarps + 1) {
+            if (lane == 0) {  // products
+                bool ok = true;
+                int slot = 0;
+                for (int i = 0; i < combos && ok && kn > 0; ++i) {
+                    const uint32_t ci = combo_no + i, d = tmem + 256 * (ci & 1);
+                    const bool release_b = !keep || i + 1 == combos || s_combos[i + 1] >> 2 != s_combos[i] >> 2;
+                    if (ci >= 2) ok = umma::bar_wait(drained + (ci & 1), ((ci >> 1) - 1) & 1);
+                    if (keep) slot = 0;
+                    for (int k0 = 0; k0 < kn && ok; k0 += kLatK) {
+                        ok = umma::bar_wait(full_b + slot, phase_b >> slot & 1) && umma::bar_wait(full + stage_no, phase);
+                        if (!ok) break;
+                        umma::fence_after();
+                        umma::product(d, d + 128, ring + stage_no * 3 * term, kLatGroup, term, ring_b + slot * 3 * term, kLatGroup, term, rows,
+                                      min(kLatK, kn - k0) / 16, k0 > 0);
+                        umma::commit(empty + stage_no);
+                        if (release_b) {
+                            umma::commit(empty_b + slot);
+                            phase_b ^= 1u << slot;
+                        }
+                        if (++slot == kLatSlotsB) slot = 0;
+                        if (++stage_no == L.stages) stage_no = 0, phase ^= 1;
+                    }
+                    umma::commit(done + (ci & 1));
                 }
                 if (!ok) s_dead = 1;
             }
             __syncwarp();
         } else {
-            float sum = 0.0f, rpa = 0.0f;
-            if (j < nl)
-                for (int w = 0; w < kLatWarps; ++w) sum += red[w * 512 + (tid & 15) * 32 + j];
+            float sum[2] = {0.0f, 0.0f};  // outputs o = 16 site + component: tid, tid + kLatWorkers
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (const int o = tid + h * kLatWorkers; o < 16 * nl)
+                    for (int w = 0; w < kLatWarps; ++w) sum[h] += red[w * 512 + (o & 15) * 32 + (o >> 4)];
             worker_sync();  // M takes the place of the sums
-            if (tid == 0) stage[rows * stride] = 0.0f;  // for the padding words
-            for (int i = 0; i < combos && chunks > 0; ++i) {
+            if (tid < 4) stage[rows * stride + tid] = 0.0f;  // for the padding words
+            float rpa[4] = {};
+            const int2 *list = reinterpret_cast<const int2 *>(a.prod_words);
+            const int *ptr = a.prod_ptr + group;
+            int w0 = 0, w1 = 0;
+            if (combos) {
+                w0 = __ldg(ptr + s_combos[0] * kLatGroups);
+                w1 = __ldg(ptr + s_combos[0] * kLatGroups + 1);
+            }
+            for (int i = 0; i < combos && kn > 0; ++i) {
                 const uint32_t ci = combo_no + i, b = ci & 1;
                 const int cb = s_combos[i];
-                int w0 = 0, w1 = 0;
-                if (j < nl) {
-                    w0 = __ldg(a.prod_ptr + cb * nl + j);
-                    w1 = __ldg(a.prod_ptr + cb * nl + j + 1);
-                }
+                int2 ahead[kLatAhead];
+#pragma unroll
+                for (int e = 0; e < kLatAhead; ++e) ahead[e] = w0 + e < w1 ? __ldg(list + w0 + e) : make_int2(rows * stride, rows * stride);
                 if (!umma::bar_wait(done + b, (ci >> 1) & 1)) s_late = 1;
                 umma::fence_after();
                 const int row = (warp & 3) * 32 + lane;
-                for (int c0 = (warp >> 2) * 16; c0 < rows; c0 += 64) {
+                for (int c0 = (warp >> 2) * 16; c0 < rows && warp < kLatReaders; c0 += 4 * kLatReaders) {
                     float hi[16], lo[16];
                     const uint32_t addr = tmem + 256 * b + (uint32_t(warp & 3) << 21) + c0;
                     umma::load16(addr, hi);
@@ -1152,44 +1278,66 @@ __global__ void __launch_bounds__(kLatThreads, 1) tri_lattice_kernel(TriArgs a) 
                     umma::load_wait();
                     if (row < rows)
 #pragma unroll
-                        for (int k = 0; k < 16; ++k) stage[row * stride + c0 + k] = hi[k] + lo[k];
+                        for (int k = 0; k < 16; k += 4)
+                            *reinterpret_cast<float4 *>(stage + row * stride + c0 + k) =
+                                make_float4(hi[k] + lo[k], hi[k + 1] + lo[k + 1], hi[k + 2] + lo[k + 2], hi[k + 3] + lo[k + 3]);
                 }
                 umma::fence_before();
                 __syncwarp();
-                if (lane == 0) umma::bar_arrive(drained + b);
+                if (lane == 0 && warp < kLatReaders) umma::bar_arrive(drained + b);
                 worker_sync();
                 if (s_late) break;  // the workers write it before this barrier alone, so they agree
-                float p0 = 0.0f, p1 = 0.0f;
-                const int4 *list = reinterpret_cast<const int4 *>(a.prod_words);
-                auto element = [&](int w) {
-                    return stage[(w & 0x7fff) + ((w >> (15 + 2 * mu)) & 3) * stride + ((unsigned(w) >> (23 + 2 * nu)) & 3)];
-                };
-#pragma unroll 4
-                for (int e = w0; e < w1; ++e) {
-                    const int4 w = __ldg(list + e);
-                    p0 += element(w.x) + element(w.y);
-                    p1 += element(w.z) + element(w.w);
+                int n0 = 0, n1 = 0;
+                if (i + 1 < combos) {
+                    n0 = __ldg(ptr + s_combos[i + 1] * kLatGroups);
+                    n1 = __ldg(ptr + s_combos[i + 1] * kLatGroups + 1);
                 }
-                // tri::rpa_sign: the inner index is the density for k1 = 3 alone
-                const float part = p0 + p1;
-                rpa += (mu == 3) == (nu == 3) && ((cb & 3) == 3) != (mu == 3) ? -part : part;
+                float part[4] = {};
+                auto pair = [&](int w) {  // row mu of the pair's element block, its columns permuted
+                    const float *m = stage + (w & 0x7fff) + ((w >> (15 + 2 * mu)) & 3) * stride;
+                    part[0] += m[(w >> 23) & 3];
+                    part[1] += m[(w >> 25) & 3];
+                    part[2] += m[(w >> 27) & 3];
+                    part[3] += m[3];
+                };
+#pragma unroll
+                for (int e = 0; e < kLatAhead; ++e) {
+                    pair(ahead[e].x);
+                    pair(ahead[e].y);
+                }
+#pragma unroll 4
+                for (int e = w0 + kLatAhead; e < w1; ++e) {
+                    const int2 w = __ldg(list + e);
+                    pair(w.x);
+                    pair(w.y);
+                }
+#pragma unroll
+                for (int nu = 0; nu < 4; ++nu)  // tri::rpa_sign: the inner index is the density for k1 = 3 alone
+                    rpa[nu] += (mu == 3) == (nu == 3) && ((cb & 3) == 3) != (mu == 3) ? -part[nu] : part[nu];
+                w0 = n0;
+                w1 = n1;
                 worker_sync();  // M is read
             }
-            if (j < nl) {
-                float *p = a.dv4 + size_t(it) * 16 * nl + (tid & 15) * nl + j;
-                const float o = *p + (sum + 2.0f * rpa) / two_pi;
-                *p = o;
-                if (isnan(o)) atomicOr(a.status, kStatusNaN);
+#pragma unroll
+            for (int nu = 0; nu < 4; ++nu) stage[16 * group + 4 * mu + nu] = rpa[nu];
+            worker_sync();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int o = tid + h * kLatWorkers, j = o >> 4;
+                if (o >= 16 * nl) continue;
+                float r = 0.0f;
+                for (int g = __ldg(a.prod_group + j); g < __ldg(a.prod_group + j + 1); ++g) r += stage[16 * g + (o & 15)];
+                float *p = a.dv4 + size_t(it) * 16 * nl + (o & 15) * nl + j;
+                const float v = *p + (sum[h] + 2.0f * r) / two_pi;
+                *p = v;
+                if (isnan(v)) atomicOr(a.status, kStatusNaN);
             }
         }
-        chunk_no += combos * chunks;
-        if (chunks > 0) combo_no += combos;
+        if (kn > 0) combo_no += combos;
         __syncthreads();  // s_dead, s_late
     }
-    if (s_dead || s_late) {  // a copy or a product did not complete in time: report it, and give them a last chance before the memory goes
-        if (tid == 0) atomicOr(a.status, kStatusProductTimeout);
-        if (tid < 2) umma::bar_wait(full + tid, 0) && umma::bar_wait(done + tid, 0);
-    }
+    // a copy or a product did not complete in time (each wait is long enough for those in flight to end)
+    if ((s_dead || s_late) && tid == 0) atomicOr(a.status, kStatusProductTimeout);
     umma::fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -1337,7 +1485,7 @@ struct spn_tri {
           *node_c = nullptr, *corr_out = nullptr;
     int *ints = nullptr;  // all integer tables in one allocation
     int *sites, *sites_perm, *inv_sites, *inv_sites_perm, *range_rid, *range_inv, *corr_rid,
-        *corr_perm, *node_cnt, *work_counter, *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr, *prod_ptr, *prod_words;
+        *corr_perm, *node_cnt, *work_counter, *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr, *prod_ptr, *prod_words, *prod_group;
     int rpa_n_seg = 0;
     unsigned char *prod_scratch = nullptr;  // tri_lattice_kernel runs when not NULL
     unsigned *status = nullptr;
@@ -1370,6 +1518,7 @@ struct spn_tri {
         a.rpa_n_seg = rpa_n_seg;
         a.prod_ptr = prod_ptr;
         a.prod_words = prod_words;
+        a.prod_group = prod_group;
         a.prod_scratch = prod_scratch;
         a.range_rid = range_rid;
         a.range_inv = range_inv;
@@ -1467,16 +1616,26 @@ void (*vertex_kernel(const spn_tri *h))(TriArgs) {
 // Whether the t channel runs on the tensor cores (tri_lattice_kernel).
 bool use_products(int nl) { return nl >= kLatMinSites && nl <= 32; }
 
-// The RPA pairs by inner components and site, as tri_lattice_kernel reads them, four words at a time: the element of the
-// staged M (15 bits) and the images of the four components under perm1 and perm2 (2 bits each).  The last
-// four of a site are filled up with words of the zero behind M.
-void product_pairs(const spn_tri_desc *d, std::vector<int> &ptr, std::vector<int> &words) {
+// The RPA pairs as tri_lattice_kernel reads them, two words at a time: the element of the staged M (15 bits) and the
+// images of the four components under perm1 and perm2 (2 bits each); an odd list ends with the zero behind M.  A site's pairs are
+// dealt to as many groups as keep every group's share below the smallest bound that suffices.
+void product_pairs(const spn_tri_desc *d, std::vector<int> &ptr, std::vector<int> &words, std::vector<int> &group) {
     const int nl = d->n_sites, stride = lat_stride(nl);
+    int bound = 1;
+    for (;; ++bound) {
+        group.assign(1, 0);
+        for (int j = 0; j < nl; ++j) group.push_back(group.back() + (d->overlap_ptr[j + 1] - d->overlap_ptr[j] + bound - 1) / bound);
+        if (group.back() <= kLatGroups) break;
+    }
+    std::vector<int> site(kLatGroups, -1);
+    for (int j = 0; j < nl; ++j) std::fill(site.begin() + group[j], site.begin() + group[j + 1], j);
     ptr.assign(1, 0);
     for (int k2 = 0; k2 < 4; ++k2)
         for (int k1 = 0; k1 < 4; ++k1)
-            for (int j = 0; j < nl; ++j) {
-                for (int i = d->overlap_ptr[j]; i < d->overlap_ptr[j + 1]; ++i) {
+            for (int g = 0; g < kLatGroups; ++g) {
+                const int j = site[g], step = j < 0 ? 1 : group[j + 1] - group[j];
+                const int first = j < 0 ? 0 : d->overlap_ptr[j] + g - group[j], last = j < 0 ? 0 : d->overlap_ptr[j + 1];
+                for (int i = first; i < last; i += step) {
                     const int p1 = d->overlap_perm1[i], p2 = d->overlap_perm2[i];
                     for (int k = 0; k < 4; ++k) {
                         if (permc(p1, k) != k1 || permc(p2, k) != k2) continue;
@@ -1485,8 +1644,8 @@ void product_pairs(const spn_tri_desc *d, std::vector<int> &ptr, std::vector<int
                         words.push_back(int(w));
                     }
                 }
-                while (words.size() % 4) words.push_back(lat_rows(nl) * stride);
-                ptr.push_back(int(words.size() / 4));
+                if (words.size() % 2) words.push_back(lat_rows(nl) * stride);
+                ptr.push_back(int(words.size() / 2));
             }
 }
 
@@ -1573,16 +1732,17 @@ extern "C" int spn_tri_create(const spn_tri_desc *d, spn_tri **out) {
             put(rpa.count.data(), 32);
             put(rpa.slot_base.data(), 32);
             put(rpa.seg_ptr.data(), nl + 1);
-            std::vector<int> prod_ptr, prod_words;
-            if (use_products(nl)) product_pairs(d, prod_ptr, prod_words);
+            std::vector<int> prod_ptr, prod_words, prod_group;
+            if (use_products(nl)) product_pairs(d, prod_ptr, prod_words, prod_group);
             put(prod_ptr.data(), int(prod_ptr.size()));
-            img.resize((img.size() + 3) / 4 * 4);  // read four words at a time
+            img.resize((img.size() + 1) / 2 * 2);  // read two words at a time
             put(prod_words.data(), int(prod_words.size()));
+            put(prod_group.data(), int(prod_group.size()));
             h->ints = dalloc<int>(img.size(), "alloc lattice tables");
             h2d(h->ints, img.data(), img.size(), h->stream);
             int **fields[] = {&h->sites, &h->sites_perm, &h->inv_sites, &h->inv_sites_perm,
                               &h->range_rid, &h->range_inv, &h->corr_rid, &h->corr_perm, &h->node_cnt, &h->work_counter,
-                              &h->rpa_sched, &h->rpa_count, &h->rpa_slot_base, &h->rpa_seg_ptr, &h->prod_ptr, &h->prod_words};
+                              &h->rpa_sched, &h->rpa_count, &h->rpa_slot_base, &h->rpa_seg_ptr, &h->prod_ptr, &h->prod_words, &h->prod_group};
             for (size_t k = 0; k < at.size(); ++k) *fields[k] = h->ints + at[k];
             h2d(h->freq, d->freq, h->n, h->stream);
             check_cuda(cudaMemsetAsync(h->v4, 0, vsz * sizeof(float), h->stream), "memset");
@@ -1596,7 +1756,7 @@ extern "C" int spn_tri_create(const spn_tri_desc *d, spn_tri **out) {
                 void *p = nullptr;
                 if (cudaFuncSetAttribute(tri_lattice_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(lat_smem(nl).total)) ==
                         cudaSuccess &&
-                    cudaMalloc(&p, lat_scratch_bytes(nl, h->max_nodes) * size_t(h->sms)) == cudaSuccess)
+                    cudaMalloc(&p, lat_scratch_bytes(h->max_nodes) * size_t(h->sms)) == cudaSuccess)
                     h->prod_scratch = static_cast<unsigned char *>(p);
                 else cudaGetLastError();
             }

@@ -1,7 +1,7 @@
 """The TRI vertex flow of lattices of at most 32 sites (a CTA per triple, the t channel's lattice sum on the tensor
-cores from 20 sites on) against the oracle at the sizes where it can go wrong: meshes of 2 to 7 points, 8, 16
-and 32 lanes a node with their edges, permuted spin components, tables that no lattice has, and loop sums of one,
-two and three operand chunks (up to 40, 80 and more nodes).
+cores from 10 sites on) against the oracle at the sizes where it can go wrong: meshes of 2 to 7 points, 8, 16
+and 32 lanes a node with their edges, permuted spin components, tables that no lattice has, and loop sums of one
+to six operand chunks (16 nodes each) with and without the second factor kept.
 
 Tolerance: 1e-5 of the largest value, the bound of the other right-hand-side tests (about 100 uncompensated FP32
 terms of the oracle, 6e-8 each, with cancellation).  The tensor-core products keep 24 bits of every operand."""
