@@ -602,8 +602,10 @@ spn_su2 *spn::create_flow(const spn_su2_desc *d, cudaStream_t stream) {
                 cuda_check(cudaMemsetAsync(h->dsd, 0, vsz * sizeof(float2), h->stream), "memset");
             }
             h->node_cnt = dev_alloc<int>(h->n, "alloc node counts");
-            h->work_counter = dev_alloc<int>(1, "alloc work counter");
-            h->status = dev_alloc<unsigned>(1, "alloc status");
+            h->status = dev_alloc<unsigned>(2, "alloc status");
+            h->work_counter = reinterpret_cast<int *>(h->status + 1);
+            h->status_host.alloc(sizeof(unsigned));
+            h->corr_host.alloc((2 * size_t(h->n_corr) + 2 * h->nl) * (f64 ? sizeof(double) : sizeof(float)));
             h->sites = dev_alloc<int>(h->nl, "alloc sites");
             h->inv_sites = dev_alloc<int>(h->nl, "alloc inv sites");
             h->ov_ptr = dev_alloc<int>(h->nl + 1, "alloc overlap ptr");
@@ -772,8 +774,7 @@ extern "C" int spn_su2_compute_step(spn_su2 *h) {
             e0 = h->event();
             cuda_check(cudaEventRecord(h->ev_pool[e0], h->stream), "event record");
         }
-        cuda_check(cudaMemsetAsync(h->status, 0, sizeof(unsigned), h->stream), "memset status");
-        cuda_check(cudaMemsetAsync(h->work_counter, 0, sizeof(int), h->stream), "memset counter");
+        cuda_check(cudaMemsetAsync(h->status, 0, 2 * sizeof(unsigned), h->stream), "memset status and counter");
         if (h->fp64()) {
             const FlowArgsT<double> a = h->args64();
             su2_self_energy_f64_kernel<<<h->n, 128, 0, h->stream>>>(a);
@@ -1007,27 +1008,17 @@ void launch_correlation(spn_su2 *h) {
 }
 
 void copy_correlation(spn_su2 *h, float *zz, float *dd, float *chi_zz, float *chi_dd) {
-        if (h->fp64()) {
-            const std::vector<double> v = download(h->corr_out64, 2 * size_t(h->n_corr) + 2 * h->nl, h->stream);
-            auto put = [&](float *out, size_t off, int cnt) {
-                if (out)
-                    for (int i = 0; i < cnt; ++i) out[i] = float(v[off + i]);
-            };
-            put(zz, 0, h->n_corr);
-            put(dd, h->n_corr, h->n_corr);
-            put(chi_zz, 2 * size_t(h->n_corr), h->nl);
-            put(chi_dd, 2 * size_t(h->n_corr) + h->nl, h->nl);
-            return;
-        }
-        if (zz) cuda_check(cudaMemcpyAsync(zz, h->corr_out, h->n_corr * sizeof(float), cudaMemcpyDeviceToHost, h->stream), "D2H");
-        if (dd)
-            cuda_check(cudaMemcpyAsync(dd, h->corr_out + h->n_corr, h->n_corr * sizeof(float), cudaMemcpyDeviceToHost, h->stream), "D2H");
-        if (chi_zz)
-            cuda_check(cudaMemcpyAsync(chi_zz, h->corr_out + 2 * h->n_corr, h->nl * sizeof(float), cudaMemcpyDeviceToHost, h->stream), "D2H");
-        if (chi_dd)
-            cuda_check(cudaMemcpyAsync(chi_dd, h->corr_out + 2 * h->n_corr + h->nl, h->nl * sizeof(float), cudaMemcpyDeviceToHost, h->stream),
-                       "D2H");
-        cuda_check(cudaStreamSynchronize(h->stream), "correlation sync");
+    const size_t count = 2 * size_t(h->n_corr) + 2 * h->nl;
+    const double *v64 = h->fp64() ? h->corr_host.fetch(h->corr_out64, count, h->stream) : nullptr;
+    const float *v = v64 ? nullptr : h->corr_host.fetch(h->corr_out, count, h->stream);
+    auto put = [&](float *out, size_t off, int cnt) {
+        if (out)
+            for (int i = 0; i < cnt; ++i) out[i] = v64 ? float(v64[off + i]) : v[off + i];
+    };
+    put(zz, 0, h->n_corr);
+    put(dd, h->n_corr, h->n_corr);
+    put(chi_zz, 2 * size_t(h->n_corr), h->nl);
+    put(chi_dd, 2 * size_t(h->n_corr) + h->nl, h->nl);
 }
 
 }  // namespace
@@ -1090,9 +1081,9 @@ extern "C" int spn_su2_measure_correlation_f64(spn_su2 *h, double *zz, double *d
         require_fp64(h);
         cuda_check(cudaSetDevice(h->device), "cudaSetDevice");
         launch_correlation(h);
-        const std::vector<double> v = download(h->corr_out64, 2 * size_t(h->n_corr) + 2 * h->nl, h->stream);
+        const double *v = h->corr_host.fetch(h->corr_out64, 2 * size_t(h->n_corr) + 2 * h->nl, h->stream);
         auto put = [&](double *out, size_t off, int cnt) {
-            if (out) std::copy(v.begin() + off, v.begin() + off + cnt, out);
+            if (out) std::copy(v + off, v + off + cnt, out);
         };
         put(zz, 0, h->n_corr);
         put(dd, h->n_corr, h->n_corr);
@@ -1121,9 +1112,7 @@ extern "C" int spn_su2_is_diverged(spn_su2 *h, int *diverged) {
     return guarded([&] {
         if (!h || !diverged) throw Error(ErrorType::Argument, "null argument");
         cuda_check(cudaSetDevice(h->device), "cudaSetDevice");
-        unsigned st = 0;
-        cuda_check(cudaMemcpyAsync(&st, h->status, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream), "D2H");
-        cuda_check(cudaStreamSynchronize(h->stream), "status sync");
+        const unsigned st = *h->status_host.fetch(h->status, 1, h->stream);
         if (st & kStatusNodeOverflow) throw Error(ErrorType::Device, "loop-frequency node table overflow");
         *diverged = (st & kStatusNaN) ? 1 : 0;
     });

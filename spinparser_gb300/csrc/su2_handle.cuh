@@ -5,6 +5,7 @@
 #include <string>
 #include <utility>
 #include <vector>
+#include "cuda_host.cuh"
 #include "su2_common.cuh"
 #include "host/capi_common.hpp"
 #include "../../include/spn_su2.h"
@@ -34,7 +35,8 @@ struct spn_su2 {
     int mesh_shift = 0;
     float *node_wp = nullptr, *node_c = nullptr, *corr_out = nullptr;
     int *node_cnt = nullptr, *work_counter = nullptr;
-    unsigned *status = nullptr;
+    unsigned *status = nullptr;  // the word after it is work_counter
+    spn::cuh::Pinned corr_host, status_host;  // measurements and the status word on the host
     int *sites = nullptr, *inv_sites = nullptr, *ov_ptr = nullptr, *ov_r1 = nullptr, *ov_r2 = nullptr;
     int *range_rid = nullptr, *range_inv = nullptr, *corr_rid = nullptr;
     double *corr_partial = nullptr;
@@ -156,7 +158,7 @@ struct spn_su2 {
         for (auto e : ev_pool) cudaEventDestroy(e);
         ev_pool.clear();
         void *ptrs[] = {freq,      sd,     dsd,       stage,     v2,           dv2,       node_wp,  node_c,
-                        corr_out,  node_cnt, work_counter, status, sites,     inv_sites,    ov_ptr,    ov_r1,
+                        corr_out,  node_cnt, status, sites,     inv_sites,    ov_ptr,    ov_r1,
                         ov_r2,     range_rid, range_inv, corr_rid, corr_partial, rpa_image, v2d,      dv2d,
                         freq64,    sd64,   dsd64,     node_wp64, node_c64,  corr_out64, mesh_lo};
         for (void *p : ptrs)

@@ -1488,7 +1488,8 @@ struct spn_tri {
         *corr_perm, *node_cnt, *work_counter, *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr, *prod_ptr, *prod_words, *prod_group;
     int rpa_n_seg = 0;
     unsigned char *prod_scratch = nullptr;  // tri_lattice_kernel runs when not NULL
-    unsigned *status = nullptr;
+    unsigned *status = nullptr;  // in ints, behind the work counters
+    spn::cuh::Pinned corr_host, status_host;  // measurements and the status word on the host
     double *partial = nullptr;
 
     long long vsize() const { return 16 * fn * nl; }
@@ -1555,7 +1556,7 @@ struct spn_tri {
 
     void release() {
         cudaSetDevice(device);
-        void *ptrs[] = {freq, v2, dv2, v4, dv4, node_wp, node_c, corr_out, ints, status, partial, prod_scratch};
+        void *ptrs[] = {freq, v2, dv2, v4, dv4, node_wp, node_c, corr_out, ints, partial, prod_scratch};
         for (void *p : ptrs)
             if (p) cudaFree(p);
         if (stream) cudaStreamDestroy(stream);
@@ -1706,7 +1707,8 @@ extern "C" int spn_tri_create(const spn_tri_desc *d, spn_tri **out) {
             h->node_c = dalloc<float>(size_t(h->n) * h->max_nodes, "alloc node table");
             h->corr_out = dalloc<float>(size_t(kCorrOut) * h->n_corr + 16 * h->nl, "alloc correlation output");
             h->partial = dalloc<double>(size_t(kMaxCorrNodes) * kCorrOut * h->nl, "alloc correlation scratch");
-            h->status = dalloc<unsigned>(1, "alloc status");
+            h->corr_host.alloc((size_t(kCorrOut) * h->n_corr + 16 * h->nl) * sizeof(float));
+            h->status_host.alloc(sizeof(unsigned));
             const int nl = h->nl, nr = h->n_range, nc = h->n_corr;
             std::vector<int> img;
             std::vector<size_t> at;
@@ -1727,7 +1729,7 @@ extern "C" int spn_tri_create(const spn_tri_desc *d, spn_tri **out) {
             put(d->corr_rid, nc);
             put(d->corr_perm, nc);
             put(nullptr, h->n);  // node counts
-            put(nullptr, 2);     // work counters
+            put(nullptr, 3);     // work counters, status
             put(rpa.sched.data(), int(rpa.sched.size()));
             put(rpa.count.data(), 32);
             put(rpa.slot_base.data(), 32);
@@ -1744,12 +1746,12 @@ extern "C" int spn_tri_create(const spn_tri_desc *d, spn_tri **out) {
                               &h->range_rid, &h->range_inv, &h->corr_rid, &h->corr_perm, &h->node_cnt, &h->work_counter,
                               &h->rpa_sched, &h->rpa_count, &h->rpa_slot_base, &h->rpa_seg_ptr, &h->prod_ptr, &h->prod_words, &h->prod_group};
             for (size_t k = 0; k < at.size(); ++k) *fields[k] = h->ints + at[k];
+            h->status = reinterpret_cast<unsigned *>(h->work_counter + 2);
             h2d(h->freq, d->freq, h->n, h->stream);
             check_cuda(cudaMemsetAsync(h->v4, 0, vsz * sizeof(float), h->stream), "memset");
             check_cuda(cudaMemsetAsync(h->dv4, 0, vsz * sizeof(float), h->stream), "memset");
             check_cuda(cudaMemsetAsync(h->v2, 0, h->n * sizeof(float), h->stream), "memset");
             check_cuda(cudaMemsetAsync(h->dv2, 0, h->n * sizeof(float), h->stream), "memset");
-            check_cuda(cudaMemsetAsync(h->status, 0, sizeof(unsigned), h->stream), "memset");
             check_cuda(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device), "device attribute");
             if (use_products(nl)) {
                 // without the memory for the scratch, or room for the kernel, the pairs are walked
@@ -1824,8 +1826,7 @@ extern "C" int spn_tri_compute_step(spn_tri *h) {
     return guarded([&] {
         if (!h) throw Error(ErrorType::Argument, "null handle");
         check_cuda(cudaSetDevice(h->device), "cudaSetDevice");
-        check_cuda(cudaMemsetAsync(h->status, 0, sizeof(unsigned), h->stream), "memset status");
-        check_cuda(cudaMemsetAsync(h->work_counter, 0, 2 * sizeof(int), h->stream), "memset counter");
+        check_cuda(cudaMemsetAsync(h->work_counter, 0, 3 * sizeof(int), h->stream), "memset counters and status");
         const TriArgs a = h->args();
         tri_self_energy_kernel<<<h->n, 128, 0, h->stream>>>(a);
         check_cuda(cudaGetLastError(), "self-energy launch");
@@ -1861,15 +1862,10 @@ extern "C" int spn_tri_measure_correlation(spn_tri *h, float *corr, float *chi) 
         if (!h) throw Error(ErrorType::Argument, "null handle");
         check_cuda(cudaSetDevice(h->device), "cudaSetDevice");
         launch_correlation(h);
-        if (corr)
-            check_cuda(cudaMemcpyAsync(corr, h->corr_out, size_t(kCorrOut) * h->n_corr * sizeof(float), cudaMemcpyDeviceToHost,
-                                       h->stream),
-                       "D2H");
-        if (chi)
-            check_cuda(cudaMemcpyAsync(chi, h->corr_out + size_t(kCorrOut) * h->n_corr, 16 * h->nl * sizeof(float),
-                                       cudaMemcpyDeviceToHost, h->stream),
-                       "D2H");
-        check_cuda(cudaStreamSynchronize(h->stream), "correlation sync");
+        const size_t n = size_t(kCorrOut) * h->n_corr;
+        const float *v = h->corr_host.fetch(h->corr_out, n + 16 * h->nl, h->stream);
+        if (corr) std::copy(v, v + n, corr);
+        if (chi) std::copy(v + n, v + n + 16 * h->nl, chi);
     });
 }
 
@@ -1877,9 +1873,7 @@ extern "C" int spn_tri_is_diverged(spn_tri *h, int *diverged) {
     return guarded([&] {
         if (!h || !diverged) throw Error(ErrorType::Argument, "null argument");
         check_cuda(cudaSetDevice(h->device), "cudaSetDevice");
-        unsigned st = 0;
-        check_cuda(cudaMemcpyAsync(&st, h->status, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream), "D2H");
-        check_cuda(cudaStreamSynchronize(h->stream), "status sync");
+        const unsigned st = *h->status_host.fetch(h->status, 1, h->stream);
         if (st & kStatusNodeOverflow) throw Error(ErrorType::Device, "loop-frequency node table overflow");
         if (st & kStatusProductTimeout) throw Error(ErrorType::Device, "a tensor-core product of the vertex flow did not complete");
         *diverged = (st & kStatusNaN) ? 1 : 0;

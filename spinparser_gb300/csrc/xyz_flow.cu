@@ -1062,7 +1062,8 @@ struct spn_xyz {
         *work_counter, *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr, *item_sched, *item_count, *item_slot_base,
         *item_seg_ptr;
     int rpa_n_seg = 0, item_n_seg = 0, site_kind = 0;
-    unsigned *status = nullptr;
+    unsigned *status = nullptr;  // in ints, behind the work counters
+    spn::cuh::Pinned corr_host, status_host;  // measurements and the status word on the host
     double *partial = nullptr;
 
     XyzArgs args() const {
@@ -1129,7 +1130,7 @@ struct spn_xyz {
 
     void release() {
         cudaSetDevice(device);
-        void *ptrs[] = {freq, v2, dv2, stage, node_wp, node_c, corr_out, sd, dsd, ints, status, partial};
+        void *ptrs[] = {freq, v2, dv2, stage, node_wp, node_c, corr_out, sd, dsd, ints, partial};
         for (void *p : ptrs)
             if (p) cudaFree(p);
         if (stream) cudaStreamDestroy(stream);
@@ -1243,7 +1244,8 @@ extern "C" int spn_xyz_create(const spn_xyz_desc *d, spn_xyz **out) {
             h->node_c = dalloc<float>(size_t(h->n) * h->max_nodes, "alloc node table");
             h->corr_out = dalloc<float>(4 * size_t(h->n_corr) + 4 * h->nl, "alloc correlation output");
             h->partial = dalloc<double>(size_t(kMaxCorrNodes) * 4 * h->nl, "alloc correlation scratch");
-            h->status = dalloc<unsigned>(1, "alloc status");
+            h->corr_host.alloc((4 * size_t(h->n_corr) + 4 * h->nl) * sizeof(float));
+            h->status_host.alloc(sizeof(unsigned));
             // integer tables, one allocation
             const int nl = h->nl, nr = h->n_range, nc = h->n_corr;
             std::vector<int> img;
@@ -1265,7 +1267,7 @@ extern "C" int spn_xyz_create(const spn_xyz_desc *d, spn_xyz **out) {
             put(d->corr_rid, nc);
             put(d->corr_perm, nc);
             put(nullptr, h->n);  // node counts
-            put(nullptr, 1);     // work counter
+            put(nullptr, 2);     // work counter, status
             put(rpa.sched.data(), int(rpa.sched.size()));
             put(rpa.count.data(), 32);
             put(rpa.slot_base.data(), 32);
@@ -1284,12 +1286,12 @@ extern "C" int spn_xyz_create(const spn_xyz_desc *d, spn_xyz **out) {
                               &h->rpa_count, &h->rpa_slot_base, &h->rpa_seg_ptr, &h->item_sched, &h->item_count,
                               &h->item_slot_base, &h->item_seg_ptr};
             for (size_t k = 0; k < at.size(); ++k) *fields[k] = h->ints + at[k];
+            h->status = reinterpret_cast<unsigned *>(h->work_counter + 1);
             h2d(h->freq, d->freq, h->n, h->stream);
             check_cuda(cudaMemsetAsync(h->sd, 0, vsz * sizeof(float4), h->stream), "memset");
             check_cuda(cudaMemsetAsync(h->dsd, 0, vsz * sizeof(float4), h->stream), "memset");
             check_cuda(cudaMemsetAsync(h->v2, 0, h->n * sizeof(float), h->stream), "memset");
             check_cuda(cudaMemsetAsync(h->dv2, 0, h->n * sizeof(float), h->stream), "memset");
-            check_cuda(cudaMemsetAsync(h->status, 0, sizeof(unsigned), h->stream), "memset");
             check_cuda(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device), "device attribute");
             int per_sm = 0;
             const void *fn = vertex_kernel(h->nl);
@@ -1380,8 +1382,7 @@ extern "C" int spn_xyz_compute_step(spn_xyz *h) {
     return guarded([&] {
         if (!h) throw Error(ErrorType::Argument, "null handle");
         check_cuda(cudaSetDevice(h->device), "cudaSetDevice");
-        check_cuda(cudaMemsetAsync(h->status, 0, sizeof(unsigned), h->stream), "memset status");
-        check_cuda(cudaMemsetAsync(h->work_counter, 0, sizeof(int), h->stream), "memset counter");
+        check_cuda(cudaMemsetAsync(h->work_counter, 0, 2 * sizeof(int), h->stream), "memset counter and status");
         const XyzArgs a = h->args();
         xyz_self_energy_kernel<<<h->n, 128, 0, h->stream>>>(a);
         check_cuda(cudaGetLastError(), "self-energy launch");
@@ -1415,17 +1416,11 @@ extern "C" int spn_xyz_measure_correlation(spn_xyz *h, float *xx, float *yy, flo
         if (!h) throw Error(ErrorType::Argument, "null handle");
         check_cuda(cudaSetDevice(h->device), "cudaSetDevice");
         launch_correlation(h);
+        const float *v = h->corr_host.fetch(h->corr_out, 4 * size_t(h->n_corr) + 4 * h->nl, h->stream);
         float *const dst[4] = {xx, yy, zz, dd};
         for (int c = 0; c < 4; ++c)
-            if (dst[c])
-                check_cuda(cudaMemcpyAsync(dst[c], h->corr_out + size_t(c) * h->n_corr, h->n_corr * sizeof(float),
-                                           cudaMemcpyDeviceToHost, h->stream),
-                           "D2H");
-        if (chi)
-            check_cuda(cudaMemcpyAsync(chi, h->corr_out + 4 * size_t(h->n_corr), 4 * h->nl * sizeof(float),
-                                       cudaMemcpyDeviceToHost, h->stream),
-                       "D2H");
-        check_cuda(cudaStreamSynchronize(h->stream), "correlation sync");
+            if (dst[c]) std::copy(v + size_t(c) * h->n_corr, v + size_t(c + 1) * h->n_corr, dst[c]);
+        if (chi) std::copy(v + 4 * size_t(h->n_corr), v + 4 * size_t(h->n_corr) + 4 * h->nl, chi);
     });
 }
 
@@ -1433,9 +1428,7 @@ extern "C" int spn_xyz_is_diverged(spn_xyz *h, int *diverged) {
     return guarded([&] {
         if (!h || !diverged) throw Error(ErrorType::Argument, "null argument");
         check_cuda(cudaSetDevice(h->device), "cudaSetDevice");
-        unsigned st = 0;
-        check_cuda(cudaMemcpyAsync(&st, h->status, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream), "D2H");
-        check_cuda(cudaStreamSynchronize(h->stream), "status sync");
+        const unsigned st = *h->status_host.fetch(h->status, 1, h->stream);
         if (st & kStatusNodeOverflow) throw Error(ErrorType::Device, "loop-frequency node table overflow");
         *diverged = (st & kStatusNaN) ? 1 : 0;
     });

@@ -73,7 +73,7 @@ def test_tri_flow_matches_oracle(lattice, rng, n, mesh, tables):
     check(tab, spin, freq, (0.4 * float(freq[0]), 0.37, float(freq[n // 2]), 1.5 * float(freq[-1])), 3 * rng + n)
 
 
-@pytest.mark.parametrize("n", [24, 40])
+@pytest.mark.parametrize("n", [12, 20, 24, 40])
 def test_tri_operand_chunks_match_oracle(n):
     tab, spin = tables_of("honeycomb", 8)
     tab, spin = arbitrary_tables(tab, spin, n)
