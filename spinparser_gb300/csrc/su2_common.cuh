@@ -169,11 +169,11 @@ int batch_vertex_blocks_per_sm(int cls, size_t smem);
 void launch_batch_vertex(const BatchVertexArgs &b, int cls, int grid, cudaStream_t stream);
 // Vertex-kernel class of a flow (one kernel instance per class): for nl <= 32 (outer-product RPA with
 // w = 8, 16, 24, 32) 0-3, a warp per item of three triples (site_exchange_kind 0), or 11-14, a warp
-// per triple; 6-10 for 33 <= nl <= 128 (outer-product RPA with w = 48, 64, 80, 96, 128, a CTA per
-// triple); 4 and 5 are unused.
-constexpr int kVertexClasses = 15;
+// per triple; for 33 <= nl <= 128 (w = 48, 64, 80, 96, 128) 6-10, a CTA per triple, or for at most
+// 64 sites and site_exchange_kind 0 15-16, a CTA per item of three; 4 and 5 are unused.
+constexpr int kVertexClasses = 17;
 int vertex_class(int nl, int inv_kind);
-bool vertex_class_big(int cls);  // 6-10
+bool vertex_class_big(int cls);  // a CTA per triple or item
 long long vertex_work_items(int n, int nl, int inv_kind);  // items of the vertex kernel's work counter
 // Lanes of the RPA schedule the vertex kernel of an nl-site flow walks: 32 (a warp per triple)
 // or the CTA's threads (33 to 128 sites).

@@ -408,5 +408,69 @@ __device__ __forceinline__ void node_eval(const float2 *sd, const ItemDesc &d, f
     if (INV && SPT > 1 && kind == 1) __syncwarp();
 }
 
+// Site-local coefficients of a node's t integrand, of T0 and T1 (ka, kb) and of their diagonal densities (kd, ke),
+// from the planes at pair 0 (as in node_eval).
+struct __align__(16) LocalCoef {
+    float2 ka, kb;
+    float kd, ke, pad[2];
+};
+__device__ __forceinline__ void item_local(const float2 *sd, const ItemDesc &d, int step, LocalCoef &k) {
+    const float4 wA = d.w[0], wB = d.w[1], wP = d.w[2], wQ = d.w[3];
+    const int fl = d.flags;
+    float2 L0 = g_value(d, sd, 0, wA, wB), L1 = g_value(d, sd, 1, wP, wQ);
+    float2 L2 = g_value(d, sd, 2, wB, wA), L3 = g_value(d, sd, 3, wQ, wP);
+    if (step != 2 && (fl & kFlDiag)) {
+        L0.y = diag_u(d, sd, 0, fl, wA, wB, L0.y);
+        L1.y = diag_u(d, sd, 1, fl, wP, wQ, L1.y);
+        L2.y = diag_u(d, sd, 2, fl, wB, wA, L2.y);
+        L3.y = diag_u(d, sd, 3, fl, wQ, wP, L3.y);
+    }
+    k.ka.x = __fmaf_rn(0.25f, __fadd_rn(L0.x, L2.x), __fadd_rn(L0.y, L2.y));
+    k.kb.x = __fmaf_rn(0.25f, __fadd_rn(L1.x, L3.x), __fadd_rn(L1.y, L3.y));
+    k.ka.y = __fmaf_rn(-0.75f, __fsub_rn(L2.x, L0.x), __fsub_rn(L2.y, L0.y));
+    k.kb.y = __fmaf_rn(-0.75f, __fsub_rn(L1.x, L3.x), __fsub_rn(L1.y, L3.y));
+    k.kd = __fmaf_rn(-0.75f, __fadd_rn(L0.x, L2.x), __fadd_rn(L0.y, L2.y));
+    k.ke = __fmaf_rn(-0.75f, __fadd_rn(L1.x, L3.x), __fadd_rn(L1.y, L3.y));
+}
+
+// node_eval at one site per lane (its element v in a slab, its own exchange) with the local coefficients given: the lanes of
+// a warp need not hold pair 0.
+__device__ __forceinline__ void site_node(const ItemDesc &d, const LocalCoef &lc, int step, const float2 *v, Acc &acc1,
+                                          Acc &acc2, Acc &acct, float2 &pa, float2 &pb) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const float4 wA = d.w[0], wB = d.w[1], wP = d.w[2], wQ = d.w[3];
+    const int fl = d.flags;
+    const float c = d.c;
+    // density output: opposite sign in the u channel
+    const float2 c1 = make_float2(c, step == 2 ? -c : c), c2 = make_float2(c, step == 0 ? c : -c);
+    const bool diag = step == 1 && __any_sync(kAll, (fl & kFlDiag) != 0);
+    const bool diag_t = __any_sync(kAll, (fl & kFlDiagT) != 0);
+    float2 G0 = g_value(d, v, 0, wA, wB), G1 = g_value(d, v, 1, wP, wQ);
+    float2 G2 = g_value(d, v, 2, wB, wA), G3 = g_value(d, v, 3, wQ, wP);
+    const float2 T0 = t_value(d, v, 0), T1 = t_value(d, v, 1);
+    const float2 r1 = su_term(G0, G1, G2, G3);
+    acc1.add(c1, r1);
+    float2 r = fma2(lc.kb, T1, mul2(lc.ka, T0));
+    pa = mul2(make_float2(c, -c), T0);  // third buffer
+    pb = make_float2(T1.x, -T1.y);      // fourth buffer
+    if (diag_t && (fl & kFlDiagT)) {
+        const float e0 = t_diag(d, v, 0), e1 = t_diag(d, v, 1);
+        r.y = __fmaf_rn(lc.ke, e1, __fmaf_rn(lc.kd, e0, r.y));
+        pa.y = __fmaf_rn(c, e0, pa.y);
+        pb.y = __fadd_rn(e1, pb.y);
+    }
+    acct.add(make_float2(c, c), r);
+    // the second target exchanges a and b: G0 and G2 trade places
+    if (diag) {
+        G0.y = diag_u(d, v, 0, fl, wA, wB, G0.y);
+        G1.y = diag_u(d, v, 1, fl, wP, wQ, G1.y);
+        G2.y = diag_u(d, v, 2, fl, wB, wA, G2.y);
+        G3.y = diag_u(d, v, 3, fl, wQ, wP, G3.y);
+    }
+    const float2 r2 = su_term(G2, G1, G0, G3);
+    acc2.add(c2, r2);
+}
+
+
 }  // namespace dev
 }  // namespace spn

@@ -24,7 +24,8 @@
 // from a per-node shared-memory panel -- and then walks the merged pair list once per t channel,
 // sum m M[rid1][rid2] per rid (every (rid1, rid2) occurs: the pair matrix is dense).  The walk
 // follows a lane-balanced schedule (host/rpa_schedule.hpp).  Lattices of 33 to 128 sites take a
-// CTA per triple (su2_vertex_big_kernel below).
+// CTA per triple (su2_vertex_big_kernel below) or, up to 64 sites whose pairs are their own exchange, per item
+// (su2_vertex_mid_kernel).
 //
 // What bounds it (cubic r6, N = 64, cutoff 2.24): the L1 data path (77 % busy: 25 segment loads of
 // 3.1 wavefronts and 24 shared loads per node) and, at 12 resident warps, dependent-issue and L1
@@ -1296,6 +1297,267 @@ __global__ void __launch_bounds__(kGroupWarps * 32, vertex_min_blocks(MB)) su2_v
 }
 
 // ------------------------------------------------------------------------------------
+// Lattices of 33 to 64 sites whose pairs are their own exchange: one CTA per item of three triples
+// (su2_vertex_mid_kernel<R>).
+//
+// Above 32 sites the t channel's outer-product matrix M = sum over nodes of (c A) x B (w x w,
+// w = 16 R >= Nl) no longer fits one warp's registers.  The CTA's threads build up to 64 node
+// descriptors at once, one per thread, with the site-local coefficients of the t channel.  A warp then takes 32 sites
+// of a node, so that a lane holds the sums of the item's three triples at one site, and writes its part of the
+// node's panel to shared memory (double-buffered: one block barrier per round of four nodes), after which the
+// threads add the round's panels to their blocks of M in registers.  After a transfer frequency M is staged in shared
+// memory; half of the threads walk the merged pair list once while the others build the next descriptors.  Each warp keeps Kahan sums over its nodes; the warps' sums and the RPA
+// term are combined in a fixed order, so results do not depend on the launch.
+//
+// Square r12 (49 sites), N = 47: 2.50 ms, triple by triple (su2_vertex_big_kernel) 2.78, bound by the barriers of the rounds, the
+// latency of slab reads and the shared-memory path (panel reads, 60 %).  Not above 64 sites, nor where the exchange
+// is another pair: the wider panels' and the exchanged planes' traffic and barriers take more than the shared slab reads
+// save (square r20, 121 sites: 5.3 ms against 4.7; pyrochlore r6, 64 sites: 14.0 against 13.7).
+// ------------------------------------------------------------------------------------
+// w = 16 R = 48 or 64: a node's sites are two warps' 32, so NN nodes make a round; the threads are a 16 x 16 grid over M
+template <int R>
+struct MidCfg {
+    static constexpr int w = 16 * R, SPT = 2, NT = 256, NN = NT / 32 / SPT, B = w / 16;
+    static_assert(R == 3 || R == 4, "two warps hold a node's sites");
+};
+constexpr int kMidThreads = 256;
+constexpr int kMidBatch = 64;    // node descriptors built at once
+constexpr int kMidWalkers = 128;  // threads that walk the pairs; the others build descriptors meanwhile
+
+struct MidSmem {
+    size_t pos, ms, desc, loc, panels, parts, rpa, total;
+};
+__host__ __device__ inline MidSmem mid_smem_layout(int R, int n_seg) {
+    const int w = 16 * R, NN = kMidThreads / 64;
+    MidSmem L;
+    size_t o = 0;
+    L.pos = o; o += align16(sizeof(float) * kMaxFreq);
+    L.ms = o; o += align16(sizeof(float2) * (size_t(w) * w + n_seg));  // M and the pair walk's segment partials
+    L.desc = o; o += kMidBatch * sizeof(ItemDesc);
+    L.loc = o; o += kMidBatch * sizeof(LocalCoef);
+    L.panels = o; o += align16(sizeof(float2) * 2 * NN * 2 * size_t(w));  // 2 buffers x nodes x (A, B)
+    L.parts = o; o += align16(sizeof(float2) * 3 * NN * size_t(w));       // per triple, node warp and site
+    L.rpa = o; o += align16(sizeof(float2) * 3 * size_t(w));
+    L.total = o;
+    return L;
+}
+
+// Adds a panel (A = c * third slab, B = fourth slab, w entries each) to the thread's block of M.
+template <int R>
+__device__ __forceinline__ void mid_outer_update(const float2 *pan, int tid, float2 (&M)[MidCfg<R>::B][MidCfg<R>::B]) {
+    using C = MidCfg<R>;
+    const int tr = tid >> 4, tc = tid & 15;
+    float2 av[C::B], bv[C::B];
+#pragma unroll
+    for (int i = 0; i < C::B; ++i) av[i] = pan[tr * C::B + i];
+#pragma unroll
+    for (int j = 0; j < C::B; ++j) bv[j] = pan[C::w + tc * C::B + j];
+#pragma unroll
+    for (int i = 0; i < C::B; ++i)
+#pragma unroll
+        for (int j = 0; j < C::B; ++j) M[i][j] = fma2(av[i], bv[j], M[i][j]);
+}
+
+// The three triples of item `item` of flow `a` by the whole CTA; `pos` the mesh in shared memory.
+template <int R>
+__device__ __forceinline__ void mid_item(const FlowArgs &a, const float *pos, int item, unsigned char *smem,
+                                         const MidSmem &L) {
+    using C = MidCfg<R>;
+    constexpr int w = C::w, NN = C::NN;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int part = warp % C::SPT, nw = warp / C::SPT;  // the warp's sites and its place among the round's nodes
+    ItemDesc *desc = reinterpret_cast<ItemDesc *>(smem + L.desc);
+    float2 *Ms = reinterpret_cast<float2 *>(smem + L.ms);
+    float2 *slots = Ms + w * w;
+    LocalCoef *loc = reinterpret_cast<LocalCoef *>(smem + L.loc);
+    float2 *panels = reinterpret_cast<float2 *>(smem + L.panels);
+    float2 *parts = reinterpret_cast<float2 *>(smem + L.parts);
+    float2 *rpa = reinterpret_cast<float2 *>(smem + L.rpa);
+    int p, q, r;
+    decode_item(item, p, q, r);
+    const int site = 32 * part + lane;
+    const bool valid = site < a.nl;
+    // a lane past the last site reads the last site's element (never used), which lies among the
+    // elements the warp's valid lanes read
+    const float2 *v = a.sd + a.sites[min(site, a.nl - 1)];
+
+    Acc A, B, T;
+    A.clear();
+    B.clear();
+    T.clear();
+    // descriptors and local coefficients of a batch of nodes, by threads first, first + 1, ...
+    auto build = [&](const ItemFreq &f, int cnt, int step, int b0, int first) {
+        const int t = tid - first, at = f.xi * a.max_nodes + b0 + t;
+        if (t < 0 || t >= min(kMidBatch, cnt - b0)) return;
+        make_item(mesh_of(a, pos), a.nl, f, __ldg(a.node_wp + at), __ldg(a.node_c + at), desc[t]);
+        item_local(a.sd, desc[t], step, loc[t]);
+    };
+    ItemFreq f = item_step(pos, 0, p, q, r);
+    int cnt = __ldg(a.node_cnt + f.xi);
+    build(f, cnt, 0, 0, 0);
+    __syncthreads();
+    float2 M[C::B][C::B];
+    int round = 0;
+#pragma unroll 1
+    for (int step = 0; step < 3; ++step) {
+#pragma unroll
+        for (int i = 0; i < C::B; ++i)
+#pragma unroll
+            for (int j = 0; j < C::B; ++j) M[i][j] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+        for (int b0 = 0; b0 < cnt; b0 += kMidBatch) {
+            const int nb = min(kMidBatch, cnt - b0);
+            if (b0) {  // the first batch is built during the pair walk before
+                __syncthreads();  // the previous batch's descriptors are no longer read
+                build(f, cnt, step, b0, 0);
+                __syncthreads();
+            }
+#pragma unroll 1
+            for (int r0 = 0; r0 < nb; r0 += NN, ++round) {
+                const int k = r0 + nw;
+                float2 *buf = panels + size_t(round & 1) * NN * 2 * w;
+                if (k < nb) {
+                    float2 pa, pb;
+                    site_node(desc[k], loc[k], step, v, A, B, T, pa, pb);
+                    if (valid) {
+                        buf[nw * 2 * w + site] = pa;
+                        buf[nw * 2 * w + w + site] = pb;
+                    }
+                }
+                __syncthreads();  // the round's panels are written
+                const int np = min(NN, nb - r0);
+                for (int n = 0; n < np; ++n) mid_outer_update<R>(buf + n * 2 * w, tid, M);
+            }
+        }
+        // RPA term: M staged, the merged pair list walked once, per-site sums
+        __syncthreads();  // every descriptor read is done
+        const int tr = tid >> 4, tc = tid & 15;
+#pragma unroll
+        for (int i = 0; i < C::B; ++i)
+#pragma unroll
+            for (int j = 0; j < C::B; ++j) Ms[(tr * C::B + i) * w + tc * C::B + j] = M[i][j];
+        __syncthreads();
+        // half of the threads walk the pairs, the others build the next transfer frequency's first descriptors
+        if (tid < kMidWalkers) {
+            const int lanes = a.rpa.lanes;
+            for (int l = tid; l < lanes; l += kMidWalkers) {
+                const int cntq = __ldg(a.rpa.count + l);
+                int slot = __ldg(a.rpa.slot_base + l);
+                const int *sched = a.rpa.sched + l;
+                float2 acc = make_float2(0.0f, 0.0f);
+                for (int i = 0; i < cntq; ++i) {
+                    const int e = __ldg(sched + size_t(i) * lanes);
+                    const float m = float((e >> 14) & 0xff);
+                    const int ra = e & 0x7f, rb = (e >> 7) & 0x7f;
+                    acc = fma2(make_float2(m, m), Ms[ra * w + rb], acc);
+                    if (e & (1 << 22)) {
+                        slots[slot++] = acc;
+                        acc = make_float2(0.0f, 0.0f);
+                    }
+                }
+            }
+        }
+        if (step < 2) {
+            f = item_step(pos, step + 1, p, q, r);
+            cnt = __ldg(a.node_cnt + f.xi);
+            build(f, cnt, step + 1, 0, kMidWalkers);
+        }
+        __syncthreads();
+        if (tid < a.nl) {
+            float2 sum = make_float2(0.0f, 0.0f);
+            for (int k = __ldg(a.rpa.seg_ptr + tid); k < __ldg(a.rpa.seg_ptr + tid + 1); ++k) sum = add2(sum, slots[k]);
+            rpa[step * w + tid] = sum;
+        }
+        if (step == 0) swap_acc(A, T);
+        if (step == 1) swap_acc(B, T);
+    }
+
+    // the warps' sums per site (a pairwise tree), then the RPA term (SU2FrgCore.cpp:265-266)
+    if (valid) {
+        parts[(0 * NN + nw) * w + site] = B.value();  // (p,q,r), t channel of step 1
+        parts[(1 * NN + nw) * w + site] = T.value();  // (p,r,q), step 2
+        parts[(2 * NN + nw) * w + site] = A.value();  // (q,p,r), step 0
+    }
+    __syncthreads();
+    const float two_pi = 2.0f * float(kPi);
+    for (int e = tid; e < 3 * a.nl; e += C::NT) {
+        const int k = e / a.nl, j = e - k * a.nl;
+        if ((k == 1 && q == r) || (k == 2 && p == q)) continue;  // the same triple again
+        float2 sums[NN];
+#pragma unroll
+        for (int n = 0; n < NN; ++n) sums[n] = parts[(k * NN + n) * w + j];
+#pragma unroll
+        for (int o = 1; o < NN; o <<= 1)
+#pragma unroll
+            for (int n = 0; n + o < NN; n += 2 * o) sums[n] = add2(sums[n], sums[n + o]);
+        const float2 s = fma2(make_float2(2.0f * a.spin, 8.0f * a.spin), rpa[((k + 1) % 3) * w + j], sums[0]);
+        const int ts = k == 2 ? q : p, tt = k == 0 ? q : (k == 1 ? r : p), tu = k == 1 ? q : r;
+        const float os = s.x / two_pi, od = s.y / two_pi;
+        a.dsd[(size_t(su_index(ts, tu)) * a.n + tt) * a.nl + j] = make_float2(os, od);
+        if (isnan(os) || isnan(od)) atomicOr(a.status, kStatusNaN);
+    }
+}
+
+template <int R>
+__global__ void __launch_bounds__(kMidThreads, 2) su2_vertex_mid_kernel(FlowArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int s_item;
+    const MidSmem L = mid_smem_layout(R, a.rpa.n_seg);
+    float *pos = reinterpret_cast<float *>(smem_raw + L.pos);
+    for (int i = threadIdx.x; i < a.n; i += blockDim.x) pos[i] = a.freq[i];
+    const int items = vertex_items(a.n);
+    for (;;) {
+        __syncthreads();  // the previous item is finished with shared memory
+        if (threadIdx.x == 0) s_item = atomicAdd(a.work_counter, 1);
+        __syncthreads();
+        const int it = s_item;
+        if (it >= items) break;
+        mid_item<R>(a, pos, it, smem_raw, L);
+    }
+}
+
+// Batched form: a persistent grid over the ragged (flow, item) list of the batch's flows of
+// the class; the CTA reloads the flow's argument block and mesh when the flow changes
+// (items are numbered flow by flow).
+template <int R>
+__global__ void __launch_bounds__(kMidThreads, 2) su2_vertex_mid_batch_kernel(BatchVertexArgs b) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int s_item;
+    __shared__ __align__(16) FlowArgs fa;
+    const MidSmem L = mid_smem_layout(R, b.n_seg_max);
+    float *pos = reinterpret_cast<float *>(smem_raw + L.pos);
+    int cur = -1, base = 0;
+    bool skip = false;
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_item = atomicAdd(b.counter, 1);
+        __syncthreads();
+        const int w = s_item;
+        if (w >= b.total) break;
+        int lo = 0, hi = b.n_list - 1;  // last f with prefix[f] <= w
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (__ldg(b.prefix + mid) <= w) lo = mid;
+            else hi = mid - 1;
+        }
+        if (lo != cur) {
+            cur = lo;
+            base = __ldg(b.prefix + lo);
+            const BatchFlow *bf = b.flows + __ldg(b.list + lo);
+            const int *src = reinterpret_cast<const int *>(&bf->a);
+            int *dst = reinterpret_cast<int *>(&fa);
+            for (int i = threadIdx.x; i < int(sizeof(FlowArgs) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
+            skip = bf->phase != kPhaseFlowing;
+            __syncthreads();
+            for (int i = threadIdx.x; i < fa.n; i += blockDim.x) pos[i] = fa.freq[i];
+            __syncthreads();
+        }
+        if (skip) continue;
+        mid_item<R>(fa, pos, w - base, smem_raw, L);
+    }
+}
+
+// ------------------------------------------------------------------------------------
 // Lattices of 33 to 128 sites: one CTA per triple (su2_vertex_big_kernel<R, NT>).
 //
 // Above 32 sites the t channel's outer-product matrix M = sum over nodes of (c A) x B (w x w,
@@ -1605,16 +1867,20 @@ int big_r_of(int nl) {
 int big_class_r(int cls) { return cls == 6 ? 3 : (cls == 7 ? 4 : (cls == 8 ? 5 : (cls == 9 ? 6 : 8))); }
 int big_threads(int r) { return r <= 3 ? 128 : 256; }
 
+// Whether the CTA takes items of three triples (su2_vertex_mid_kernel; classes 15 and 16 for R = 3, 4).
+bool mid_of(int nl, int inv_kind) { return nl > 32 && nl <= 64 && !inv_kind; }
+
 // items of three triples, or single triples
 long long vertex_work_items(int n, int nl, int inv_kind) {
-    return big_r_of(nl) || inv_kind ? (long long)n * n * (n + 1) / 2 : vertex_items(n);
+    return mid_of(nl, inv_kind) || (!big_r_of(nl) && !inv_kind) ? vertex_items(n) : (long long)n * n * (n + 1) / 2;
 }
 
 int vertex_rpa_lanes(int nl) { return big_r_of(nl) ? big_threads(big_r_of(nl)) : 32; }
 
-bool vertex_class_big(int cls) { return cls >= 6 && cls <= 10; }
+bool vertex_class_big(int cls) { return (cls >= 6 && cls <= 10) || cls >= 15; }
 
 int vertex_class(int nl, int inv_kind) {
+    if (mid_of(nl, inv_kind)) return nl <= 48 ? 15 : 16;
     switch (big_r_of(nl)) {
         case 0: return (inv_kind ? 11 : 0) + rpa_outer_width(nl) / 8 - 1;
         case 3: return 6;
@@ -1636,6 +1902,7 @@ size_t warp_area_bytes(int nl, int n_seg, int inv_kind) {
 }  // namespace
 
 size_t vertex_flow_smem_bytes(int nl, const RpaSchedule &rpa, int inv_kind) {
+    if (mid_of(nl, inv_kind)) return mid_smem_layout(big_r_of(nl), rpa.n_seg).total;
     if (const int r = big_r_of(nl)) return big_smem_layout(r, big_threads(r), rpa.n_seg).total;
     return kMaxFreq * sizeof(float) + sched_bytes(rpa, nl) + kWarps * warp_area_bytes(nl, rpa.n_seg, inv_kind);
 }
@@ -1656,10 +1923,12 @@ VertexKernel vertex_kernel(int cls) {
         case 7: return su2_vertex_big_kernel<4, 256>;
         case 8: return su2_vertex_big_kernel<5, 256>;
         case 9: return su2_vertex_big_kernel<6, 256>;
+        case 15: return su2_vertex_mid_kernel<3>;
+        case 16: return su2_vertex_mid_kernel<4>;
         default: return su2_vertex_big_kernel<8, 256>;
     }
 }
-int threads_of(int cls) { return vertex_class_big(cls) ? big_threads(big_class_r(cls)) : kThreads; }
+int threads_of(int cls) { return cls >= 15 ? kMidThreads : (vertex_class_big(cls) ? big_threads(big_class_r(cls)) : kThreads); }
 }  // namespace
 
 // The CTA-per-triple kernel (33..128 sites) reads the schedule from global memory wherever
@@ -1705,12 +1974,15 @@ BatchKernel batch_kernel(int cls) {
         case 7: return su2_vertex_big_batch_kernel<4, 256>;
         case 8: return su2_vertex_big_batch_kernel<5, 256>;
         case 9: return su2_vertex_big_batch_kernel<6, 256>;
+        case 15: return su2_vertex_mid_batch_kernel<3>;
+        case 16: return su2_vertex_mid_batch_kernel<4>;
         default: return su2_vertex_big_batch_kernel<8, 256>;
     }
 }
 }  // namespace
 
 size_t batch_big_smem_bytes(int cls, int n_seg_max) {
+    if (cls >= 15) return mid_smem_layout(cls - 12, n_seg_max).total;
     const int r = big_class_r(cls);
     return big_smem_layout(r, big_threads(r), n_seg_max).total;
 }

@@ -65,3 +65,27 @@ def test_items_match_oracle(lattice, rng, n, mesh, tables):
         for what, a, b in zip(("spin", "density"), got, want):
             assert normwise(a, b) < 1e-5, (what, cutoff)
     flow.close()
+
+
+@pytest.mark.parametrize("lattice,rng,n", [("square", 10, 40), ("square", 13, 40)])
+def test_many_nodes_match_oracle(lattice, rng, n):
+    """More loop frequencies than a CTA builds descriptors at once (64), on the first, middle and last triples.  In 64
+    bits: at the highest frequencies of a random state the oracle's FP32 frequency sums cost it 6e-5."""
+    model, params = LATTICES[lattice]
+    tab = spn.Lattice(lattice, rng, model, params).tables()
+    freq = spn.frequency_exponential(0.02, 20.0, n)
+    g = np.random.RandomState(rng)
+    fn = n * n * (n + 1) // 2
+    v2 = (0.2 * freq).astype(np.float32)
+    ss = g.uniform(-1, 1, fn * tab.n_sites).astype(np.float32)
+    dd = g.uniform(-1, 1, fn * tab.n_sites).astype(np.float32)
+    oracle = Oracle(tab, freq)
+    flow = spn.Su2Flow(tab, freq)
+    flow.set_state(0.01, v2, ss, dd)
+    flow.compute_step()
+    dv2, *got = flow.get_flow()
+    for at in (0, fn // 2, fn - 150):
+        want = oracle.vertex_range(float(np.float32(0.01)), v2, dv2, ss, dd, at, at + 150, fp64=True)
+        for a, b in zip(got, want):
+            assert normwise(a[at * tab.n_sites:(at + 150) * tab.n_sites], b) < 1e-5, at
+    flow.close()
