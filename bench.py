@@ -997,8 +997,13 @@ def main():
     nominal = flops_nominal(tab, n)
     achieved = nominal / (avg_vertex_ms * 1e-3) / 1e12
     achieved_eval = flops_eval / (prof["vertex_ms"] * 1e-3) / 1e12
-    # the dominant kernel: a warp per triple up to 32 sites, a CTA per triple above
-    kernel = "su2_vertex_flow_kernel" if tab.n_sites <= 32 else "su2_vertex_big_kernel"
+    # the dominant kernel: items of three triples where every pair is its own exchange (a warp's up to 32 sites, a
+    # CTA's up to 64), else single triples
+    own = np.array_equal(tab.inv_sites_rid, np.arange(tab.n_sites)) and np.array_equal(tab.sites_rid, np.arange(tab.n_sites))
+    if tab.n_sites <= 32:
+        kernel = "su2_vertex_flow_kernel" if own else "su2_triple_flow_kernel"
+    else:
+        kernel = "su2_vertex_mid_kernel" if own and tab.n_sites <= 64 else "su2_vertex_big_kernel"
     traffic = None
     prof_file = os.path.join(ROOT, "profiles", f"{kernel.replace('su2_', '').replace('_kernel', '')}_{args.workload}.json")
     if os.path.exists(prof_file):

@@ -193,7 +193,7 @@ struct spn_batch {
     // per vertex class (vertex_class): work lists, prefixes, shared memory, grid
     int off_cv[kVertexClasses] = {}, n_cv[kVertexClasses] = {}, off_cp[kVertexClasses] = {}, total_cv[kVertexClasses] = {};
     int warp_area[kVertexClasses] = {}, nl_max = 1, vgrid[kVertexClasses] = {}, sched_ints[kVertexClasses] = {};
-    int nseg_v[kVertexClasses] = {};  // the CTA-per-triple classes: the largest RPA segment count of the list
+    int nseg_v[kVertexClasses] = {};  // the CTA classes: the largest RPA segment count of the list
     // per grouped class: subgroup member table, item prefix, grid
     int off_gm[kGroupClasses] = {}, off_gp[kGroupClasses] = {}, n_sg[kGroupClasses] = {}, total_g[kGroupClasses] = {};
     int nseg_g[kGroupClasses] = {}, ggrid[kGroupClasses] = {};
@@ -368,7 +368,7 @@ struct spn_batch {
             total_cv[c] = prefix.back();
             warp_area[c] = int((area + 15) / 16 * 16);
             // each warp stages its flow's RPA schedule when the largest one is small (warp-per-
-            // triple classes; the CTA-per-triple classes 6-8 read it from global memory)
+            // item and warp-per-triple classes; the CTA classes read it from global memory)
             sched_ints[c] = (!vertex_class_big(c) && stage_sched && sched <= kBatchSchedMaxInts) ? sched : 0;
             vgrid[c] = 0;
             if (n_cv[c] > 0) {

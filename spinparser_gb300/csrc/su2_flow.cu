@@ -11,8 +11,9 @@
 //   3. su2_vertex_flow_kernel   Gamma-dot for every (s,t,u) triple (SU2FrgCore.cpp:171-431)
 // and finalize_step is su2_euler_kernel (SU2FrgCore.cpp:111-137).
 //
-// Vertex-flow work distribution: a persistent grid whose warps pull triples from a device
-// atomic counter (this replaces the reference's MPI/OpenMP LoadManager).  Inside a warp the
+// Vertex-flow work distribution: a persistent grid whose warps (CTAs above 32 sites) pull items of three
+// triples, or single triples, from a device atomic counter (this replaces the reference's MPI/OpenMP
+// LoadManager); which kernel a flow takes is vertex_class's rule (su2_vertex.cu).  Inside a warp the
 // lanes are split into G groups of W lanes: lane = (loop-frequency node group, lattice site),
 // so each group evaluates one loop-frequency node for all Nl sites at once, the slab reads of
 // a support are one coalesced segment, and the group results are combined with warp shuffles.
@@ -639,7 +640,7 @@ spn_su2 *spn::create_flow(const spn_su2_desc *d, cudaStream_t stream) {
             cuda_check(cudaMemsetAsync(h->dv2d, 0, h->n * sizeof(double), h->stream), "memset");
             cuda_check(cudaMemsetAsync(h->status, 0, sizeof(unsigned), h->stream), "memset");
             // RPA schedule balanced over the lanes that walk it (a warp's 32, or the 128 or 256
-            // threads of the CTA-per-triple kernel above 32 sites)
+            // of a CTA's threads above 32 sites)
             RpaHostSchedule rpa = build_rpa_schedule(h->nl, d->overlap_ptr, d->overlap_rid1, d->overlap_rid2,
                                                      vertex_rpa_lanes(h->nl));
             h->rpa_lanes = rpa.lanes;

@@ -1859,8 +1859,8 @@ __global__ void __launch_bounds__(NT, big_min_blocks(R, NT)) su2_vertex_big_batc
 
 }  // namespace
 
-// Lattices of 33 to 128 sites use the CTA-per-triple kernel: w = 16 R >= Nl, R = 3 with 128
-// threads, R = 4, 5, 6, 8 with 256 (classes 6..10).
+// Lattices of 33 to 128 sites: w = 16 R >= Nl.  The CTA-per-triple kernel has 128 threads for R = 3, 256 for
+// R = 4, 5, 6, 8 (classes 6..10).
 int big_r_of(int nl) {
     return nl <= 32 ? 0 : (nl <= 48 ? 3 : (nl <= 64 ? 4 : (nl <= 80 ? 5 : (nl <= 96 ? 6 : 8))));
 }
@@ -1931,7 +1931,7 @@ VertexKernel vertex_kernel(int cls) {
 int threads_of(int cls) { return cls >= 15 ? kMidThreads : (vertex_class_big(cls) ? big_threads(big_class_r(cls)) : kThreads); }
 }  // namespace
 
-// The CTA-per-triple kernel (33..128 sites) reads the schedule from global memory wherever
+// The CTA kernels (33..128 sites) read the schedule from global memory wherever
 // rpa.in_smem says.
 int vertex_flow_blocks_per_sm(int nl, const RpaSchedule &rpa, int inv_kind) {
     const size_t smem = vertex_flow_smem_bytes(nl, rpa, inv_kind);
