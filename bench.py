@@ -22,7 +22,8 @@ JSON line (rank 0):
             F_RHS = F_N (2N+8) (3*100*Nl + 4*sum O) over its CUDA-event launch time, against
             the FP32 FMA throughput measured in-run on the same GPU; "evaluated" uses the
             node counts the step actually used instead of 2N+8; "gather": the kernel's slab
-            gathers (16 segments of Nl pairs per evaluated node) per second against a pure
+            gathers (16 segments of Nl pairs per evaluated node, half of them where the kernel
+            takes three triples at a time, whose nodes share theirs) per second against a pure
             gather kernel timed in-run on the same GPU (spn_measure_gather_peak)
   cpu_baseline  the CPU port of the reference's SU(2) core (the oracle's sources built with the
             reference's flags, -O3 -fopenmp) on all of this host's cores: three complete
@@ -980,6 +981,13 @@ def main():
         full = {"steps": len(cut) - 1, "seconds": fs, "steps_per_s": (len(cut) - 1) / fs,
                 "diverged": flow.is_diverged()}
 
+    # the dominant kernel: items of three triples where every pair is its own exchange (a warp's up to 32 sites, a
+    # CTA's up to 64), else single triples
+    own = np.array_equal(tab.inv_sites_rid, np.arange(tab.n_sites)) and np.array_equal(tab.sites_rid, np.arange(tab.n_sites))
+    if tab.n_sites <= 32:
+        kernel = "su2_vertex_flow_kernel" if own else "su2_triple_flow_kernel"
+    else:
+        kernel = "su2_vertex_mid_kernel" if own and tab.n_sites <= 64 else "su2_vertex_big_kernel"
     fp32_peak, clk = spn.measure_fp32_peak(local)
     gather = None
     if tab.n_sites <= 32:
@@ -987,8 +995,8 @@ def main():
         # L1-resident working sets; the larger rate is the denominator
         g_l2 = spn.measure_gather_peak(tab.n_sites, flow.fn, local)
         g_l1 = spn.measure_gather_peak(tab.n_sites, 512, local)
-        g_ach = gathers_eval / (prof["vertex_ms"] * 1e-3)
-        gather = {"kernel": "su2_vertex_flow_kernel", "achieved": g_ach / 1e9, "peak": max(g_l1, g_l2) / 1e9,
+        g_ach = gathers_eval * (0.5 if own else 1.0) / (prof["vertex_ms"] * 1e-3)
+        gather = {"kernel": kernel, "achieved": g_ach / 1e9, "peak": max(g_l1, g_l2) / 1e9,
                   "unit": "G segments/s", "frac": g_ach / max(g_l1, g_l2), "peak_l2_resident": g_l2 / 1e9,
                   "peak_l1_resident": g_l1 / 1e9,
                   "segment": f"{tab.n_sites} float2 pairs (one interpolation support of one access buffer)",
@@ -997,13 +1005,6 @@ def main():
     nominal = flops_nominal(tab, n)
     achieved = nominal / (avg_vertex_ms * 1e-3) / 1e12
     achieved_eval = flops_eval / (prof["vertex_ms"] * 1e-3) / 1e12
-    # the dominant kernel: items of three triples where every pair is its own exchange (a warp's up to 32 sites, a
-    # CTA's up to 64), else single triples
-    own = np.array_equal(tab.inv_sites_rid, np.arange(tab.n_sites)) and np.array_equal(tab.sites_rid, np.arange(tab.n_sites))
-    if tab.n_sites <= 32:
-        kernel = "su2_vertex_flow_kernel" if own else "su2_triple_flow_kernel"
-    else:
-        kernel = "su2_vertex_mid_kernel" if own and tab.n_sites <= 64 else "su2_vertex_big_kernel"
     traffic = None
     prof_file = os.path.join(ROOT, "profiles", f"{kernel.replace('su2_', '').replace('_kernel', '')}_{args.workload}.json")
     if os.path.exists(prof_file):
