@@ -107,6 +107,21 @@ struct BatchFlow {
     unsigned flags;
 };
 
+// Lets a kernel's launches take any amount of dynamic shared memory up to the device's limit; an error if `bytes` are
+// more than that.  The attribute belongs to the kernel and the device, not to a launch: one set to what a
+// flow needs could be lowered by another thread's smaller flow before the launch.
+template <class K>
+cudaError_t allow_shared(K kernel, size_t bytes) {
+    cudaFuncAttributes at;
+    int device = 0, limit = 0;
+    cudaError_t e = cudaFuncGetAttributes(&at, kernel);
+    if (e == cudaSuccess) e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e != cudaSuccess) return e;
+    if (bytes + at.sharedSizeBytes > size_t(limit)) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit - int(at.sharedSizeBytes));
+}
+
 // Site exchange of a flow: 0, every site's pair and its exchanged pair are the site's own; 1,
 // site j's pair is pair j and the exchange is an involution that fixes pair 0 (every lattice of
 // the factory is one of these); 2, any other tables.

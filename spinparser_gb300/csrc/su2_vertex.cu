@@ -1937,17 +1937,17 @@ int vertex_flow_blocks_per_sm(int nl, const RpaSchedule &rpa, int inv_kind) {
     const size_t smem = vertex_flow_smem_bytes(nl, rpa, inv_kind);
     const int cls = vertex_class(nl, inv_kind);
     VertexKernel k = vertex_kernel(cls);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -1;
+    if (allow_shared(k, smem) != cudaSuccess) return -1;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads_of(cls), smem) != cudaSuccess) return -1;
     return per_sm;
 }
 
+// The kernel's shared-memory limit is raised by vertex_flow_blocks_per_sm when the variant is selected.
 void launch_vertex_flow(const FlowArgs &a, int grid, cudaStream_t stream) {
     const size_t smem = vertex_flow_smem_bytes(a.nl, a.rpa, a.inv_kind);
     const int cls = vertex_class(a.nl, a.inv_kind);
     VertexKernel k = vertex_kernel(cls);
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     k<<<grid, threads_of(cls), smem, stream>>>(a);
 }
 
@@ -1989,7 +1989,7 @@ size_t batch_big_smem_bytes(int cls, int n_seg_max) {
 
 int batch_vertex_blocks_per_sm(int cls, size_t smem) {
     BatchKernel k = batch_kernel(cls);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -1;
+    if (allow_shared(k, smem) != cudaSuccess) return -1;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads_of(cls), smem) != cudaSuccess) return -1;
     return per_sm;
@@ -2024,7 +2024,7 @@ size_t group_vertex_smem_bytes(int cls, int n_seg_max) { return group_smem_layou
 int group_vertex_blocks_per_sm(int cls, int n_seg_max) {
     GroupKernel k = group_kernel(cls);
     const size_t smem = group_vertex_smem_bytes(cls, n_seg_max);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -1;
+    if (allow_shared(k, smem) != cudaSuccess) return -1;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kGroupWarps * 32, smem) != cudaSuccess) return -1;
     return per_sm;

@@ -550,7 +550,7 @@ size_t smem64(int nl, int n_seg) {
 
 int vertex_flow_f64_blocks_per_sm(int nl, const RpaSchedule &rpa) {
     const size_t smem = smem64(nl, rpa.n_seg);
-    if (cudaFuncSetAttribute(kernel64(nl), cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -1;
+    if (allow_shared(kernel64(nl), smem) != cudaSuccess) return -1;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel64(nl), kThreads64, smem) != cudaSuccess) return -1;
     return per_sm;
@@ -558,7 +558,6 @@ int vertex_flow_f64_blocks_per_sm(int nl, const RpaSchedule &rpa) {
 
 void launch_vertex_flow_f64(const FlowArgsT<double> &a, int grid, cudaStream_t stream) {
     const size_t smem = smem64(a.nl, a.rpa.n_seg);
-    cudaFuncSetAttribute(kernel64(a.nl), cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     kernel64(a.nl)<<<grid, kThreads64, smem, stream>>>(a);
 }
 

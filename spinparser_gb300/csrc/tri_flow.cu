@@ -1671,8 +1671,6 @@ std::vector<int> order_rpa_pairs(const spn_tri_desc *d) {
 void launch_correlation(spn_tri *h) {
     const TriArgs a = h->args();
     const size_t smem = size_t(kCorrTWarps) * kCorrOut * h->nl * sizeof(double);
-    check_cuda(cudaFuncSetAttribute(tri_corr_inner_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-               "shared memory limit");
     tri_corr_inner_kernel<<<2 * h->n + 4, kCorrTThreads, smem, h->stream>>>(a);
     check_cuda(cudaGetLastError(), "correlation launch");
     tri_corr_final_kernel<<<1, kCorrThreads, tri_final_smem(h->nl), h->stream>>>(a);
@@ -1756,15 +1754,15 @@ extern "C" int spn_tri_create(const spn_tri_desc *d, spn_tri **out) {
             if (use_products(nl)) {
                 // without the memory for the scratch, or room for the kernel, the pairs are walked
                 void *p = nullptr;
-                if (cudaFuncSetAttribute(tri_lattice_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(lat_smem(nl).total)) ==
-                        cudaSuccess &&
+                if (allow_shared(tri_lattice_kernel, lat_smem(nl).total) == cudaSuccess &&
                     cudaMalloc(&p, lat_scratch_bytes(h->max_nodes) * size_t(h->sms)) == cudaSuccess)
                     h->prod_scratch = static_cast<unsigned char *>(p);
                 else cudaGetLastError();
             }
             int per_sm = 0;
             const auto fn = vertex_kernel(h);
-            check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(vertex_smem(h))), "shared memory limit");
+            check_cuda(allow_shared(fn, vertex_smem(h)), "shared memory limit");
+            check_cuda(allow_shared(tri_corr_inner_kernel, size_t(kCorrTWarps) * kCorrOut * nl * sizeof(double)), "shared memory limit");
             check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, vertex_smem(h)), "occupancy");
             if (per_sm < 1) throw Error(ErrorType::Unsupported, "TRI vertex-flow kernel does not fit on this device");
             h->grid = h->sms * per_sm;
@@ -1833,12 +1831,10 @@ extern "C" int spn_tri_compute_step(spn_tri *h) {
         tri_node_table_kernel<<<h->n, kNodeThreads, 0, h->stream>>>(h->node_args());
         check_cuda(cudaGetLastError(), "node table launch");
         const auto fn = vertex_kernel(h);
-        check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(vertex_smem(h))), "shared memory limit");
         fn<<<h->grid, kThreads, vertex_smem(h), h->stream>>>(a);
         if (h->prod_scratch) {
             check_cuda(cudaGetLastError(), "vertex flow launch");
             const size_t smem = lat_smem(h->nl).total;
-            check_cuda(cudaFuncSetAttribute(tri_lattice_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)), "shared memory limit");
             tri_lattice_kernel<<<h->sms, kLatThreads, smem, h->stream>>>(a);
         }
         check_cuda(cudaGetLastError(), "vertex flow launch");

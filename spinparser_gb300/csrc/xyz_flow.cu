@@ -1295,8 +1295,7 @@ extern "C" int spn_xyz_create(const spn_xyz_desc *d, spn_xyz **out) {
             check_cuda(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device), "device attribute");
             int per_sm = 0;
             const void *fn = vertex_kernel(h->nl);
-            check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(vertex_smem(h))),
-                       "shared memory limit");
+            check_cuda(allow_shared(fn, vertex_smem(h)), "shared memory limit");
             check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, vertex_threads(h->nl), vertex_smem(h)), "occupancy");
             if (per_sm < 1) throw Error(ErrorType::Unsupported, "XYZ vertex-flow kernel does not fit on this device");
             h->grid = h->sms * per_sm;
@@ -1389,7 +1388,6 @@ extern "C" int spn_xyz_compute_step(spn_xyz *h) {
         xyz_node_table_kernel<<<h->n, kNodeThreads, 0, h->stream>>>(h->node_args());
         check_cuda(cudaGetLastError(), "node table launch");
         const void *fn = vertex_kernel(h->nl);
-        check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(vertex_smem(h))), "shared memory limit");
         XyzArgs arg = a;
         void *params[] = {&arg};
         check_cuda(cudaLaunchKernel(fn, dim3(h->grid), dim3(vertex_threads(h->nl)), params, vertex_smem(h), h->stream), "vertex flow launch");
