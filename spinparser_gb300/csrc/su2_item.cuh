@@ -224,12 +224,6 @@ __device__ __forceinline__ void make_item(const Mesh &mi, int nl, const ItemFreq
     d.flags = flags;
 }
 
-// A lane's sites: site k of lane jl is jl + k W (W lanes hold a node); a lane without a site has
-// the last one's.  Element of the site's pair and of its exchanged pair in a slab.
-struct SiteRef {
-    int site, isite;
-};
-
 // (spin, density) of G plane i at one site (v: the site's element of slab 0): four loads,
 // interpolated along u (wo), then along t (wi).
 __device__ __forceinline__ float2 g_value(const ItemDesc &d, const float2 *v, int i, const float4 &wi, const float4 &wo) {
@@ -279,38 +273,32 @@ __device__ __forceinline__ float2 su_term(float2 g0, float2 g1, float2 g2, float
     return r;
 }
 
-// One node at the SPT sites of a lane: adds the two s/u targets to acc1, acc2 and the t target's
+// One node at the SPT sites of a lane, every pair its own exchange: adds the two s/u targets to acc1, acc2 and the t target's
 // local terms to acct, and returns the t channel's panel entries pa = c * (third buffer),
 // pb = fourth buffer per site.  `step` 0: both targets are s-channel nodes; 1: the first is, the
 // second is a u-channel node; 2: both are u-channel nodes.  Every lane of the warp calls it, W
-// lanes per node (jl: the lane's place among them); lanes whose node is not `active` add nothing.
-// INV: false, every site is its own pair and its own exchange.  Otherwise `kind`
-// (site_exchange_kind): 1, site j's pair is pair j and the exchange is an involution that fixes
-// pair 0, so the second target's exchanged planes are another site's of the same node (shuffles,
-// or for SPT > 1 through xch, one float4 per site of the node); 2, any tables: they are read again.
-template <int SPT, int W, bool INV>
-__device__ __forceinline__ void node_eval(const float2 *sd, const ItemDesc &d, float c, int step, bool active, int kind,
-                                          const SiteRef (&sr)[SPT], int jl, float4 *xch, Acc (&acc1)[SPT],
-                                          Acc (&acc2)[SPT], Acc (&acct)[SPT], float2 (&pa)[SPT], float2 (&pb)[SPT]) {
+// lanes per node; lanes whose node is not `active` add nothing.
+template <int SPT, int W>
+__device__ __forceinline__ void node_eval(const float2 *sd, const ItemDesc &d, float c, int step, bool active,
+                                          const int (&site)[SPT], Acc (&acc1)[SPT], Acc (&acc2)[SPT], Acc (&acct)[SPT],
+                                          float2 (&pa)[SPT], float2 (&pb)[SPT]) {
     constexpr unsigned kAll = 0xffffffffu;
     const float4 wA = d.w[0], wB = d.w[1], wP = d.w[2], wQ = d.w[3];
     const int fl = d.flags;
     // density output: opposite sign in the u channel
     const float2 c1 = make_float2(c, step == 2 ? -c : c), c2 = make_float2(c, step == 0 ? c : -c);
     const bool diag = step != 2 && __any_sync(kAll, (fl & kFlDiag) != 0);
-    const bool diag_t = __any_sync(kAll, (fl & (kFlDiagT | kFlExT)) != 0);
+    const bool diag_t = __any_sync(kAll, (fl & kFlDiagT) != 0);
     // the t integrand's site-local coefficients: of T0 and T1, and of their diagonal densities
     float2 ka, kb;
-    float kd = 0.0f, ke = 0.0f, l3 = 0.0f, m3 = 0.0f;
+    float kd = 0.0f, ke = 0.0f;
     float2 q0[SPT], q1[SPT], q2[SPT], q3[SPT];  // the second target's planes
-    auto at = [&](int k, int bit) { return sd + (INV && (fl & bit) ? sr[k].isite : sr[k].site); };
 #pragma unroll
     for (int k = 0; k < SPT; ++k) {
-        const float2 *v0 = at(k, kFlE0), *v1 = at(k, kFlE1), *v2 = at(k, kFlE2), *v3 = at(k, kFlE3);
-        const float2 *vt0 = at(k, kFlT0), *vt1 = at(k, kFlT1);
-        const float2 G0 = g_value(d, v0, 0, wA, wB), G1 = g_value(d, v1, 1, wP, wQ);
-        const float2 G2 = g_value(d, v2, 2, wB, wA), G3 = g_value(d, v3, 3, wQ, wP);
-        const float2 T0 = t_value(d, vt0, 0), T1 = t_value(d, vt1, 1);
+        const float2 *v = sd + site[k];
+        const float2 G0 = g_value(d, v, 0, wA, wB), G1 = g_value(d, v, 1, wP, wQ);
+        const float2 G2 = g_value(d, v, 2, wB, wA), G3 = g_value(d, v, 3, wQ, wP);
+        const float2 T0 = t_value(d, v, 0), T1 = t_value(d, v, 1);
         const float2 r1 = su_term(G0, G1, G2, G3);
         if (active) acc1[k].add(c1, r1);
         q0[k] = G0;
@@ -319,28 +307,15 @@ __device__ __forceinline__ void node_eval(const float2 *sd, const ItemDesc &d, f
         q3[k] = G3;
         float u0 = G0.y, u1 = G1.y, u2 = G2.y, u3 = G3.y;  // densities with the u channel's signs
         if (diag) {
-            u0 = diag_u(d, v0, 0, fl, wA, wB, u0);
-            u1 = diag_u(d, v1, 1, fl, wP, wQ, u1);
-            u2 = diag_u(d, v2, 2, fl, wB, wA, u2);
-            u3 = diag_u(d, v3, 3, fl, wQ, wP, u3);
+            u0 = diag_u(d, v, 0, fl, wA, wB, u0);
+            u1 = diag_u(d, v, 1, fl, wP, wQ, u1);
+            u2 = diag_u(d, v, 2, fl, wB, wA, u2);
+            u3 = diag_u(d, v, 3, fl, wQ, wP, u3);
             if (step == 1) q0[k].y = u0, q1[k].y = u1, q2[k].y = u2, q3[k].y = u3;
         }
-        if (INV && SPT > 1 && kind == 1) xch[jl + k * W] = make_float4(q0[k].x, q0[k].y, q2[k].x, q2[k].y);
         // t channel, SU2FrgCore.cpp:286-302: buffer 0 takes plane G2 at pair 0, 1 G1, 2 G0, 3 G3
         if (k == 0) {
             float2 L0 = make_float2(G0.x, u0), L1 = make_float2(G1.x, u1), L2 = make_float2(G2.x, u2), L3 = make_float2(G3.x, u3);
-            if (INV && kind == 2) {  // pair 0 itself
-                L0 = g_value(d, sd, 0, wA, wB);
-                L1 = g_value(d, sd, 1, wP, wQ);
-                L2 = g_value(d, sd, 2, wB, wA);
-                L3 = g_value(d, sd, 3, wQ, wP);
-                if (diag) {
-                    L0.y = diag_u(d, sd, 0, fl, wA, wB, L0.y);
-                    L1.y = diag_u(d, sd, 1, fl, wP, wQ, L1.y);
-                    L2.y = diag_u(d, sd, 2, fl, wB, wA, L2.y);
-                    L3.y = diag_u(d, sd, 3, fl, wQ, wP, L3.y);
-                }
-            }
             // spin: buffers 0 and 2 (1 and 3) have equal slabs; density: opposite ones
             ka.x = __fmaf_rn(0.25f, __fadd_rn(L0.x, L2.x), __fadd_rn(L0.y, L2.y));
             kb.x = __fmaf_rn(0.25f, __fadd_rn(L1.x, L3.x), __fadd_rn(L1.y, L3.y));
@@ -353,59 +328,25 @@ __device__ __forceinline__ void node_eval(const float2 *sd, const ItemDesc &d, f
             if (diag_t) {
                 kd = __shfl_sync(kAll, __fmaf_rn(-0.75f, __fadd_rn(L0.x, L2.x), __fadd_rn(L0.y, L2.y)), 0, W);
                 ke = __shfl_sync(kAll, __fmaf_rn(-0.75f, __fadd_rn(L1.x, L3.x), __fadd_rn(L1.y, L3.y)), 0, W);
-                if constexpr (INV) {
-                    l3 = __shfl_sync(kAll, __fmaf_rn(0.25f, L3.x, L3.y), 0, W);
-                    m3 = __shfl_sync(kAll, __fmaf_rn(-0.75f, L3.x, L3.y), 0, W);
-                }
             }
         }
         float2 r = fma2(kb, T1, mul2(ka, T0));
         pa[k] = mul2(make_float2(c, -c), T0);  // third buffer
         pb[k] = make_float2(T1.x, -T1.y);      // fourth buffer
-        if (diag_t && (fl & (kFlDiagT | kFlExT))) {
-            const float e0 = t_diag(d, vt0, 0), e1 = t_diag(d, vt1, 1);
+        if (diag_t && (fl & kFlDiagT)) {
+            const float e0 = t_diag(d, v, 0), e1 = t_diag(d, v, 1);
             r.y = __fmaf_rn(ke, e1, __fmaf_rn(kd, e0, r.y));
             pa[k].y = __fmaf_rn(c, e0, pa[k].y);
             pb[k].y = __fadd_rn(e1, pb[k].y);
-            if (INV && (fl & kFlExT)) {  // the fourth buffer reads the other site
-                const float2 *vt3 = at(k, kFlT3);
-                const float2 T3 = t_value(d, vt3, 1);
-                const float y3 = __fsub_rn(t_diag(d, vt3, 1), T3.y);
-                r.x = __fmaf_rn(l3, __fsub_rn(T3.x, T1.x), r.x);
-                r.y = __fmaf_rn(m3, __fsub_rn(y3, pb[k].y), r.y);
-                pb[k] = make_float2(T3.x, y3);
-            }
         }
         if (active) acct[k].add(make_float2(c, c), r);
     }
-    // the second target exchanges a and b: G0 and G2 trade places, with their own site exchange
-    if (INV && SPT > 1 && kind == 1) __syncwarp();
+    // the second target exchanges a and b: G0 and G2 trade places
 #pragma unroll
     for (int k = 0; k < SPT; ++k) {
-        if constexpr (INV) {
-            const bool f0 = ((fl & kFlE0) != 0) != ((fl & kFlF0) != 0), f2 = ((fl & kFlE2) != 0) != ((fl & kFlF2) != 0);
-            if (kind == 2) {
-                const float2 *b0 = at(k, kFlF0), *b2 = at(k, kFlF2);
-                q0[k] = g_value(d, b0, 0, wA, wB);
-                q2[k] = g_value(d, b2, 2, wB, wA);
-                if (diag && step == 1) {
-                    q0[k].y = diag_u(d, b0, 0, fl, wA, wB, q0[k].y);
-                    q2[k].y = diag_u(d, b2, 2, fl, wB, wA, q2[k].y);
-                }
-            } else if (kind == 1 && SPT == 1) {
-                const int s0 = f0 ? sr[k].isite : jl, s2 = f2 ? sr[k].isite : jl;
-                q0[k] = make_float2(__shfl_sync(kAll, q0[k].x, s0, W), __shfl_sync(kAll, q0[k].y, s0, W));
-                q2[k] = make_float2(__shfl_sync(kAll, q2[k].x, s2, W), __shfl_sync(kAll, q2[k].y, s2, W));
-            } else if (kind == 1) {
-                const float4 o = xch[sr[k].isite];
-                if (f0) q0[k] = make_float2(o.x, o.y);
-                if (f2) q2[k] = make_float2(o.z, o.w);
-            }
-        }
         const float2 r = su_term(q2[k], q1[k], q0[k], q3[k]);
         if (active) acc2[k].add(c2, r);
     }
-    if (INV && SPT > 1 && kind == 1) __syncwarp();
 }
 
 // Site-local coefficients of a node's t integrand, of T0 and T1 (ka, kb) and of their diagonal densities (kd, ke),

@@ -442,7 +442,7 @@ struct WarpCtx {
     ItemDesc *desc;
     float2 *panel;  // first panel (A2[w], B2[w]) of the warp; the lane's group has panel g
     const int *sched, *count, *slot_base, *seg_ptr;
-    SiteRef sr[kSpt];
+    int site[kSpt];  // element of the lane's site in a slab
     int g, jl;
 };
 
@@ -463,8 +463,7 @@ __device__ __forceinline__ void setup_ctx(const FlowArgs &a, int lane, unsigned 
 #pragma unroll
     for (int k = 0; k < kSpt; ++k) {
         const int j = min(c.jl + k * W, a.nl - 1);
-        c.sr[k].site = a.sites[j];
-        c.sr[k].isite = a.inv_sites[j];
+        c.site[k] = a.sites[j];
     }
     __syncwarp();
 }
@@ -548,7 +547,7 @@ __device__ __forceinline__ void item_nodes(const float2 *sd, int nl, const ItemD
         const bool active = G == 1 || k < nb;
         const int kk = active ? k : 0;
         float2 pa[kSpt], pb[kSpt];
-        node_eval<kSpt, W, false>(sd, desc[kk], coef(kk), step, active, 0, c.sr, c.jl, nullptr, A, B, T, pa, pb);
+        node_eval<kSpt, W>(sd, desc[kk], coef(kk), step, active, c.site, A, B, T, pa, pb);
         float2 *pan = c.panel + c.g * 16 * MB + c.jl;
 #pragma unroll
         for (int s = 0; s < kSpt; ++s)

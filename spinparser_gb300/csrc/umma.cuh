@@ -30,9 +30,6 @@ __device__ __forceinline__ void tmem_free(uint32_t addr, uint32_t cols) {
 }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// shared-memory writes of this thread become visible to the tensor core's reads
-__device__ __forceinline__ void fence_operands() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
 // generic-proxy accesses of this thread, to shared and global memory, come before later bulk copies
 __device__ __forceinline__ void fence_copies() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
@@ -116,16 +113,7 @@ __device__ __forceinline__ void product(uint32_t d_hi, uint32_t d_lo, uint32_t a
     }
 }
 
-// Four columns of this thread's lane (lane 32 (warp % 4) + lane id of the addressed rows).
-__device__ __forceinline__ void load4(uint32_t addr, float (&v)[4]) {
-    uint32_t r[4];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
-}
-// The same for 16 columns.
+// 16 columns of this thread's lane (lane 32 (warp % 4) + lane id of the addressed rows).
 __device__ __forceinline__ void load16(uint32_t addr, float (&v)[16]) {
     uint32_t r[16];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
