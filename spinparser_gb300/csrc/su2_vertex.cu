@@ -30,7 +30,7 @@
 // What bounds it (cubic r6, N = 64, cutoff 2.24): the L1 data path (77 % busy: 25 segment loads of
 // 3.1 wavefronts and 24 shared loads per node) and, at 12 resident warps, dependent-issue and L1
 // latency (issue 48 %).  Evaluated triple by triple, each channel with its own gathers, the same
-// launch took 5.73 ms (the L1 data path at 95 %); by items it takes 3.56 ms.  Padding the slabs to
+// launch took 5.73 ms (the L1 data path at 95 %); by items it takes 3.50 ms.  Padding the slabs to
 // whole cache lines takes the loads to 2.0 wavefronts but not the time down (3.55 ms).
 #include <type_traits>
 #include "su2_common.cuh"
