@@ -1037,18 +1037,28 @@ __device__ __forceinline__ void worker_sync() { asm volatile("bar.sync 1, %0;" :
 
 // Stores the lane's rows 4 lane .. 4 lane + 3 of slab pair k, four operands of three terms: x[operand][row].  The lanes fill
 // whole sectors.
-__device__ __forceinline__ void lat_store(unsigned char *dst, int blocks, int k, int lane, const float (&x)[4][4]) {
+template <class Split>
+__device__ __forceinline__ void lat_store(unsigned char *dst, int blocks, int k, int lane, const float (&x)[4][4], Split &&split) {
     unsigned char *p = dst + (k >> 3) * kLatGroup + (lane >> 4) * 1024 + umma::block_offset(lane & 15, k & 7);
     const size_t term = size_t(blocks) * kLatGroup;
 #pragma unroll
     for (int o = 0; o < 4; ++o) {
         uint2 h, m, l;
-        umma::split2(x[o][0], x[o][1], h.x, m.x, l.x);
-        umma::split2(x[o][2], x[o][3], h.y, m.y, l.y);
+        split(x[o][0], x[o][1], h.x, m.x, l.x);
+        split(x[o][2], x[o][3], h.y, m.y, l.y);
         *reinterpret_cast<uint2 *>(p + 3 * o * term) = h;
         *reinterpret_cast<uint2 *>(p + (3 * o + 1) * term) = m;
         *reinterpret_cast<uint2 *>(p + (3 * o + 2) * term) = l;
     }
+}
+__device__ __forceinline__ void lat_store(unsigned char *dst, int blocks, int k, int lane, const float (&x)[4][4]) {
+    float top = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) top = fmaxf(top, fabsf(x[i >> 2][i & 3]));
+    if (top <= umma::kSplitMax)
+        lat_store(dst, blocks, k, lane, x, [](float u, float v, uint32_t &h, uint32_t &m, uint32_t &l) { umma::split2(u, v, h, m, l); });
+    else
+        lat_store(dst, blocks, k, lane, x, [](float u, float v, uint32_t &h, uint32_t &m, uint32_t &l) { umma::split2_any(u, v, h, m, l); });
 }
 
 // Copies the three terms of a chunk.
@@ -1280,7 +1290,8 @@ __global__ void __launch_bounds__(kLatThreads, 1) tri_lattice_kernel(TriArgs a) 
 #pragma unroll
                         for (int k = 0; k < 16; k += 4)
                             *reinterpret_cast<float4 *>(stage + row * stride + c0 + k) =
-                                make_float4(hi[k] + lo[k], hi[k + 1] + lo[k + 1], hi[k + 2] + lo[k + 2], hi[k + 3] + lo[k + 3]);
+                                make_float4(umma::add_terms(hi[k], lo[k]), umma::add_terms(hi[k + 1], lo[k + 1]),
+                                            umma::add_terms(hi[k + 2], lo[k + 2]), umma::add_terms(hi[k + 3], lo[k + 3]));
                 }
                 umma::fence_before();
                 __syncwarp();

@@ -12,6 +12,7 @@
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <cfloat>
 #include <cstdint>
 
 namespace spn {
@@ -125,16 +126,29 @@ __device__ __forceinline__ void load16(uint32_t addr, float (&v)[16]) {
 }
 __device__ __forceinline__ void load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// The three bf16 terms of two values.  An infinite, NaN or overflowing value keeps its leading term alone.
+// The three bf16 terms of two values of magnitudes up to kSplitMax, above which rounding to bf16 may give infinity.
+constexpr float kSplitMax = 3.3e38f;
 __device__ __forceinline__ void split2(float u, float v, uint32_t &h, uint32_t &m, uint32_t &l) {
     const __nv_bfloat162 p = __floats2bfloat162_rn(u, v);
-    const float ru = fabsf(u) < 3.3e38f ? u - __low2float(p) : 0.0f, rv = fabsf(v) < 3.3e38f ? v - __high2float(p) : 0.0f;
+    const float ru = u - __low2float(p), rv = v - __high2float(p);
     const __nv_bfloat162 q = __floats2bfloat162_rn(ru, rv);
     const __nv_bfloat162 s = __floats2bfloat162_rn(ru - __low2float(q), rv - __high2float(q));
     h = *reinterpret_cast<const uint32_t *>(&p);
     m = *reinterpret_cast<const uint32_t *>(&q);
     l = *reinterpret_cast<const uint32_t *>(&s);
 }
+// The terms of any two values: the leading one is cut instead of rounded above kSplitMax, so that every finite value keeps all three.  An
+// infinite value is its leading term alone: what the small terms' accumulator then holds is no part of the product (add_terms).
+__device__ __forceinline__ void split2_any(float u, float v, uint32_t &h, uint32_t &m, uint32_t &l) {
+    const float cu = __uint_as_float(__float_as_uint(u) & 0xffff0000u), cv = __uint_as_float(__float_as_uint(v) & 0xffff0000u);
+    const bool bu = fabsf(u) > kSplitMax, bv = fabsf(v) > kSplitMax;
+    split2(bu ? (isinf(u) ? 0.0f : u - cu) : u, bv ? (isinf(v) ? 0.0f : v - cv) : v, h, m, l);
+    if (bu) l = (l & 0xffff0000u) | (m & 0xffffu), m = (m & 0xffff0000u) | (h & 0xffffu), h = (h & 0xffff0000u) | (__float_as_uint(cu) >> 16);
+    if (bv) l = (l & 0xffffu) | (m & 0xffff0000u), m = (m & 0xffffu) | (h & 0xffff0000u), h = (h & 0xffffu) | __float_as_uint(cv);
+}
+// An element of a product from its two accumulators.  An infinite operand makes the large one infinite (or NaN, as the FP32 sum is)
+// and the small one NaN, from infinity times a term that is zero or of the other sign.
+__device__ __forceinline__ float add_terms(float hi, float lo) { return fabsf(hi) <= FLT_MAX ? hi + lo : hi; }
 
 }  // namespace umma
 }  // namespace dev
