@@ -546,7 +546,10 @@ typedef spn_xyz_desc spn_tri_desc; /* the same lattice and spin-permutation tabl
  * v4[it][a][b][rid] += 0.25 J^ab(rid) / normalization for spin components a, b. */
 int spn_tri_initial_state(const spn_lattice *lat, int n_freq, float normalization, float *v2, float *v4);
 
-/* The flow cycle (TRIFrgCore::computeStep / finalizeStep, TRIFrgCore.cpp:76-120). */
+/* The flow cycle (TRIFrgCore::computeStep / finalizeStep, TRIFrgCore.cpp:76-120).  Besides the state
+ * and the flow, a flow of 10 to 32 sites takes the operand scratch of its lattice sum on the device
+ * (spn_tri_scratch: 128 MiB at 32 frequencies on 152 SMs, 926 MiB at 256); where there is no memory
+ * for all of it, fewer CTAs share a smaller one, with the same results. */
 int spn_tri_create(const spn_tri_desc *desc, spn_tri **out);
 int spn_tri_destroy(spn_tri *h);
 int spn_tri_set_state(spn_tri *h, float cutoff, const float *v2, const float *v4);
@@ -560,6 +563,11 @@ int spn_tri_finalize_step(spn_tri *h, float new_cutoff);
  * pointer may be NULL. */
 int spn_tri_measure_correlation(spn_tri *h, float *corr, float *chi);
 int spn_tri_is_diverged(spn_tri *h, int *diverged);
+
+/* The operand scratch that spn_tri_create allocates on a device of n_ctas SMs with free_bytes left
+ * for it: its CTAs and bytes, 0 for flows that take none; SPN_E_CUDA if there is no room for one CTA.
+ * Host only (no device use). */
+int spn_tri_scratch(int n_freq, int n_sites, int n_ctas, long long free_bytes, int *ctas, long long *bytes);
 
 /* One vertex read of the TRI kernels on the host with their code (diagnostics; no device use), on
  * a state v4 in the reference layout, with the arguments of spn_xyz_vertex_probe: value[16] =

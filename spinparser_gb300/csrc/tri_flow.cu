@@ -1498,7 +1498,8 @@ struct spn_tri {
     int *sites, *sites_perm, *inv_sites, *inv_sites_perm, *range_rid, *range_inv, *corr_rid,
         *corr_perm, *node_cnt, *work_counter, *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr, *prod_ptr, *prod_words, *prod_group;
     int rpa_n_seg = 0;
-    unsigned char *prod_scratch = nullptr;  // tri_lattice_kernel runs when not NULL
+    unsigned char *prod_scratch = nullptr;  // tri_lattice_kernel's, of prod_ctas CTAs; it runs when not NULL
+    int prod_ctas = 0;
     unsigned *status = nullptr;  // in ints, behind the work counters
     spn::cuh::Pinned corr_host, status_host;  // measurements and the status word on the host
     double *partial = nullptr;
@@ -1627,6 +1628,15 @@ void (*vertex_kernel(const spn_tri *h))(TriArgs) {
 
 // Whether the t channel runs on the tensor cores (tri_lattice_kernel).
 bool use_products(int nl) { return nl >= kLatMinSites && nl <= 32; }
+
+// CTAs of tri_lattice_kernel: `want`, or as many of them as the device has memory for, by halves; 0 if there is none for one.  The flow
+// is the same with any number, as each triple is one CTA's.
+template <class TryAlloc>
+int scratch_ctas(int want, size_t bytes, TryAlloc &&try_alloc) {
+    for (; want > 0; want /= 2)
+        if (try_alloc(want * bytes)) return want;
+    return 0;
+}
 
 // The RPA pairs as tri_lattice_kernel reads them, two words at a time: the element of the staged M (15 bits) and the
 // images of the four components under perm1 and perm2 (2 bits each); an odd list ends with the zero behind M.  A site's pairs are
@@ -1763,12 +1773,15 @@ extern "C" int spn_tri_create(const spn_tri_desc *d, spn_tri **out) {
             check_cuda(cudaMemsetAsync(h->dv2, 0, h->n * sizeof(float), h->stream), "memset");
             check_cuda(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device), "device attribute");
             if (use_products(nl)) {
-                // without the memory for the scratch, or room for the kernel, the pairs are walked
+                check_cuda(allow_shared(tri_lattice_kernel, lat_smem(nl).total), "shared memory limit");
                 void *p = nullptr;
-                if (allow_shared(tri_lattice_kernel, lat_smem(nl).total) == cudaSuccess &&
-                    cudaMalloc(&p, lat_scratch_bytes(h->max_nodes) * size_t(h->sms)) == cudaSuccess)
-                    h->prod_scratch = static_cast<unsigned char *>(p);
-                else cudaGetLastError();
+                h->prod_ctas = scratch_ctas(h->sms, lat_scratch_bytes(h->max_nodes), [&](size_t bytes) {
+                    const bool ok = cudaMalloc(&p, bytes) == cudaSuccess;
+                    if (!ok) cudaGetLastError();
+                    return ok;
+                });
+                if (!h->prod_ctas) throw Error(ErrorType::Cuda, "alloc operand scratch: out of memory");
+                h->prod_scratch = static_cast<unsigned char *>(p);
             }
             int per_sm = 0;
             const auto fn = vertex_kernel(h);
@@ -1846,7 +1859,7 @@ extern "C" int spn_tri_compute_step(spn_tri *h) {
         if (h->prod_scratch) {
             check_cuda(cudaGetLastError(), "vertex flow launch");
             const size_t smem = lat_smem(h->nl).total;
-            tri_lattice_kernel<<<h->sms, kLatThreads, smem, h->stream>>>(a);
+            tri_lattice_kernel<<<h->prod_ctas, kLatThreads, smem, h->stream>>>(a);
         }
         check_cuda(cudaGetLastError(), "vertex flow launch");
     });
@@ -1873,6 +1886,22 @@ extern "C" int spn_tri_measure_correlation(spn_tri *h, float *corr, float *chi) 
         const float *v = h->corr_host.fetch(h->corr_out, n + 16 * h->nl, h->stream);
         if (corr) std::copy(v, v + n, corr);
         if (chi) std::copy(v + n, v + n + 16 * h->nl, chi);
+    });
+}
+
+extern "C" int spn_tri_scratch(int n_freq, int n_sites, int n_ctas, long long free_bytes, int *ctas, long long *bytes) {
+    return guarded([&] {
+        if (n_freq < 2 || n_freq > kMaxFreq || n_sites < 1 || n_sites > kMaxSites || n_ctas < 1 || free_bytes < 0 || !ctas || !bytes)
+            throw Error(ErrorType::Argument, "spn_tri_scratch: bad argument");
+        *ctas = 0;
+        *bytes = 0;
+        if (!use_products(n_sites)) return;
+        *ctas = scratch_ctas(n_ctas, lat_scratch_bytes(2 * n_freq + 8), [&](size_t want) {
+            if (want > size_t(free_bytes)) return false;
+            *bytes = (long long)want;
+            return true;
+        });
+        if (!*ctas) throw Error(ErrorType::Cuda, "alloc operand scratch: out of memory");
     });
 }
 
