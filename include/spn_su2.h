@@ -370,8 +370,10 @@ int spn_batch_set_variant(spn_batch *b, int npi, int use_graph);
  * flows of one lattice, range and frequency count, admitted together) have the same
  * loop-frequency nodes and interpolation supports; groups of at least min_group such flows
  * (0 = off, the default; spn_batch_autotune may switch it on) are evaluated by a kernel that
- * builds each node's supports once per subgroup and evaluates them for all its flows.  Subgroups hold at most the kernel's flows
- * per block divided by cap_divisor (1, 2 or 4; default 1).  No counterpart in the reference,
+ * builds each node's supports once per subgroup and evaluates them for all its flows.  Subgroups
+ * hold at most the kernel's flows per block divided by cap_divisor (1, 2 or 4; default 1).  Of
+ * lattices on which a pair's exchange is another pair, only subgroups that fill the kernel's block,
+ * of at most 24 sites, are evaluated so: smaller ones are faster flow by flow.  No counterpart in the reference,
  * which runs one flow per process.  Results are bit-identical to the per-flow kernel's. */
 int spn_batch_set_grouping(spn_batch *b, int min_group, int cap_divisor);
 /* Holds a flow out of the following steps (paused = 1) or lets it take part again (0).  A

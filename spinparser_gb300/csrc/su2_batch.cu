@@ -34,7 +34,6 @@ namespace {
 
 constexpr int kClasses = 3;  // measurement classes: sites per lane 1, 2, 4
 constexpr int kBatchSchedMaxInts = 3072;  // per-warp staged RPA schedule (12 KB) at most
-constexpr int kGroupClasses = 4;  // grouped vertex classes: vertex classes 0..3
 constexpr int kCounters = kVertexClasses + kGroupClasses;
 
 __global__ void batch_prepare_kernel(BatchFlow *flows, const int *list, int n, int *counters) {
@@ -299,14 +298,14 @@ struct spn_batch {
             nl_max = std::max(nl_max, f.h->nl);
             if (f.phase == kPhaseFlowing) {
                 flowing.push_back(int(i));
-                if (min_group > 0 && vc < kGroupClasses && group_vertex_eligible(f.h->nl, f.h->inv_kind))
+                if (min_group > 0 && group_vertex_class(f.h->nl, f.h->inv_kind) >= 0)
                     buckets[{f.share_id, f.step}].push_back(int(i));
                 else
                     cv[vc].push_back(int(i));
             }
         }
         // groups large enough go to the grouped kernel in balanced subgroups of at most
-        // gmax / group_cap_div flows; the rest to the per-flow kernel
+        // gmax / group_cap_div flows (in full ones alone where only those pay); the rest to the per-flow kernel
         std::vector<int> gm[kGroupClasses], gp[kGroupClasses];
         n_grouped = 0;
         for (int c = 0; c < kGroupClasses; ++c) {
@@ -315,22 +314,23 @@ struct spn_batch {
         }
         for (auto &kv : buckets) {
             const std::vector<int> &v = kv.second;
-            const int vc = vertex_class(flows[v[0]].h->nl, 0);
-            if (int(v.size()) < min_group) {
-                cv[vc].insert(cv[vc].end(), v.begin(), v.end());
-                continue;
-            }
-            const int gmax = group_vertex_gmax();
+            const spn_su2 *h = flows[v[0]].h;
+            const int gc = group_vertex_class(h->nl, h->inv_kind);
+            const int gmax = group_vertex_gmax(gc);
             const int cap = std::max(1, gmax / group_cap_div);
-            const int parts = (int(v.size()) + cap - 1) / cap;
+            size_t shared = int(v.size()) < min_group ? 0 : v.size();  // flows that go to the grouped kernel
+            if (group_full_only(gc)) shared = cap < gmax ? 0 : shared / gmax * gmax;
+            const int vc = vertex_class(h->nl, h->inv_kind);
+            cv[vc].insert(cv[vc].end(), v.begin() + shared, v.end());
+            const int parts = (int(shared) + cap - 1) / cap;
             size_t at = 0;
             for (int q = 0; q < parts; ++q) {
-                const size_t take = (v.size() - at) / size_t(parts - q);  // balanced sizes
-                for (int m = 0; m < gmax; ++m) gm[vc].push_back(m < int(take) ? v[at + m] : -1);
-                const long long next = gp[vc].back() + vertex_work_items(flows[v[at]].h->n, flows[v[at]].h->nl, 0);
+                const size_t take = (shared - at) / size_t(parts - q);  // balanced sizes
+                for (int m = 0; m < gmax; ++m) gm[gc].push_back(m < int(take) ? v[at + m] : -1);
+                const long long next = gp[gc].back() + vertex_work_items(h->n, h->nl, h->inv_kind);
                 if (next >= (1ll << 31)) throw Error(ErrorType::Unsupported, "batch work list beyond 2^31 items");
-                gp[vc].push_back(int(next));
-                for (size_t m = 0; m < take; ++m) nseg_g[vc] = std::max(nseg_g[vc], flows[v[at + m]].h->rpa_n_seg);
+                gp[gc].push_back(int(next));
+                for (size_t m = 0; m < take; ++m) nseg_g[gc] = std::max(nseg_g[gc], flows[v[at + m]].h->rpa_n_seg);
                 at += take;
                 n_grouped += int(take);
             }
@@ -454,7 +454,7 @@ struct spn_batch {
                 g.prefix = L + off_gp[c];
                 g.n_sg = n_sg[c];
                 g.total = total_g[c];
-                g.gmax = group_vertex_gmax();
+                g.gmax = group_vertex_gmax(c);
                 g.counter = d_counters + kVertexClasses + c;
                 g.n_seg_max = nseg_g[c];
                 launch_group_vertex(g, c, ggrid[c], stream);

@@ -162,8 +162,8 @@ struct BatchVertexArgs {
     int n_seg_max;  // classes 6-8 (CTA per triple): the largest RPA segment count of the list
 };
 // Grouped batches (flows sharing mesh, lattice tables and cutoff; see su2_vertex.cu): one
-// persistent launch per vertex class 0..3 over (subgroup, triple) items.  A subgroup holds up
-// to group_vertex_gmax() flows: members[sg * gmax + q] is the record index of member q, -1
+// persistent launch per group class over (subgroup, item) pairs.  A subgroup holds up
+// to group_vertex_gmax(cls) flows: members[sg * gmax + q] is the record index of member q, -1
 // after the last; its items are prefix[sg] .. prefix[sg + 1] - 1 (its flows' vertex_work_items).
 // n_seg_max: the largest RPA segment count of the flows in the launch.
 struct GroupVertexArgs {
@@ -173,8 +173,12 @@ struct GroupVertexArgs {
     int *counter;
     int n_seg_max;
 };
-bool group_vertex_eligible(int nl, int inv_kind);  // 5 <= nl <= 32, every pair its own exchange
-int group_vertex_gmax();  // flows of a subgroup
+// Group classes: 0-3, the flows of vertex classes 0-3 (by items) of 5 to 32 sites, and 4-6, those of 11-13 (by triples) of 5 to
+// 24, whose subgroups are full; -1 for others.
+constexpr int kGroupClasses = 7;
+int group_vertex_class(int nl, int inv_kind);
+inline bool group_full_only(int cls) { return cls >= 4; }
+int group_vertex_gmax(int cls);  // flows of a subgroup
 size_t group_vertex_smem_bytes(int cls, int n_seg_max);
 int group_vertex_blocks_per_sm(int cls, int n_seg_max);
 void launch_group_vertex(const GroupVertexArgs &g, int cls, int grid, cudaStream_t stream);

@@ -45,6 +45,7 @@ using namespace spn::dev;
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
 constexpr int kBatch = 32;  // nodes whose descriptors a warp builds at once (phase A)
+constexpr int kGroupWarps = 4;  // warps of a grouped kernel's CTA
 constexpr double kPi = 3.14159265358979323846;
 
 struct __align__(16) NodeDesc {
@@ -1152,6 +1153,410 @@ __global__ void __launch_bounds__(kThreads) su2_triple_batch_kernel(BatchVertexA
     }
 }
 
+// Grouped batches of such flows (see below, su2_vertex_group_kernel).  A CTA takes one triple for a
+// subgroup of up to kGroupWarps * 32 / W flows: its threads build each node's supports once, in chunks of 32
+// nodes, and every warp evaluates them for 32 / W flows at once, lane = (flow, site).  The node coefficients
+// and the t channel's site-local values are per flow.
+//
+// The result of every flow is the single-flow kernel's, bit for bit: a flow's W lanes keep the
+// single-flow kernel's G = 32 / W Kahan accumulator pairs (node k of a channel adds into pair
+// k mod G, the RPA term into pair 0 after the t channel) and combine them in its order, and
+// the outer-product matrix M adds the nodes' panels in ascending order.  The pair walk follows
+// the same 32-chunk schedule, each of the flow's W lanes walking chunks l, l + W, ...
+//
+// Only full subgroups of at most 24 sites take it (us a step of 8 flows, alone and here, early and late in the flow: pyrochlore r3,
+// 9 sites, N = 32, one subgroup: 1020, 727 and 2866, 2381; r4, 18 sites, N = 24, two: 648, 599 and 1762, 1719; half
+// subgroups: 1020, 1299 and 648, 1087; four flows of r5, 31 sites, N = 24: 490, 506 and 1153, 1142).
+// Supports of the four site-local access buffers of a t-channel node (the values cbs ... icad2
+// of make_desc are local_pair of these with a flow's state).
+struct LocDesc {
+    int4 off[4];
+    float4 w[4];
+    float4 sw[4];
+};
+
+// A node's supports, as make_desc builds them, split over the four threads of a quad (q = 0..3), for a CTA
+// that builds 32 nodes with 128 threads.  Thread q builds main buffer b(q) and, in the t channel,
+// local buffer l(q), from the two magnitudes (y1, y2) that those buffers interpolate; the
+// coordinates come from selects, so the quad runs one instruction stream.  Every coordinate is the
+// value make_desc passes (negations are exact), so the supports are the same bits.  Returns the
+// exchange and sign bits of the thread's buffer; the quad ORs them into d.exch.
+template <int CH>
+__device__ __forceinline__ int make_part(const FlowArgs &a, const float *pos, const Transfer &f, float wp, int q,
+                                         NodeDesc &d, LocDesc &loc) {
+    AB4 ab;
+    const int nl = a.nl, n = a.n;
+    const MeshIndex m{pos, a.n, a.mesh_lo, a.mesh_base, a.mesh_shift};
+    const bool lo2 = q < 2, odd = q & 1;
+    if (CH == kS) {
+        // buffers (t, u): 0 (-A, -B), 1 (P, -Q), 2 (B, A), 3 (-Q, P); (y1, y2) = (A, B) or (P, Q)
+        const float y1 = odd ? f.w1p + wp : f.w1 + wp, y2 = odd ? f.w2p + wp : f.w2 + wp;
+        const Interp<float> i1 = interp_abs(m, y1), i2 = interp_abs(m, y2);
+        const float t = lo2 ? (odd ? y1 : -y1) : (odd ? -y2 : y2);
+        const float u = lo2 ? -y2 : y1;
+        access4i<kS>(n, nl, f.s, t, u, lo2 ? i1 : i2, lo2 ? i2 : i1, f.si, ab);
+        return put_ab(d, q, ab) | (int(ab.exch) << q);
+    } else if (CH == kU) {
+        // buffers (s, t): 0 (A, -D), 1 (P, E), 2 (D, -A), 3 (E, P); (y1, y2) = (A, D) or (P, E)
+        const float y1 = odd ? f.w1p + wp : f.w1 + wp, y2 = odd ? f.w2 - wp : f.w2p - wp;
+        const Interp<float> i1 = interp_abs(m, y1), i2 = interp_abs(m, y2);
+        const float sv = lo2 ? y1 : y2;
+        const float t = lo2 ? (odd ? y2 : -y2) : (odd ? y1 : -y1);
+        access4i<kU>(n, nl, sv, t, f.u, lo2 ? i1 : i2, lo2 ? i2 : i1, f.ui, ab);
+        return put_ab(d, q, ab) | (int(ab.exch) << q);
+    } else {
+        // main buffers (s, u): 0 (C, P), 2 (P, C), 1 (D, -B), 3 (B, -D); local buffers (s, t, u):
+        // 1 (C, -P, -t), 3 (P, -C, -t), 0 (D, -B, t), 2 (B, -D, t); (y1, y2) = (C, P), (P, C),
+        // (D, B), (B, D) for q = 0..3
+        const float C = f.w1 - wp, P = f.w1p + wp, D = f.w2p - wp, B = f.w2 + wp;
+        const float x1 = lo2 ? C : D, x2 = lo2 ? P : B;
+        const float y1 = odd ? x2 : x1, y2 = odd ? x1 : x2;
+        const Interp<float> i1 = interp_abs(m, y1), i2 = interp_abs(m, y2);
+        const int bi = (int(odd) << 1) | (q >> 1), li = (int(odd) << 1) | (1 - (q >> 1));
+        access4i<kT>(n, nl, y1, f.t, lo2 ? y2 : -y2, i1, i2, f.ti, ab);
+        const int bits = put_ab(d, bi, ab) | (int(ab.exch) << bi);
+        access4i<kU>(n, nl, y1, -y2, lo2 ? -f.t : f.t, i1, i2, f.ti, ab);
+        loc.off[li] = make_int4(ab.off[0], ab.off[1], ab.off[2], ab.off[3]);
+        loc.w[li] = make_float4(ab.w[0], ab.w[1], ab.w[2], ab.w[3]);
+        loc.sw[li] = make_float4(ab.sw[0], ab.sw[1], ab.sw[2], ab.sw[3]);
+        return bits;
+    }
+}
+
+// The t channel's eight site-local values of one node for one flow's state (make_desc's
+// local_pair of each local buffer, in the same order).
+__device__ __forceinline__ void triple_local_values(const float2 *sd, const LocDesc &loc, float *lv) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int4 o = loc.off[i];
+        const float4 w = loc.w[i], sw = loc.sw[i];
+        float2 g = make_float2(0.0f, 0.0f);
+        g = fma2(make_float2(w.x, sw.x), __ldg(sd + o.x), g);
+        g = fma2(make_float2(w.y, sw.y), __ldg(sd + o.y), g);
+        g = fma2(make_float2(w.z, sw.z), __ldg(sd + o.z), g);
+        g = fma2(make_float2(w.w, sw.w), __ldg(sd + o.w), g);
+        lv[2 * i] = g.x;
+        lv[2 * i + 1] = g.y;
+    }
+}
+
+constexpr int kTripleChunk = 32;  // nodes whose supports the CTA builds at once (four threads per node)
+static_assert(kGroupWarps * 32 == 4 * kTripleChunk, "the grouped kernel builds a chunk with four threads per node");
+
+// What a lane of a grouped warp needs of its flow (node_term reads a.sd and a.spin).
+struct GroupLaneArgs {
+    const float2 *sd;
+    float spin;
+};
+
+__host__ __device__ constexpr int triple_group_cb(int W) { return W == 8 ? 2 : 4; }
+
+// Adds the outer product of the flow's panel (A2 = c * third slab, B2 = fourth slab; w entries
+// each) to the lane's R x C block of M; the flow's W lanes form a (W / Cb) x Cb grid.
+template <int W, int MB>
+__device__ __forceinline__ void triple_group_outer(const float2 *pan, int jl, float2 (*m)[8 * MB / triple_group_cb(W)]) {
+    constexpr int w = 8 * MB, Cb = triple_group_cb(W), Rb = W / Cb, R = w / Rb, C = w / Cb;
+    const int rb = jl / Cb, cb = jl % Cb;
+    float2 av[R], bv[C];
+#pragma unroll
+    for (int i = 0; i < R; ++i) av[i] = pan[rb * R + i];
+#pragma unroll
+    for (int j = 0; j < C; ++j) bv[j] = pan[w + cb * C + j];
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < C; ++j) m[i][j] = fma2(av[i], bv[j], m[i][j]);
+}
+
+template <int W, int MB>
+struct GroupShape {
+    static constexpr int F = 32 / W;                 // flows per warp
+    static constexpr int GMAX = kGroupWarps * F;     // flows per CTA
+    static constexpr int G = 32 / W;                 // single-flow node groups (accumulator pairs)
+    static constexpr int w = 8 * MB;                 // outer-product width
+    static constexpr int Cb = triple_group_cb(W), R = w / (W / Cb), C = w / Cb;
+};
+
+// Shared-memory layout of the grouped kernel (bytes from the dynamic base, all 16-aligned).
+struct TripleGroupSmem {
+    size_t fa, ptrs, pos, build_desc, build_loc, build_c, build_lv, stage, panels, total;
+};
+__host__ __device__ inline TripleGroupSmem triple_group_smem(int W, int MB, int n_seg_max) {
+    const int F = 32 / W, GMAX = kGroupWarps * F, w = 8 * MB;
+    TripleGroupSmem L;
+    size_t o = 0;
+    L.fa = o; o += align16(sizeof(FlowArgs));
+    L.ptrs = o; o += align16(size_t(GMAX) * (2 * sizeof(void *) + sizeof(void *) + sizeof(void *) + sizeof(int)));
+    L.pos = o; o += align16(sizeof(float) * kMaxFreq);
+    // union: the chunk build area, or (after the t channel) each flow's staged M and slots
+    const size_t u0 = o;
+    L.build_desc = o; o += kTripleChunk * sizeof(NodeDesc);
+    L.build_loc = o; o += kTripleChunk * sizeof(LocDesc);
+    L.build_c = o; o += align16(sizeof(float) * kTripleChunk * GMAX);
+    L.build_lv = o; o += align16(sizeof(float) * 8 * kTripleChunk * GMAX);
+    const size_t build_end = o;
+    L.stage = u0;
+    const size_t stage_end = u0 + align16(sizeof(float2) * size_t(GMAX) * (size_t(w) * w + n_seg_max));
+    o = build_end > stage_end ? build_end : stage_end;
+    L.panels = o; o += align16(sizeof(float2) * size_t(GMAX) * 2 * w);
+    L.total = o;
+    return L;
+}
+
+template <int W, int MB>
+__global__ void __launch_bounds__(kGroupWarps * 32) su2_triple_group_kernel(GroupVertexArgs g) {
+    using S = GroupShape<W, MB>;
+    constexpr int F = S::F, GMAX = S::GMAX, G = S::G, w = S::w, R = S::R, C = S::C;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int s_item;
+    const TripleGroupSmem L = triple_group_smem(W, MB, g.n_seg_max);
+    FlowArgs *fa = reinterpret_cast<FlowArgs *>(smem_raw + L.fa);
+    unsigned char *pb = smem_raw + L.ptrs;
+    const float2 **m_sd = reinterpret_cast<const float2 **>(pb);
+    float2 **m_dsd = reinterpret_cast<float2 **>(pb + GMAX * sizeof(void *));
+    const float **m_nc = reinterpret_cast<const float **>(pb + 2 * GMAX * sizeof(void *));
+    unsigned **m_status = reinterpret_cast<unsigned **>(pb + 3 * GMAX * sizeof(void *));
+    int *m_on = reinterpret_cast<int *>(pb + 4 * GMAX * sizeof(void *));  // member flowing this step
+    float *pos = reinterpret_cast<float *>(smem_raw + L.pos);
+    NodeDesc *desc = reinterpret_cast<NodeDesc *>(smem_raw + L.build_desc);
+    LocDesc *loc = reinterpret_cast<LocDesc *>(smem_raw + L.build_loc);
+    float *ctab = reinterpret_cast<float *>(smem_raw + L.build_c);   // [node][member]
+    float *lvtab = reinterpret_cast<float *>(smem_raw + L.build_lv);  // [node][member][8]
+    float2 *stage = reinterpret_cast<float2 *>(smem_raw + L.stage);
+    float2 *panels = reinterpret_cast<float2 *>(smem_raw + L.panels);
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int gg = lane / W, jl = lane - gg * W;  // flow slot in the warp, site
+    const int fs = warp * F + gg;                 // member index in the subgroup
+    float2 *pan = panels + size_t(fs) * 2 * w;
+    // panel entries of sites >= Nl are never written and stay zero
+    for (int i = tid; i < GMAX * 2 * w; i += blockDim.x) panels[i] = make_float2(0.0f, 0.0f);
+
+    int cur = -1, base = 0, nf = 0;
+    bool live = false;
+    for (;;) {
+        __syncthreads();  // the previous item is finished with the shared areas
+        if (tid == 0) s_item = atomicAdd(g.counter, 1);
+        __syncthreads();
+        const int item = s_item;
+        if (item >= g.total) break;
+        int lo = 0, hi = g.n_sg - 1;  // last subgroup with prefix <= item
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (__ldg(g.prefix + mid) <= item) lo = mid;
+            else hi = mid - 1;
+        }
+        if (lo != cur) {
+            cur = lo;
+            base = __ldg(g.prefix + lo);
+            // leader: the first member that is flowing this step (its node tables are current)
+            int lead = -1, cnt = 0;
+            for (int q = 0; q < GMAX; ++q) {
+                const int fi = __ldg(g.members + size_t(lo) * GMAX + q);
+                if (fi < 0) break;
+                ++cnt;
+                if (lead < 0 && g.flows[fi].phase == kPhaseFlowing) lead = fi;
+            }
+            nf = cnt;
+            live = lead >= 0;
+            if (live) {
+                const BatchFlow *lf = g.flows + lead;
+                const int *src = reinterpret_cast<const int *>(&lf->a);
+                int *dst = reinterpret_cast<int *>(fa);
+                for (int i = tid; i < int(sizeof(FlowArgs) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
+                if (tid < GMAX) {
+                    const int fi = tid < cnt ? __ldg(g.members + size_t(lo) * GMAX + tid) : -1;
+                    const bool on = fi >= 0 && g.flows[fi].phase == kPhaseFlowing;
+                    const BatchFlow *bf = g.flows + (on ? fi : lead);  // idle slots read the leader's data
+                    m_sd[tid] = bf->a.sd;
+                    m_dsd[tid] = bf->a.dsd;
+                    m_nc[tid] = bf->a.node_c;
+                    m_status[tid] = bf->a.status;
+                    m_on[tid] = on ? 1 : 0;
+                }
+            }
+            __syncthreads();
+            if (live)
+                for (int i = tid; i < fa->n; i += blockDim.x) pos[i] = fa->freq[i];
+            __syncthreads();
+        }
+        if (!live) continue;
+        const int it = item - base;
+        const FlowArgs &a = *fa;
+
+        // the triple (as vertex_triple decodes it)
+        const int su = it / a.n, ti = it - su * a.n;
+        int si = int((sqrtf(8.0f * float(su) + 1.0f) - 1.0f) * 0.5f);
+        while (si * (si + 1) / 2 > su) --si;
+        while ((si + 1) * (si + 2) / 2 <= su) ++si;
+        const int ui = su - si * (si + 1) / 2;
+        Transfer f;
+        f.s = pos[si];
+        f.t = pos[ti];
+        f.u = pos[ui];
+        f.w1p = 0.5f * (f.s + f.t + f.u);
+        f.w1 = 0.5f * (f.s - f.t + f.u);
+        f.w2p = 0.5f * (f.s - f.t - f.u);
+        f.w2 = 0.5f * (f.s + f.t - f.u);
+        f.si = si;
+        f.ti = ti;
+        f.ui = ui;
+
+        const bool mine = fs < nf && m_on[fs];
+        const GroupLaneArgs la{m_sd[fs < nf ? fs : 0], a.spin};
+        Lane<1> ln;
+        ln.j[0] = jl;
+        ln.valid[0] = jl < a.nl;
+        ln.site[0] = ln.valid[0] ? a.sites[jl] : 0;
+        ln.isite[0] = ln.valid[0] ? a.inv_sites[jl] : 0;
+        TExchange tx;
+        tx.A2 = pan;
+        tx.B2 = pan + w;
+
+        float acc_s[G], cmp_s[G], acc_d[G], cmp_d[G];
+#pragma unroll
+        for (int q = 0; q < G; ++q) acc_s[q] = cmp_s[q] = acc_d[q] = cmp_d[q] = 0.0f;
+        float2 M[R][C];
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+            for (int j = 0; j < C; ++j) M[i][j] = make_float2(0.0f, 0.0f);
+
+        // node k of a channel adds into pair k mod G: the pairs rotate after every node, and
+        // pair 0 is realigned at the end of each channel
+        auto rotate = [&]() {
+#pragma unroll
+            for (int q = 0; q + 1 < G; ++q) {
+                float t;
+                t = acc_s[q]; acc_s[q] = acc_s[q + 1]; acc_s[q + 1] = t;
+                t = cmp_s[q]; cmp_s[q] = cmp_s[q + 1]; cmp_s[q + 1] = t;
+                t = acc_d[q]; acc_d[q] = acc_d[q + 1]; acc_d[q + 1] = t;
+                t = cmp_d[q]; cmp_d[q] = cmp_d[q + 1]; cmp_d[q + 1] = t;
+            }
+        };
+
+        auto channel = [&](auto chc, int xi) {
+            constexpr int CH = decltype(chc)::value;
+            const int cnt = __ldg(a.node_cnt + xi);
+            const float *nwp = a.node_wp + size_t(xi) * a.max_nodes;
+            for (int b0 = 0; b0 < cnt; b0 += kTripleChunk) {
+                const int nb = min(kTripleChunk, cnt - b0);
+                __syncthreads();  // the previous chunk is consumed
+                {  // four threads per node build its supports (the CTA's 128 threads: 32 nodes)
+                    const int k = tid >> 2, q = tid & 3;
+                    int bits = 0;
+                    if (k < nb) bits = make_part<CH>(a, pos, f, __ldg(nwp + b0 + k), q, desc[k], loc[k]);
+                    bits |= __shfl_xor_sync(0xffffffffu, bits, 1);
+                    bits |= __shfl_xor_sync(0xffffffffu, bits, 2);
+                    if (k < nb && q == 0) {
+                        desc[k].exch = bits;
+                        desc[k].c = 0.0f;
+                    }
+                    for (int p = tid; p < nb * GMAX; p += blockDim.x) {
+                        const int kk = p / GMAX, qq = p - kk * GMAX;
+                        float c = __ldg(m_nc[qq] + size_t(xi) * a.max_nodes + b0 + kk);
+                        if (CH == kU) c = -c;
+                        ctab[p] = c;
+                    }
+                }
+                __syncthreads();
+                if constexpr (CH == kT) {
+                    for (int p = tid; p < nb * GMAX; p += blockDim.x) {
+                        const int k = p / GMAX, q = p - k * GMAX;
+                        triple_local_values(m_sd[q], loc[k], lvtab + size_t(p) * 8);
+                    }
+                    __syncthreads();
+                }
+                for (int k = 0; k < nb; ++k) {
+                    const int p = k * GMAX + fs;
+                    NodeView v{&desc[k], ctab[p], lvtab + size_t(p) * 8};
+                    float rs[1][1], rd[1][1];
+                    node_term<CH, 1, 1>(la, &v, ln, jl, &tx, rs, rd);
+                    kahan_add(acc_s[0], cmp_s[0], v.c * rs[0][0]);
+                    kahan_add(acc_d[0], cmp_d[0], v.c * rd[0][0]);
+                    rotate();
+                    if constexpr (CH == kT) {
+                        __syncwarp();  // panel written
+                        triple_group_outer<W, MB>(pan, jl, M);
+                        __syncwarp();  // panel read
+                    }
+                }
+            }
+            // realign: pair 0 holds residue 0 again
+            const int extra = (G - cnt % G) % G;
+            for (int r = 0; r < extra; ++r) rotate();
+        };
+
+        channel(std::integral_constant<int, kS>{}, si);
+        channel(std::integral_constant<int, kT>{}, ti);
+
+        // RPA term: stage each flow's M, walk the 32-chunk schedule (chunks jl, jl + W, ...)
+        __syncthreads();  // the build area is free
+        {
+            float2 *Ms = stage + size_t(fs) * (size_t(w) * w + g.n_seg_max);
+            float2 *slots = Ms + w * w;
+            const int rb = jl / S::Cb, cb = jl % S::Cb;
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+#pragma unroll
+                for (int j = 0; j < C; ++j) Ms[(rb * R + i) * w + cb * C + j] = M[i][j];
+            __syncwarp();
+            const int lanes = a.rpa.lanes;
+            const char *mb = reinterpret_cast<const char *>(Ms);
+            for (int ch = jl; ch < lanes; ch += W) {
+                const int cntq = __ldg(a.rpa.count + ch);
+                int slot = __ldg(a.rpa.slot_base + ch);
+                const int *sched = a.rpa.sched + ch;
+                float2 acc = make_float2(0.0f, 0.0f);
+                for (int i = 0; i < cntq; ++i) {
+                    const int e = __ldg(sched + size_t(i) * lanes);
+                    const float2 v = *reinterpret_cast<const float2 *>(mb + (e & 0xffff));
+                    const float m = float((e >> 16) & 0xff);
+                    acc = fma2(make_float2(m, m), v, acc);
+                    if (e < 0) {
+                        slots[slot++] = acc;
+                        acc = make_float2(0.0f, 0.0f);
+                    }
+                }
+            }
+            __syncwarp();
+            if (ln.valid[0]) {
+                float os = 0.0f, od = 0.0f;
+                for (int q = __ldg(a.rpa.seg_ptr + jl); q < __ldg(a.rpa.seg_ptr + jl + 1); ++q) {
+                    const float2 p = slots[q];
+                    os += p.x;
+                    od += p.y;
+                }
+                kahan_add(acc_s[0], cmp_s[0], (2.0f * a.spin) * os);  // SU2FrgCore.cpp:265-266
+                kahan_add(acc_d[0], cmp_d[0], (8.0f * a.spin) * od);
+            }
+        }
+        channel(std::integral_constant<int, kU>{}, ui);
+
+        // the single-flow kernel's combination of its groups: xor-shuffle order
+        float vs[G], vd[G];
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            vs[q] = acc_s[q] - cmp_s[q];
+            vd[q] = acc_d[q] - cmp_d[q];
+        }
+        float ts = vs[0], td = vd[0];
+        if constexpr (G == 2) {
+            ts = vs[0] + vs[1];
+            td = vd[0] + vd[1];
+        } else if constexpr (G == 4) {
+            ts = (vs[0] + vs[1]) + (vs[2] + vs[3]);
+            td = (vd[0] + vd[1]) + (vd[2] + vd[3]);
+        }
+        if (mine && ln.valid[0]) {
+            const float two_pi = 2.0f * float(kPi);
+            const float os = ts / two_pi, od = td / two_pi;
+            m_dsd[fs][size_t(it) * a.nl + jl] = make_float2(os, od);
+            if (isnan(os) || isnan(od)) atomicOr(m_status[fs], kStatusNaN);
+        }
+    }
+}
+
 }  // namespace triple
 
 // ------------------------------------------------------------------------------------
@@ -1164,7 +1569,6 @@ __global__ void __launch_bounds__(kThreads) su2_triple_batch_kernel(BatchVertexA
 // with the single-flow kernel's code, so every flow's result is the single-flow kernel's, bit for
 // bit.
 // ------------------------------------------------------------------------------------
-constexpr int kGroupWarps = 4;
 constexpr int kGroupChunk = kGroupWarps * 32;  // nodes whose supports the CTA builds at once
 static_assert(kGroupChunk % kBatch == 0, "node k must fall to the same node group as in the single-flow kernel");
 
@@ -2009,16 +2413,25 @@ GroupKernel group_kernel(int cls) {
         case 0: return su2_vertex_group_kernel<1>;
         case 1: return su2_vertex_group_kernel<2>;
         case 2: return su2_vertex_group_kernel<3>;
-        default: return su2_vertex_group_kernel<4>;
+        case 3: return su2_vertex_group_kernel<4>;
+        case 4: return triple::su2_triple_group_kernel<8, 1>;
+        case 5: return triple::su2_triple_group_kernel<16, 2>;
+        default: return triple::su2_triple_group_kernel<32, 3>;
     }
 }
+int group_w(int cls) { return lanes_of(cls % 4 + 1); }
 }  // namespace
 
-bool group_vertex_eligible(int nl, int inv_kind) { return nl >= 5 && nl <= 32 && inv_kind == 0; }
+int group_vertex_class(int nl, int inv_kind) {
+    if (nl < 5 || nl > (inv_kind ? 24 : 32)) return -1;
+    return (inv_kind ? 4 : 0) + rpa_outer_width(nl) / 8 - 1;
+}
 
-int group_vertex_gmax() { return kGroupWarps; }
+int group_vertex_gmax(int cls) { return cls < 4 ? kGroupWarps : kGroupWarps * (32 / group_w(cls)); }
 
-size_t group_vertex_smem_bytes(int cls, int n_seg_max) { return group_smem_layout(cls + 1, n_seg_max).total; }
+size_t group_vertex_smem_bytes(int cls, int n_seg_max) {
+    return cls < 4 ? group_smem_layout(cls + 1, n_seg_max).total : triple::triple_group_smem(group_w(cls), cls - 3, n_seg_max).total;
+}
 
 int group_vertex_blocks_per_sm(int cls, int n_seg_max) {
     GroupKernel k = group_kernel(cls);
