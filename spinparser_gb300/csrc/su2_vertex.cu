@@ -421,6 +421,7 @@ __host__ __device__ inline size_t align16(size_t x) { return (x + 15) / 16 * 16;
 // Two sites per lane (half the address arithmetic, descriptor reads and control per node) need so
 // many more registers that they lose: cubic r6 at a mid cutoff 4.32 ms against 3.61.
 constexpr int kSpt = 1;
+constexpr size_t kItemPanels = kBatch * sizeof(ItemDesc);  // a warp's panels follow its descriptors
 // CTAs per SM the register budget is sized for: M takes 4 MB^2 registers a lane, and a budget that
 // spills loses more than the resident warps gain (ms at a mid cutoff with 2, 3, 4 CTAs: 20 sites
 // (MB 3) 4.41, 3.69, 5.06; 31 sites (MB 4) 9.70, 12.26, 16.84; 12 sites (MB 2) 0.96, 0.76, 0.82;
@@ -448,11 +449,11 @@ struct WarpCtx {
 };
 
 template <int MB>
-__device__ __forceinline__ void setup_ctx(const FlowArgs &a, int lane, unsigned char *area, const int *sched,
+__device__ __forceinline__ void setup_ctx(const FlowArgs &a, int lane, unsigned char *area, size_t panel_at, const int *sched,
                                           const int *count, const int *slot_base, const int *seg_ptr, WarpCtx &c) {
     constexpr int W = lanes_of(MB), G = 32 / W;
     c.desc = reinterpret_cast<ItemDesc *>(area);
-    c.panel = reinterpret_cast<float2 *>(area + kBatch * sizeof(ItemDesc));
+    c.panel = reinterpret_cast<float2 *>(area + panel_at);
     c.sched = sched;
     c.count = count;
     c.slot_base = slot_base;
@@ -686,8 +687,8 @@ __global__ void __launch_bounds__(kThreads, vertex_min_blocks(MB)) su2_vertex_fl
         seg_ptr = a.rpa.seg_ptr;
     }
     WarpCtx c;
-    setup_ctx<MB>(a, lane, sbase + sched_bytes(a.rpa, a.nl) + warp * warp_bytes(MB, a.rpa.n_seg), sched, count,
-                  slot_base, seg_ptr, c);
+    setup_ctx<MB>(a, lane, sbase + sched_bytes(a.rpa, a.nl) + warp * warp_bytes(MB, a.rpa.n_seg), kItemPanels, sched,
+                  count, slot_base, seg_ptr, c);
     __syncthreads();
 
     const int items = vertex_items(a.n);
@@ -753,9 +754,9 @@ __global__ void __launch_bounds__(kThreads, vertex_min_blocks(MB)) su2_vertex_ba
                     sch[ns + nc + i] = __ldg(r.slot_base + i);
                 }
                 for (int i = lane; i <= fa->nl; i += 32) sch[ns + 2 * nc + i] = __ldg(r.seg_ptr + i);
-                setup_ctx<MB>(*fa, lane, area, sch, sch + ns, sch + ns + nc, sch + ns + 2 * nc, c);
+                setup_ctx<MB>(*fa, lane, area, kItemPanels, sch, sch + ns, sch + ns + nc, sch + ns + 2 * nc, c);
             } else {
-                setup_ctx<MB>(*fa, lane, area, fa->rpa.sched, fa->rpa.count, fa->rpa.slot_base, fa->rpa.seg_ptr, c);
+                setup_ctx<MB>(*fa, lane, area, kItemPanels, fa->rpa.sched, fa->rpa.count, fa->rpa.slot_base, fa->rpa.seg_ptr, c);
             }
             __syncwarp();
         }
@@ -1564,53 +1565,81 @@ __global__ void __launch_bounds__(kGroupWarps * 32) su2_triple_group_kernel(Grou
 // cutoff (a parameter scan's members of one lattice, range and frequency count, started
 // together) have the same loop-frequency node positions and the same interpolation supports
 // for every (item, node); only the state and the node coefficients (through the self-energy)
-// differ.  A CTA takes one item for a subgroup of up to kGroupWarps flows: its threads build
-// each node's supports once, one node per thread, and every warp evaluates them for its own flow
-// with the single-flow kernel's code, so every flow's result is the single-flow kernel's, bit for
-// bit.
+// differ.  A CTA takes one item for a subgroup of up to kGroupWarps * 32 / W flows: its threads build
+// each node's supports once, one node per thread, and every warp evaluates them for its flows one after the
+// other with the single-flow kernel's code, so every flow's result is the single-flow kernel's, bit for
+// bit.  Where a warp has several flows, their sums wait in shared memory.
+//
+// us a step, flow by flow and here (square lattices, N = 32, early and late in the flow): 6 sites, 16 flows, 917 and 878, 2390 and 2250;
+// 12 sites, 8 flows, 692 and 739, 1982 and 1937; 20 sites, 8 flows, 1075 and 1306, 3414 and 4022.  With one flow a warp at any size (as
+// for 20 sites) the first two took 1138, 2537 and 867, 2302; subgroups of a half and a quarter of the flows 955, 2318
+// and 1109, 2502 at 6 sites.
 // ------------------------------------------------------------------------------------
-constexpr int kGroupChunk = kGroupWarps * 32;  // nodes whose supports the CTA builds at once
-static_assert(kGroupChunk % kBatch == 0, "node k must fall to the same node group as in the single-flow kernel");
+template <int MB>
+struct GroupCfg {
+    static constexpr int F = 32 / lanes_of(MB);      // flows of a warp
+    static constexpr int flows = kGroupWarps * F;    // member m is flow m / kGroupWarps of warp m % kGroupWarps
+    static constexpr int chunk = F > 1 ? 64 : 128;   // nodes whose supports the CTA builds at once
+    static constexpr int sums = F > 1 ? 6 + 2 * MB * MB : 0;  // float2 a lane keeps per flow: three Acc and its block of M
+    static_assert(chunk % kBatch == 0, "node k must fall to the same node group as in the single-flow kernel");
+};
 
 // Shared-memory layout of the grouped kernel (bytes from the dynamic base, all 16-aligned).
 struct GroupSmem {
-    size_t fa, ptrs, pos, desc, coef, warps, warp_size, total;
+    size_t fa, ptrs, pos, desc, coef, sums, warps, panel, warp_size, total;
 };
-__host__ __device__ inline GroupSmem group_smem_layout(int MB, int n_seg_max) {
+template <int MB>
+__host__ __device__ inline GroupSmem group_smem_layout(int n_seg_max) {
+    using C = GroupCfg<MB>;
+    constexpr size_t w = 8 * MB;
     GroupSmem L;
     size_t o = 0;
     L.fa = o; o += align16(sizeof(FlowArgs));
-    L.ptrs = o; o += align16(size_t(kGroupWarps) * (4 * sizeof(void *) + sizeof(int)));
+    L.ptrs = o; o += align16(size_t(C::flows) * (4 * sizeof(void *) + sizeof(int)));
     L.pos = o; o += align16(sizeof(float) * kMaxFreq);
-    L.desc = o; o += kGroupChunk * sizeof(ItemDesc);
-    L.coef = o; o += align16(sizeof(float) * kGroupChunk * kGroupWarps);
-    L.warps = o;  // per warp: as the single-flow kernel's area (its descriptors only as room for M)
-    L.warp_size = warp_bytes(MB, n_seg_max);
+    L.desc = o; o += C::chunk * sizeof(ItemDesc);
+    L.coef = o; o += align16(sizeof(float) * C::chunk * C::flows);
+    L.sums = o; o += size_t(C::flows) * C::sums * 32 * sizeof(float2);
+    L.warps = o;  // per warp: M and the segment partials, and the panels
+    L.panel = align16(sizeof(float2) * (w * w + n_seg_max));
+    L.warp_size = L.panel + 32 / lanes_of(MB) * sizeof(float2) * 2 * w;
     L.total = o + kGroupWarps * L.warp_size;
     return L;
 }
 
+__device__ __forceinline__ void put_acc(float2 *p, const Acc &a) {
+    p[0] = a.sum;
+    p[32] = a.lost;
+}
+__device__ __forceinline__ void get_acc(const float2 *p, Acc &a) {
+    a.sum = p[0];
+    a.lost = p[32];
+}
+
 template <int MB>
 __global__ void __launch_bounds__(kGroupWarps * 32, vertex_min_blocks(MB)) su2_vertex_group_kernel(GroupVertexArgs g) {
+    using C = GroupCfg<MB>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_item;
-    const GroupSmem L = group_smem_layout(MB, g.n_seg_max);
+    const GroupSmem L = group_smem_layout<MB>(g.n_seg_max);
     FlowArgs *fa = reinterpret_cast<FlowArgs *>(smem_raw + L.fa);
     unsigned char *pb = smem_raw + L.ptrs;
     const float2 **m_sd = reinterpret_cast<const float2 **>(pb);
-    float2 **m_dsd = reinterpret_cast<float2 **>(pb + kGroupWarps * sizeof(void *));
-    const float **m_nc = reinterpret_cast<const float **>(pb + 2 * kGroupWarps * sizeof(void *));
-    unsigned **m_status = reinterpret_cast<unsigned **>(pb + 3 * kGroupWarps * sizeof(void *));
-    int *m_on = reinterpret_cast<int *>(pb + 4 * kGroupWarps * sizeof(void *));  // member flowing this step
+    float2 **m_dsd = reinterpret_cast<float2 **>(pb + C::flows * sizeof(void *));
+    const float **m_nc = reinterpret_cast<const float **>(pb + 2 * C::flows * sizeof(void *));
+    unsigned **m_status = reinterpret_cast<unsigned **>(pb + 3 * C::flows * sizeof(void *));
+    int *m_on = reinterpret_cast<int *>(pb + 4 * C::flows * sizeof(void *));  // member flowing this step
     float *pos = reinterpret_cast<float *>(smem_raw + L.pos);
     ItemDesc *desc = reinterpret_cast<ItemDesc *>(smem_raw + L.desc);
     float *ctab = reinterpret_cast<float *>(smem_raw + L.coef);  // [member][node]
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     unsigned char *area = smem_raw + L.warps + warp * L.warp_size;
+    float2 *sums = reinterpret_cast<float2 *>(smem_raw + L.sums) + lane;
     WarpCtx c;
     int cur = -1, base = 0;
     bool live = false;
+    int flows = C::flows;  // places up to the last member that flows
     for (;;) {
         __syncthreads();  // the previous item is finished with the shared areas
         if (tid == 0) s_item = atomicAdd(g.counter, 1);
@@ -1628,8 +1657,8 @@ __global__ void __launch_bounds__(kGroupWarps * 32, vertex_min_blocks(MB)) su2_v
             base = __ldg(g.prefix + lo);
             // leader: the first member that is flowing this step (its node tables are current)
             int lead = -1, cnt = 0;
-            for (int q = 0; q < kGroupWarps; ++q) {
-                const int fi = __ldg(g.members + size_t(lo) * kGroupWarps + q);
+            for (int q = 0; q < C::flows; ++q) {
+                const int fi = __ldg(g.members + size_t(lo) * C::flows + q);
                 if (fi < 0) break;
                 ++cnt;
                 if (lead < 0 && g.flows[fi].phase == kPhaseFlowing) lead = fi;
@@ -1640,10 +1669,10 @@ __global__ void __launch_bounds__(kGroupWarps * 32, vertex_min_blocks(MB)) su2_v
                 const int *src = reinterpret_cast<const int *>(&lf->a);
                 int *dst = reinterpret_cast<int *>(fa);
                 for (int i = tid; i < int(sizeof(FlowArgs) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
-                if (tid < kGroupWarps) {
-                    const int fi = tid < cnt ? __ldg(g.members + size_t(lo) * kGroupWarps + tid) : -1;
+                if (tid < C::flows) {
+                    const int fi = tid < cnt ? __ldg(g.members + size_t(lo) * C::flows + tid) : -1;
                     const bool on = fi >= 0 && g.flows[fi].phase == kPhaseFlowing;
-                    const BatchFlow *bf = g.flows + (on ? fi : lead);  // idle warps have no flow of their own
+                    const BatchFlow *bf = g.flows + (on ? fi : lead);  // idle places have no flow of their own
                     m_sd[tid] = bf->a.sd;
                     m_dsd[tid] = bf->a.dsd;
                     m_nc[tid] = bf->a.node_c;
@@ -1654,47 +1683,75 @@ __global__ void __launch_bounds__(kGroupWarps * 32, vertex_min_blocks(MB)) su2_v
             __syncthreads();
             if (live) {
                 for (int i = tid; i < fa->n; i += blockDim.x) pos[i] = fa->freq[i];
-                setup_ctx<MB>(*fa, lane, area, fa->rpa.sched, fa->rpa.count, fa->rpa.slot_base, fa->rpa.seg_ptr, c);
+                if constexpr (C::F > 1) {
+                    flows = C::flows;
+                    while (!m_on[flows - 1]) --flows;
+                }
+                setup_ctx<MB>(*fa, lane, area, L.panel, fa->rpa.sched, fa->rpa.count, fa->rpa.slot_base, fa->rpa.seg_ptr, c);
             }
             __syncthreads();
         }
         if (!live) continue;
         const FlowArgs &a = *fa;
-        const bool mine = m_on[warp] != 0;
         int p, q, r;
         decode_item(item - base, p, q, r);
-        Acc A[kSpt], B[kSpt], T[kSpt];
-#pragma unroll
-        for (int k = 0; k < kSpt; ++k) {
-            A[k].clear();
-            B[k].clear();
-            T[k].clear();
-        }
+        Acc A[kSpt], B[kSpt], T[kSpt];  // of one flow
+        OuterAcc<MB> M;
 #pragma unroll 1
         for (int step = 0; step < 3; ++step) {
             const ItemFreq f = item_step(pos, step, p, q, r);
-            OuterAcc<MB> M;
-            clear_outer(M);
             const int cnt = __ldg(a.node_cnt + f.xi);
             const float *nwp = a.node_wp + size_t(f.xi) * a.max_nodes;
-            for (int b0 = 0; b0 < cnt; b0 += kGroupChunk) {
-                const int nb = min(kGroupChunk, cnt - b0);
+            for (int b0 = 0; b0 < cnt; b0 += C::chunk) {
+                const int nb = min(C::chunk, cnt - b0);
                 __syncthreads();  // the previous chunk is consumed
                 if (tid < nb) make_item(mesh_of(a, pos), a.nl, f, __ldg(nwp + b0 + tid), 0.0f, desc[tid]);
-                for (int k = lane; k < nb; k += 32)
-                    ctab[warp * kGroupChunk + k] = __ldg(m_nc[warp] + size_t(f.xi) * a.max_nodes + b0 + k);
+                for (int m = warp; m < (C::F > 1 ? flows : C::flows); m += kGroupWarps)
+                    for (int k = lane; k < nb; k += 32)
+                        ctab[m * C::chunk + k] = __ldg(m_nc[m] + size_t(f.xi) * a.max_nodes + b0 + k);
                 __syncthreads();
-                if (mine)
-                    item_nodes<MB>(m_sd[warp], a.nl, desc, nb, step, c, lane,
-                                         [&](int k) { return ctab[warp * kGroupChunk + k]; }, A, B, T, M);
+#pragma unroll 1
+                for (int m = warp; m < (C::F > 1 ? flows : C::flows); m += kGroupWarps) {
+                    if (!m_on[m]) continue;
+                    float2 *kept = sums + m * C::sums * 32;
+                    if (step == 0 && b0 == 0) {
+#pragma unroll
+                        for (int k = 0; k < kSpt; ++k) {
+                            A[k].clear();
+                            B[k].clear();
+                            T[k].clear();
+                        }
+                    } else if constexpr (C::F > 1) {
+                        get_acc(kept, A[0]);
+                        get_acc(kept + 64, B[0]);
+                        get_acc(kept + 128, T[0]);
+                    }
+                    if (b0 == 0) {
+                        clear_outer(M);
+                    } else if constexpr (C::F > 1) {
+#pragma unroll
+                        for (int i = 0; i < 2 * MB * MB; ++i) M.m[i / (2 * MB)][i % (2 * MB)] = kept[(6 + i) * 32];
+                    }
+                    item_nodes<MB>(m_sd[m], a.nl, desc, nb, step, c, lane, [&](int k) { return ctab[m * C::chunk + k]; }, A, B, T, M);
+                    if (b0 + C::chunk >= cnt) {
+                        outer_gather<MB>(a, c, reinterpret_cast<float2 *>(area), lane, M, T);
+                        turn_accs(step, A, B, T);
+                        if (step == 2) {
+                            store_triple<MB>(a, m_dsd[m], m_status[m], c, B, p, q, r);
+                            if (q != r) store_triple<MB>(a, m_dsd[m], m_status[m], c, T, p, r, q);
+                            if (p != q) store_triple<MB>(a, m_dsd[m], m_status[m], c, A, q, p, r);
+                        }
+                    } else if constexpr (C::F > 1) {
+#pragma unroll
+                        for (int i = 0; i < 2 * MB * MB; ++i) kept[(6 + i) * 32] = M.m[i / (2 * MB)][i % (2 * MB)];
+                    }
+                    if constexpr (C::F > 1) {
+                        put_acc(kept, A[0]);
+                        put_acc(kept + 64, B[0]);
+                        put_acc(kept + 128, T[0]);
+                    }
+                }
             }
-            if (mine) outer_gather<MB>(a, c, reinterpret_cast<float2 *>(area), lane, M, T);
-            turn_accs(step, A, B, T);
-        }
-        if (mine) {
-            store_triple<MB>(a, m_dsd[warp], m_status[warp], c, B, p, q, r);
-            if (q != r) store_triple<MB>(a, m_dsd[warp], m_status[warp], c, T, p, r, q);
-            if (p != q) store_triple<MB>(a, m_dsd[warp], m_status[warp], c, A, q, p, r);
         }
     }
 }
@@ -2427,10 +2484,16 @@ int group_vertex_class(int nl, int inv_kind) {
     return (inv_kind ? 4 : 0) + rpa_outer_width(nl) / 8 - 1;
 }
 
-int group_vertex_gmax(int cls) { return cls < 4 ? kGroupWarps : kGroupWarps * (32 / group_w(cls)); }
+int group_vertex_gmax(int cls) { return kGroupWarps * (32 / group_w(cls)); }
 
 size_t group_vertex_smem_bytes(int cls, int n_seg_max) {
-    return cls < 4 ? group_smem_layout(cls + 1, n_seg_max).total : triple::triple_group_smem(group_w(cls), cls - 3, n_seg_max).total;
+    switch (cls) {
+        case 0: return group_smem_layout<1>(n_seg_max).total;
+        case 1: return group_smem_layout<2>(n_seg_max).total;
+        case 2: return group_smem_layout<3>(n_seg_max).total;
+        case 3: return group_smem_layout<4>(n_seg_max).total;
+        default: return triple::triple_group_smem(group_w(cls), cls - 3, n_seg_max).total;
+    }
 }
 
 int group_vertex_blocks_per_sm(int cls, int n_seg_max) {
