@@ -1,9 +1,12 @@
-// Host-side CUDA helpers of the XYZ and TRI cores: status check, device allocation, host to
-// device copy and the grid of elementwise kernels.
+// Host-side CUDA helpers: status check, device allocation, host to device copy, small results on
+// the host and the grid of elementwise kernels.
 #pragma once
 
 #include <cuda_runtime.h>
+#include <unistd.h>
 #include <algorithm>
+#include <cstdlib>
+#include <new>
 #include <string>
 #include "host/capi_common.hpp"
 
@@ -27,30 +30,47 @@ void h2d(T *dst, const T *src, size_t count, cudaStream_t s) {
     if (count) check_cuda(cudaMemcpyAsync(dst, src, count * sizeof(T), cudaMemcpyHostToDevice, s), "cudaMemcpyAsync H2D");
 }
 
-// Page-locked memory that a handle's small results are copied to.  The driver stages a copy to pageable memory and waits for
-// each by itself; a measurement's four or five arrays come in one copy here (square r2, N = 16: 277 -> 214 us for a cutoff
-// step, two measurements and the state in and out).
-class Pinned {
+// Host memory that a handle's small results (a measurement, the status word) are copied to, in one copy each: four copies take 39 us,
+// one 14, and 12.4 to page-locked memory.  It is taken with the first copy, so a flow whose results are not fetched by itself (a batch's)
+// has none, and pages of its own are locked in place: cudaHostAlloc and cudaFreeHost cost 240 us a handle, which a flow of a few
+// steps does not earn back; registering and unregistering 16.
+class HostResults {
   public:
-    Pinned() = default;
-    Pinned(const Pinned &) = delete;
-    Pinned &operator=(const Pinned &) = delete;
-    ~Pinned() { release(); }
-    void alloc(size_t bytes) { check_cuda(cudaHostAlloc(&p_, std::max<size_t>(bytes, 16), cudaHostAllocDefault), "cudaHostAlloc"); }
-    void release() {
-        if (p_) cudaFreeHost(p_);
-        p_ = nullptr;
-    }
-    // `count` elements from the device, once the stream's work so far is done
+    HostResults() = default;
+    HostResults(const HostResults &) = delete;
+    HostResults &operator=(const HostResults &) = delete;
+    ~HostResults() { release(); }
+    // `count` elements from the device, once the stream's work so far is done; valid until the next fetch
     template <class T>
     const T *fetch(const T *src, size_t count, cudaStream_t s) {
+        reserve(count * sizeof(T));
         if (count) check_cuda(cudaMemcpyAsync(p_, src, count * sizeof(T), cudaMemcpyDeviceToHost, s), "D2H");
         check_cuda(cudaStreamSynchronize(s), "D2H sync");
         return static_cast<const T *>(p_);
     }
 
   private:
+    void reserve(size_t bytes) {
+        if (p_ && bytes <= size_) return;
+        release();
+        const size_t page = size_t(sysconf(_SC_PAGESIZE));
+        const size_t size = (std::max<size_t>(bytes, 1) + page - 1) / page * page;
+        p_ = std::aligned_alloc(page, size);
+        if (!p_) throw std::bad_alloc();
+        size_ = size;
+        locked_ = cudaHostRegister(p_, size, cudaHostRegisterDefault) == cudaSuccess;
+        if (!locked_) cudaGetLastError();  // the copies are staged by the driver then
+    }
+    void release() {
+        if (locked_) cudaHostUnregister(p_);
+        std::free(p_);
+        p_ = nullptr;
+        size_ = 0;
+        locked_ = false;
+    }
     void *p_ = nullptr;
+    size_t size_ = 0;
+    bool locked_ = false;
 };
 
 // blocks of 256 threads for an elementwise kernel over n items (grid-stride beyond 4096 blocks)

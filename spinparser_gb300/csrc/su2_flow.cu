@@ -605,8 +605,6 @@ spn_su2 *spn::create_flow(const spn_su2_desc *d, cudaStream_t stream) {
             h->node_cnt = dev_alloc<int>(h->n, "alloc node counts");
             h->status = dev_alloc<unsigned>(2, "alloc status");
             h->work_counter = reinterpret_cast<int *>(h->status + 1);
-            h->status_host.alloc(sizeof(unsigned));
-            h->corr_host.alloc((2 * size_t(h->n_corr) + 2 * h->nl) * (f64 ? sizeof(double) : sizeof(float)));
             h->sites = dev_alloc<int>(h->nl, "alloc sites");
             h->inv_sites = dev_alloc<int>(h->nl, "alloc inv sites");
             h->ov_ptr = dev_alloc<int>(h->nl + 1, "alloc overlap ptr");
@@ -1010,8 +1008,8 @@ void launch_correlation(spn_su2 *h) {
 
 void copy_correlation(spn_su2 *h, float *zz, float *dd, float *chi_zz, float *chi_dd) {
     const size_t count = 2 * size_t(h->n_corr) + 2 * h->nl;
-    const double *v64 = h->fp64() ? h->corr_host.fetch(h->corr_out64, count, h->stream) : nullptr;
-    const float *v = v64 ? nullptr : h->corr_host.fetch(h->corr_out, count, h->stream);
+    const double *v64 = h->fp64() ? h->results.fetch(h->corr_out64, count, h->stream) : nullptr;
+    const float *v = v64 ? nullptr : h->results.fetch(h->corr_out, count, h->stream);
     auto put = [&](float *out, size_t off, int cnt) {
         if (out)
             for (int i = 0; i < cnt; ++i) out[i] = v64 ? float(v64[off + i]) : v[off + i];
@@ -1082,7 +1080,7 @@ extern "C" int spn_su2_measure_correlation_f64(spn_su2 *h, double *zz, double *d
         require_fp64(h);
         cuda_check(cudaSetDevice(h->device), "cudaSetDevice");
         launch_correlation(h);
-        const double *v = h->corr_host.fetch(h->corr_out64, 2 * size_t(h->n_corr) + 2 * h->nl, h->stream);
+        const double *v = h->results.fetch(h->corr_out64, 2 * size_t(h->n_corr) + 2 * h->nl, h->stream);
         auto put = [&](double *out, size_t off, int cnt) {
             if (out) std::copy(v + off, v + off + cnt, out);
         };
@@ -1113,7 +1111,7 @@ extern "C" int spn_su2_is_diverged(spn_su2 *h, int *diverged) {
     return guarded([&] {
         if (!h || !diverged) throw Error(ErrorType::Argument, "null argument");
         cuda_check(cudaSetDevice(h->device), "cudaSetDevice");
-        const unsigned st = *h->status_host.fetch(h->status, 1, h->stream);
+        const unsigned st = *h->results.fetch(h->status, 1, h->stream);
         if (st & kStatusNodeOverflow) throw Error(ErrorType::Device, "loop-frequency node table overflow");
         *diverged = (st & kStatusNaN) ? 1 : 0;
     });

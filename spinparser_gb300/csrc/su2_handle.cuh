@@ -36,7 +36,7 @@ struct spn_su2 {
     float *node_wp = nullptr, *node_c = nullptr, *corr_out = nullptr;
     int *node_cnt = nullptr, *work_counter = nullptr;
     unsigned *status = nullptr;  // the word after it is work_counter
-    spn::cuh::Pinned corr_host, status_host;  // measurements and the status word on the host
+    spn::cuh::HostResults results;  // measurements and the status word on the host
     int *sites = nullptr, *inv_sites = nullptr, *ov_ptr = nullptr, *ov_r1 = nullptr, *ov_r2 = nullptr;
     int *range_rid = nullptr, *range_inv = nullptr, *corr_rid = nullptr;
     double *corr_partial = nullptr;

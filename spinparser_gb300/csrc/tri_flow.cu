@@ -1501,7 +1501,7 @@ struct spn_tri {
     unsigned char *prod_scratch = nullptr;  // tri_lattice_kernel's, of prod_ctas CTAs; it runs when not NULL
     int prod_ctas = 0;
     unsigned *status = nullptr;  // in ints, behind the work counters
-    spn::cuh::Pinned corr_host, status_host;  // measurements and the status word on the host
+    spn::cuh::HostResults results;  // measurements and the status word on the host
     double *partial = nullptr;
 
     long long vsize() const { return 16 * fn * nl; }
@@ -1726,8 +1726,6 @@ extern "C" int spn_tri_create(const spn_tri_desc *d, spn_tri **out) {
             h->node_c = dalloc<float>(size_t(h->n) * h->max_nodes, "alloc node table");
             h->corr_out = dalloc<float>(size_t(kCorrOut) * h->n_corr + 16 * h->nl, "alloc correlation output");
             h->partial = dalloc<double>(size_t(kMaxCorrNodes) * kCorrOut * h->nl, "alloc correlation scratch");
-            h->corr_host.alloc((size_t(kCorrOut) * h->n_corr + 16 * h->nl) * sizeof(float));
-            h->status_host.alloc(sizeof(unsigned));
             const int nl = h->nl, nr = h->n_range, nc = h->n_corr;
             std::vector<int> img;
             std::vector<size_t> at;
@@ -1883,7 +1881,7 @@ extern "C" int spn_tri_measure_correlation(spn_tri *h, float *corr, float *chi) 
         check_cuda(cudaSetDevice(h->device), "cudaSetDevice");
         launch_correlation(h);
         const size_t n = size_t(kCorrOut) * h->n_corr;
-        const float *v = h->corr_host.fetch(h->corr_out, n + 16 * h->nl, h->stream);
+        const float *v = h->results.fetch(h->corr_out, n + 16 * h->nl, h->stream);
         if (corr) std::copy(v, v + n, corr);
         if (chi) std::copy(v + n, v + n + 16 * h->nl, chi);
     });
@@ -1909,7 +1907,7 @@ extern "C" int spn_tri_is_diverged(spn_tri *h, int *diverged) {
     return guarded([&] {
         if (!h || !diverged) throw Error(ErrorType::Argument, "null argument");
         check_cuda(cudaSetDevice(h->device), "cudaSetDevice");
-        const unsigned st = *h->status_host.fetch(h->status, 1, h->stream);
+        const unsigned st = *h->results.fetch(h->status, 1, h->stream);
         if (st & kStatusNodeOverflow) throw Error(ErrorType::Device, "loop-frequency node table overflow");
         if (st & kStatusProductTimeout) throw Error(ErrorType::Device, "a tensor-core product of the vertex flow did not complete");
         *diverged = (st & kStatusNaN) ? 1 : 0;

@@ -1063,7 +1063,7 @@ struct spn_xyz {
         *item_seg_ptr;
     int rpa_n_seg = 0, item_n_seg = 0, site_kind = 0;
     unsigned *status = nullptr;  // in ints, behind the work counters
-    spn::cuh::Pinned corr_host, status_host;  // measurements and the status word on the host
+    spn::cuh::HostResults results;  // measurements and the status word on the host
     double *partial = nullptr;
 
     XyzArgs args() const {
@@ -1244,8 +1244,6 @@ extern "C" int spn_xyz_create(const spn_xyz_desc *d, spn_xyz **out) {
             h->node_c = dalloc<float>(size_t(h->n) * h->max_nodes, "alloc node table");
             h->corr_out = dalloc<float>(4 * size_t(h->n_corr) + 4 * h->nl, "alloc correlation output");
             h->partial = dalloc<double>(size_t(kMaxCorrNodes) * 4 * h->nl, "alloc correlation scratch");
-            h->corr_host.alloc((4 * size_t(h->n_corr) + 4 * h->nl) * sizeof(float));
-            h->status_host.alloc(sizeof(unsigned));
             // integer tables, one allocation
             const int nl = h->nl, nr = h->n_range, nc = h->n_corr;
             std::vector<int> img;
@@ -1414,7 +1412,7 @@ extern "C" int spn_xyz_measure_correlation(spn_xyz *h, float *xx, float *yy, flo
         if (!h) throw Error(ErrorType::Argument, "null handle");
         check_cuda(cudaSetDevice(h->device), "cudaSetDevice");
         launch_correlation(h);
-        const float *v = h->corr_host.fetch(h->corr_out, 4 * size_t(h->n_corr) + 4 * h->nl, h->stream);
+        const float *v = h->results.fetch(h->corr_out, 4 * size_t(h->n_corr) + 4 * h->nl, h->stream);
         float *const dst[4] = {xx, yy, zz, dd};
         for (int c = 0; c < 4; ++c)
             if (dst[c]) std::copy(v + size_t(c) * h->n_corr, v + size_t(c + 1) * h->n_corr, dst[c]);
@@ -1426,7 +1424,7 @@ extern "C" int spn_xyz_is_diverged(spn_xyz *h, int *diverged) {
     return guarded([&] {
         if (!h || !diverged) throw Error(ErrorType::Argument, "null argument");
         check_cuda(cudaSetDevice(h->device), "cudaSetDevice");
-        const unsigned st = *h->status_host.fetch(h->status, 1, h->stream);
+        const unsigned st = *h->results.fetch(h->status, 1, h->stream);
         if (st & kStatusNodeOverflow) throw Error(ErrorType::Device, "loop-frequency node table overflow");
         *diverged = (st & kStatusNaN) ? 1 : 0;
     });
