@@ -69,7 +69,7 @@ struct TriArgs {
     // slot_base[l], ... and site j sums slots seg_ptr[j] .. seg_ptr[j + 1] - 1
     const int *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr;
     int rpa_n_seg;
-    // the same pairs for the lattice sum on the tensor cores (tri_lattice_kernel): site j's are dealt to groups
+    // instead of them, the pairs for the lattice sum on the tensor cores (tri_lattice_kernel): site j's are dealt to groups
     // prod_group[j] .. prod_group[j + 1] - 1; the words of the inner components (k2, k1) and group g at
     // prod_words[2 prod_ptr[(4 k2 + k1) kLatGroups + g]] ..; the CTAs' operand scratch
     const int *prod_ptr, *prod_words, *prod_group;
@@ -1738,8 +1738,8 @@ extern "C" int spn_tri_create(const spn_tri_desc *d, spn_tri **out) {
             put(d->sites_perm, nl);
             put(d->inv_sites_rid, nl);
             put(d->inv_sites_perm, nl);
-            const std::vector<int> packed = order_rpa_pairs(d);
-            const LaneSchedule rpa = tri_lane_schedule(nl, d->overlap_ptr, packed);
+            LaneSchedule rpa;  // of the flows whose pairs are walked
+            if (!use_products(nl)) rpa = tri_lane_schedule(nl, d->overlap_ptr, order_rpa_pairs(d));
             h->rpa_n_seg = rpa.n_seg;
             put(d->range_rid, nr);
             put(d->range_inv_rid, nr);
@@ -1748,9 +1748,9 @@ extern "C" int spn_tri_create(const spn_tri_desc *d, spn_tri **out) {
             put(nullptr, h->n);  // node counts
             put(nullptr, 3);     // work counters, status
             put(rpa.sched.data(), int(rpa.sched.size()));
-            put(rpa.count.data(), 32);
-            put(rpa.slot_base.data(), 32);
-            put(rpa.seg_ptr.data(), nl + 1);
+            put(rpa.count.data(), int(rpa.count.size()));
+            put(rpa.slot_base.data(), int(rpa.slot_base.size()));
+            put(rpa.seg_ptr.data(), int(rpa.seg_ptr.size()));
             std::vector<int> prod_ptr, prod_words, prod_group;
             if (use_products(nl)) product_pairs(d, prod_ptr, prod_words, prod_group);
             put(prod_ptr.data(), int(prod_ptr.size()));

@@ -66,10 +66,7 @@ struct XyzArgs {
     // seg_ptr[j] .. seg_ptr[j + 1] - 1
     const int *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr;
     int rpa_n_seg;
-    // lattices of at most 32 sites: site_kind (below) and the same walk cut into kItemThreads chunks
-    int site_kind;
-    const int *item_sched, *item_count, *item_slot_base, *item_seg_ptr;
-    int item_n_seg;
+    int site_kind;  // lattices of at most 32 sites: xyz_site_kind (below); their walk is cut into kItemThreads chunks
     const int *range_rid, *range_inv;
     const float *node_wp, *node_c;
     const int *node_cnt;
@@ -754,7 +751,7 @@ __global__ void __launch_bounds__(kItemThreads, 2) xyz_item_kernel(XyzArgs a) {
     __shared__ float pos[kMaxFreq];
     __shared__ int s_item;
     unsigned char *smem = reinterpret_cast<unsigned char *>(xs);
-    const XyzItemSmem L = xyz_item_smem(R, a.item_n_seg);
+    const XyzItemSmem L = xyz_item_smem(R, a.rpa_n_seg);
     ItemDesc *desc = reinterpret_cast<ItemDesc *>(smem + L.u);
     float *Ms = reinterpret_cast<float *>(smem + L.u);  // spin (3w x 3w), then density (w x w)
     float4 *slots = reinterpret_cast<float4 *>(Ms + 10 * w * w);
@@ -767,7 +764,7 @@ __global__ void __launch_bounds__(kItemThreads, 2) xyz_item_kernel(XyzArgs a) {
     const bool valid = lane < nl;
     const int sc = min(lane, nl - 1);  // a lane without a site reads the last one's elements
     const int rid = a.sites[sc], prm = a.sites_perm[sc], irid = a.inv_sites[sc], iprm = a.inv_sites_perm[sc];
-    const int rpa_cnt = a.item_count[tid], rpa_base = a.item_slot_base[tid];
+    const int rpa_cnt = a.rpa_count[tid], rpa_base = a.rpa_slot_base[tid];
     const float two_pi = 2.0f * float(kPiD);
     const int items = vertex_items(n);
     const MeshSearch<float> mesh{pos, n};
@@ -843,7 +840,7 @@ __global__ void __launch_bounds__(kItemThreads, 2) xyz_item_kernel(XyzArgs a) {
                 float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 int slot = rpa_base;
                 for (int i = 0; i < rpa_cnt; ++i) {
-                    const int e = __ldg(a.item_sched + kItemThreads * i + tid);
+                    const int e = __ldg(a.rpa_sched + kItemThreads * i + tid);
                     const int r1 = e & 127, r2 = (e >> 7) & 127, p1 = (e >> 14) & 7, p2 = (e >> 17) & 7;
                     sum.x += Ms[(perm_c(p1, 0) * w + r1) * 3 * w + perm_c(p2, 0) * w + r2];
                     sum.y += Ms[(perm_c(p1, 1) * w + r1) * 3 * w + perm_c(p2, 1) * w + r2];
@@ -858,7 +855,7 @@ __global__ void __launch_bounds__(kItemThreads, 2) xyz_item_kernel(XyzArgs a) {
             __syncthreads();
             if (tid < nl) {
                 float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                for (int k = a.item_seg_ptr[tid]; k < a.item_seg_ptr[tid + 1]; ++k) {
+                for (int k = a.rpa_seg_ptr[tid]; k < a.rpa_seg_ptr[tid + 1]; ++k) {
                     const float4 v = slots[k];
                     sum.x += v.x;
                     sum.y += v.y;
@@ -1059,9 +1056,8 @@ struct spn_xyz {
     float4 *sd = nullptr, *dsd = nullptr;
     int *ints = nullptr;  // all integer tables in one allocation
     int *sites, *sites_perm, *inv_sites, *inv_sites_perm, *range_rid, *range_inv, *corr_rid, *corr_perm, *node_cnt,
-        *work_counter, *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr, *item_sched, *item_count, *item_slot_base,
-        *item_seg_ptr;
-    int rpa_n_seg = 0, item_n_seg = 0, site_kind = 0;
+        *work_counter, *rpa_sched, *rpa_count, *rpa_slot_base, *rpa_seg_ptr;
+    int rpa_n_seg = 0, site_kind = 0;
     unsigned *status = nullptr;  // in ints, behind the work counters
     spn::cuh::HostResults results;  // measurements and the status word on the host
     double *partial = nullptr;
@@ -1090,11 +1086,6 @@ struct spn_xyz {
         a.rpa_seg_ptr = rpa_seg_ptr;
         a.rpa_n_seg = rpa_n_seg;
         a.site_kind = site_kind;
-        a.item_sched = item_sched;
-        a.item_count = item_count;
-        a.item_slot_base = item_slot_base;
-        a.item_seg_ptr = item_seg_ptr;
-        a.item_n_seg = item_n_seg;
         a.range_rid = range_rid;
         a.range_inv = range_inv;
         a.node_wp = node_wp;
@@ -1204,7 +1195,7 @@ std::vector<int> order_rpa_pairs(const spn_xyz_desc *d) {
 }
 
 size_t vertex_smem(const spn_xyz *h) {
-    if (h->nl <= 32) return xyz_item_smem(h->nl <= 16 ? 1 : 2, h->item_n_seg).total;
+    if (h->nl <= 32) return xyz_item_smem(h->nl <= 16 ? 1 : 2, h->rpa_n_seg).total;
     return size_t(kWarps) * (kXBatch * sizeof(XDesc) + (12 * size_t(h->nl) + size_t(h->rpa_n_seg)) * sizeof(float4));
 }
 
@@ -1258,7 +1249,9 @@ extern "C" int spn_xyz_create(const spn_xyz_desc *d, spn_xyz **out) {
             put(d->inv_sites_rid, nl);
             put(d->inv_sites_perm, nl);
             const std::vector<int> packed = order_rpa_pairs(d);
-            const LaneSchedule rpa = xyz_lane_schedule(nl, d->overlap_ptr, packed);
+            const int lanes = nl <= 32 ? kItemThreads : 32;
+            const LaneSchedule rpa = nl <= 32 ? lane_schedule(nl, d->overlap_ptr, packed, kItemThreads, 20)
+                                              : xyz_lane_schedule(nl, d->overlap_ptr, packed);
             h->rpa_n_seg = rpa.n_seg;
             put(d->range_rid, nr);
             put(d->range_inv_rid, nr);
@@ -1267,22 +1260,15 @@ extern "C" int spn_xyz_create(const spn_xyz_desc *d, spn_xyz **out) {
             put(nullptr, h->n);  // node counts
             put(nullptr, 2);     // work counter, status
             put(rpa.sched.data(), int(rpa.sched.size()));
-            put(rpa.count.data(), 32);
-            put(rpa.slot_base.data(), 32);
+            put(rpa.count.data(), lanes);
+            put(rpa.slot_base.data(), lanes);
             put(rpa.seg_ptr.data(), nl + 1);
             h->site_kind = xyz_site_kind(nl, d->sites_rid, d->sites_perm, d->inv_sites_rid, d->inv_sites_perm);
-            const LaneSchedule items = lane_schedule(nl, d->overlap_ptr, packed, kItemThreads, 20);
-            h->item_n_seg = items.n_seg;
-            put(items.sched.data(), int(items.sched.size()));
-            put(items.count.data(), kItemThreads);
-            put(items.slot_base.data(), kItemThreads);
-            put(items.seg_ptr.data(), nl + 1);
             h->ints = dalloc<int>(img.size(), "alloc lattice tables");
             h2d(h->ints, img.data(), img.size(), h->stream);
             int **fields[] = {&h->sites, &h->sites_perm, &h->inv_sites, &h->inv_sites_perm, &h->range_rid, &h->range_inv,
                               &h->corr_rid, &h->corr_perm, &h->node_cnt, &h->work_counter, &h->rpa_sched,
-                              &h->rpa_count, &h->rpa_slot_base, &h->rpa_seg_ptr, &h->item_sched, &h->item_count,
-                              &h->item_slot_base, &h->item_seg_ptr};
+                              &h->rpa_count, &h->rpa_slot_base, &h->rpa_seg_ptr};
             for (size_t k = 0; k < at.size(); ++k) *fields[k] = h->ints + at[k];
             h->status = reinterpret_cast<unsigned *>(h->work_counter + 1);
             h2d(h->freq, d->freq, h->n, h->stream);
