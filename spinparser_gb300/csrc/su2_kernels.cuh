@@ -61,6 +61,18 @@ __device__ __forceinline__ void self_energy_body(const FlowArgsT<T> &a, int blk)
 // ------------------------------------------------------------------------------------
 // 2. loop-frequency node tables
 // ------------------------------------------------------------------------------------
+// Of transfer frequency x = pos[xi] at cutoff L: the conventional nodes (SU2FrgCore.cpp:351-371: L, and -L if x > 2 L) and the rules of the
+// Katanin contribution (SU2FrgCore.cpp:374-424), cnt[] nodes each.
+template <class T>
+SPN_HDI int node_rules(const T *pos, int n, int xi, T L, QuadRule<T> (&r)[3], int (&cnt)[3]) {
+    const T x = pos[xi];
+    cnt[0] = cnt[1] = cnt[2] = 0;
+    if (-(x + L) > -pos[n - 1]) r[0] = rule_right(pos, n, -(x + L)), cnt[0] = r[0].count;
+    if (x - L > L) r[1] = rule_both(pos, n, L - x, -L), cnt[1] = r[1].count;
+    if (L < pos[n - 1]) r[2] = rule_left(pos, n, L), cnt[2] = r[2].count;
+    return x > T(2) * L ? 2 : 1;
+}
+
 // One block per transfer frequency x, one thread per node.  A thread that walked a frequency's list
 // alone (2N + 8 nodes of three FP64 reads and a division each, at 2 FP64 FMAs per clock and SM) took
 // 150 us at N = 32 and 230 us at N = 64; the nodes side by side take 10 us.
@@ -81,14 +93,9 @@ __device__ __forceinline__ void node_table_body(const FlowArgsT<T> &a, int xi) {
         double d1 = double(w1) + sig(w1);
         return dsig(w1) / (d1 * d1 * (double(w2) + sig(w2)));
     };
-    // conventional contribution (SU2FrgCore.cpp:351-371): L, and -L if x > 2 L
-    const int conv = x > T(2) * L ? 2 : 1;
-    // Katanin contribution (SU2FrgCore.cpp:374-424)
     QuadRule<T> r[3];
-    int cnt[3] = {0, 0, 0};
-    if (-(x + L) > -pos[n - 1]) r[0] = rule_right(pos, n, -(x + L)), cnt[0] = r[0].count;
-    if (x - L > L) r[1] = rule_both(pos, n, L - x, -L), cnt[1] = r[1].count;
-    if (L < pos[n - 1]) r[2] = rule_left(pos, n, L), cnt[2] = r[2].count;
+    int cnt[3];
+    const int conv = node_rules(pos, n, xi, L, r, cnt);
     const int total = conv + cnt[0] + cnt[1] + cnt[2];
     for (int k = threadIdx.x; k < min(total, a.max_nodes); k += blockDim.x) {
         T wp;

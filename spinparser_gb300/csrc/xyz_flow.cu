@@ -688,16 +688,17 @@ __device__ __forceinline__ void xyz_node(const XyzArgs &a, const ItemDesc &d, in
 }
 
 struct XyzItemSmem {
-    size_t u, panels, parts, rpa, total;
+    size_t u, ms, panels, parts, rpa, total;
 };
-__host__ __device__ inline XyzItemSmem xyz_item_smem(int R, int n_seg) {
+__host__ __device__ inline XyzItemSmem xyz_item_smem(int R, bool once, int n_seg) {
     const int w = 16 * R;
     XyzItemSmem L;
     size_t o = 0;
-    // union: a batch's descriptors, or (after a transfer frequency) the product matrices and the walk's partials
+    // a batch's descriptors and (after a transfer frequency) the product matrices and the walk's partials, in a union but for `once`
     L.u = o;
     const size_t d = kItemBatch * sizeof(ItemDesc), m = sizeof(float) * size_t(10 * w * w) + sizeof(float4) * size_t(n_seg);
-    o += ((d > m ? d : m) + 15) / 16 * 16;
+    L.ms = once ? o + d : o;
+    o += ((once ? d + m : (d > m ? d : m)) + 15) / 16 * 16;
     L.panels = o; o += sizeof(float) * 2 * kItemWarps * 8 * size_t(w);  // 2 buffers x nodes x (A, B) x 4 components
     L.parts = o; o += sizeof(float4) * 3 * kItemWarps * size_t(w);
     L.rpa = o; o += sizeof(float4) * 3 * size_t(w);
@@ -744,16 +745,20 @@ __device__ __forceinline__ void xyz_outer(const float *pan, int tr, int tc, floa
         for (int j = 0; j < R; ++j) Dm[i][j] = fmaf(ad[i], bd[j], Dm[i][j]);
 }
 
-template <int R>
+// ONCE: the nodes of any three transfer frequencies together are at most kItemBatch, so an item's descriptors are built at once.  At so few nodes,
+// as early in a flow, the builds before each transfer frequency are most of an item's time: at 3 sites, N = 32, cutoff 20 a
+// right-hand side took 496 us with them (429 triple by triple), 416 without; later in the flow the form costs 1 to 2 %
+// (registers), so it is a kernel by itself.
+template <int R, bool ONCE>
 __global__ void __launch_bounds__(kItemThreads, 2) xyz_item_kernel(XyzArgs a) {
     constexpr int w = 16 * R, K = 3 * R, K2 = (K + 1) / 2;
     extern __shared__ float4 xs[];
     __shared__ float pos[kMaxFreq];
     __shared__ int s_item;
     unsigned char *smem = reinterpret_cast<unsigned char *>(xs);
-    const XyzItemSmem L = xyz_item_smem(R, a.rpa_n_seg);
+    const XyzItemSmem L = xyz_item_smem(R, ONCE, a.rpa_n_seg);
     ItemDesc *desc = reinterpret_cast<ItemDesc *>(smem + L.u);
-    float *Ms = reinterpret_cast<float *>(smem + L.u);  // spin (3w x 3w), then density (w x w)
+    float *Ms = reinterpret_cast<float *>(smem + L.ms);  // spin (3w x 3w), then density (w x w)
     float4 *slots = reinterpret_cast<float4 *>(Ms + 10 * w * w);
     float *panels = reinterpret_cast<float *>(smem + L.panels);
     float4 *parts = reinterpret_cast<float4 *>(smem + L.parts);
@@ -780,6 +785,15 @@ __global__ void __launch_bounds__(kItemThreads, 2) xyz_item_kernel(XyzArgs a) {
         float4 A = make_float4(0.0f, 0.0f, 0.0f, 0.0f), B = A, T = A;
         // transfer p: targets (p,q,r), (p,r,q) and the t channel of (q,p,r); q: (q,p,r), (p,r,q), t of (p,q,r);
         // r: (q,p,r), (p,q,r), t of (p,r,q)
+        [[maybe_unused]] int first = 0;  // the transfer frequency's first descriptor
+        if constexpr (ONCE) {
+            const int n0 = __ldg(a.node_cnt + p), n1 = __ldg(a.node_cnt + q), step = tid < n0 ? 0 : (tid < n0 + n1 ? 1 : 2);
+            const ItemFreq f = item_freq(pos, step == 0 ? p : (step == 1 ? q : r), step == 0 ? q : p, step == 2 ? q : r, step == 2);
+            const int node = tid - (step == 0 ? 0 : (step == 1 ? n0 : n0 + n1));
+            const size_t k = size_t(f.xi) * a.max_nodes + node;
+            if (node < __ldg(a.node_cnt + f.xi)) make_item(mesh, nl, f, __ldg(a.node_wp + k), __ldg(a.node_c + k), desc[tid]);
+            __syncthreads();
+        }
 #pragma unroll 1
         for (int step = 0; step < 3; ++step) {
             const ItemFreq f = item_freq(pos, step == 0 ? p : (step == 1 ? q : r), step == 0 ? q : p, step == 2 ? q : r, step == 2);
@@ -799,15 +813,17 @@ __global__ void __launch_bounds__(kItemThreads, 2) xyz_item_kernel(XyzArgs a) {
 #pragma unroll 1
             for (int b0 = 0; b0 < cnt; b0 += kItemBatch) {
                 const int nb = min(kItemBatch, cnt - b0);
-                __syncthreads();  // the previous batch's descriptors (or the matrices) are no longer read
-                if (tid < nb) make_item(mesh, nl, f, __ldg(nwp + b0 + tid), __ldg(nc + b0 + tid), desc[tid]);
-                __syncthreads();
+                if constexpr (!ONCE) {
+                    __syncthreads();  // the previous batch's descriptors (or the matrices) are no longer read
+                    if (tid < nb) make_item(mesh, nl, f, __ldg(nwp + b0 + tid), __ldg(nc + b0 + tid), desc[tid]);
+                    __syncthreads();
+                }
 #pragma unroll 1
                 for (int r0 = 0; r0 < nb; r0 += kItemWarps, ++round) {
                     float *buf = panels + size_t(round & 1) * kItemWarps * 8 * w;
                     if (r0 + warp < nb) {
                         Quad pa, pb;
-                        xyz_node(a, desc[r0 + warp], step, rid, prm, irid, iprm, lane, A, B, T, pa, pb);
+                        xyz_node(a, desc[ONCE ? first + r0 + warp : r0 + warp], step, rid, prm, irid, iprm, lane, A, B, T, pa, pb);
                         if (valid) {
                             float *pan = buf + warp * 8 * w + lane;
                             pan[0] = pa.a.x;
@@ -864,6 +880,7 @@ __global__ void __launch_bounds__(kItemThreads, 2) xyz_item_kernel(XyzArgs a) {
                 }
                 rpa[step * w + tid] = sum;
             }
+            if constexpr (ONCE) first += cnt;
             if (step == 0) { const float4 t = A; A = T; T = t; }
             if (step == 1) { const float4 t = B; B = T; T = t; }
         }
@@ -1050,6 +1067,7 @@ struct spn_xyz {
     int device = 0, n = 0, nl = 0, n_range = 0, n_corr = 0, n_overlap = 0, max_nodes = 0, sms = 0, grid = 0;
     long long fn = 0;
     float cutoff = 0.0f;
+    std::vector<float> mesh;
     cudaStream_t stream = nullptr;
     float *freq = nullptr, *v2 = nullptr, *dv2 = nullptr, *stage = nullptr, *node_wp = nullptr, *node_c = nullptr,
           *corr_out = nullptr;
@@ -1171,9 +1189,9 @@ void validate(const spn_xyz_desc *d) {
 }
 
 // The vertex kernel: by items for Nl <= 32, else by triples with SPT sites per lane (2 for Nl <= 64, else 4).
-const void *vertex_kernel(int nl) {
-    if (nl <= 16) return reinterpret_cast<const void *>(&xyz_item_kernel<1>);
-    if (nl <= 32) return reinterpret_cast<const void *>(&xyz_item_kernel<2>);
+const void *vertex_kernel(int nl, bool once) {
+    if (nl <= 16) return once ? reinterpret_cast<const void *>(&xyz_item_kernel<1, true>) : reinterpret_cast<const void *>(&xyz_item_kernel<1, false>);
+    if (nl <= 32) return reinterpret_cast<const void *>(&xyz_item_kernel<2, false>);
     if (nl <= 64) return reinterpret_cast<const void *>(&xyz_vertex_kernel<2>);
     return reinterpret_cast<const void *>(&xyz_vertex_kernel<4>);
 }
@@ -1194,9 +1212,22 @@ std::vector<int> order_rpa_pairs(const spn_xyz_desc *d) {
     return out;
 }
 
-size_t vertex_smem(const spn_xyz *h) {
-    if (h->nl <= 32) return xyz_item_smem(h->nl <= 16 ? 1 : 2, h->rpa_n_seg).total;
+size_t vertex_smem(const spn_xyz *h, bool once) {
+    if (h->nl <= 32) return xyz_item_smem(h->nl <= 16 ? 1 : 2, once, h->rpa_n_seg).total;
     return size_t(kWarps) * (kXBatch * sizeof(XDesc) + (12 * size_t(h->nl) + size_t(h->rpa_n_seg)) * sizeof(float4));
+}
+
+// Whether the items' descriptors are built at once (xyz_item_kernel<1, true>), at the flow's cutoff.
+bool build_once(const spn_xyz *h) {
+    if (h->nl > 16) return false;
+    int most = 0;
+    for (int i = 0; i < h->n; ++i) {
+        QuadRule<float> r[3];
+        int cnt[3];
+        const int conv = node_rules(h->mesh.data(), h->n, i, h->cutoff, r, cnt);
+        most = std::max(most, conv + cnt[0] + cnt[1] + cnt[2]);
+    }
+    return 3 * most <= kItemBatch;
 }
 
 void launch_correlation(spn_xyz *h) {
@@ -1277,12 +1308,16 @@ extern "C" int spn_xyz_create(const spn_xyz_desc *d, spn_xyz **out) {
             check_cuda(cudaMemsetAsync(h->v2, 0, h->n * sizeof(float), h->stream), "memset");
             check_cuda(cudaMemsetAsync(h->dv2, 0, h->n * sizeof(float), h->stream), "memset");
             check_cuda(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device), "device attribute");
-            int per_sm = 0;
-            const void *fn = vertex_kernel(h->nl);
-            check_cuda(allow_shared(fn, vertex_smem(h)), "shared memory limit");
-            check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, vertex_threads(h->nl), vertex_smem(h)), "occupancy");
-            if (per_sm < 1) throw Error(ErrorType::Unsupported, "XYZ vertex-flow kernel does not fit on this device");
-            h->grid = h->sms * per_sm;
+            h->mesh.assign(d->freq, d->freq + h->n);
+            for (const bool once : {true, false}) {
+                if (once && h->nl > 16) continue;
+                int per_sm = 0;
+                const void *fn = vertex_kernel(h->nl, once);
+                check_cuda(allow_shared(fn, vertex_smem(h, once)), "shared memory limit");
+                check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, vertex_threads(h->nl), vertex_smem(h, once)), "occupancy");
+                if (per_sm < 1) throw Error(ErrorType::Unsupported, "XYZ vertex-flow kernel does not fit on this device");
+                h->grid = h->sms * per_sm;
+            }
             check_cuda(cudaStreamSynchronize(h->stream), "create sync");
         } catch (...) {
             h->release();
@@ -1371,10 +1406,11 @@ extern "C" int spn_xyz_compute_step(spn_xyz *h) {
         check_cuda(cudaGetLastError(), "self-energy launch");
         xyz_node_table_kernel<<<h->n, kNodeThreads, 0, h->stream>>>(h->node_args());
         check_cuda(cudaGetLastError(), "node table launch");
-        const void *fn = vertex_kernel(h->nl);
+        const bool once = build_once(h);
+        const void *fn = vertex_kernel(h->nl, once);
         XyzArgs arg = a;
         void *params[] = {&arg};
-        check_cuda(cudaLaunchKernel(fn, dim3(h->grid), dim3(vertex_threads(h->nl)), params, vertex_smem(h), h->stream), "vertex flow launch");
+        check_cuda(cudaLaunchKernel(fn, dim3(h->grid), dim3(vertex_threads(h->nl)), params, vertex_smem(h, once), h->stream), "vertex flow launch");
         check_cuda(cudaGetLastError(), "vertex flow launch");
     });
 }
