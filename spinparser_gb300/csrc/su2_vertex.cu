@@ -1818,10 +1818,12 @@ __device__ __forceinline__ void mid_outer_update(const float2 *pan, int tid, flo
         for (int j = 0; j < C::B; ++j) M[i][j] = fma2(av[i], bv[j], M[i][j]);
 }
 
-// The three triples of item `item` of flow `a` by the whole CTA; `pos` the mesh in shared memory.
-template <int R>
-__device__ __forceinline__ void mid_item(const FlowArgs &a, const float *pos, int item, unsigned char *smem,
-                                         const MidSmem &L) {
+// The three triples of item (p, q, r) of flow `a` by the whole CTA; `pos` the mesh in shared memory.  ONCE: the nodes of all transfer
+// frequencies together are at most kMidBatch, so their descriptors are built at once and every thread walks the pairs (at few nodes, as early in
+// a flow, the builds before each transfer frequency and the walk by half of the threads are most of an item's time).
+template <int R, bool ONCE>
+__device__ __forceinline__ void mid_triples(const FlowArgs &a, const float *pos, int p, int q, int r, unsigned char *smem,
+                                            const MidSmem &L) {
     using C = MidCfg<R>;
     constexpr int w = C::w, NN = C::NN;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1833,8 +1835,6 @@ __device__ __forceinline__ void mid_item(const FlowArgs &a, const float *pos, in
     float2 *panels = reinterpret_cast<float2 *>(smem + L.panels);
     float2 *parts = reinterpret_cast<float2 *>(smem + L.parts);
     float2 *rpa = reinterpret_cast<float2 *>(smem + L.rpa);
-    int p, q, r;
-    decode_item(item, p, q, r);
     const int site = 32 * part + lane;
     const bool valid = site < a.nl;
     // a lane past the last site reads the last site's element (never used), which lies among the
@@ -1849,12 +1849,19 @@ __device__ __forceinline__ void mid_item(const FlowArgs &a, const float *pos, in
     auto build = [&](const ItemFreq &f, int cnt, int step, int b0, int first) {
         const int t = tid - first, at = f.xi * a.max_nodes + b0 + t;
         if (t < 0 || t >= min(kMidBatch, cnt - b0)) return;
-        make_item(mesh_of(a, pos), a.nl, f, __ldg(a.node_wp + at), __ldg(a.node_c + at), desc[t]);
-        item_local(a.sd, desc[t], step, loc[t]);
+        const int place = ONCE ? tid : t;
+        make_item(mesh_of(a, pos), a.nl, f, __ldg(a.node_wp + at), __ldg(a.node_c + at), desc[place]);
+        item_local(a.sd, desc[place], step, loc[place]);
     };
     ItemFreq f = item_step(pos, 0, p, q, r);
-    int cnt = __ldg(a.node_cnt + f.xi);
-    build(f, cnt, 0, 0, 0);
+    int cnt = __ldg(a.node_cnt + f.xi), first = 0;  // first: the transfer frequency's first descriptor
+    if constexpr (ONCE) {
+        const int n1 = __ldg(a.node_cnt + q), step = tid < cnt ? 0 : (tid < cnt + n1 ? 1 : 2);
+        const ItemFreq g = item_step(pos, step, p, q, r);
+        build(g, __ldg(a.node_cnt + g.xi), step, 0, step == 0 ? 0 : (step == 1 ? cnt : cnt + n1));
+    } else {
+        build(f, cnt, 0, 0, 0);
+    }
     __syncthreads();
     float2 M[C::B][C::B];
     int round = 0;
@@ -1867,7 +1874,7 @@ __device__ __forceinline__ void mid_item(const FlowArgs &a, const float *pos, in
 #pragma unroll 1
         for (int b0 = 0; b0 < cnt; b0 += kMidBatch) {
             const int nb = min(kMidBatch, cnt - b0);
-            if (b0) {  // the first batch is built during the pair walk before
+            if (!ONCE && b0) {  // the first batch is built during the pair walk before
                 __syncthreads();  // the previous batch's descriptors are no longer read
                 build(f, cnt, step, b0, 0);
                 __syncthreads();
@@ -1878,7 +1885,7 @@ __device__ __forceinline__ void mid_item(const FlowArgs &a, const float *pos, in
                 float2 *buf = panels + size_t(round & 1) * NN * 2 * w;
                 if (k < nb) {
                     float2 pa, pb;
-                    site_node(desc[k], loc[k], step, v, A, B, T, pa, pb);
+                    site_node(desc[ONCE ? first + k : k], loc[ONCE ? first + k : k], step, v, A, B, T, pa, pb);
                     if (valid) {
                         buf[nw * 2 * w + site] = pa;
                         buf[nw * 2 * w + w + site] = pb;
@@ -1898,9 +1905,10 @@ __device__ __forceinline__ void mid_item(const FlowArgs &a, const float *pos, in
             for (int j = 0; j < C::B; ++j) Ms[(tr * C::B + i) * w + tc * C::B + j] = M[i][j];
         __syncthreads();
         // half of the threads walk the pairs, the others build the next transfer frequency's first descriptors
-        if (tid < kMidWalkers) {
+        constexpr int walkers = ONCE ? kMidThreads : kMidWalkers;
+        if (tid < walkers) {
             const int lanes = a.rpa.lanes;
-            for (int l = tid; l < lanes; l += kMidWalkers) {
+            for (int l = tid; l < lanes; l += walkers) {
                 const int cntq = __ldg(a.rpa.count + l);
                 int slot = __ldg(a.rpa.slot_base + l);
                 const int *sched = a.rpa.sched + l;
@@ -1918,9 +1926,14 @@ __device__ __forceinline__ void mid_item(const FlowArgs &a, const float *pos, in
             }
         }
         if (step < 2) {
-            f = item_step(pos, step + 1, p, q, r);
-            cnt = __ldg(a.node_cnt + f.xi);
-            build(f, cnt, step + 1, 0, kMidWalkers);
+            first += cnt;
+            if constexpr (ONCE) {
+                cnt = __ldg(a.node_cnt + (step == 0 ? q : r));
+            } else {
+                f = item_step(pos, step + 1, p, q, r);
+                cnt = __ldg(a.node_cnt + f.xi);
+                build(f, cnt, step + 1, 0, kMidWalkers);
+            }
         }
         __syncthreads();
         if (tid < a.nl) {
@@ -1956,6 +1969,22 @@ __device__ __forceinline__ void mid_item(const FlowArgs &a, const float *pos, in
         a.dsd[(size_t(su_index(ts, tu)) * a.n + tt) * a.nl + j] = make_float2(os, od);
         if (isnan(os) || isnan(od)) atomicOr(a.status, kStatusNaN);
     }
+}
+
+template <int R>
+__device__ __forceinline__ void mid_item(const FlowArgs &a, const float *pos, int item, unsigned char *smem, const MidSmem &L) {
+    int p, q, r;
+    decode_item(item, p, q, r);
+    // Both forms in one kernel cost registers: at R = 4 less than 1 % late in a flow (64 sites, N = 20, cutoffs 20 and 0.01: 222 and 521 us a
+    // right-hand side without the second form, 207 and 618 triple by triple, 183 and 525 with it), at R = 3, where early
+    // flows are fast without it (41 sites: 156 us triple by triple, 138), 3 %.
+    if constexpr (R == 4) {
+        if (__ldg(a.node_cnt + p) + __ldg(a.node_cnt + q) + __ldg(a.node_cnt + r) <= kMidBatch) {
+            mid_triples<R, true>(a, pos, p, q, r, smem, L);
+            return;
+        }
+    }
+    mid_triples<R, false>(a, pos, p, q, r, smem, L);
 }
 
 template <int R>
