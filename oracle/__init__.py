@@ -327,6 +327,8 @@ class TriOracle:
         dsc = C.POINTER(XyzOracleDesc)
         lib.oracle_tri_rhs_f32.argtypes = [dsc, C.c_float, fp, fp, fp, fp, i4]
         lib.oracle_tri_vertex_f32.argtypes = [dsc, C.c_float, fp, fp, fp, fp, i4]
+        dp = C.POINTER(C.c_double)
+        lib.oracle_tri_vertex_sample_f64.argtypes = [dsc, C.c_double, dp, dp, dp, C.POINTER(C.c_int), i4, dp, i4]
         lib.oracle_tri_correlation_f32.argtypes = [dsc, C.c_float, fp, fp, fp]
         lib.oracle_tri_flow_f32.argtypes = [dsc, fp, i4, fp, fp, fp, i4]
         lib.oracle_tri_tables.argtypes = [C.POINTER(C.c_int)]
@@ -374,6 +376,17 @@ class TriOracle:
         assert self.lib.oracle_tri_vertex_f32(C.byref(self.desc), cutoff, _p(v2, C.c_float), _p(dv2, C.c_float),
                                               _p(v4, C.c_float), _p(dv4, C.c_float), threads) == 0
         return dv4
+
+    def vertex_sample64(self, cutoff, v2, dv2, v4, triples, threads: int = 0):
+        """dv4[len(triples), 16*Nl] of the listed triples in 64 bits, with the given self-energy flow dv2[N]."""
+        v2, dv2, v4 = (np.ascontiguousarray(x, np.float64).reshape(-1) for x in (v2, dv2, v4))
+        assert v4.size == self.size
+        its = np.ascontiguousarray(triples, np.int32)
+        assert its.min() >= 0 and its.max() < self.fn
+        out = np.empty((len(its), 16 * self.nl))
+        assert self.lib.oracle_tri_vertex_sample_f64(C.byref(self.desc), cutoff, _p(v2, C.c_double), _p(dv2, C.c_double),
+                                                     _p(v4, C.c_double), _p(its, C.c_int), len(its), _p(out, C.c_double), threads) == 0
+        return out
 
     def correlation(self, cutoff, v2, v4):
         """chi[16][Nl] at the state (the mixed spin/density components are zero)."""

@@ -61,10 +61,6 @@ constexpr int kPerm[6][3] = {{0, 1, 2}, {0, 2, 1}, {1, 0, 2}, {1, 2, 0}, {2, 0, 
 constexpr int D = 3;
 constexpr int kSpinOrder[4] = {3, 2, 1, 0};  // density, Z, Y, X: the reference's order of inner indices
 
-const float kTwoPiProd = 2.0f * float(M_PI);          // 2.0f * (float)M_PI
-const float kTwoPiCast = float(2.0f * M_PI);          // float(2.0f * M_PI)
-const float kFourPi2Cast = float(4.0f * M_PI * M_PI);  // float(4.0f * M_PI * M_PI)
-
 inline float zeta(int c) { return c <= 2 ? -1.0f : 1.0f; }
 inline int permc(int p, int c) { return c == D ? D : kPerm[p][c]; }
 
@@ -160,38 +156,39 @@ const Tables &tables() {
     return T;
 }
 
-struct Mesh {
+template <class Real>
+struct MeshT {
     int n;
-    std::vector<float> full;  // 2N values: -w[N-1] .. -w[0], w[0] .. w[N-1]
-    const float *pos;
-    explicit Mesh(const TriOracleDesc &d) : n(d.n_freq), full(2 * d.n_freq) {
+    std::vector<Real> full;  // 2N values: -w[N-1] .. -w[0], w[0] .. w[N-1]
+    const Real *pos;
+    explicit MeshT(const TriOracleDesc &d) : n(d.n_freq), full(2 * d.n_freq) {
         for (int i = 0; i < n; ++i) {
             full[n + i] = d.freq[i];
             full[n - 1 - i] = -d.freq[i];
         }
         pos = full.data() + n;
     }
-    int lesser(float w) const {
+    int lesser(Real w) const {
         if (w < 0) return n - (greater(-w) - n + 1);
         if (w <= pos[0]) return n;
         for (int i = 1; i < n; ++i)
             if (pos[i] > w) return n + i - 1;
         return n + n - 1;
     }
-    int greater(float w) const {
+    int greater(Real w) const {
         if (w < 0) return n - (lesser(-w) - n + 1);
         if (w <= pos[0]) return n;
         for (int i = 1; i < n; ++i)
             if (pos[i] > w) return n + i;
         return n + n - 1;
     }
-    int offset(float w) const {
+    int offset(Real w) const {
         if (w <= pos[0]) return 0;
         for (int i = 1; i < n; ++i)
             if (pos[i] >= w) return i;
         return n - 1;
     }
-    void interpolate(float w, int &lo, int &hi, float &bias) const {
+    void interpolate(Real w, int &lo, int &hi, Real &bias) const {
         if (w <= pos[0]) {
             lo = hi = 0;
             bias = 0.0f;
@@ -212,15 +209,15 @@ struct Mesh {
 // TRIVertexTwoParticleAccessBuffer<K>: the sign table sign[i][a][b] is the product of
 // zeta(a) zeta(b) when exactly one of t, u was negated, and, for a support whose s and u
 // offsets were exchanged, -zeta(a) (pair exchange) or -zeta(b).
-template <int K>
-struct AccessBuffer {
+template <class Real, int K>
+struct AccessBufferT {
     int off[K];
-    float wgt[K];
+    Real wgt[K];
     bool fx[K];
     bool exch = false;
     bool tu = false;
-    float sign(int i, int a, int b) const {
-        float s = 1.0f;
+    Real sign(int i, int a, int b) const {
+        Real s = 1.0f;
         if (tu) s *= zeta(a) * zeta(b);
         if (fx[i]) s *= -(exch ? zeta(a) : zeta(b));
         return s;
@@ -228,9 +225,11 @@ struct AccessBuffer {
 };
 
 // ValueSuperbundle<float, 16>
-struct Bundle16 {
-    std::vector<float> c[16];
-    explicit Bundle16(int nl = 0) {
+template <class Real>
+struct Bundle16T {
+    using real = Real;
+    std::vector<Real> c[16];
+    explicit Bundle16T(int nl = 0) {
         for (auto &v : c) v.assign(nl, 0.0f);
     }
     void reset() {
@@ -238,39 +237,51 @@ struct Bundle16 {
     }
 };
 
-void axpy(Bundle16 &y, float a, const Bundle16 &x) {
+template <class B>
+void axpy(B &y, typename B::real a, const B &x) {
     for (int k = 0; k < 16; ++k)
         for (size_t i = 0; i < y.c[k].size(); ++i) y.c[k][i] += a * x.c[k][i];
 }
-void add(Bundle16 &y, const Bundle16 &x) {
+template <class B>
+void add(B &y, const B &x) {
     for (int k = 0; k < 16; ++k)
         for (size_t i = 0; i < y.c[k].size(); ++i) y.c[k][i] += x.c[k][i];
 }
-void scale(Bundle16 &y, float a) {
+template <class B>
+void scale(B &y, typename B::real a) {
     for (auto &v : y.c)
         for (auto &e : v) e *= a;
 }
 
-struct Tri {
+// In 32 bits (every operation rounded as the reference's) or in 64.
+template <class Real>
+struct TriT {
+    using Mesh = MeshT<Real>;
+    using Bundle16 = Bundle16T<Real>;
+    template <int K>
+    using AccessBuffer = AccessBufferT<Real, K>;
+    static constexpr Real kTwoPiProd = Real(2) * Real(M_PI);           // 2.0f * (float)M_PI
+    static constexpr Real kTwoPiCast = Real(2.0f * M_PI);              // float(2.0f * M_PI)
+    static constexpr Real kFourPi2Cast = Real(4.0f * M_PI * M_PI);     // float(4.0f * M_PI * M_PI)
     const TriOracleDesc &dsc;
     Mesh mesh;
     int N, Nl;
     long long stepT, stepSU;  // 16 Nl per t, N 16 Nl per (s,u)
-    const float *v2, *dv2;
-    const float *v4;          // [F_N][16][Nl]
+    const Real *v2, *dv2;
+    const Real *v4;          // [F_N][16][Nl]
 
-    Tri(const TriOracleDesc &d, const float *v2_, const float *dv2_, const float *v4_)
+    TriT(const TriOracleDesc &d, const Real *v2_, const Real *dv2_, const Real *v4_)
         : dsc(d), mesh(d), N(d.n_freq), Nl(d.n_sites), stepT(16LL * d.n_sites), stepSU(16LL * d.n_sites * d.n_freq),
           v2(v2_), dv2(dv2_), v4(v4_) {}
 
-    float sigma(const float *data, float w) const {
-        float sign = 1.0f;
+    Real sigma(const Real *data, Real w) const {
+        Real sign = 1.0f;
         if (w < 0) {
             w = -w;
             sign = -1.0f;
         }
         int lo, hi;
-        float b;
+        Real b;
         mesh.interpolate(w, lo, hi, b);
         return sign * ((1 - b) * data[lo] + b * data[hi]);
     }
@@ -287,7 +298,7 @@ struct Tri {
     }
 
     template <int K>
-    static void fold(float &s, float &t, float &u, AccessBuffer<K> &ab) {
+    static void fold(Real &s, Real &t, Real &u, AccessBuffer<K> &ab) {
         if (s < 0) {
             s = -s;
             ab.exch = !ab.exch;
@@ -303,11 +314,11 @@ struct Tri {
         }
     }
 
-    AccessBuffer<4> access4(float s, float t, float u, int channel) const {
+    AccessBuffer<4> access4(Real s, Real t, Real u, int channel) const {
         AccessBuffer<4> ab;
         fold(s, t, u, ab);
         int e, la, ua, lb, ub;
-        float ba, bb;
+        Real ba, bb;
         if (channel == 0) {
             e = mesh.offset(s);
             mesh.interpolate(t, la, ua, ba);
@@ -336,11 +347,11 @@ struct Tri {
         return ab;
     }
 
-    AccessBuffer<8> access8(float s, float t, float u) const {
+    AccessBuffer<8> access8(Real s, Real t, Real u) const {
         AccessBuffer<8> ab;
         fold(s, t, u, ab);
         int ls, us, lt, ut, lu, uu;
-        float bs, bt, bu;
+        Real bs, bt, bu;
         mesh.interpolate(s, ls, us, bs);
         mesh.interpolate(t, lt, ut, bt);
         mesh.interpolate(u, lu, uu, bu);
@@ -365,7 +376,7 @@ struct Tri {
         for (int i = 0; i < K; ++i)
             for (int a = 0; a < 4; ++a)
                 for (int b = 0; b < 4; ++b) {
-                    const float sw = ab.sign(i, a, b) * ab.wgt[i];
+                    const Real sw = ab.sign(i, a, b) * ab.wgt[i];
                     for (int j = 0; j < Nl; ++j) {
                         const int a1 = permc(prm[j], ab.exch ? b : a);
                         const int b1 = permc(prm[j], ab.exch ? a : b);
@@ -377,22 +388,22 @@ struct Tri {
     // getValueLocal: the components are exchanged first and the sign is indexed by the
     // exchanged pair.
     template <int K>
-    float local(int a, int b, const AccessBuffer<K> &ab) const {
+    Real local(int a, int b, const AccessBuffer<K> &ab) const {
         if (ab.exch) std::swap(a, b);
-        float v = 0.0f;
+        Real v = 0.0f;
         for (int i = 0; i < K; ++i) v += ab.sign(i, a, b) * ab.wgt[i] * v4[ab.off[i] + (4 * a + b) * Nl];
         return v;
     }
 
-    float direct(int site, int so, int to, int uo, int a, int b) const {
+    Real direct(int site, int so, int to, int uo, int a, int b) const {
         if (so >= uo) return v4[stepSU * (so * (so + 1) / 2 + uo) + stepT * to + (4 * a + b) * Nl + site];
         return -zeta(b) * v4[stepSU * (uo * (uo + 1) / 2 + so) + stepT * to + (4 * a + b) * Nl + site];
     }
 
     // getValue(i1, i2, s, t, u, a, b, FrequencyChannel::None) for the pairs the self-energy
     // reads: (origin, j) through rid12 / rid21 with identity spin maps, a == b.
-    float value_none(int rid12, int rid21, float s, float t, float u, int a, int b) const {
-        float sign = 1.0f;
+    Real value_none(int rid12, int rid21, Real s, Real t, Real u, int a, int b) const {
+        Real sign = 1.0f;
         bool swapped = false;
         if (s < 0) {
             s = -s;
@@ -411,7 +422,7 @@ struct Tri {
         }
         const int site = swapped ? rid21 : rid12;
         int ls, us, lt, ut, lu, uu;
-        float bs, bt, bu;
+        Real bs, bt, bu;
         mesh.interpolate(s, ls, us, bs);
         mesh.interpolate(t, lt, ut, bt);
         mesh.interpolate(u, lu, uu, bu);
@@ -424,11 +435,11 @@ struct Tri {
 
     // ---- trapezoid rules with off-mesh boundaries (Integrator.hpp:137-287) ----
     template <class F>
-    void int_left(float min, F &&f, Bundle16 &ib, Bundle16 &res) const {
+    void int_left(Real min, F &&f, Bundle16 &ib, Bundle16 &res) const {
         res.reset();
         const int maxi = 2 * N - 1;
         int um = mesh.greater(min);
-        const float *fl = mesh.full.data();
+        const Real *fl = mesh.full.data();
         if (um != maxi) {
             f(min, ib); axpy(res, fl[um] - min, ib);
             f(fl[um], ib); axpy(res, fl[um + 1] - min, ib);
@@ -445,9 +456,9 @@ struct Tri {
         }
     }
     template <class F>
-    void int_right(float max, F &&f, Bundle16 &ib, Bundle16 &res) const {
+    void int_right(Real max, F &&f, Bundle16 &ib, Bundle16 &res) const {
         res.reset();
-        const float *fl = mesh.full.data();
+        const Real *fl = mesh.full.data();
         int um = 0;
         int ux = mesh.lesser(max);
         if (um != ux) {
@@ -466,9 +477,9 @@ struct Tri {
         }
     }
     template <class F>
-    void int_both(float min, float max, F &&f, Bundle16 &ib, Bundle16 &res) const {
+    void int_both(Real min, Real max, F &&f, Bundle16 &ib, Bundle16 &res) const {
         res.reset();
-        const float *fl = mesh.full.data();
+        const Real *fl = mesh.full.data();
         int um = mesh.greater(min);
         int ux = mesh.lesser(max);
         if (ux >= um) {
@@ -493,10 +504,10 @@ struct Tri {
     }
 
     // ---- self-energy flow, one frequency (TRIFrgCore.cpp:122-151) ----
-    float self_energy_flow(int i, float cutoff) const {
-        const float w = mesh.pos[i];
-        float val = 0.0f;
-        float sum = 0.0f;
+    Real self_energy_flow(int i, Real cutoff) const {
+        const Real w = mesh.pos[i];
+        Real val = 0.0f;
+        Real sum = 0.0f;
         for (int j = 0; j < dsc.n_range; ++j) {
             sum += value_none(dsc.range_rid[j], dsc.range_inv_rid[j], w + cutoff, 0.0f, w - cutoff, D, D);
             sum -= value_none(dsc.range_rid[j], dsc.range_inv_rid[j], w - cutoff, 0.0f, w + cutoff, D, D);
@@ -528,24 +539,24 @@ struct Tri {
             }
     }
 
-    void vertex_flow(int it, float cutoff, Scratch &sc, float *out) const {
+    void vertex_flow(int it, Real cutoff, Scratch &sc, Real *out) const {
         const Tables &T = tables();
         const int su = it / N;
-        const float t = mesh.pos[it % N];
-        float s = 0.0f, u = 0.0f;
+        const Real t = mesh.pos[it % N];
+        Real s = 0.0f, u = 0.0f;
         for (int so = 0; so <= su; ++so)
             for (int uo = 0; uo <= so; ++uo)
                 if (su == so * (so + 1) / 2 + uo) {
                     s = mesh.pos[so];
                     u = mesh.pos[uo];
                 }
-        const float w1p = 0.5f * (s + t + u);
-        const float w1 = 0.5f * (s - t + u);
-        const float w2p = 0.5f * (s - t - u);
-        const float w2 = 0.5f * (s + t - u);
+        const Real w1p = 0.5f * (s + t + u);
+        const Real w1 = 0.5f * (s - t + u);
+        const Real w2p = 0.5f * (s - t - u);
+        const Real w2 = 0.5f * (s + t - u);
         Bundle16 *sb = sc.st;
 
-        auto kernelS = [&](float wp, Bundle16 &r) {  // TRIFrgCore.cpp:181-712
+        auto kernelS = [&](Real wp, Bundle16 &r) {  // TRIFrgCore.cpp:181-712
             superbundle(access4(s, w2 + wp, w1 + wp, 0), sb[0]);
             superbundle(access4(s, -w2p - wp, w1p + wp, 0), sb[1]);
             superbundle(access4(s, -w1 - wp, -w2 - wp, 0), sb[2]);
@@ -553,7 +564,7 @@ struct Tri {
             ladder(T.pp, sb, r);
         };
 
-        auto kernelT = [&](float wp, Bundle16 &r) {  // TRIFrgCore.cpp:714-2369
+        auto kernelT = [&](Real wp, Bundle16 &r) {  // TRIFrgCore.cpp:714-2369
             superbundle(access4(w1 - wp, t, w1p + wp, 1), sb[0]);
             superbundle(access4(w2p - wp, t, -w2 - wp, 1), sb[1]);
             superbundle(access4(w1p + wp, t, w1 - wp, 1), sb[2]);
@@ -570,8 +581,8 @@ struct Tri {
                         for (int p = 0; p < 4; p += 2)
                             for (int i = i0; i < i1; ++i) {
                                 const int P1 = dsc.overlap_perm1[i], P2 = dsc.overlap_perm2[i];
-                                const float x = sb[p].c[4 * permc(P1, mu) + permc(P1, k)][dsc.overlap_rid1[i]];
-                                const float y = sb[p + 1].c[4 * permc(P2, k) + permc(P2, nu)][dsc.overlap_rid2[i]];
+                                const Real x = sb[p].c[4 * permc(P1, mu) + permc(P1, k)][dsc.overlap_rid1[i]];
+                                const Real y = sb[p + 1].c[4 * permc(P2, k) + permc(P2, nu)][dsc.overlap_rid2[i]];
                                 if (sg > 0) sc.rpa.c[c][rid] += 2 * x * y;
                                 else sc.rpa.c[c][rid] -= 2 * x * y;
                             }
@@ -581,7 +592,7 @@ struct Tri {
             add(r, sc.rpa);
             const AccessBuffer<4> a4 = access4(w2p - wp, -w2 - wp, t, 2);
             const AccessBuffer<4> a5 = access4(w2 + wp, -w2p + wp, t, 2);
-            float L4[16], L5[16];
+            Real L4[16], L5[16];
             for (int l = 0; l < 16; ++l) {
                 L4[l] = local(l >> 2, l & 3, a4);
                 L5[l] = local(l >> 2, l & 3, a5);
@@ -601,7 +612,7 @@ struct Tri {
                 }
             const AccessBuffer<4> a6 = access4(w1 - wp, -w1p - wp, -t, 2);
             const AccessBuffer<4> a7 = access4(w1p + wp, -w1 + wp, -t, 2);
-            float L6[16], L7[16];
+            Real L6[16], L7[16];
             for (int l = 0; l < 16; ++l) {
                 L6[l] = local(l >> 2, l & 3, a6);
                 L7[l] = local(l >> 2, l & 3, a7);
@@ -621,7 +632,7 @@ struct Tri {
                 }
         };
 
-        auto kernelU = [&](float wp, Bundle16 &r) {  // TRIFrgCore.cpp:2371-2903
+        auto kernelU = [&](Real wp, Bundle16 &r) {  // TRIFrgCore.cpp:2371-2903
             superbundle(access4(w1 + wp, -w2p + wp, u, 2), sb[0]);
             superbundle(access4(w1p + wp, w2 - wp, u, 2), sb[1]);
             superbundle(access4(w2p - wp, -w1 - wp, u, 2), sb[2]);
@@ -629,9 +640,9 @@ struct Tri {
             ladder(T.ph, sb, r);
         };
 
-        auto p = [&](float a, float b) { return 1.0f / ((a + sigma(v2, a)) * (b + sigma(v2, b))); };
-        auto pK = [&](float a, float b) {
-            const float den = a + sigma(v2, a);
+        auto p = [&](Real a, Real b) { return 1.0f / ((a + sigma(v2, a)) * (b + sigma(v2, b))); };
+        auto pK = [&](Real a, Real b) {
+            const Real den = a + sigma(v2, a);
             return sigma(dv2, a) / (den * den * (b + sigma(v2, b)));
         };
 
@@ -644,12 +655,12 @@ struct Tri {
         kernelU(cutoff, sc.b1); axpy(acc, p(cutoff, cutoff + u), sc.b1);
         if (u > 2.0f * cutoff) { kernelU(-cutoff, sc.b1); axpy(acc, p(cutoff, cutoff - u), sc.b1); }
 
-        auto kS = [&](float wp, Bundle16 &r) { kernelS(wp, r); scale(r, pK(wp, s + wp)); };
-        auto kT = [&](float wp, Bundle16 &r) { kernelT(wp, r); scale(r, pK(wp, t + wp)); };
-        auto kU = [&](float wp, Bundle16 &r) { kernelU(wp, r); scale(r, pK(wp, u + wp)); };
-        const float wmax = mesh.pos[N - 1];
-        const float wneg = mesh.full[0];
-        auto katanin = [&](float x, auto &kern) {
+        auto kS = [&](Real wp, Bundle16 &r) { kernelS(wp, r); scale(r, pK(wp, s + wp)); };
+        auto kT = [&](Real wp, Bundle16 &r) { kernelT(wp, r); scale(r, pK(wp, t + wp)); };
+        auto kU = [&](Real wp, Bundle16 &r) { kernelU(wp, r); scale(r, pK(wp, u + wp)); };
+        const Real wmax = mesh.pos[N - 1];
+        const Real wneg = mesh.full[0];
+        auto katanin = [&](Real x, auto &kern) {
             if (-(x + cutoff) > wneg) { int_right(-(x + cutoff), kern, sc.b1, sc.b2); add(acc, sc.b2); }
             if (x - cutoff > cutoff) { int_both(cutoff - x, -cutoff, kern, sc.b1, sc.b2); add(acc, sc.b2); }
             if (cutoff < wmax) { int_left(cutoff, kern, sc.b1, sc.b2); add(acc, sc.b2); }
@@ -663,25 +674,25 @@ struct Tri {
     }
 
     // ---- static susceptibility at nu = 0 (TRIMeasurementCorrelation.cpp:147-285) ----
-    void correlation(float cut, float *chi) const {
+    void correlation(Real cut, Real *chi) const {
         const Tables &T = tables();
-        const float nu = 0.0f;
+        const Real nu = 0.0f;
         Bundle16 sus(Nl), stk(Nl), b1(Nl), b2(Nl), b3(Nl), b4(Nl);
-        const float wmax = mesh.pos[N - 1];
-        const float wneg = mesh.full[0];
+        const Real wmax = mesh.pos[N - 1];
+        const Real wneg = mesh.full[0];
         static const int kOut[10] = {15, 0, 1, 2, 4, 5, 6, 8, 9, 10};
-        auto outer = [&](float w, Bundle16 &ret) {
+        auto outer = [&](Real w, Bundle16 &ret) {
             ret.reset();
-            const float term1 = 1.0f / ((w + sigma(v2, w)) * (w + nu + sigma(v2, w + nu)));
+            const Real term1 = 1.0f / ((w + sigma(v2, w)) * (w + nu + sigma(v2, w + nu)));
             ret.c[15][0] += 2.0f * term1 / kTwoPiCast;
             ret.c[0][0] += 0.5f * term1 / kTwoPiCast;
             ret.c[5][0] += 0.5f * term1 / kTwoPiCast;
             ret.c[10][0] += 0.5f * term1 / kTwoPiCast;
-            auto inner = [&](float wp, Bundle16 &r) {
+            auto inner = [&](Real wp, Bundle16 &r) {
                 r.reset();
                 superbundle(access8(w + wp + nu, nu, w - wp), stk);
                 const AccessBuffer<8> ab1 = access8(w + wp + nu, w - wp, nu);
-                float L[16];
+                Real L[16];
                 for (int l = 0; l < 16; ++l) L[l] = local(l >> 2, l & 3, ab1);
                 // dumbbell
                 for (int j = 0; j < Nl; ++j) r.c[15][j] -= 4.0f * stk.c[15][j];
@@ -690,14 +701,14 @@ struct Tri {
                 // egg
                 for (int q = 0; q < 10; ++q) {
                     const int c = kOut[q];
-                    const float f = c == 15 ? 2.0f : 0.5f;
+                    const Real f = c == 15 ? 2.0f : 0.5f;
                     for (int n = 0; n < 4; ++n) {
                         const Pair &e = T.egg[c][n];
                         if (e.sg > 0) r.c[c][0] += f * L[e.a];
                         else if (e.sg < 0) r.c[c][0] -= f * L[e.a];
                     }
                 }
-                const float norm = 1.0f / ((w + sigma(v2, w)) * (w + nu + sigma(v2, w + nu)) * (wp + sigma(v2, wp)) *
+                const Real norm = 1.0f / ((w + sigma(v2, w)) * (w + nu + sigma(v2, w + nu)) * (wp + sigma(v2, wp)) *
                                            (wp + nu + sigma(v2, wp + nu)) * kFourPi2Cast);
                 scale(r, norm);
             };
@@ -712,6 +723,7 @@ struct Tri {
             for (int j = 0; j < Nl; ++j) chi[c * Nl + j] = sus.c[c][j];
     }
 };
+using Tri = TriT<float>;
 
 }  // namespace
 
@@ -758,6 +770,27 @@ int oracle_tri_vertex_f32(const TriOracleDesc *d, float cutoff, const float *v2,
 #pragma omp for schedule(dynamic, 8)
 #endif
         for (int it = 0; it < FN; ++it) core.vertex_flow(it, cutoff, sc, dv4 + (long long)it * 16 * Nl);
+    }
+    return 0;
+}
+
+// The vertex flow of `count` triples, out[count][16*Nl], in 64 bits, with a given self-energy flow.
+int oracle_tri_vertex_sample_f64(const TriOracleDesc *d, double cutoff, const double *v2, const double *dv2, const double *v4,
+                                 const int *triples, int count, double *out, int nthreads) {
+    if (!d || d->n_freq < 2 || d->n_sites < 1) return -2;
+    if (tables().bad) return -3;
+    const int Nl = d->n_sites;
+    TriT<double> core(*d, v2, dv2, v4);
+#ifdef _OPENMP
+    if (nthreads > 0) omp_set_num_threads(nthreads);
+#pragma omp parallel
+#endif
+    {
+        TriT<double>::Scratch sc(Nl);
+#ifdef _OPENMP
+#pragma omp for schedule(dynamic, 1)
+#endif
+        for (int i = 0; i < count; ++i) core.vertex_flow(triples[i], cutoff, sc, out + (long long)i * 16 * Nl);
     }
     return 0;
 }

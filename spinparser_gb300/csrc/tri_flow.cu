@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 #include "su2_common.cuh"
 #include "su2_device.cuh"
@@ -998,6 +999,13 @@ constexpr int kLatK = 32;        // slab pairs of a chunk
 // Chunks of A in shared memory (as many as fit) and of B, which are kept for all products of a k2 where its K has no
 // more.
 constexpr int kLatStages = 4, kLatSlotsB = 3;
+constexpr int kLatKeep = kLatSlotsB * kLatK;
+// Slab pairs that one accumulator takes where there are more than kLatKeep.  The tensor cores cut what they add, by 0.4 units in the last
+// place of the sum for every 16 slab pairs and always towards zero.  A right-hand side of operands of one sign is 2.6e-7 off in norm
+// over 90 slab pairs, with the pairs walked in FP32 3.9e-7; over 144 (N = 32), 240 (N = 56) and 416 (N = 100) it would be 5.0e-7,
+// 1.1e-6 and 2.1e-6 off, walked 3.8e-7, 3.6e-7 and 7.5e-7.  So longer sums are made of parts, added rounded: 3.0e-7, 1.2e-7 and
+// 3.6e-7 (with parts of 96 6.4e-7 at N = 56; parts of 32 take 7 % longer).
+constexpr int kLatPart = 2 * kLatK;
 constexpr int kLatNodes = kLatWorkers / 4;  // nodes whose descriptors are built at once (a quad of threads each)
 constexpr uint32_t kLatCols = 512;  // tensor memory: accumulator b's high products at column 256 b, low ones 128 on
 
@@ -1153,7 +1161,7 @@ __global__ void __launch_bounds__(kLatThreads, 1) tri_lattice_kernel(TriArgs a) 
                 worker_sync();
 #pragma unroll 1
                 for (int task = warp; task < 2 * nb; task += kLatWarps) {  // slabs q and q + 2 of a node
-                    const int q = task & 1, k = 2 * (b0 + (task >> 1));
+                    const int q = task & 1, k = 2 * (cnt - 1 - b0 - (task >> 1));
                     const TDesc &d = desc[task >> 1];
                     float x[16], y[16], v[16], f[4][4], g[4][4];
                     const float lv = local_value(a, d, 32 * q + lane);
@@ -1197,7 +1205,8 @@ __global__ void __launch_bounds__(kLatThreads, 1) tri_lattice_kernel(TriArgs a) 
         }
         __syncthreads();
 
-        const bool keep = kn <= kLatSlotsB * kLatK;  // the whole B of a k2 stays in shared memory
+        const bool keep = kn <= kLatKeep;  // the whole B of a k2 stays in shared memory
+        const int part_len = keep ? kLatKeep : kLatPart, parts = keep ? 1 : (kn + kLatPart - 1) / kLatPart;
         if (warp == kLatWarps) {
             if (lane == 0) {  // copies
                 bool ok = true;
@@ -1231,26 +1240,29 @@ __global__ void __launch_bounds__(kLatThreads, 1) tri_lattice_kernel(TriArgs a) 
             if (lane == 0) {  // products
                 bool ok = true;
                 int slot = 0;
-                for (int i = 0; i < combos && ok && kn > 0; ++i) {
-                    const uint32_t ci = combo_no + i, d = tmem + 256 * (ci & 1);
+                uint32_t ci = combo_no;
+                for (int i = 0; i < combos && ok; ++i) {
                     const bool release_b = !keep || i + 1 == combos || s_combos[i + 1] >> 2 != s_combos[i] >> 2;
-                    if (ci >= 2) ok = umma::bar_wait(drained + (ci & 1), ((ci >> 1) - 1) & 1);
                     if (keep) slot = 0;
-                    for (int k0 = 0; k0 < kn && ok; k0 += kLatK) {
-                        ok = umma::bar_wait(full_b + slot, phase_b >> slot & 1) && umma::bar_wait(full + stage_no, phase);
-                        if (!ok) break;
-                        umma::fence_after();
-                        umma::product(d, d + 128, ring + stage_no * 3 * term, kLatGroup, term, ring_b + slot * 3 * term, kLatGroup, term, rows,
-                                      min(kLatK, kn - k0) / 16, k0 > 0);
-                        umma::commit(empty + stage_no);
-                        if (release_b) {
-                            umma::commit(empty_b + slot);
-                            phase_b ^= 1u << slot;
+                    for (int part = 0; part < kn && ok; part += part_len, ++ci) {
+                        const uint32_t d = tmem + 256 * (ci & 1);
+                        if (ci >= 2) ok = umma::bar_wait(drained + (ci & 1), ((ci >> 1) - 1) & 1);
+                        for (int k0 = part; k0 < min(kn, part + part_len) && ok; k0 += kLatK) {
+                            ok = umma::bar_wait(full_b + slot, phase_b >> slot & 1) && umma::bar_wait(full + stage_no, phase);
+                            if (!ok) break;
+                            umma::fence_after();
+                            umma::product(d, d + 128, ring + stage_no * 3 * term, kLatGroup, term, ring_b + slot * 3 * term, kLatGroup, term, rows,
+                                          min(kLatK, kn - k0) / 16, k0 > part);
+                            umma::commit(empty + stage_no);
+                            if (release_b) {
+                                umma::commit(empty_b + slot);
+                                phase_b ^= 1u << slot;
+                            }
+                            if (++slot == kLatSlotsB) slot = 0;
+                            if (++stage_no == L.stages) stage_no = 0, phase ^= 1;
                         }
-                        if (++slot == kLatSlotsB) slot = 0;
-                        if (++stage_no == L.stages) stage_no = 0, phase ^= 1;
+                        umma::commit(done + (ci & 1));
                     }
-                    umma::commit(done + (ci & 1));
                 }
                 if (!ok) s_dead = 1;
             }
@@ -1271,31 +1283,47 @@ __global__ void __launch_bounds__(kLatThreads, 1) tri_lattice_kernel(TriArgs a) 
                 w0 = __ldg(ptr + s_combos[0] * kLatGroups);
                 w1 = __ldg(ptr + s_combos[0] * kLatGroups + 1);
             }
+            uint32_t ci = combo_no;
             for (int i = 0; i < combos && kn > 0; ++i) {
-                const uint32_t ci = combo_no + i, b = ci & 1;
                 const int cb = s_combos[i];
                 int2 ahead[kLatAhead];
 #pragma unroll
                 for (int e = 0; e < kLatAhead; ++e) ahead[e] = w0 + e < w1 ? __ldg(list + w0 + e) : make_int2(rows * stride, rows * stride);
-                if (!umma::bar_wait(done + b, (ci >> 1) & 1)) s_late = 1;
-                umma::fence_after();
-                const int row = (warp & 3) * 32 + lane;
-                for (int c0 = (warp >> 2) * 16; c0 < rows && warp < kLatReaders; c0 += 4 * kLatReaders) {
-                    float hi[16], lo[16];
-                    const uint32_t addr = tmem + 256 * b + (uint32_t(warp & 3) << 21) + c0;
-                    umma::load16(addr, hi);
-                    umma::load16(addr + 128, lo);
-                    umma::load_wait();
-                    if (row < rows)
+                // the reading warps alone wait for the products: the others are not held to their pace, and would miss a phase
+                auto drain = [&](auto more) {
+                    const uint32_t b = ci & 1;
+                    if (!umma::bar_wait(done + b, (ci >> 1) & 1)) s_late = 1;
+                    umma::fence_after();
+                    const int row = (warp & 3) * 32 + lane;
+                    for (int c0 = (warp >> 2) * 16; c0 < rows; c0 += 4 * kLatReaders) {
+                        float hi[16], lo[16];
+                        const uint32_t addr = tmem + 256 * b + (uint32_t(warp & 3) << 21) + c0;
+                        umma::load16(addr, hi);
+                        umma::load16(addr + 128, lo);
+                        umma::load_wait();
+                        if (row < rows)
 #pragma unroll
-                        for (int k = 0; k < 16; k += 4)
-                            *reinterpret_cast<float4 *>(stage + row * stride + c0 + k) =
-                                make_float4(umma::add_terms(hi[k], lo[k]), umma::add_terms(hi[k + 1], lo[k + 1]),
-                                            umma::add_terms(hi[k + 2], lo[k + 2]), umma::add_terms(hi[k + 3], lo[k + 3]));
+                            for (int k = 0; k < 16; k += 4) {
+                                float4 v = make_float4(umma::add_terms(hi[k], lo[k]), umma::add_terms(hi[k + 1], lo[k + 1]),
+                                                       umma::add_terms(hi[k + 2], lo[k + 2]), umma::add_terms(hi[k + 3], lo[k + 3]));
+                                float4 *m = reinterpret_cast<float4 *>(stage + row * stride + c0 + k);
+                                if constexpr (decltype(more)::value) {  // this thread's own elements
+                                    const float4 u = *m;
+                                    v = make_float4(u.x + v.x, u.y + v.y, u.z + v.z, u.w + v.w);
+                                }
+                                *m = v;
+                            }
+                    }
+                    umma::fence_before();
+                    __syncwarp();
+                    if (lane == 0) umma::bar_arrive(drained + b);
+                    ++ci;
+                };
+                if (warp < kLatReaders) {
+                    drain(std::false_type{});
+#pragma unroll 1
+                    for (int part = 1; part < parts; ++part) drain(std::true_type{});
                 }
-                umma::fence_before();
-                __syncwarp();
-                if (lane == 0 && warp < kLatReaders) umma::bar_arrive(drained + b);
                 worker_sync();
                 if (s_late) break;  // the workers write it before this barrier alone, so they agree
                 int n0 = 0, n1 = 0;
@@ -1344,7 +1372,7 @@ __global__ void __launch_bounds__(kLatThreads, 1) tri_lattice_kernel(TriArgs a) 
                 if (isnan(v)) atomicOr(a.status, kStatusNaN);
             }
         }
-        if (kn > 0) combo_no += combos;
+        combo_no += combos * parts;
         __syncthreads();  // s_dead, s_late
     }
     // a copy or a product did not complete in time (each wait is long enough for those in flight to end)
