@@ -237,8 +237,8 @@ typedef struct {
  * and the measurement (the precision reference for FP32 flows of the same task; the cutoff
  * list and the frequency mesh keep the task's float values).  The float entry points convert
  * on the host; the _f64 entry points below move the double arrays themselves.  Such a flow is
- * evaluated by a plain FP64 kernel (one warp per frequency triple): correct, not fast.  Not
- * accepted by spn_batch_add. */
+ * evaluated by FP64 kernels (a warp per item of three triples up to 32 sites, per triple above),
+ * at the FP64 rate.  Not accepted by spn_batch_add. */
 #define SPN_SU2_FP64 0x2
 
 /* Creates a flow (allocates its device memory).  State starts at zero, cutoff 0.
@@ -270,15 +270,16 @@ int spn_su2_get_node_counts(spn_su2 *h, int *counts);
 int spn_su2_compute_step(spn_su2 *h);
 
 /* Picks the vertex-flow kernel variant for this flow by timing the candidates on the current
- * state (`reps` launches each): nodes a site group evaluates per iteration (1 or 2) and
- * whether the RPA schedule is staged in shared memory.  All variants give identical results.
- * Leaves the state unchanged; reports the choice and the persistent grid size.  Replaces the
+ * state (`reps` launches each): whether the RPA schedule is staged in shared memory.  All
+ * variants give identical results.  Leaves the state unchanged; reports the choice and the
+ * persistent grid size, and npi as it was set (one kernel serves both values).  Replaces the
  * reference LoadManager's throughput model (src/lib/LoadManager.hpp:796-852) as the tuning
  * step of the work distribution. */
 int spn_su2_autotune(spn_su2 *h, int reps, int *npi, int *sched_in_smem, int *grid);
 
-/* Selects a vertex-flow variant explicitly (npi = 1 or 2; schedule in shared memory or not).
- * SPN_E_UNSUPPORTED if it does not fit for this lattice. */
+/* Selects a vertex-flow variant explicitly (schedule in shared memory or not).  npi = 1 or 2 is
+ * accepted and kept, without effect.  SPN_E_UNSUPPORTED if the variant does not fit for this
+ * lattice. */
 int spn_su2_set_variant(spn_su2 *h, int npi, int sched_in_smem);
 
 /* Copies the flow computed by the last compute_step: dv2[N], dv4ss/dv4dd[F_N*Nl]. */
@@ -362,8 +363,7 @@ typedef struct spn_batch spn_batch;
 
 int spn_batch_create(int device, spn_batch **out);
 int spn_batch_destroy(spn_batch *b);
-/* Vertex-flow variant of the batch (npi = 1 or 2) and whether steps are replayed as graphs.
- * Variants do not change results. */
+/* Whether steps are replayed as graphs; npi = 1 or 2 is accepted and kept, without effect. */
 int spn_batch_set_variant(spn_batch *b, int npi, int use_graph);
 /* Cross-flow sharing in the vertex flow.  Flows of a batch that have the same frequency mesh,
  * lattice tables, spin length and cutoff list and stand at the same cutoff (a parameter scan's
@@ -383,9 +383,9 @@ int spn_batch_set_paused(spn_batch *b, int flow_id, int paused);
 /* Flows the current plan evaluates with the grouped kernel. */
 int spn_batch_grouped_flows(spn_batch *b, int *n_grouped);
 /* Batch autotuner: times the vertex flow of the current flows, `reps` launches per candidate,
- * over nodes per iteration (1, 2) x RPA schedule staging (without sharing) and, if sharing is
- * enabled (spn_batch_set_grouping), x sharing (full or half subgroups), and keeps the fastest
- * (returned, with its time per launch in ms).
+ * over RPA schedule staging (without sharing) and, if sharing is enabled
+ * (spn_batch_set_grouping), sharing in full or half subgroups, and keeps the fastest (returned,
+ * with its time per launch in ms; npi as it was set).
  * Touches no flow's state or results; call it between steps, after the flows of interest are
  * admitted.  Replaces the reference LoadManager's chunk-size choice
  * (src/lib/LoadManager.hpp:796-852). */

@@ -51,7 +51,7 @@ class Su2Batch:
         self.close()
 
     def set_variant(self, nodes_per_iteration: int = 1, use_graph: bool = True) -> None:
-        """Kernel variant and graph replay; results do not change."""
+        """Graph replay; results do not change.  nodes_per_iteration (1 or 2) has no effect."""
         check(self._lib.spn_batch_set_variant(self._h, nodes_per_iteration, int(use_graph)))
 
     def set_grouping(self, min_group: int = 2, cap_divisor: int = 1) -> None:
@@ -63,7 +63,7 @@ class Su2Batch:
 
     def autotune(self, reps: int = 2) -> dict:
         """Times the vertex flow of the current flows under each candidate configuration
-        (nodes per iteration x cross-flow sharing) and keeps the fastest; no state changes."""
+        (schedule staging, cross-flow sharing) and keeps the fastest; no state changes."""
         a, m, c, t = C.c_int(), C.c_int(), C.c_int(), C.c_float()
         check(self._lib.spn_batch_autotune(self._h, int(reps), C.byref(a), C.byref(m), C.byref(c), C.byref(t)))
         return {"nodes_per_iteration": a.value, "min_group": m.value, "cap_divisor": c.value, "vertex_ms": t.value}

@@ -303,7 +303,7 @@ class Su2Flow:
         return {"nodes_per_iteration": npi.value, "schedule_in_smem": bool(sm.value), "grid": grid.value}
 
     def set_variant(self, nodes_per_iteration: int, schedule_in_smem: bool) -> None:
-        """Kernel variant (all variants give identical results)."""
+        """Kernel variant (all variants give identical results).  nodes_per_iteration (1 or 2) has no effect."""
         check(self._lib.spn_su2_set_variant(self._h, nodes_per_iteration, int(schedule_in_smem)))
 
     def get_flow(self):

@@ -11,8 +11,8 @@
 //            row-major W x W matrix, W = rpa_outer_width(Nl).  The kernel accumulates
 //            M = sum over nodes of (c A) x B first and walks the schedule once per triple:
 //            acc += m * M[rid1][rid2];
-//   Nl > 32: rid1 | rid2 << 7 | m << 14 | last << 22; the kernel accumulates
-//            acc += (A[rid1] * m) * B[rid2] per node.
+//   Nl > 32: rid1 | rid2 << 7 | m << 14 | last << 22, for the same walk:
+//            acc += m * M[rid1][rid2].
 #pragma once
 #include <vector>
 

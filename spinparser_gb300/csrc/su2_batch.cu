@@ -454,7 +454,6 @@ struct spn_batch {
                 g.prefix = L + off_gp[c];
                 g.n_sg = n_sg[c];
                 g.total = total_g[c];
-                g.gmax = group_vertex_gmax(c);
                 g.counter = d_counters + kVertexClasses + c;
                 g.n_seg_max = nseg_g[c];
                 launch_group_vertex(g, c, ggrid[c], stream);
@@ -803,8 +802,8 @@ extern "C" int spn_batch_autotune(spn_batch *b, int reps, int *npi, int *min_gro
         };
         const Cand cands[] = {{b->npi, 0, 1, false}, {b->npi, 0, 1, true}, {b->npi, 2, 1, false}, {b->npi, 2, 2, false}};
         const Cand keep{b->npi, b->min_group, b->group_cap_div, b->stage_sched};
-        // sharing is a candidate only when the caller enabled it (spn_batch_set_grouping): on
-        // a scan it wins in the first steps and loses in the later ones, which dominate
+        // sharing is a candidate only when the caller enabled it (spn_batch_set_grouping): it wins
+        // by a few percent with full subgroups of small lattices and loses elsewhere (su2_vertex.cu)
         const bool sharing = b->min_group > 0;
         Cand best = keep;
         float best_t = -1.0f;

@@ -159,7 +159,7 @@ struct BatchVertexArgs {
     int *counter;
     int warp_area;
     int sched_ints;
-    int n_seg_max;  // classes 6-8 (CTA per triple): the largest RPA segment count of the list
+    int n_seg_max;  // the CTA classes (vertex_class_big): the largest RPA segment count of the list
 };
 // Grouped batches (flows sharing mesh, lattice tables and cutoff; see su2_vertex.cu): one
 // persistent launch per group class over (subgroup, item) pairs.  A subgroup holds up
@@ -169,7 +169,7 @@ struct BatchVertexArgs {
 struct GroupVertexArgs {
     BatchFlow *flows;
     const int *members, *prefix;
-    int n_sg, total, gmax;
+    int n_sg, total;
     int *counter;
     int n_seg_max;
 };

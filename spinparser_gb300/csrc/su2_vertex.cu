@@ -259,9 +259,8 @@ struct NodeView {
     const float *lv;
 };
 
-// K_X at NPI nodes for this lane's sites (one group evaluates NPI nodes per iteration so that
-// the t channel decodes each RPA schedule entry once for all of them).  `a` provides the
-// state (a.sd), the spin length and, for SPT > 1, the RPA schedule.
+// K_X at NPI nodes for this lane's sites (one; see namespace triple).  `a` provides the
+// state (a.sd) and the spin length.
 // The t channel writes the node's panel (c * third slab, fourth slab) for every site of the
 // lane; the caller adds its outer product to M and walks the RPA pair list once per triple.
 template <int CH, int SPT, int NPI, class A>
@@ -776,7 +775,9 @@ __global__ void __launch_bounds__(kThreads, vertex_min_blocks(MB)) su2_vertex_ba
 // reference's coordinates.
 // ------------------------------------------------------------------------------------
 namespace triple {
-constexpr int SPT = 1, NPI = 1;  // one site per lane, one node per group and step
+// One site per lane, one node per group and step.  Kept as parameters: with the loops over them written out the compiler orders the
+// reads otherwise, and launches of one wave take 4 % longer (18 and 31 sites, N = 8: 55 -> 57 us a right-hand side; the same bits).
+constexpr int SPT = 1, NPI = 1;
 
 // Adds the outer products of the panels of nodes k = (r*NPI+n)*G+gg < nb (ascending k) to the
 // lane's block of M.  `pan`: the warp's first panel; panel (gg, n) starts pstride float2 later
@@ -1772,7 +1773,7 @@ __global__ void __launch_bounds__(kGroupWarps * 32, vertex_min_blocks(MB)) su2_v
 // Square r12 (49 sites), N = 47: 2.50 ms, triple by triple (su2_vertex_big_kernel) 2.78, bound by the barriers of the rounds, the
 // latency of slab reads and the shared-memory path (panel reads, 60 %).  Not above 64 sites, nor where the exchange
 // is another pair: the wider panels' and the exchanged planes' traffic and barriers take more than the shared slab reads
-// save (square r20, 121 sites: 5.3 ms against 4.7; pyrochlore r6, 64 sites: 14.0 against 13.7).
+// save (square r20, 121 sites: 5.3 ms against 4.7; pyrochlore r6, 48 sites: 14.0 against 13.7).
 // ------------------------------------------------------------------------------------
 // w = 16 R = 48 or 64: a node's sites are two warps' 32, so NN nodes make a round; the threads are a 16 x 16 grid over M
 template <int R>
@@ -2356,7 +2357,9 @@ int big_r_of(int nl) {
 int big_class_r(int cls) { return cls == 6 ? 3 : (cls == 7 ? 4 : (cls == 8 ? 5 : (cls == 9 ? 6 : 8))); }
 int big_threads(int r) { return r <= 3 ? 128 : 256; }
 
-// Whether the CTA takes items of three triples (su2_vertex_mid_kernel; classes 15 and 16 for R = 3, 4).
+// Whether the CTA takes items of three triples (su2_vertex_mid_kernel; classes 15 and 16 for R = 3, 4).  Right-hand sides of 36 to 42 sites are
+// 1.08 to 2.3 times as fast as triple by triple at N = 4 to 48 and cutoffs from 20 to 0.01, of 49 to 64 sites 1.02 to 1.9 times, but
+// for N = 6 at cutoff 20 (49, 56, 64 sites: 45, 46, 49 us triple by triple, 45, 47, 51).
 bool mid_of(int nl, int inv_kind) { return nl > 32 && nl <= 64 && !inv_kind; }
 
 // items of three triples, or single triples

@@ -980,7 +980,8 @@ __global__ void __launch_bounds__(kThreads, 4) tri_site_kernel(TriArgs a) {
 // adds 128 products for every pair and node.
 //
 // A CTA takes a triple.  Its 14 worker warps gather the nodes' slabs, a slab at a time, add the chalice terms and leave
-// the slabs as operands (three bf16 terms of each FP32 value, umma.cuh) in a scratch that stays in L2.  Then one
+// the slabs as operands (three bf16 terms of each FP32 value, umma.cuh) in the CTA's scratch (0.4 MB at the nodes of N = 32 and
+// cutoff 0.5, room for 0.9: with 152 CTAs 65 MB are in use, of which L2 writes 4.5 GB a launch back to DRAM).  Then one
 // thread copies the operands of every (k2, k1) to shared memory in chunks of 32 slab pairs, another issues the products, up
 // to two accumulators ahead of the workers, which stage M in shared memory and add their outputs' elements.
 //
@@ -988,8 +989,11 @@ __global__ void __launch_bounds__(kThreads, 4) tri_site_kernel(TriArgs a) {
 // cycles: 47,000 gather and split the slabs (latency of the slab reads, sectors written), 29,000 add the pairs' elements, 20,000
 // are the products (62 cycles each, the reads of their operands), the rest is waiting between the stages.
 // ------------------------------------------------------------------------------------
-// From here on the products pay (honeycomb, N = 24, cutoff 0.5, a right-hand side): 8 sites 2.41 ms, with the pairs walked
-// 2.22; 11 sites 2.64 and 3.08; 28 sites 3.4 and 9.1.
+// From here on the products pay, but for the fewest nodes (honeycomb, a right-hand side at cutoffs 20 and 0.1, us, by products and with
+// the pairs walked): 8 sites, N = 8 91, 128 and 62, 103; N = 32 3103, 9239 and 2139, 9719.  11 sites, N = 8 93, 140 and 64, 118; N = 16 406, 851
+// and 290, 974; N = 32 3315, 10091 and 2759, 12777.  14 sites, N = 8 95, 142 and 73, 145; N = 32 3369, 10351 and 3340, 16651.  28 sites, N = 4
+// 89, 103 and 150, 217; N = 32 4686, 13697 and 7124, 39820.  A product takes 16 slab pairs at least and its staging and pair sums
+// do not shrink with N; most of a flow's time is at low cutoffs, where the line is between 8 and 11 sites from N = 12 on.
 constexpr int kLatMinSites = 10;
 constexpr int kLatWarps = 14, kLatWorkers = 32 * kLatWarps, kLatThreads = kLatWorkers + 64;
 constexpr int kLatReaders = kLatWarps / 4 * 4;  // warps that stage M: every four of them, the 128 rows
