@@ -791,7 +791,7 @@ __global__ void __launch_bounds__(kItemThreads, 2) xyz_item_kernel(XyzArgs a) {
             const ItemFreq f = item_freq(pos, step == 0 ? p : (step == 1 ? q : r), step == 0 ? q : p, step == 2 ? q : r, step == 2);
             const int node = tid - (step == 0 ? 0 : (step == 1 ? n0 : n0 + n1));
             const size_t k = size_t(f.xi) * a.max_nodes + node;
-            if (node < __ldg(a.node_cnt + f.xi)) make_item(mesh, nl, f, __ldg(a.node_wp + k), __ldg(a.node_c + k), desc[tid]);
+            if (tid < kItemBatch && node < __ldg(a.node_cnt + f.xi)) make_item(mesh, nl, f, __ldg(a.node_wp + k), __ldg(a.node_c + k), desc[tid]);
             __syncthreads();
         }
 #pragma unroll 1
